@@ -446,6 +446,21 @@ def test_gemm_32_bit_is_true_32_bit_and_row_independent(kernels, M, N, K_):
     assert torch.equal(one[0, 0], out[0, M // 2]), "a row's result must not depend on the other rows"
 
 
+# few tokens on 8 and on 16 features a block; either side of the border to tiles (32 tokens; 200 tiles of 64 x 64); rows that do
+# not start on 16-byte borders; inner sizes behind one segment of 128, behind the eight classes, and that fill none
+@pytest.mark.parametrize("M,N,K_", [(4, 2367, 128), (9, 2400, 1153), (16, 100, 4100), (17, 33, 1025), (32, 12801, 132), (33, 12737, 260),
+                                    (65, 6401, 1029), (613, 1100, 2052), (200, 1100, 96)])
+def test_gemm_32_bit_is_one_sum_in_every_kernel(kernels, M, N, K_):
+    K = kernels("float32")
+    x, w = _randn(M, K_, seed=74).float().cuda(), _randn(N, K_, seed=75).float().cuda()
+    out = K.gemm_store(x, w)
+    assert helpers.rel_err(out, x.double() @ w.double().T) < 2e-6
+    for m in (0, M // 2, M - 1):
+        assert torch.equal(K.gemm_store(x[m:m + 1].contiguous(), w)[0], out[m]), "a row's result must not depend on the other rows"
+    half = K.gemm_store(x, w[:N // 2].contiguous())       # (fewer features: another kernel or tile for many of the sizes)
+    assert torch.equal(half, out[:, :N // 2])
+
+
 # Token counts on both sides of every border between kernels and tile shapes (16, 32, 64, 128 tokens on
 # the lanes of one kernel; 128- and 256-token tiles of another above that).
 CUTS = (1, 2, 16, 17, 32, 33, 64, 65, 128, 129, 200, 256, 257, 300)
