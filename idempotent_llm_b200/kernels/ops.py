@@ -68,8 +68,8 @@ SIGNATURES = {
     "idm_ssd_chunk_tokens": (c_int, ""),
     "idm_ssd_scan": (c_int, "piiiipiiippppqpippiiiiippipip"),
     "idm_ssd_group_norm": (c_int, "piipffpiiip"),
-    "idm_attention_sink": (c_int, "ppiifpppippipppppiiiiifip"),
-    "idm_attention_biased": (c_int, "ppiifpppiipppiipppppiiiiififiipp"),
+    "idm_attention_sink": (c_int, "ppiifpppippipppppiiiipiiiifip"),
+    "idm_attention_biased": (c_int, "ppiifpppiipppiipppppiiiipiiiififiipp"),
     "idm_head_finish": (c_int, "piiiipppppiiifipfiiiippppiipppip"),
     "idm_cols_cast": (c_int, "piiipiip"),
     "idm_delta_prep": (c_int, "piiipiipiiipppiiiip"),
@@ -88,7 +88,8 @@ SIGNATURES = {
     "idm_sample_scratch_floats": (c_longlong, "ii"),
     "idm_sample": (c_int, "piifpppp"),
     "idm_decode_advance": (c_int, "pppppppiip"),
-    "idm_attention_generic": (c_int, "pppppiipppppppiiiifip"),
+    "idm_attention_generic": (c_int, "pppppiipppppppiiiipiiifip"),
+    "idm_attention_generic_scratch_floats": (c_longlong, "iiiiiiii"),
     "idm_attention_decode_supports": (c_int, "i"),
     "idm_attention_decode_chunk": (c_int, ""),
     "idm_attention_decode_scratch_floats": (c_longlong, "iiii"),
@@ -456,8 +457,9 @@ class Kernels:
         self._check(self.lib.idm_attention_sink(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], _p(sink), (gate.data_ptr() if gate is not None else None), gate_stride,
-            _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q), n, n_q,
-            kv.n_kv_heads, dk, dv, scale, 0, self._stream()))
+            _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
+            *self._generic_step(ctx, n, n_q, kv.n_kv_heads, dv, False), n_q, kv.n_kv_heads, dk, dv, scale, 0, self._stream()),
+            self._generic_launches)
 
     def attention_biased(self, q, kv, ctx, scale: float, out, out_col: int, out_scale: float = 1.0, sink=None,
                          slopes=None, gate=None, gate_stride: int = 0, gate_per_head: bool = False, window=None,
@@ -476,9 +478,18 @@ class Kernels:
         self._check(self.lib.idm_attention_biased(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table), kv.table.shape[1],
             kv.ring, _p(sink), _p(slopes), _p(gate), gate_stride, 1 if gate_per_head else 0, _p(ctx.token_seq),
-            _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q), n, n_q, kv.n_kv_heads, dk, kv.v_head_dim,
-            float(scale), int(window) if window else 0, float(softcap or 0.0), int(keep_first or 0), int(chunk or 0),
-            _p(score_bias), self._stream()))
+            _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
+            *self._generic_step(ctx, n, n_q, kv.n_kv_heads, kv.v_head_dim, bool(window or chunk)), n_q, kv.n_kv_heads, dk,
+            kv.v_head_dim, float(scale), int(window) if window else 0, float(softcap or 0.0), int(keep_first or 0),
+            int(chunk or 0), _p(score_bias), self._stream()), self._generic_launches)
+
+    def _generic_step(self, ctx, n: int, n_q: int, n_kv: int, dv: int, bounded: bool):
+        """What the general attention kernel is told of a step: tokens, sequences, bounds on a sequence's new tokens and
+        keys, and scratch for the runs of steps with few tiles (``bounded``: a window or chunks, whose walk is short)."""
+        need = self.lib.idm_attention_generic_scratch_floats(n, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, n_q, n_kv, dv,
+                                                             1 if bounded else 0)
+        self._generic_launches = 2 if need else 1
+        return n, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, _p(self.scratch("attention_generic", need) if need else None)
 
     def head_finish(self, proj, col_q: int, col_k: int, col_v, n_q: int, n_kv: int, dk: int, dv: int, biases, gammas,
                     eps: float, cs, mag: float, kv, ctx, norm_all: bool = False, v_norm: bool = False,
@@ -830,8 +841,8 @@ class Kernels:
             _p(q), _p(out), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], kv.ring, _p(k_new), _p(v_new),
             _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots),
-            _p(ctx.q_start), _p(ctx.cu_q), n, n_q, kv.n_kv_heads,
-            hd, scale, (int(window) if window else 0), self._stream()))
+            _p(ctx.q_start), _p(ctx.cu_q), *self._generic_step(ctx, n, n_q, kv.n_kv_heads, hd, bool(window)),
+            n_q, kv.n_kv_heads, hd, scale, (int(window) if window else 0), self._stream()), self._generic_launches)
         return out
 
     def attention_decode(self, q, kv, slots, kv_len, max_kv_len: int, scale: float, window: int,

@@ -421,6 +421,81 @@ def test_ring_write_keeps_the_last_ring_tokens(kernels, dtype):
             assert torch.equal(kv.v[page, :, r], v_new[off + j - st])
 
 
+def _attention_64(q, k, v, positions, scale, window=None, keep_first=0, chunk=None, softcap=0.0, sink=None, slopes=None, score_bias=None):
+    """q [T, H, d] at ``positions`` against one sequence's k [L, G, d], v [L, G, dv], in 64 bits."""
+    T, H, _ = q.shape
+    per = H // k.shape[1]
+    j = torch.arange(k.shape[0])
+    out = torch.zeros(T, H, v.shape[2], dtype=torch.float64)
+    for t, p in enumerate(positions):
+        lo = p - p % chunk if chunk else max(0, p - window + 1) if window else 0
+        see = (j <= p) & ((j >= lo) | ((j < keep_first) if window else (j < 0)))
+        for h in range(H):
+            s = (k[see, h // per] @ q[t, h]) * scale
+            if softcap:
+                s = softcap * torch.tanh(s / softcap)
+            if slopes is not None:
+                s = s - slopes[h] * (p - j[see])
+            if score_bias is not None:
+                w = torch.sigmoid(s + score_bias[h])
+            else:
+                e = torch.cat([s, sink[h:h + 1]]) if sink is not None else s
+                w = torch.softmax(e, dim=0)[:s.numel()]
+            out[t, h] = w @ v[see, h // per]
+    return out
+
+
+# tiles of 4, 16 and 32 rows (and a group of heads wider than a tile), rows that fill no tile, one to three runs of 128 keys, every
+# option, and odd widths; single tokens of few sequences leave their runs in scratch, the prompt walks them
+@pytest.mark.parametrize("n_q,n_kv,hd,dv,length,opts", [
+    (4, 2, 64, 64, 300, {}), (6, 2, 36, 20, 131, {"window": 70}), (16, 8, 128, 128, 257, {"sink": True}),
+    (3, 1, 128, 72, 200, {"window": 40, "keep_first": 5}), (40, 1, 24, 136, 129, {"softcap": 3.0}), (16, 1, 256, 256, 140, {"slopes": True}),
+    (5, 5, 7, 9, 260, {"chunk": 100}), (8, 2, 96, 128, 190, {"score_bias": True})])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_general_attention_is_one_sum_in_every_tile(kernels, dtype, n_q, n_kv, hd, dv, length, opts):
+    K = kernels(dtype)
+    if dtype == "bfloat16" and (hd % 8 or dv % 8) and hd != 7:
+        pytest.skip("the odd widths run in 32-bit")
+    lens = [length, 37, 64]
+    need = CacheNeed("full", n_kv, hd, k_row=(n_kv, hd), v_row=(n_kv, dv))
+    cache = SequenceCache({0: need}, 64 * 16, DT[dtype], "cuda:0", max_seqs=3)
+    slots = [cache.alloc_slot() for _ in lens]
+    cache.reserve(list(zip(slots, lens))); cache.flush()
+    kv = cache.view(0)
+    kv.k.fill_(float("nan")); kv.v.fill_(float("nan"))           # what no query sees is never touched
+    q = _randn(sum(lens), n_q, hd, seed=90).to(DT[dtype])
+    k, v = _randn(sum(lens), n_kv, hd, seed=91).to(DT[dtype]), _randn(sum(lens), n_kv, dv, seed=92).to(DT[dtype])
+    at = 0
+    for s, n in zip(slots, lens):
+        for j in range(n):
+            page = int(kv.table[s, j // 64])
+            kv.k[page, :, j % 64], kv.v[page, :, j % 64] = k[at + j].cuda(), v[at + j].cuda()
+        at += n
+    args = {n: (_randn(n_q, seed=93).float() if x is True else x) for n, x in opts.items()}
+    dev = {n: (x.cuda() if isinstance(x, torch.Tensor) else x) for n, x in args.items()}
+
+    def run(rows, starts, counts):
+        packed, n, q_lens = pack_step_host(slots, starts, [[0] * c for c in counts])
+        ctx = context_from_packed(packed.cuda(), n, slots, q_lens, starts)
+        out = torch.empty((n, n_q * dv), dtype=DT[dtype], device="cuda")
+        K.attention_biased(q[rows].contiguous().cuda(), kv, ctx, hd ** -0.5, out, 0, **dev)
+        return out.view(n, n_q, dv)
+    whole = run(list(range(sum(lens))), [0, 0, 0], lens)
+    at = 0
+    for i, n in enumerate(lens):
+        ref = _attention_64(q[at:at + n].double(), k[at:at + n].double(), v[at:at + n].double(), range(n), hd ** -0.5,
+                            **{m: (x.double() if isinstance(x, torch.Tensor) else x) for m, x in args.items()})
+        # 32-bit sums of up to 256 products, softmax over up to 300 keys (bfloat16 rounds the result); a slope times the distance makes
+        # scores as large as max|slope| * (n - 1), which 32 bits hold to 2^-24 of that, and a weight is off by as much as its score
+        tol = max(KTOL[dtype], float(args["slopes"].abs().max()) * (n - 1) * 2.0 ** -24 if "slopes" in args else 0.0)
+        assert helpers.rel_err(whole[at:at + n], ref) < tol, f"sequence {i}"
+        at += n
+    first = [0, lens[0], lens[0] + lens[1]]
+    for few in (1, 3, 7):                                         # the last tokens of each sequence, so many at once
+        rows = [first[i] + lens[i] - few + j for i in range(3) for j in range(few)]
+        assert torch.equal(run(rows, [n - few for n in lens], [few] * 3), whole[rows]), f"{few} tokens a sequence"
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_swiglu(kernels, dtype):
     K = kernels(dtype)
