@@ -580,7 +580,7 @@ def decode_kernel_times(lm, lens, seed: int):
              "ssd_scan", "ssd_group_norm", "token_gate", "gated_act", "attention_lse_gate", "add_dyt", "latent_kv_finish",
              "headwise", "latent_attention", "experts_few", "act_cast", "concat_cast", "logit_cap", "add_rmsnorm2", "head_finish",
              "attention_biased", "cols_cast", "delta_prep", "delta_scan", "delta_out", "gate_scale", "embed_bigram", "post_layernorm",
-             "add_layernorm", "route", "experts_identity", "sum_norm", "grouped_rmsnorm", "experts_dense", "experts_grouped_step", "conv_state_update",
+             "add_layernorm", "route", "experts_identity", "sum_norm", "grouped_rmsnorm", "experts_by_expert", "conv_state_update",
              "retention", "diff_combine"]
     names = [n for n in names if hasattr(K, n)]
     out, saved = {}, {n: getattr(K, n) for n in names}

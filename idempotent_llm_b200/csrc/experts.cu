@@ -1,9 +1,9 @@
 // Feed-forward experts chosen per token: out[t] = weight * sum_k down_e (act(gate_e x_t) * up_e x_t), e = the
 // k-th expert of token t = table[token id of t, k] (a table of integers [vocabulary, top]).  These kernels serve steps of few tokens (single tokens above all): every (token,
 // choice) streams its expert's matrices once, a warp per output row, sums in 32-bit in a fixed order, so a
-// token's result does not depend on what else the step holds.  Steps of many tokens group their rows by expert
-// on the host and run one matrix product per expert instead; the kernels below then gather the rows
-// (rows_gather) and add the experts' outputs back in the order of a token's choices (experts_combine).
+// token's result does not depend on what else the step holds.  Steps of many tokens group their rows by expert: in bfloat16 on
+// the device, with one product over all experts (idm_experts_by_expert); in 32-bit on the host, with one product per expert
+// between rows_gather and experts_combine, which adds the experts' outputs back in the order of a token's choices.
 //
 // A learned router names a token's experts on the device: then `tokens` holds the step's row numbers and `table` the
 // step's choices [rows, top], and `pair_w` [rows, top] (null: 1) is the weight of every (token, choice) beside the
@@ -187,29 +187,74 @@ extern "C" int idm_rows_gather(const void* x, const int* src, void* out, int n_r
     return 0;
 }
 
-// h[t, :] += weight * sum_k z[place[t, k], :] in ascending k  (z 32-bit: the experts' outputs, grouped rows)
-__global__ void __launch_bounds__(256) experts_combine_kernel(const float* __restrict__ z, const int* __restrict__ place,
-                                                              const float* __restrict__ pair_w, float* __restrict__ h, int width,
-                                                              int top, float weight) {
+// h[t, :] += weight * sum_k z[place[t, k], :] in ascending k  (z 32-bit: the experts' outputs, grouped rows), and with x then
+// += x[t, :] * (the weights of t's pairs whose expert table[tokens[t], k] is n_real or more: experts that hand their input on).
+// Four elements a thread where rows allow it, four pairs' loads at a time: bound by the bytes of z.
+struct CombineArgs {
+    const float* z; const int* place; const float* pair_w; float* h;
+    int width, top; float weight;
+    const T* x; const int* tokens; const int* table; int n_real;
+};
+template <int V>
+__global__ void __launch_bounds__(256) experts_combine_kernel(CombineArgs a) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t t = blockIdx.x;
-    for (int d = threadIdx.x; d < width; d += blockDim.x) {
-        float s = 0.f;
-        for (int k = 0; k < top; ++k) {
-            const int r = place ? place[t * top + k] : (int)(t * top + k);      // (no places: pair by pair as they lie)
-            if (r >= 0) s = pair_w ? fmaf(pair_w[t * top + k], z[(size_t)r * width + d], s) : s + z[(size_t)r * width + d];
+    const int top = a.top;
+    float same = 0.f;                                                        // the identity experts' weight
+    if (a.x)
+        for (int k = 0; k < top; ++k)
+            if (a.table[(size_t)a.tokens[t] * top + k] >= a.n_real) same += a.pair_w[t * top + k];
+    for (int d = threadIdx.x * V; d < a.width; d += blockDim.x * V) {
+        float s[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) s[i] = 0.f;
+        for (int k0 = 0; k0 < top; k0 += 4) {
+            float v[4][V], pw[4];
+            int r[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const size_t p = t * top + k0 + j;
+                r[j] = k0 + j >= top ? -1 : a.place ? a.place[p] : (int)p;   // (no places: pair by pair as they lie)
+                pw[j] = r[j] >= 0 && a.pair_w ? a.pair_w[p] : 1.f;
+                if (r[j] < 0) continue;
+                const float* z = a.z + (size_t)r[j] * a.width + d;
+                if (V == 4) *reinterpret_cast<float4*>(v[j]) = *reinterpret_cast<const float4*>(z);
+                else v[j][0] = *z;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (r[j] >= 0) {
+#pragma unroll
+                    for (int i = 0; i < V; ++i) s[i] = a.pair_w ? fmaf(pw[j], v[j][i], s[i]) : s[i] + v[j][i];
+                }
         }
-        h[t * width + d] += s * weight;
+        float* h = a.h + t * a.width + d;
+        float o[V];
+        if (V == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(h);
+        else o[0] = *h;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            o[i] += s[i] * a.weight;
+            if (a.x && same != 0.f) o[i] = fmaf(same, to_f32(a.x[t * a.width + d + i]), o[i]);
+        }
+        if (V == 4) *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(o);
+        else *h = o[0];
     }
+}
+
+static int experts_combine(const CombineArgs& a, int n_tokens, cudaStream_t stream) {
+    const bool vec = a.width % 4 == 0 && (((uintptr_t)a.z | (uintptr_t)a.h) & 15) == 0;
+    const int threads = vec ? min(256, (a.width / 4 + 31) / 32 * 32) : 256;
+    idm_launch(vec ? experts_combine_kernel<4> : experts_combine_kernel<1>, dim3(n_tokens), dim3(threads), 0, stream, a);
+    IDM_LAUNCH_CHECK("experts_combine");
+    return 0;
 }
 
 extern "C" int idm_experts_combine(const float* z, const int* place, const float* pair_w, float* h, int n_tokens, int width,
                                    int top, float weight, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
-    idm_launch(experts_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, z, place, pair_w, h, width, top, weight);
-    IDM_LAUNCH_CHECK("experts_combine");
-    return 0;
+    return experts_combine(CombineArgs{z, place, pair_w, h, width, top, weight, nullptr, nullptr, nullptr, 0}, n_tokens, stream);
 }
 
 // out[place[p]] = pair_w[p] for every (token, choice) p that has a grouped row
@@ -363,119 +408,144 @@ extern "C" int idm_experts_major(const void* x, const int* tokens, const int* ta
     idm_launch(experts_major_kernel<1>, dim3(n_experts, by2), dim3(256), s2, stream, (const T*)nullptr, (const float*)a, tokens, table, (const float*)nullptr,
                (const T*)down, (long long)width * ff, (long long)ff, 0LL, z, n_tokens, top, ff, width, act, 0);
     IDM_LAUNCH_CHECK("experts_major down");
-    idm_launch(experts_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, (const float*)z, (const int*)nullptr, (const float*)nullptr, h,
-               width, top, weight);
-    IDM_LAUNCH_CHECK("experts_combine");
-    return 0;
+    return experts_combine(CombineArgs{z, nullptr, nullptr, h, width, top, weight, nullptr, nullptr, nullptr, 0}, n_tokens, stream);
 }
 
 #if defined(IDM_BF16)
-// Every expert's gated feed-forward over its slice of rows grouped by expert: the library's own matrix products (the
-// gate/up product with the activation as its epilogue, then the down product), expert after expert, from one call.
-// counts: on the HOST, rows of each expert; gate_up [E, tiles * 128, width] alternating rows; down [E, width, ff].
-// row_w (or null): a number per grouped row that multiplies the row's pre-activations (a weight on the expert's input).
-extern "C" int idm_gemm_bf16_gated_rows(const void* x, const void* w, void* y, int M, int inter, int K, int act, const float* row_w, cudaStream_t stream);
-extern "C" int idm_gemm_bf16(const void* x, const void* w, float* out, int M, int N, int K, cudaStream_t stream);
-
-static int experts_grouped(const void* xg, const float* row_w, const int* counts, int n_experts, const void* gate_up,
-                                   long long gate_up_stride, const void* down, long long down_stride, void* y, float* z,
-                                   int width, int ff, int act, cudaStream_t stream) {
-    IDM_REQUIRE(width > 0 && ff > 0 && width % 8 == 0 && ff % 8 == 0, "experts_grouped: width=%d ff=%d (multiples of 8)", width, ff);
-    long long at = 0;
-    for (int e = 0; e < n_experts; ++e) {
-        const int c = counts[e];
-        if (c <= 0) continue;
-        const T* xe = (const T*)xg + at * width;
-        T* ye = (T*)y + at * ff;
-        if (idm_gemm_bf16_gated_rows(xe, (const T*)gate_up + (long long)e * gate_up_stride, ye, c, ff, width, act, row_w ? row_w + at : nullptr, stream)) return 1;
-        if (idm_gemm_bf16(ye, (const T*)down + (long long)e * down_stride, z + at * width, c, width, ff, stream)) return 1;
-        at += c;
-    }
-    return 0;
+// ------------------------------------------------------------------ steps of many (token, choice) pairs, grouped by expert
+// The pairs in the order of their experts, ascending inside an expert: offsets [E + 1] (an expert's first row), place [N, top] (a
+// pair's row, -1 for a pair that names no expert), xg [rows, width] (the pairs' input rows) and, if asked for, row_w [rows]
+// (their weights).  A block has some tokens and counts for itself how many pairs of each expert lie before them (the pairs
+// are a few hundred KB at most, in the L2), so one launch does it all, without a count from the host; then it copies
+// its tokens' rows, each read once.  Bound by the bytes of xg.
+#define EG_THREADS 512
+struct GroupArgs {
+    const T* x; const int* tokens; const int* table; const float* pair_w;
+    int n_tokens, top, n_experts, width, block_tokens;
+    int* place; int* offsets; float* row_w; T* xg;
+};
+__device__ __forceinline__ int pair_expert(const GroupArgs& a, int p) {      // of pair p = token * top + choice, or -1
+    const int t = p / a.top, e = a.table[(size_t)a.tokens[t] * a.top + (p - t * a.top)];
+    return e >= 0 && e < a.n_experts ? e : -1;
 }
-
-extern "C" int idm_experts_grouped(const void* xg, const int* counts, int n_experts, const void* gate_up,
-                                   long long gate_up_stride, const void* down, long long down_stride, void* y, float* z,
-                                   int width, int ff, int act, cudaStream_t stream) {
-    return experts_grouped(xg, nullptr, counts, n_experts, gate_up, gate_up_stride, down, down_stride, y, z, width, ff, act, stream);
-}
-
-// The grouped feed-forward of a step from one call: rows gathered in the order of their experts (src: grouped row ->
-// token), every expert's two products, outputs added into the stream in the order of a token's choices (place:
-// (token, choice) -> grouped row).  xg, y, z: scratch [n_tokens * top, width | ff | width].  row_w (scratch [n_tokens *
-// top], or null): the pairs' weights belong on the experts' inputs; they are put in the order of the grouped rows there.
-extern "C" int idm_experts_grouped_step(const void* x, const int* src, const int* place, const float* pair_w, const int* counts, int n_experts,
-                                        const void* gate_up, long long gate_up_stride, const void* down, long long down_stride,
-                                        void* xg, void* y, float* z, float* h, int n_tokens, int top, int width, int ff, int act,
-                                        float weight, float* row_w, cudaStream_t stream) {
-    if (n_tokens == 0) return 0;
-    IDM_REQUIRE(row_w == nullptr || pair_w != nullptr, "experts_grouped_step: weights on the inputs need the pairs' weights");
-    if (idm_rows_gather(x, src, xg, n_tokens * top, width, stream)) return 1;
-    if (row_w && idm_rows_weight(pair_w, place, row_w, n_tokens * top, stream)) return 1;
-    if (experts_grouped(xg, row_w, counts, n_experts, gate_up, gate_up_stride, down, down_stride, y, z, width, ff, act, stream)) return 1;
-    return idm_experts_combine(z, place, row_w ? nullptr : pair_w, h, n_tokens, width, top, weight, stream);
-}
-
-// Single-token steps of many sequences, whose ids exist on the device only and whose shapes must not change from
-// step to step: EVERY expert's feed-forward over ALL the step's tokens with the library's matrix products (what such a
-// step has to do anyway is to stream every expert's matrices once: the products it does not need ride along), then
-// each token takes the outputs of its own experts.  z_all: [E, n_tokens, width] 32-bit; y: [n_tokens, ff] scratch.
-__global__ void __launch_bounds__(256) experts_pick_kernel(const float* __restrict__ z_all, const int* __restrict__ tokens,
-                                                           const int* __restrict__ table, const float* __restrict__ pair_w,
-                                                           float* __restrict__ h, int n_tokens, int width, int top, int n_experts,
-                                                           float weight) {
+__global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) {
     pdl_launch_dependents();
     pdl_wait();
-    const size_t t = blockIdx.x;
-    for (int d = threadIdx.x; d < width; d += blockDim.x) {
-        float s = 0.f;
-        for (int k = 0; k < top; ++k) {
-            const int e = table[(size_t)tokens[t] * top + k];
-            if (e >= 0 && e < n_experts) {
-                const float z = z_all[((size_t)e * n_tokens + t) * width + d];
-                s = pair_w ? fmaf(pair_w[t * top + k], z, s) : s + z;
+    extern __shared__ int group_sm[];
+    int* total = group_sm;                                                         // pairs of an expert; then the expert's first row
+    int* before = total + a.n_experts;                                       // those before this block's; then before the next pair
+    int* at = before + a.n_experts;                                          // [block_tokens * top]: this block's pairs' rows
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * a.block_tokens, t1 = min(t0 + a.block_tokens, a.n_tokens);
+    const int pairs = a.n_tokens * a.top, p0 = t0 * a.top, p1 = t1 * a.top;
+    for (int e = threadIdx.x; e < a.n_experts; e += EG_THREADS) { total[e] = 0; before[e] = 0; }
+    __syncthreads();
+    for (int c0 = warp * 32; c0 < pairs; c0 += 8 * EG_THREADS) {             // eight looks at the table on their way at a time
+        int named[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int p = c0 + j * EG_THREADS + lane;
+            named[j] = p < pairs ? pair_expert(a, p) : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = named[j];
+            const unsigned same = __match_any_sync(0xffffffffu, e), early = __ballot_sync(0xffffffffu, c0 + j * EG_THREADS + lane < p0);
+            if (e >= 0 && lane == __ffs(same) - 1) {
+                atomicAdd(&total[e], __popc(same));
+                if (same & early) atomicAdd(&before[e], __popc(same & early));
             }
         }
-        h[t * width + d] += s * weight;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int rows = 0;                                                        // of the experts so far
+        for (int e0 = 0; e0 < a.n_experts; e0 += 32) {
+            const int e = e0 + lane, n = e < a.n_experts ? total[e] : 0;
+            int upto = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
+            if (e < a.n_experts) {
+                total[e] = rows + upto - n;
+                if (blockIdx.x == 0) a.offsets[e] = rows + upto - n;
+            }
+            rows += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (blockIdx.x == 0 && lane == 0) a.offsets[a.n_experts] = rows;
+        __syncwarp();
+        for (int c = p0; c < p1; c += 32) {
+            const int p = c + lane, e = p < p1 ? pair_expert(a, p) : -1;
+            const unsigned same = __match_any_sync(0xffffffffu, e);
+            const int row = e >= 0 ? total[e] + before[e] + __popc(same & ((1u << lane) - 1u)) : -1;
+            __syncwarp();
+            if (e >= 0 && lane == __ffs(same) - 1) before[e] += __popc(same);
+            __syncwarp();
+            if (p < p1) {
+                at[p - p0] = row;
+                a.place[p] = row;
+                if (row >= 0 && a.row_w) a.row_w[row] = a.pair_w[p];
+            }
+        }
+    }
+    __syncthreads();
+    // 16-byte pieces of this block's rows (whole pieces, width % 8 == 0), one after another over all threads, four on their way
+    const int pieces = a.width / Vec16<T>::N, all = (t1 - t0) * pieces;
+    const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)t0 * a.width);
+    uint4* dst = reinterpret_cast<uint4*>(a.xg);
+    for (int i0 = threadIdx.x; i0 < all; i0 += 4 * EG_THREADS) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i0 + j * EG_THREADS < all) v[j] = src[i0 + j * EG_THREADS];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + j * EG_THREADS, t = i / pieces, piece = i - t * pieces;
+            if (i >= all) break;
+            for (int k = 0; k < a.top; ++k) {
+                const int row = at[t * a.top + k];
+                if (row >= 0) dst[(size_t)row * pieces + piece] = v[j];
+            }
+        }
     }
 }
 
-// out[e, t] = the weight of token t's pair that names expert e (0 where none does): one thread per (expert, token)
-__global__ void __launch_bounds__(256) experts_weight_table_kernel(const int* __restrict__ tokens, const int* __restrict__ table,
-                                                                   const float* __restrict__ pair_w, float* __restrict__ out,
-                                                                   int n_tokens, int top, int n_experts) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_tokens * n_experts) return;
-    const int e = i / n_tokens, t = i % n_tokens;
-    float w = 0.f;
-    for (int k = 0; k < top; ++k)
-        if (table[(size_t)tokens[t] * top + k] == e) w = pair_w[t * top + k];
-    out[i] = w;
-}
+int gemm_experts_store(const void* x, const void* w, float* out, const int* offsets, int n_experts, int n_rows, int N, int K, cudaStream_t stream);
+int gemm_experts_gated(const void* x, const void* w_tiled, void* y, const int* offsets, int n_experts, int n_rows, int inter, int K, int act,
+                       const float* row_w, cudaStream_t stream);
 
-// weights_in (scratch [E, n_tokens], or null): the pairs' weights belong on the experts' inputs
-extern "C" int idm_experts_dense(const void* x, const int* tokens, const int* table, const float* pair_w, int n_experts, const void* gate_up,
-                                 long long gate_up_stride, const void* down, long long down_stride, void* y, float* z_all,
-                                 float* h, int n_tokens, int width, int ff, int top, int act, float weight, float* weights_in,
-                                 cudaStream_t stream) {
+// h[t] += weight * sum_k ff_e(x_t), e = table[tokens[t], k], with the pairs grouped by expert: one launch groups them, one makes every
+// expert's gated product (gate_up [E, tiles * 128, width], gate and up rows alternating), one every expert's down product (down
+// [E, width, ff]), one adds the outputs up in the order of a token's choices.  Nothing depends on the host: steps can be captured.
+// pair_w [N, top] (or null: 1) weighs the outputs, or (weight_in) the inputs; `identity`: pairs that name expert E or more add
+// their weight times x_t itself.  scratch: xg, y [N * top, width | ff], z 32-bit [N * top, width], ints [E + 1 + N * top], row_w [N * top].
+extern "C" int idm_experts_by_expert(const void* x, const int* tokens, const int* table, const float* pair_w, int n_experts, const void* gate_up,
+                                     const void* down, void* xg, void* y, float* z, int* ints, float* row_w, float* h, int n_tokens, int top,
+                                     int width, int ff, int act, float weight, int weight_in, int identity, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
-    IDM_REQUIRE(weights_in == nullptr || pair_w != nullptr, "experts_dense: weights on the inputs need the pairs' weights");
-    if (weights_in) {
-        idm_launch(experts_weight_table_kernel, dim3((n_tokens * n_experts + 255) / 256), dim3(256), 0, stream, tokens, table, pair_w, weights_in,
-                   n_tokens, top, n_experts);
-        IDM_LAUNCH_CHECK("experts_weight_table");
-    }
-    IDM_REQUIRE(width > 0 && ff > 0 && width % 8 == 0 && ff % 8 == 0, "experts_dense: width=%d ff=%d (multiples of 8)", width, ff);
-    for (int e = 0; e < n_experts; ++e) {
-        if (idm_gemm_bf16_gated_rows(x, (const T*)gate_up + (long long)e * gate_up_stride, y, n_tokens, ff, width, act,
-                                     weights_in ? weights_in + (size_t)e * n_tokens : nullptr, stream)) return 1;
-        if (idm_gemm_bf16(y, (const T*)down + (long long)e * down_stride, z_all + (size_t)e * n_tokens * width, n_tokens, width, ff, stream)) return 1;
-    }
-    idm_launch(experts_pick_kernel, dim3(n_tokens), dim3(256), 0, stream, (const float*)z_all, tokens, table, weights_in ? (const float*)nullptr : pair_w, h,
-               n_tokens, width, top, n_experts, weight);
-    IDM_LAUNCH_CHECK("experts_pick");
-    return 0;
+    IDM_REQUIRE(width > 0 && ff > 0 && width % 8 == 0 && ff % 8 == 0, "experts_by_expert: width=%d ff=%d (multiples of 8)", width, ff);
+    IDM_REQUIRE(n_experts > 0 && top > 0 && (long long)n_tokens * top < (1ll << 31), "experts_by_expert: %d experts, %d x %d pairs", n_experts, n_tokens, top);
+    IDM_REQUIRE(!(weight_in || identity) || pair_w, "experts_by_expert: weights on the inputs, or identity experts, need the pairs' weights");
+    IDM_REQUIRE(((uintptr_t)x & 15) == 0, "experts_by_expert: rows must start on 16-byte borders");
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    GroupArgs g;
+    g.x = (const T*)x; g.tokens = tokens; g.table = table; g.pair_w = pair_w;
+    g.n_tokens = n_tokens; g.top = top; g.n_experts = n_experts; g.width = width;
+    // two blocks an SM, so that few blocks count all pairs; no more pairs a block than one warp places in a moment
+    const int even = (n_tokens + 2 * sms - 1) / (2 * sms), most = 512 / top > 0 ? 512 / top : 1;
+    g.block_tokens = even < most ? even : most;
+    g.offsets = ints; g.place = ints + n_experts + 1; g.row_w = weight_in ? row_w : nullptr; g.xg = (T*)xg;
+    const size_t smem = (size_t)(2 * n_experts + g.block_tokens * top) * sizeof(int);
+    IDM_REQUIRE(smem <= 200 * 1024, "experts_by_expert: %d experts do not fit shared memory", n_experts);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(experts_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    idm_launch(experts_group_kernel, dim3((n_tokens + g.block_tokens - 1) / g.block_tokens), dim3(EG_THREADS), smem, stream, g);
+    IDM_LAUNCH_CHECK("experts_group");
+    const int rows = n_tokens * top;
+    if (gemm_experts_gated(xg, gate_up, y, g.offsets, n_experts, rows, ff, width, act, g.row_w, stream)) return 1;
+    if (gemm_experts_store(y, down, z, g.offsets, n_experts, rows, width, ff, stream)) return 1;
+    CombineArgs c{z, g.place, weight_in ? nullptr : pair_w, h, width, top, weight, nullptr, nullptr, nullptr, n_experts};
+    if (identity) { c.x = (const T*)x; c.tokens = tokens; c.table = table; }
+    return experts_combine(c, n_tokens, stream);
 }
 #endif

@@ -172,9 +172,11 @@ __device__ __forceinline__ void persistent_tile_epilogue(const GemmEpi& e, uint3
     // the accumulator columns of a chunk are asked for while the chunk before is worked on (two sets of
     // registers in turn; the loop is unrolled so that which set is which is known at compile time)
     uint32_t raw[2][GP_CHUNK];
+    constexpr int PASSES = (BN + GP_GROUPS * GP_CHUNK - 1) / (GP_GROUPS * GP_CHUNK);
+    if (BN < GP_GROUPS * GP_CHUNK && grp * GP_CHUNK >= BN) return;     // (a narrow tile: only the first groups have a chunk)
     if (t0 + grp * GP_CHUNK < n_tokens) tc_ld16_issue(tmem_acc + lane_base + (uint32_t)(grp * GP_CHUNK), raw[0]);
 #pragma unroll
-    for (int ci = 0; ci < BN / (GP_GROUPS * GP_CHUNK); ++ci) {
+    for (int ci = 0; ci < PASSES; ++ci) {
         const int c0 = grp * GP_CHUNK + ci * GP_GROUPS * GP_CHUNK;
         if (t0 + c0 >= n_tokens) break;                    // uniform over the group
         const int cols = min(GP_CHUNK, n_tokens - t0 - c0);
@@ -182,7 +184,7 @@ __device__ __forceinline__ void persistent_tile_epilogue(const GemmEpi& e, uint3
         tc_ld_wait();
 #pragma unroll
         for (int j = 0; j < GP_CHUNK; ++j) v[j] = __uint_as_float(raw[ci & 1][j]);
-        if (ci + 1 < BN / (GP_GROUPS * GP_CHUNK) && t0 + c0 + GP_GROUPS * GP_CHUNK < n_tokens)
+        if (ci + 1 < PASSES && t0 + c0 + GP_GROUPS * GP_CHUNK < n_tokens)
             tc_ld16_issue(tmem_acc + lane_base + (uint32_t)(c0 + GP_GROUPS * GP_CHUNK), raw[(ci + 1) & 1]);
         if (EPI == EPI_STORE || EPI == EPI_RESIDUAL) {
             if (f < n_features) {
@@ -336,6 +338,134 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_persistent_kernel(const __gri
             if (!ok) break;
             tc_fence_after();
             persistent_tile_epilogue<BN, EPI>(e, tmem + acc * BN, xs, grp, quarter, lane, tx, t0, n_tokens, n_features);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty_bar(acc));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == GP_EPI_WARPS + 1) tmem_dealloc(tmem, TMEM_COLS);
+}
+
+// ------------------------------------------------------------------- rows grouped by expert (persistent)
+// The persistent scheme over the tiles of ALL experts in one launch: rows [offsets[e], offsets[e + 1]) of x meet expert e's
+// matrix, rows [e * expert_rows, ...) of w.  How many rows an expert has is read from the device, so a step needs nothing
+// from the host and can be captured; a block finds its tiles by walking the experts (each role for itself, from shared
+// memory).  An expert's tiles go feature tile after feature tile, so that neighbouring blocks read the same 128 rows of the
+// weight.  One product per expert and launch, which this replaces, leaves most SMs without a tile and pays 5
+// us or more each: 16 experts of 1024 x 768, 4 a token, 64 tokens 165 -> 28 us, 2 048 tokens some 350 -> 92 us (205 TFLOP/s, of
+// which 30 us are the grouping and the sum); 14 experts of 4096 x 3072 with 3 250 tokens 946 us (1 037 TFLOP/s).
+#define GE_SMEM_EXPERTS 400        // offsets of up to so many experts wait in shared memory (what is left beside the rings)
+struct ExpertWalk {
+    const int* offs;
+    int n_experts, tiles_x, bn;
+    int e, row0, row1, first, across;                              // the expert, its rows, its first tile, tiles over its rows
+    __device__ __forceinline__ ExpertWalk(const int* o, int n, int tx, int b) : offs(o), n_experts(n), tiles_x(tx), bn(b), e(-1), row1(0), first(0), across(0) { next(); }
+    __device__ __forceinline__ void next() {
+        first += tiles_x * across;
+        row0 = row1;
+        if (++e < n_experts) { row1 = offs[e + 1]; across = (row1 - row0 + bn - 1) / bn; }
+    }
+    // the place of tile number `tile` (asked for in ascending order); false: there are no more
+    __device__ __forceinline__ bool place(int tile, int& fx, int& t0) {
+        while (e < n_experts && tile >= first + tiles_x * across) next();
+        if (e >= n_experts) return false;
+        const int r = tile - first;
+        fx = r / across;
+        t0 = row0 + (r - fx * across) * bn;
+        return true;
+    }
+};
+
+template <int BN, int STAGES, int EPI>
+__global__ void __launch_bounds__(GP_THREADS) gemm_experts_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                                  const __grid_constant__ CUtensorMap map_x, const GemmEpi e,
+                                                                  const int* __restrict__ offsets, int n_experts, int expert_rows,
+                                                                  int n_features, int kb_total, int tiles_x) {
+    using S = PersistSmem<BN, STAGES>;
+    constexpr int TMEM_COLS = 2 * BN;                              // 64 to 512
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t bars = base + S::BAR_OFF;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+    auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
+    auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + S::BAR_OFF + 8 * (2 * STAGES + 4));
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    int* held = (int*)(gen_base + S::BAR_OFF + 256);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), GP_EPI_WARPS); }
+        *abort_flag = 0;
+        mbar_init_fence();
+    }
+    if (warp == GP_EPI_WARPS + 1) tmem_alloc(smem_u32((const void*)tmem_slot), TMEM_COLS);
+    pdl_wait();
+    if (n_experts <= GE_SMEM_EXPERTS)
+        for (int i = threadIdx.x; i <= n_experts; i += GP_THREADS) held[i] = offsets[i];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    ExpertWalk walk(n_experts <= GE_SMEM_EXPERTS ? held : offsets, n_experts, tiles_x, BN);
+    int fx, t0;
+
+    if (warp == GP_EPI_WARPS) {
+        if (lane == 0) {
+            uint32_t cnt = 0;                                      // k-blocks issued so far, over all tiles
+            bool ok = true;
+            for (int tile = blockIdx.x; ok && walk.place(tile, fx, t0); tile += gridDim.x) {
+                const int wrow = walk.e * expert_rows + fx * GT_BM;
+                for (int i = 0; i < kb_total; ++i, ++cnt) {
+                    const int s = cnt % STAGES;
+                    ok = mbar_wait(empty_bar(s), ((cnt / STAGES) & 1) ^ 1, abort_flag, &g_gemm_error);
+                    if (!ok) break;
+                    mbar_expect_tx(full_bar(s), S::STAGE_BYTES);
+                    const uint32_t a_dst = base + s * S::STAGE_BYTES;
+                    tma_load_2d(a_dst, &map_w, i * GT_BK, wrow, full_bar(s));
+                    tma_load_2d(a_dst + S::A_BYTES, &map_x, i * GT_BK, t0, full_bar(s));
+                }
+            }
+        }
+    } else if (warp == GP_EPI_WARPS + 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = umma_idesc(GT_BM, BN);
+            uint32_t cnt = 0, it = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; ok && walk.place(tile, fx, t0); tile += gridDim.x, ++it) {
+                const uint32_t acc = it & 1;
+                ok = mbar_wait(tempty_bar(acc), ((it >> 1) & 1) ^ 1, abort_flag, &g_gemm_error);   // epilogue drained it
+                if (!ok) break;
+                tc_fence_after();
+                bool ready = mbar_try(full_bar(cnt % STAGES), (cnt / STAGES) & 1);               // (asked ahead, as above)
+                for (int i = 0; i < kb_total && ok; ++i, ++cnt) {
+                    const int s = cnt % STAGES;
+                    if (!ready) ok = mbar_wait(full_bar(s), (cnt / STAGES) & 1, abort_flag, &g_gemm_error);
+                    if (!ok) break;
+                    tc_fence_after();
+                    ready = i + 1 < kb_total && mbar_try(full_bar((cnt + 1) % STAGES), ((cnt + 1) / STAGES) & 1);
+                    const uint32_t a_addr = base + s * S::STAGE_BYTES;
+                    tc_mma_bf16_kblock(tmem + acc * BN, umma_desc_kmajor(a_addr), umma_desc_kmajor(a_addr + S::A_BYTES), idesc, i > 0 ? 1u : 0u);
+                    tc_commit(empty_bar(s));
+                }
+                if (ok) tc_commit(tfull_bar(acc));
+            }
+        }
+    } else {
+        const int quarter = warp & 3, grp = warp >> 2;
+        float* xs = (float*)(gen_base + S::XS_OFF) + grp * (GP_CHUNK * GT_BM);
+        uint32_t it = 0;
+        for (int tile = blockIdx.x; walk.place(tile, fx, t0); tile += gridDim.x, ++it) {
+            const uint32_t acc = it & 1;
+            if (!mbar_wait(tfull_bar(acc), (it >> 1) & 1, abort_flag, &g_gemm_error)) break;
+            tc_fence_after();
+            persistent_tile_epilogue<BN, EPI>(e, tmem + acc * BN, xs, grp, quarter, lane, fx, t0, walk.row1, n_features);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(acc));
@@ -1448,6 +1578,58 @@ static int gemm_any(const void* x, const void* w, GemmEpi e, int M, int N, int K
     if (make_map(&mx, x, M, K, wide ? 256 : 128)) return 1;
     return wide ? launch_persistent<256, 4, EPI>(mw, mx, e, M, N, kb_total, stream)
                 : launch_persistent<128, 6, EPI>(mw, mx, e, M, N, kb_total, stream);
+}
+
+// Every expert's product over its rows of x [n_rows, K] (see gemm_experts_kernel): `out` 32-bit [n_rows, n_features], or the gated
+// activation y [n_rows, inter] of alternating gate and up rows.  w [n_experts * expert_rows, K]; offsets [n_experts + 1] on the device.
+template <int BN, int STAGES, int EPI>
+static int launch_experts(const void* x, const void* w, const GemmEpi& e, const int* offsets, int n_experts, int expert_rows, int n_rows,
+                          int n_features, int K, cudaStream_t stream) {
+    using S = PersistSmem<BN, STAGES>;
+    constexpr int BYTES = S::TOTAL + (GE_SMEM_EXPERTS + 1) * 4;
+    static_assert(BYTES <= 227 * 1024, "shared memory");
+    cudaError_t err = cudaFuncSetAttribute(gemm_experts_kernel<BN, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+    IDM_REQUIRE(err == cudaSuccess, "gemm_experts: cannot get %d bytes of shared memory: %s", BYTES, cudaGetErrorString(err));
+    CUtensorMap mw, mx;
+    if (make_map(&mw, w, n_experts * expert_rows, K, GT_BM)) return 1;
+    if (make_map(&mx, x, n_rows, K, BN)) return 1;
+    const int tiles_x = (n_features + GT_BM - 1) / GT_BM, sms = device_sms();
+    const long long most = (long long)tiles_x * (n_rows / BN + (n_experts < n_rows ? n_experts : n_rows));
+    idm_launch(gemm_experts_kernel<BN, STAGES, EPI>, dim3(most < sms ? (int)most : sms), dim3(GP_THREADS), (size_t)BYTES, stream, mw, mx, e, offsets,
+               n_experts, expert_rows, n_features, (K + GT_BK - 1) / GT_BK, tiles_x);
+    IDM_LAUNCH_CHECK("gemm_experts");
+    return 0;
+}
+
+template <int EPI>
+static int gemm_experts(const void* x, const void* w, const GemmEpi& e, const int* offsets, int n_experts, int expert_rows, int n_rows,
+                        int n_features, int K, cudaStream_t stream) {
+    IDM_REQUIRE(n_experts > 0 && n_rows > 0 && n_features > 0 && K > 0 && K % 8 == 0, "gemm_experts: %d experts, %d rows, %d x %d", n_experts, n_rows, n_features, K);
+    IDM_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0, "gemm_experts: operands must be 16-byte aligned");
+    IDM_REQUIRE((long long)n_experts * expert_rows < (1ll << 31), "gemm_experts: %d experts of %d rows", n_experts, expert_rows);
+    // Rows of an expert per tile, by the mean (us for a step, 16 experts of 1024 x 768, 4 a token, tiles of 32 / 64 / 128 / 256 rows): 16 rows an
+    // expert 28.1 / 29.4 / 29.8 / -; 32 34.6 / 31.1 / 32.0 / -; 128 68 / 56 / 44.8 / 43.9; 512 204 / 126 / 93.5 / 92.0; 2 048
+    // - / 457 / 318 / 272; 14 experts of 4096 x 3072 at 5 rows 202 / 207 / 213 / -, at 929 3816 / 1989 / 1344 / 946.
+    if (n_rows <= 24 * n_experts) return launch_experts<32, 9, EPI>(x, w, e, offsets, n_experts, expert_rows, n_rows, n_features, K, stream);
+    if (n_rows <= 64 * n_experts) return launch_experts<64, 8, EPI>(x, w, e, offsets, n_experts, expert_rows, n_rows, n_features, K, stream);
+    return launch_experts<256, 4, EPI>(x, w, e, offsets, n_experts, expert_rows, n_rows, n_features, K, stream);
+}
+
+int gemm_experts_store(const void* x, const void* w, float* out, const int* offsets, int n_experts, int n_rows, int N, int K, cudaStream_t stream) {
+    GemmEpi e = {};
+    e.out = out;
+    return gemm_experts<EPI_STORE>(x, w, e, offsets, n_experts, N, n_rows, N, K, stream);
+}
+
+// row_w (or null): a number per row that multiplies gate and up before the activation
+int gemm_experts_gated(const void* x, const void* w_tiled, void* y, const int* offsets, int n_experts, int n_rows, int inter, int K, int act,
+                       const float* row_w, cudaStream_t stream) {
+    IDM_REQUIRE(act >= 0 && act < IDM_ACT_CLAMPED, "gemm_experts: activation %d takes constants or is not built", act);
+    GemmEpi e = {};
+    e.y = (T*)y; e.inter = inter; e.act = act; e.row_w = row_w;
+    const int rows = (inter + 63) / 64 * GT_BM;
+    return act == 0 && row_w == nullptr ? gemm_experts<EPI_SWIGLU>(x, w_tiled, e, offsets, n_experts, rows, n_rows, rows, K, stream)
+                                        : gemm_experts<EPI_GATED>(x, w_tiled, e, offsets, n_experts, rows, n_rows, rows, K, stream);
 }
 
 // out [M, N] = x . w^T (32-bit)

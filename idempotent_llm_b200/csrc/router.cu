@@ -11,7 +11,9 @@
 //
 // A column behind the E logits may hold a gate's pre-activation (a shared expert's): its sigmoid goes to gate_out[t].
 //
-// One warp per token; s and c wait in shared memory.  Nothing here depends on the other tokens of the step.
+// One warp per token.  Up to 32 experts a lane holds an expert's s and c (route_lanes_kernel: 2 048 tokens of 16 experts 4.7
+// us, where loops over shared memory by single lanes took 19 us); more wait in shared memory.  Both make the same
+// comparisons and sums.  Nothing here depends on the other tokens of the step.
 #include "common.cuh"
 
 #define RT_WARPS 4
@@ -110,6 +112,73 @@ __global__ void __launch_bounds__(RT_WARPS * 32) route_kernel(const float* __res
     for (int k = lane; k < top; k += 32) weight[(size_t)t * top + k] *= f;
 }
 
+// The same for up to 32 experts: lane e is expert e, a group's members read one another by shuffles.
+#define RL_WARPS 8
+__global__ void __launch_bounds__(RL_WARPS * 32) route_lanes_kernel(const float* __restrict__ z, int z_stride,
+                                                                    const float* __restrict__ correction, int* __restrict__ chosen,
+                                                                    float* __restrict__ weight, int n_tokens, int E, int top,
+                                                                    int count, int keep, int group_top, float scale, int sigmoid,
+                                                                    int renorm, float* __restrict__ gate_out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, t = blockIdx.x * RL_WARPS + (threadIdx.x >> 5);
+    if (t >= n_tokens) return;                                   // whole warps leave
+    const float* zr = z + (size_t)t * z_stride;
+    const bool real = lane < E;
+    const float v = real ? zr[lane] : -INFINITY;
+    if (gate_out && lane == 0) gate_out[t] = 1.0f / (1.0f + expf(-zr[E]));
+    float s, c;
+    if (sigmoid) {
+        s = 1.0f / (1.0f + expf(-v));
+        c = real ? correction ? s + correction[lane] : v : -INFINITY;
+    } else {
+        const float m = warp_max(v), p = real ? expf(v - m) : 0.f;
+        s = p / warp_sum(p);
+        c = real ? s + (correction ? correction[lane] : 0.f) : -INFINITY;
+    }
+    if (count > 1 && keep < count) {
+        const int per = E / count, g = min(lane / per, count - 1), g0 = g * per;
+        float best = -INFINITY;
+        for (int j = 0; j < per; ++j) best = fmaxf(best, __shfl_sync(ALL, c, g0 + j));
+        int at = -1;
+        for (int j = 0; j < per; ++j) { const float o = __shfl_sync(ALL, c, g0 + j); if (at < 0 && o == best) at = g0 + j; }
+        float score = best, last = best;
+        for (int k = 1; k < group_top && k < per; ++k) {         // the next one down: smaller, or equal and further up
+            float nv = -INFINITY;
+            int idx = -1;
+            for (int j = 0; j < per; ++j) {
+                const float o = __shfl_sync(ALL, c, g0 + j);
+                const int e = g0 + j;
+                if ((o < last || (o == last && e > at)) && (idx < 0 || o > nv)) { nv = o; idx = e; }
+            }
+            if (idx >= 0) { score += nv; last = nv; at = idx; }
+        }
+        // the `keep` best groups, one after another, by their first lanes; a kept group's score becomes +infinity as its mark
+        const bool first = real && lane == g0;
+        for (int k = 0; k < keep; ++k) {
+            float bv = -INFINITY; int idx = 0x7fffffff;
+            if (first && score != INFINITY) { bv = score; idx = g; }
+            warp_argmax(bv, idx);
+            if (g == idx) score = INFINITY;
+        }
+        if (score != INFINITY) c = -INFINITY;
+    }
+    float total = 0.f, mine_w = 0.f;
+    int mine = -1;
+    for (int k = 0; k < top; ++k) {
+        float bv = c > -INFINITY ? c : -INFINITY; int idx = c > -INFINITY ? lane : 0x7fffffff;
+        warp_argmax(bv, idx);
+        if (idx == 0x7fffffff) idx = -1;                         // fewer experts open than `top`: the pair names no expert
+        const float sv = __shfl_sync(ALL, s, idx < 0 ? 0 : idx);
+        if (idx >= 0) total += sv;
+        if (lane == k) { mine = idx; mine_w = idx >= 0 ? sv : 0.f; }
+        if (lane == idx) c = -INFINITY;
+    }
+    const float f = renorm ? scale / (total + 1e-20f) : scale;
+    if (lane < top) { chosen[(size_t)t * top + lane] = mine; weight[(size_t)t * top + lane] = mine_w * f; }
+}
+
 extern "C" int idm_route(const float* z, int z_stride, const float* correction, int* chosen, float* weight, int n_tokens,
                          int n_experts, int top, int groups, int keep, int group_top, float scale, int sigmoid, int renorm,
                          float* gate_out, cudaStream_t stream) {
@@ -119,6 +188,12 @@ extern "C" int idm_route(const float* z, int z_stride, const float* correction, 
     IDM_REQUIRE(group_top >= 1, "route: a group's score is the sum of its %d largest", group_top);
     IDM_REQUIRE(groups >= 1 && n_experts % groups == 0 && keep >= 1 && keep <= groups, "route: %d experts in %d groups of which %d are kept",
                 n_experts, groups, keep);
+    if (n_experts <= 32) {
+        idm_launch(route_lanes_kernel, dim3((n_tokens + RL_WARPS - 1) / RL_WARPS), dim3(RL_WARPS * 32), 0, stream, z, z_stride, correction,
+                   chosen, weight, n_tokens, n_experts, top, groups, keep, group_top, scale, sigmoid, renorm, gate_out);
+        IDM_LAUNCH_CHECK("route");
+        return 0;
+    }
     const size_t smem = (size_t)RT_WARPS * (2 * n_experts + groups) * sizeof(float);
     IDM_REQUIRE(smem <= 160 * 1024, "route: %d experts do not fit shared memory", n_experts);
     if (smem > 48 * 1024) cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

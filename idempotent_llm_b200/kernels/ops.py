@@ -117,9 +117,7 @@ SIGNATURES = {
     "idm_experts_few": (c_int, "pppppqqqpppiiiiiifip"),
     "idm_experts_major": (c_int, "pppppqqqppppiiiiiifip"),
     "idm_rows_gather": (c_int, "pppiip"),
-    "idm_experts_grouped": (c_int, "ppipqpqppiiip"),
-    "idm_experts_dense": (c_int, "ppppipqpqpppiiiiifpp"),
-    "idm_experts_grouped_step": (c_int, "pppppipqpqppppiiiiifpp"),
+    "idm_experts_by_expert": (c_int, "ppppippppppppiiiiifiip"),
     "idm_dense_ff": (c_int, "ppppppiiiip"),
     "idm_experts_combine": (c_int, "ppppiiifp"),
     "idm_rows_weight": (c_int, "pppip"),
@@ -1207,43 +1205,31 @@ class Kernels:
         self._check(self.lib.idm_rows_weight(_p(pair_w), _p(place), _p(out), place.numel(), self._stream()))
         return out
 
-    def experts_dense(self, x, tokens, table, gate_up, down, h, act: int, weight: float, pair_w=None,
-                      weight_in: bool = False) -> None:
-        """``h[t] += weight * sum_k ff_e(x_t)``, ``e = table[tokens[t], k]``, by running EVERY expert over all the step's
-        tokens with the library's matrix products and letting each token pick its own (single-token steps of many
-        sequences: every expert's matrices are streamed once, in shapes that do not change from step to step)."""
+    def experts_by_expert(self, x, tokens, table, gate_up, down, h, act: int, weight: float, pair_w=None, weight_in: bool = False,
+                          identity: bool = False) -> None:
+        """``h[t] += weight * sum_k ff_e(x_t)``, ``e = table[tokens[t], k]``, with the (token, choice) pairs grouped by expert on the
+        device: an expert's matrices (``gate_up`` in the layout of ``tile_gate_up``) are read once a step, by one product over
+        all experts each way (bfloat16; steps of many pairs, captured ones too).  ``pair_w [N, top]`` weighs the pairs' outputs, or
+        with ``weight_in`` their inputs; ``identity``: a pair that names expert ``E`` or more adds its weight times ``x_t`` itself."""
         self._need(x, self.dtype, "experts input")
         self._need(h, torch.float32, "residual stream")
+        self._need(gate_up, self.dtype, "experts' gate and up rows")
+        self._need(down, self.dtype, "experts' down matrices")
+        self._need(tokens, torch.int32, "tokens")
+        self._need(table, torch.int32, "expert table")
         n, width = x.shape
         E, _, ff = down.shape
-        y = torch.empty((n, ff), dtype=self.dtype, device=self.device)
-        z = torch.empty((E, n, width), dtype=torch.float32, device=self.device)
-        w_in = torch.empty((E, n), dtype=torch.float32, device=self.device) if weight_in else None
-        self._check(self.lib.idm_experts_dense(_p(x), _p(tokens), _p(table), _p(pair_w), E, _p(gate_up), gate_up.shape[1] * width, _p(down),
-                                               width * ff, _p(y), _p(z), _p(h), n, width, ff, table.shape[1], act, float(weight),
-                                               _p(w_in), self._stream()), 2 * E + 1 + (1 if weight_in else 0))
-
-    def experts_grouped_step(self, x, src, place, counts, gate_up, down, h, act: int, weight: float, pair_w=None,
-                             weight_in: bool = False) -> None:
-        """A step's rows grouped by expert through every expert's gated feed-forward, from one call into the library:
-        rows gathered in the order of their experts (``src [rows]``: grouped row -> token), the gated product (activation
-        in its epilogue, ``gate_up`` in the layout of ``tile_gate_up``) and the down product of every expert that has
-        rows (``counts``: rows per expert, a contiguous int32 numpy array on the host), and the outputs added into ``h``
-        in the order of a token's choices (``place [tokens, top]``: (token, choice) -> grouped row)."""
-        self._need(x, self.dtype, "experts input")
-        self._need(h, torch.float32, "residual stream")
-        n, width = x.shape
-        E, _, ff = down.shape
-        top = place.shape[1]
+        top = table.shape[1]
+        if tuple(gate_up.shape) != (E, -(-ff // 64) * 128, width) or down.shape[1] != width or tuple(h.shape) != (n, width):
+            raise KernelError(f"experts: gate/up {tuple(gate_up.shape)}, down {tuple(down.shape)}, stream {tuple(h.shape)} for rows of {width}")
         xg = torch.empty((n * top, width), dtype=self.dtype, device=self.device)
         y = torch.empty((n * top, ff), dtype=self.dtype, device=self.device)
         z = torch.empty((n * top, width), dtype=torch.float32, device=self.device)
+        ints = torch.empty((E + 1 + n * top,), dtype=torch.int32, device=self.device)
         row_w = torch.empty((n * top,), dtype=torch.float32, device=self.device) if weight_in else None
-        with_rows = int((counts > 0).sum())
-        self._check(self.lib.idm_experts_grouped_step(_p(x), _p(src), _p(place), _p(pair_w), counts.ctypes.data, E, _p(gate_up),
-                                                      gate_up.shape[1] * width, _p(down), width * ff, _p(xg), _p(y), _p(z), _p(h),
-                                                      n, top, width, ff, act, float(weight), _p(row_w), self._stream()),
-                    2 * with_rows + 2 + (1 if weight_in else 0))
+        self._check(self.lib.idm_experts_by_expert(_p(x), _p(tokens), _p(table), _p(pair_w), E, _p(gate_up), _p(down), _p(xg), _p(y), _p(z),
+                                                   _p(ints), _p(row_w), _p(h), n, top, width, ff, act, float(weight), 1 if weight_in else 0,
+                                                   1 if identity else 0, self._stream()), 4)
 
     def dense_ff(self, x, w_up, w_down, h, act: int) -> None:
         """``h += w_down . act(w_up . x)`` from one call: the up product, the activation, the down product with the sum

@@ -2,14 +2,12 @@
 
     out_t = (1 / top) * sum_k  down_e (act(gate_e x_t) * up_e x_t),   e = table[token_t, k]
 
-There is no learned router: which experts a token uses depends on its id alone, so the host knows a step's
-grouping wherever it holds the step's token ids.  Steps of many tokens use that: rows are gathered in the order of
-their experts, every expert with rows runs the gated feed-forward's two matrix products on its slice, and the
-outputs are added back in the order of a token's choices.  Steps of few tokens (and steps whose tokens exist on the
-device only: captured single-token steps) look the experts up on the device, and every (token, choice) streams its
-expert's matrices; from a few pairs per expert on, such a step instead runs every expert over all its tokens with the
-library's matrix products and lets each token pick its own experts' outputs.  All add into the 32-bit stream; they
-differ in the order of their sums, not in what is summed.
+There is no learned router: which experts a token uses depends on its id alone.  Steps of few tokens look the experts up on
+the device, and every (token, choice) streams its expert's matrices.  From some pairs per expert on the rows are gathered in
+the order of their experts, every expert with rows runs the gated feed-forward's two products on its rows, and the outputs
+are added back in the order of a token's choices: in bfloat16 all of it on the device, one product over all experts each
+way; in 32-bit grouped on the host, where it holds the step's token ids.  All add into the 32-bit stream; they differ in
+the order of their sums, not in what is summed.
 """
 
 from __future__ import annotations
@@ -21,19 +19,19 @@ from ..weights.loader import TensorDecl
 from .base import FEED_FORWARDS, FeedForward
 from .mlp import ACTIVATIONS
 
-# steps with at least this many (token, choice) pairs group their rows by expert (where the host has the tokens)
+# steps outside a captured graph with at least this many (token, choice) pairs group their rows by expert (in 32-bit, where
+# the grouping is the host's, only if the host has the tokens)
 GROUP_FROM = 256
-# steps that cannot group (their token ids, or choices, are on the device only) with at least this many (token, choice)
-# pairs per expert run every expert over all tokens with the library's matrix products.  A pair that streams its expert pays
-# for the bytes, an expert's two products for their launches: experts of 5 MB break even at about 13 pairs each (16 of
-# them, 128 pairs: 99 us against 161 us; 256 pairs: 185 us against 169 us), experts of 75 MB at about 2
-# inside a captured step (8 sequences, 36 layers: 19.7 ms against 19.0 ms a step).
+# (token, choice) pairs per expert from which a captured bfloat16 step groups its rows as well.  By time alone the line would lie at 2
+# (experts of 5 MB, us pair by pair / grouped: 1 pair per expert 19 / 22, 2 31 / 28, 4 52 / 28, 8 96 / 28; experts of 75 MB: 0.3
+# pairs 75 / 86, 0.6 127 / 124, 2.3 366 / 201), but the kernels that run pair by pair keep an expert's activations in 32-bit and
+# the products round them to bfloat16: steps that had the former keep it.
 DENSE_FROM = 12
 LARGE_EXPERT, DENSE_FROM_LARGE = 16 << 20, 2
 
 
 def dense_from(spec, dtype) -> float:
-    """(token, choice) pairs from which a step that cannot group runs every expert over all its tokens."""
+    """(token, choice) pairs from which a captured bfloat16 step groups them by expert."""
     size = 3 * spec.hidden * spec.intermediate * torch.empty((), dtype=dtype).element_size()
     return (DENSE_FROM_LARGE if size >= LARGE_EXPERT else DENSE_FROM) * spec.n_experts
 
@@ -88,13 +86,14 @@ class TableExperts(FeedForward):
         n = x.shape[0]
         h = residual if residual is not None else torch.zeros((n, s.hidden), dtype=torch.float32, device=x.device)
         toks = getattr(ctx, "host_tokens", None)
-        if toks is not None and self.can_group and n * s.top >= GROUP_FROM:
+        grouped = n * s.top >= GROUP_FROM and toks is not None
+        if self.fused and (grouped or n * s.top >= self.dense_from):
+            K.experts_by_expert(x, ctx.tokens, self.table, self.gate_up, self.down, h, self.act, 1.0 / s.top)
+        elif grouped and not self.fused and self.can_group:
             ids = ctx.memo.get("host_token_array")           # the step's token ids as one array, made once a step
             if ids is None:
                 ids = ctx.memo["host_token_array"] = np.concatenate([np.asarray(t, dtype=np.int64) for t in toks])
             self._grouped(x, ids, h)
-        elif self.fused and n * s.top >= self.dense_from:
-            K.experts_dense(x, ctx.tokens, self.table, self.gate_up, self.down, h, self.act, 1.0 / s.top)
         else:
             K.experts_few(x, ctx.tokens, self.table, self.gate_up, self.row_stride, self.up_off, self.down, h, self.act, 1.0 / s.top)
         return None if residual is not None else h.unsqueeze(0)
@@ -109,10 +108,6 @@ class TableExperts(FeedForward):
         place = np.empty(n * top, dtype=np.int32)
         place[order] = np.arange(n * top, dtype=np.int32)                  # (token, k) -> grouped row
         both = torch.from_numpy(np.concatenate([(order // top).astype(np.int32), place])).to(x.device, non_blocking=True)
-        if self.fused:                      # gather, every expert's two products and the sum back: one call into the library
-            K.experts_grouped_step(x, both[:n * top], both[n * top:].view(n, top), np.ascontiguousarray(counts, dtype=np.int32),
-                                   self.gate_up, self.down, h, self.act, 1.0 / top)
-            return
         xg = K.rows_gather(x, both[:n * top])
         z = torch.empty((n * top, s.hidden), dtype=torch.float32, device=x.device)
         at = 0
@@ -120,7 +115,7 @@ class TableExperts(FeedForward):
             c = int(counts[e])
             if not c:
                 continue
-            y = K.gated_act(K.gemm_store(xg[at:at + c], self.gate_up[e]), self.act)      # (no fused epilogue here: 32-bit)
+            y = K.gated_act(K.gemm_store(xg[at:at + c], self.gate_up[e]), self.act)
             K.gemm_store(y, self.down[e], out=z[at:at + c])
             at += c
         K.experts_combine(z, both[n * top:].view(n, top), h, 1.0 / top)
@@ -137,8 +132,8 @@ class RoutedExperts(FeedForward):
     everything behind it (softmax, groups, choice, weights) is 32-bit and runs on the device, one warp per token, so a
     captured single-token step needs nothing from the host.  The experts then run the way table-routed experts do, on
     the same kernels: a step's row numbers take the place of token ids and the step's choices the place of the table;
-    every (token, choice) pair carries its weight.  Steps of many tokens, outside a captured graph, read the choices
-    back and group the rows by expert for one matrix product per expert.  The sum goes into the stream, or is returned as
+    every (token, choice) pair carries its weight.  (In 32-bit, steps of many tokens outside a captured graph read the choices
+    back to group the rows.)  The sum goes into the stream, or is returned as
     a delta where a norm sits behind the feed-forward.
 
     Options: ``s = sigmoid(z)`` instead of the softmax, no correction, weights left as they are (not over their sum), and
@@ -241,11 +236,13 @@ class RoutedExperts(FeedForward):
             h = torch.zeros((n, s.hidden), dtype=torch.float32, device=x.device)
         if s.n_experts:
             rows = self._row_numbers(n, x.device)
-            in_eager_step = getattr(ctx, "host_tokens", None) is not None
-            if in_eager_step and self.can_group and n * s.top >= GROUP_FROM:
+            grouped = n * s.top >= GROUP_FROM and getattr(ctx, "host_tokens", None) is not None
+            if self.fused and (grouped or n * s.top >= self.dense_from):
+                K.experts_by_expert(x, rows, chosen, self.gate_up, self.down, h, self.act, 1.0, pair_w=weight, weight_in=self.weight_in,
+                                    identity=s.n_identity > 0)
+                return None if residual is not None else h.unsqueeze(0)
+            if grouped and not self.fused and self.can_group:
                 self._grouped(x, chosen, weight, h)
-            elif self.fused and n * s.top >= self.dense_from:
-                K.experts_dense(x, rows, chosen, self.gate_up, self.down, h, self.act, 1.0, pair_w=weight, weight_in=self.weight_in)
             else:
                 K.experts_few(x, rows, chosen, self.gate_up, self.row_stride, self.up_off, self.down, h, self.act, 1.0,
                               pair_w=weight, weight_in=self.weight_in)
@@ -265,10 +262,6 @@ class RoutedExperts(FeedForward):
         place[order[:n_rows]] = np.arange(n_rows, dtype=np.int32)           # (token, k) -> grouped row, or -1
         both = torch.from_numpy(np.concatenate([(order // top).astype(np.int32), place])).to(x.device, non_blocking=True)
         src, place_d = both[:n * top], both[n * top:].view(n, top)
-        if self.fused:
-            K.experts_grouped_step(x, src, place_d, np.ascontiguousarray(counts, dtype=np.int32), self.gate_up, self.down, h,
-                                   self.act, 1.0, pair_w=weight, weight_in=self.weight_in)
-            return
         row_w = K.rows_weight(weight, place_d) if self.weight_in else None
         xg = K.rows_gather(x, src)
         z = torch.empty((n * top, s.hidden), dtype=torch.float32, device=x.device)

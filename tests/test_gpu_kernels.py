@@ -793,3 +793,84 @@ def test_a_bounded_wait_that_runs_out_reports_and_the_kernel_ends_normally(kerne
     assert helpers.rel_err(K.gemm_store(x, w), x.double().cpu() @ w.double().cpu().T) < 2e-5
     with pytest.raises(Exception, match="limit"):
         K.wait_probe(0)
+
+
+# Mean rows per expert on either side of the tiles' sizes (32, 64, 256 rows), tiles with one row, experts without rows, one that has
+# all, pairs that name no expert, inner sizes that are no whole k-blocks, feature counts that are no whole tiles, more experts than
+# a block keeps the offsets of
+@pytest.mark.parametrize("n,E,top,width,ff,spread", [
+    (1, 16, 4, 1024, 768, "even"), (33, 8, 2, 72, 40, "even"), (64, 16, 4, 256, 264, "one"), (97, 6, 4, 136, 200, "holes"),
+    (300, 3, 2, 128, 128, "even"), (700, 5, 3, 192, 72, "holes"), (515, 2, 1, 64, 320, "one"), (200, 450, 3, 64, 64, "even")])
+@pytest.mark.parametrize("weight_in", [False, True])
+def test_experts_grouped_on_the_device(kernels, n, E, top, width, ff, spread, weight_in):
+    K = kernels("bfloat16")
+    x = _randn(n, width, seed=80).bfloat16().cuda()
+    gate, up = ((_randn(E, ff, width, seed=81 + i) * width ** -0.5).bfloat16().cuda() for i in range(2))
+    down = (_randn(E, width, ff, seed=83) * ff ** -0.5).bfloat16().cuda()
+    gate_up = torch.stack([K.tile_gate_up(g, u) for g, u in zip(gate, up)]).contiguous()
+    g = torch.Generator().manual_seed(84)
+    table = torch.rand(n, max(E, top), generator=g).argsort(dim=1)[:, :top].to(torch.int32)
+    if spread == "one":
+        table = torch.where(table == 0, table, torch.full_like(table, E - 1))
+    if spread == "holes":
+        table[torch.rand(n, top, generator=g) < 0.3] = -1
+        table[torch.rand(n, top, generator=g) < 0.2] = E + 1           # hand the input on
+        table[table == 1] = 0                                          # (nobody names expert 1)
+    table, pw = table.cuda(), torch.rand(n, top, generator=g).cuda()
+    h0 = _randn(n, width, seed=85).float().cuda()
+    rows = torch.arange(n, dtype=torch.int32, device="cuda")
+    want = h0.double()
+    for e in range(E):
+        t, k = (table == e).nonzero(as_tuple=True)
+        if not len(t):
+            continue
+        w = pw[t, k].double()[:, None]
+        a, b = x[t].double() @ gate[e].double().T, x[t].double() @ up[e].double().T
+        if weight_in:
+            a, b, w = a * w, b * w, torch.ones_like(w)
+        want.index_put_((t,), w * ((a * torch.sigmoid(a) * b) @ down[e].double().T), accumulate=True)
+    same = (pw.double() * (table >= E)).sum(dim=1, keepdim=True) * x.double()
+    identity = spread == "holes" and not weight_in
+    out = []
+    for _ in range(2):
+        h = h0.clone()
+        K.experts_by_expert(x, rows, table, gate_up, down, h, 0, 1.0, pair_w=pw, weight_in=weight_in, identity=identity)
+        out.append(h)
+    assert K.gemm_status() == 0, "a bounded wait inside the kernel ran out"
+    assert torch.equal(out[0], out[1])
+    # the activations are rounded to bfloat16 between the two products
+    assert helpers.rel_err(out[0], want + same if identity else want) < KTOL["bfloat16"]
+    if n > 40:                                                         # a token's result does not depend on the step's other tokens
+        h = h0[7:27].clone()
+        K.experts_by_expert(x[7:27].contiguous(), rows[:20], table[7:27].contiguous(), gate_up, down, h, 0, 1.0,
+                            pair_w=pw[7:27].contiguous(), weight_in=weight_in, identity=identity)
+        assert torch.equal(h, out[0][7:27])
+
+
+# both kernels of the router: up to 32 experts a lane each, more in shared memory; the second's choices by padding the first's logits
+@pytest.mark.parametrize("E,groups,keep,top,group_top", [(1, 1, 1, 1, 1), (16, 4, 2, 4, 2), (32, 1, 1, 8, 1), (30, 5, 3, 6, 3), (12, 12, 7, 7, 1)])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_route_by_lanes_is_route(kernels, E, groups, keep, top, group_top, sigmoid):
+    K = kernels("float32")
+    z = _randn(203, E, seed=95).float()
+    z[:40] = z[:40].round()                                            # ties: the lower index wins
+    corr = _randn(E, seed=96).float().cuda() * 0.3
+    per, pad = E // groups, 33 // (E // groups) + 1
+    # more groups of the same size that nobody chooses: their logits and corrections lie far below
+    wide = torch.cat([z, torch.full((203, per * pad), -60.0)], dim=1).cuda()
+    corr_wide = torch.cat([corr, torch.full((per * pad,), -60.0, device="cuda")])
+    a = K.route(z.cuda(), corr, top, groups, keep, 1.7, sigmoid=sigmoid, group_top=group_top)
+    b = K.route(wide, corr_wide, top, groups + pad, keep, 1.7, sigmoid=sigmoid, group_top=group_top)
+    if groups > 1:
+        assert torch.equal(a[0], b[0])
+        assert helpers.rel_err(a[1], b[1]) < 1e-6                      # (the softmax's sum runs over the padding's 1e-26 too)
+    s = torch.sigmoid(z.double()) if sigmoid else torch.softmax(z.double(), dim=1)
+    s = s.cuda()
+    picked = s.gather(1, a[0].long())
+    assert helpers.rel_err(a[1], picked / picked.sum(dim=1, keepdim=True) * 1.7) < 1e-5
+    c = (s + corr.double()).view(203, groups, per)
+    score = c.topk(min(group_top, per), dim=2).values.sum(dim=2)
+    kept = score.topk(keep, dim=1).values[:, -1:]
+    open_ = torch.where((score >= kept - 1e-6)[:, :, None], c, torch.full_like(c, -9.0)).flatten(1)
+    # the choice is the top of what is open, up to sums that differ in 32 bits
+    assert (open_.gather(1, a[0].long()).sum(dim=1) > open_.topk(top, dim=1).values.sum(dim=1) - 1e-5).all()
