@@ -1,0 +1,398 @@
+// Linear recurrences over long portions, as products of tiles.  Per head, with a state S [dk, dv],
+//
+//   S_t = f_t S_(t-1) + a_t k_t v_t^T,      o_t = S_t^T q_t
+//
+// (f_t, a_t numbers; q and k shared by the heads of a group).  A portion is cut into chunks of CP_C tokens that run side by
+// side.  Over a chunk that starts from S_in, with n tokens counted from 0 and F(t, s) = f_(s+1) ... f_t,
+//
+//   o_t   = F(t, -1) S_in^T q_t + sum_(s<=t) F(t, s) a_s (k_s . q_t) v_s
+//   S_out = F(n-1, -1) S_in + sum_s F(n-1, s) a_s k_s v_s^T
+//
+// so the work is what a chunk adds to the state (chunk_state_kernel), the chunks' states one after another
+// (chunk_carry_kernel: S_in of every chunk, from and to the sequence's state), and the read-outs (chunk_out_kernel).  The
+// sums are those of the token by token walk in another order; everything is 32-bit multiply-adds, which is what bounds it.
+//
+// A thread block has (chunk, group) and some of the group's panels: a panel is 64 columns of one head's values.  What a
+// panel does not depend on is done once for all of them: the keys' tile, the queries' tile and the pair scores k_s . q_t
+// (a thread keeps its 4 x 4 of them in registers, and lays them down weighed for each head).  A panel's slices of the
+// state and its values come by asynchronous copies, one slice ahead.
+//
+// A recurrence brings its numbers as a policy W (a kernel argument):
+//   struct W::Head                               what a head's numbers over a chunk take in shared memory
+//   prepare(Head&, head, t0, n)                  made by the whole block (it may synchronise; the caller synchronises behind it)
+//   state(Head&, t) = F(t, -1);  pair(Head&, t, s) = F(t, s) a_s;  end(Head&, n, s) = F(n-1, s) a_s
+//   store_end(Head&, chunk, head, n), end_factor(chunk, head, n)     F(n-1, -1), stored by chunk_state_kernel, read by the carry
+//   finish(t, head, j, o, v)                     what goes out for column j of a head's read-out o, given the token's v
+#pragma once
+#include "common.cuh"
+
+#define CP_C 64                 // tokens of a chunk
+#define CP_LD 68                // row stride of a tile of 64 columns in shared memory (16-byte rows, banks spread)
+#define CP_TILE (64 * CP_LD)
+#define CP_THREADS 256          // of the state's kernel
+#define CP_OUT_THREADS 128      // of the read-outs': 8 tokens x 4 columns a thread (4 x 4 read shared memory nearly as long as they multiply)
+
+struct ChunkArgs {
+    const float* q; const float* k; const float* v;          // rows of packed tokens: q + t * q_stride + group * dk, v + t * v_stride + head * dv
+    int q_stride, k_stride, v_stride;
+    float* o; int o_stride;                                  // o[t, head * dv + j]
+    float* state; long long state_stride;                    // state + slot * stride : [heads][dk][dv]
+    const int* slots;
+    const int* chunk_t0; const int* seq_chunk0;              // the chunks' first packed tokens [n_chunks + 1], each sequence's first chunk
+    float* chunk_state;                                      // [n_chunks][heads][dk][dv]
+    int groups, heads, dk, dv;
+    int panels;                                              // of a block
+    int vec;                                                 // tiles may be read and written in 16-byte pieces
+};
+
+// a tile of 64 rows of `width` (a multiple of 64) floats into shared memory: rows r < n_rows at src + r * ld, columns c < n_cols;
+// zeros elsewhere.  16-byte copies are asynchronous.
+template <int THREADS>
+__device__ __forceinline__ void cp_tile(float* dst, int dst_ld, int width, const float* __restrict__ src, size_t ld, int n_rows, int n_cols, int vec) {
+    if (vec) {
+        const int per = width / 4;
+        for (int e = threadIdx.x; e < 64 * per; e += THREADS) {
+            const int r = e / per, c = (e - r * per) * 4;
+            float* to = dst + r * dst_ld + c;
+            if (r < n_rows && c < n_cols)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(src + (size_t)r * ld + c) : "memory");
+            else *reinterpret_cast<float4*>(to) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    } else {
+        for (int e = threadIdx.x; e < 64 * width; e += THREADS) {
+            const int r = e / width, c = e - r * width;
+            dst[r * dst_ld + c] = (r < n_rows && c < n_cols) ? src[(size_t)r * ld + c] : 0.f;
+        }
+    }
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
+
+// panel p of a group: its head and first column
+__device__ __forceinline__ void panel_place(const ChunkArgs& a, int group, int p, int& head, int& j0) {
+    const int across = (a.dv + 63) / 64;
+    head = group * (a.heads / a.groups) + p / across;
+    j0 = p % across * 64;
+}
+__device__ __forceinline__ int panel_count(const ChunkArgs& a) { return a.heads / a.groups * ((a.dv + 63) / 64); }
+
+__device__ __forceinline__ void store_row4(float* p, const float* x, int left, int vec) {
+    if (vec && left >= 4) { *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]); return; }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k < left) p[k] = x[k];
+}
+
+// chunk_state[c, head, d, j] = sum_s end(s) k_s[d] v_s[j]: 128 dims at a time, 8 x 4 of them a thread
+static int chunk_state_smem() { return (64 * (128 + 4) + 2 * CP_TILE) * (int)sizeof(float); }
+template <typename W>
+__global__ void __launch_bounds__(CP_THREADS) chunk_state_kernel(ChunkArgs a, W w) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    __shared__ typename W::Head hd;
+    __shared__ float weight[CP_C];
+    constexpr int LDK = 128 + 4;
+    float* sk = sm;                                          // [tokens][128 dims]
+    float* sv2 = sk + 64 * LDK;                              // [tokens][columns] of this panel and the next
+    const int c = blockIdx.x, g = blockIdx.y, t0 = a.chunk_t0[c], n = a.chunk_t0[c + 1] - t0;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int p0 = blockIdx.z * a.panels, p1 = min(p0 + a.panels, panel_count(a));
+    for (int d0 = 0; d0 < a.dk; d0 += 128) {
+        __syncthreads();
+        cp_tile<CP_THREADS>(sk, LDK, 128, a.k + (size_t)t0 * a.k_stride + g * a.dk + d0, a.k_stride, n, a.dk - d0, a.vec);
+        auto copy_values = [&](int p) {
+            int head, j0;
+            panel_place(a, g, p, head, j0);
+            cp_tile<CP_THREADS>(sv2 + (p & 1) * CP_TILE, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
+            cp_commit();
+        };
+        copy_values(p0);
+        int last = -1;
+        for (int p = p0; p < p1; ++p) {
+            int head, j0;
+            panel_place(a, g, p, head, j0);
+            const float* sv = sv2 + (p & 1) * CP_TILE;
+            if (p + 1 < p1) copy_values(p + 1); else cp_commit();
+            if (head != last) {
+                w.prepare(hd, head, t0, n);
+                __syncthreads();
+                if (threadIdx.x < CP_C) weight[threadIdx.x] = threadIdx.x < n ? w.end(hd, n, threadIdx.x) : 0.f;
+                if (threadIdx.x == 0 && d0 == 0) w.store_end(hd, c, head, n);
+                last = head;
+            }
+            cp_wait<1>();
+            __syncthreads();
+            const bool two = a.dk - d0 > 64;                 // (a second tile of 64 dims)
+            float acc[2][4][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) acc[m][i][k] = 0.f;
+#pragma unroll 4
+            for (int t = 0; t < n; ++t) {
+                const float4 v4 = *reinterpret_cast<const float4*>(sv + t * CP_LD + tx * 4);
+                const float f = weight[t];
+                const float vx[4] = {v4.x * f, v4.y * f, v4.z * f, v4.w * f};
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    if (m == 1 && !two) break;
+                    const float4 k4 = *reinterpret_cast<const float4*>(sk + t * LDK + m * 64 + ty * 4);
+                    const float kx[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[m][i][k] = fmaf(kx[i], vx[k], acc[m][i][k]);
+                }
+            }
+            float* dst = a.chunk_state + ((size_t)c * a.heads + head) * a.dk * a.dv + j0 + tx * 4;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int d = d0 + 64 * m + ty * 4 + i;
+                    if (d < a.dk) store_row4(dst + (size_t)d * a.dv, acc[m][i], a.dv - j0 - tx * 4, a.vec);
+                }
+            __syncthreads();                                 // everyone is through with the values
+        }
+    }
+}
+
+// chunk after chunk: what a chunk starts from takes the place of what it adds, and the state moves on.  A thread has V
+// elements side by side; the chunks of a batch are on their way together, only the sums are a chain.
+#define CP_BATCH 8
+template <int V, typename W>
+__global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs a, W w) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int s = blockIdx.z, h = blockIdx.y;
+    const size_t per = (size_t)a.dk * a.dv, e = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= per) return;                                    // (V == 4: dv is a multiple of 4)
+    const int c0 = a.seq_chunk0[s], c1 = a.seq_chunk0[s + 1];
+    float* st = a.state + (size_t)a.slots[s] * a.state_stride + (size_t)h * per + e;
+    float* cs = a.chunk_state + ((size_t)c0 * a.heads + h) * per + e;
+    const size_t step = (size_t)a.heads * per;
+    float S[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) S[i] = st[i];
+    for (int b = c0; b < c1; b += CP_BATCH, cs += CP_BATCH * step) {
+        float add[CP_BATCH][V], f[CP_BATCH];
+#pragma unroll
+        for (int u = 0; u < CP_BATCH; ++u)
+            if (b + u < c1) {
+                if constexpr (V == 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(cs + u * step);
+                    add[u][0] = x.x; add[u][1] = x.y; add[u][2] = x.z; add[u][3] = x.w;
+                } else add[u][0] = cs[u * step];
+                f[u] = w.end_factor(b + u, h, a.chunk_t0[b + u + 1] - a.chunk_t0[b + u]);
+            }
+#pragma unroll
+        for (int u = 0; u < CP_BATCH; ++u)
+            if (b + u < c1) {
+                if constexpr (V == 4) *reinterpret_cast<float4*>(cs + u * step) = make_float4(S[0], S[1], S[2], S[3]);
+                else cs[u * step] = S[0];
+#pragma unroll
+                for (int i = 0; i < V; ++i) S[i] = fmaf(f[u], S[i], add[u][i]);
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) st[i] = S[i];
+}
+
+// four tokens' weighed scores times their values for eight rows; FROM: of the four, row i sees those at or below i - FROM (8: all)
+template <int FROM>
+__device__ __forceinline__ void add_values(float (&out)[8][4], const float* pr, const float* vc) {
+    float4 p4[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * CP_LD);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float4 v4 = *reinterpret_cast<const float4*>(vc + e * CP_LD);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (FROM < 8 && i < e + FROM) continue;
+            const float x = e == 0 ? p4[i].x : e == 1 ? p4[i].y : e == 2 ? p4[i].z : p4[i].w;
+            out[i][0] = fmaf(x, v4.x, out[i][0]); out[i][1] = fmaf(x, v4.y, out[i][1]);
+            out[i][2] = fmaf(x, v4.z, out[i][2]); out[i][3] = fmaf(x, v4.w, out[i][3]);
+        }
+    }
+}
+
+// read-outs: pair scores once, then panel after panel: q S_in over the dims (slices of 64), times state(t), plus the masked
+// and weighed scores times v.  A thread has 8 tokens x 4 columns.
+__host__ __device__ __forceinline__ int cp_q_ld(int dk) { return (dk + 63) / 64 * 64 + 4; }
+static int chunk_out_smem(int dk) { return (64 * cp_q_ld(dk) + 4 * CP_TILE) * (int)sizeof(float); }
+template <typename W>
+__global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, W w) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    __shared__ typename W::Head hd;
+    const int ldq = cp_q_ld(a.dk), slices = (a.dk + 63) / 64;
+    float* sq = sm;                                          // [tokens][dims]
+    float* ss = sq + 64 * ldq;                               // two slices of the state [64 dims][columns]; the keys' tiles before that
+    float* sv = ss + 2 * CP_TILE;                            // [tokens][columns]
+    float* sp = sv + CP_TILE;                                // [t][s]: the head's weighed scores
+    const int c = blockIdx.x, g = blockIdx.y, t0 = a.chunk_t0[c], n = a.chunk_t0[c + 1] - t0;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;  // tokens 8 ty .., columns 4 tx ..
+    const int p0 = blockIdx.z * a.panels, p1 = min(p0 + a.panels, panel_count(a));
+    const int nk = (8 * (ty | 1) + 7) / 16 + 1;              // groups of 16 tokens that a warp's rows (two ty) may see
+    const float* kbase = a.k + (size_t)t0 * a.k_stride + g * a.dk;
+
+    // pair[i][k]: tokens t = 8 ty + i, s = tx + 16 k
+    float pair[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) pair[i][k] = 0.f;
+    cp_tile<CP_OUT_THREADS>(sq, ldq, ldq - 4, a.q + (size_t)t0 * a.q_stride + g * a.dk, a.q_stride, n, a.dk, a.vec);
+    cp_tile<CP_OUT_THREADS>(ss, CP_LD, 64, kbase, a.k_stride, n, a.dk, a.vec);
+    cp_commit();
+    for (int i = 0; i < slices; ++i) {
+        if (i + 1 < slices)
+            cp_tile<CP_OUT_THREADS>(ss + ((i + 1) & 1) * CP_TILE, CP_LD, 64, kbase + (i + 1) * 64, a.k_stride, n, a.dk - (i + 1) * 64, a.vec);
+        cp_commit();
+        cp_wait<1>();
+        __syncthreads();
+        const float* sk = ss + (i & 1) * CP_TILE;
+#pragma unroll 2
+        for (int d = 0; d < 64; d += 4) {
+            float4 q4[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) q4[u] = *reinterpret_cast<const float4*>(sq + (8 * ty + u) * ldq + i * 64 + d);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k >= nk) break;                          // (a warp's rows all lie before these tokens)
+                const float4 k4 = *reinterpret_cast<const float4*>(sk + (tx + 16 * k) * CP_LD + d);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    pair[u][k] = fmaf(q4[u].x, k4.x, pair[u][k]); pair[u][k] = fmaf(q4[u].y, k4.y, pair[u][k]);
+                    pair[u][k] = fmaf(q4[u].z, k4.z, pair[u][k]); pair[u][k] = fmaf(q4[u].w, k4.w, pair[u][k]);
+                }
+            }
+        }
+        __syncthreads();                                     // the tile's place is free
+    }
+
+    // the steps of the panels, slice after slice; a panel's values come with its first slice
+    auto copy_slice = [&](int step) {
+        int head, j0;
+        const int p = p0 + step / slices, i = step % slices;
+        panel_place(a, g, p, head, j0);
+        cp_tile<CP_OUT_THREADS>(ss + (step & 1) * CP_TILE, CP_LD, 64, a.chunk_state + (((size_t)c * a.heads + head) * a.dk + i * 64) * a.dv + j0, a.dv,
+                                a.dk - i * 64, a.dv - j0, a.vec);
+    };
+    auto copy_values = [&](int p) {
+        int head, j0;
+        panel_place(a, g, p, head, j0);
+        cp_tile<CP_OUT_THREADS>(sv, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
+    };
+    const int steps = (p1 - p0) * slices;
+    copy_slice(0);
+    copy_values(p0);
+    cp_commit();
+    int last = -1;
+    for (int p = p0, step = 0; p < p1; ++p) {
+        int head, j0;
+        panel_place(a, g, p, head, j0);
+        if (head != last) {
+            w.prepare(hd, head, t0, n);
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int t = 8 * ty + i, s = tx + 16 * k;
+                    sp[t * CP_LD + s] = s <= t && t < n ? pair[i][k] * w.pair(hd, t, s) : 0.f;
+                }
+            last = head;
+        }
+        float out[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) out[i][k] = 0.f;
+        for (int i = 0; i < slices; ++i, ++step) {
+            if (step + 1 < steps) copy_slice(step + 1);
+            cp_commit();
+            cp_wait<1>();
+            __syncthreads();
+            const float* st = ss + (step & 1) * CP_TILE + 4 * tx;
+            const float* qr = sq + 8 * ty * ldq + i * 64;
+#pragma unroll 2
+            for (int d = 0; d < 64; d += 4) {
+                float4 q4[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) q4[u] = *reinterpret_cast<const float4*>(qr + u * ldq + d);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float4 s4 = *reinterpret_cast<const float4*>(st + (d + e) * CP_LD);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const float q = e == 0 ? q4[u].x : e == 1 ? q4[u].y : e == 2 ? q4[u].z : q4[u].w;
+                        out[u][0] = fmaf(q, s4.x, out[u][0]); out[u][1] = fmaf(q, s4.y, out[u][1]);
+                        out[u][2] = fmaf(q, s4.z, out[u][2]); out[u][3] = fmaf(q, s4.w, out[u][3]);
+                    }
+                }
+            }
+            __syncthreads();                                 // the slice's place is free
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float f = 8 * ty + i < n ? w.state(hd, 8 * ty + i) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) out[i][k] *= f;
+        }
+        const float* pr = sp + 8 * ty * CP_LD;
+        const float* vc = sv + 4 * tx;
+#pragma unroll 2
+        for (int s = 0; s < 8 * ty; s += 4) add_values<8>(out, pr + s, vc + s * CP_LD);
+        add_values<0>(out, pr + 8 * ty, vc + 8 * ty * CP_LD);      // (the tokens behind a row's own are not touched, whatever they hold)
+        add_values<4>(out, pr + 8 * ty + 4, vc + (8 * ty + 4) * CP_LD);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = 8 * ty + i, left = a.dv - j0 - 4 * tx;
+            if (t >= n || left <= 0) continue;
+            const float4 v4 = *reinterpret_cast<const float4*>(sv + t * CP_LD + 4 * tx);
+            const float vx[4] = {v4.x, v4.y, v4.z, v4.w};
+            w.finish(t0 + t, head, j0 + 4 * tx, out[i], vx, min(left, 4), a.vec);
+            store_row4(a.o + (size_t)(t0 + t) * a.o_stride + head * a.dv + j0 + 4 * tx, out[i], left, a.vec);
+        }
+        __syncthreads();                                     // everyone is through with the values and the scores
+        if (p + 1 < p1) copy_values(p + 1);                  // (its slice is on its way already: both are waited for together)
+        cp_commit();
+    }
+}
+
+// How many of a group's panels a block takes: all that still leaves two blocks an SM (the pair scores and the keys are then read once for
+// them), at least one
+static int chunk_panels(int n_chunks, int groups, int panels) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int z = (int)((2ll * sms + (long long)n_chunks * groups - 1) / ((long long)n_chunks * groups));
+    if (z > panels) z = panels;
+    if (z < 1) z = 1;
+    return (panels + z - 1) / z;
+}
+
+template <typename W>
+static int chunk_products(ChunkArgs a, const W& w, int n_chunks, int n_seqs, const char* what, cudaStream_t stream) {
+    const int panels = a.heads / a.groups * ((a.dv + 63) / 64), out_smem = chunk_out_smem(a.dk);
+    IDM_REQUIRE(n_chunks > 0 && a.heads % a.groups == 0 && a.dk <= 256 && a.groups <= 65535 && n_seqs <= 65535, "%s: %d chunks, %d heads in %d groups, keys of %d",
+                what, n_chunks, a.heads, a.groups, a.dk);
+    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_state_smem());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem);
+    IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused (%s)", what, out_smem, cudaGetErrorString(e));
+    a.panels = chunk_panels(n_chunks, a.groups, panels);
+    const dim3 grid(n_chunks, a.groups, (panels + a.panels - 1) / a.panels);
+    idm_launch(chunk_state_kernel<W>, grid, dim3(CP_THREADS), chunk_state_smem(), stream, a, w);
+    const size_t per = (size_t)a.dk * a.dv;
+    if (a.vec) idm_launch(chunk_carry_kernel<4, W>, dim3((unsigned)((per / 4 + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);
+    else idm_launch(chunk_carry_kernel<1, W>, dim3((unsigned)((per + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);
+    idm_launch(chunk_out_kernel<W>, grid, dim3(CP_OUT_THREADS), out_smem, stream, a, w);
+    IDM_LAUNCH_CHECK(what);
+    return 0;
+}

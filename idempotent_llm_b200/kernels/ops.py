@@ -352,12 +352,14 @@ class Kernels:
                                                    self._state_stride(state), _p(ctx.slots), _p(ctx.q_start),
                                                    _p(ctx.cu_q), _p(ctx.kv_len), ctx.n_seqs, self._stream()))
 
+    # portions of up to so many tokens are walked token by token (the same bits however they are cut), longer ones run in chunks
+    SSD_WALK = 128
+
     def ssd_chunks(self, ctx):
         """How a step's long portions are cut for the state-space recurrence: (chunk borders in packed tokens
         [n_chunks + 1], each sequence's first chunk [n_seqs + 1], n_chunks), on the device, made once a step; None
-        when no sequence brings more than a chunk's tokens (then every sequence runs token by token from its state)."""
-        L = self.lib.idm_ssd_chunk_tokens()
-        return None if ctx.single_token or ctx.max_q_len <= L else self._chunks(ctx, L)
+        when no sequence brings more than ``SSD_WALK`` tokens (then every sequence runs token by token from its state)."""
+        return None if ctx.single_token or ctx.max_q_len <= self.SSD_WALK else self._chunks(ctx, self.lib.idm_ssd_chunk_tokens())
 
     def _chunks(self, ctx, L: int):
         """Portions cut into chunks of ``L`` tokens: what ``ssd_chunks`` returns."""
@@ -388,7 +390,7 @@ class Kernels:
         n_chunks = 0
         if plan is not None:
             _, chunk_t0, seq_chunk0, n_chunks = plan
-            scratch = self.scratch("ssd_scan", n_chunks * heads * N * P + n * heads)
+            scratch = self.scratch("ssd_scan", n_chunks * heads * (N * P + 1))
         self._check(self.lib.idm_ssd_scan(_p(xbc), xbc.shape[1], cols[0], cols[1], cols[2], _p(proj), proj.shape[1],
                                           z_col, dt_col, _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
                                           self._state_stride(state), _p(y), heads * P, _p(ctx.cu_q), _p(ctx.slots),
