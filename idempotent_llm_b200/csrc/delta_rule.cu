@@ -79,6 +79,52 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(DeltaPrepArgs p) {
         p.beta[(size_t)t * p.H + h] = 1.0f / (1.0f + expf(-p.proj[(size_t)t * p.p_stride + p.b_col + h]));
 }
 
+// The same with heads of up to 128 channels in pieces of four on their borders: a warp has four heads' rows on their way at a time, a
+// decay per head is made once a token and spread from shared memory.  Bound by the bytes of the decays.
+#define DP_HEADS 256
+__global__ void __launch_bounds__(128) delta_prep_vec_kernel(DeltaPrepArgs p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float decay[DP_HEADS];
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d = lane * 4;
+    float* row = p.c + (size_t)t * p.c_stride;
+    const float q_scale = 1.0f / sqrtf((float)p.dk);
+    if (p.head_col >= 0)
+        for (int h = threadIdx.x; h < p.H; h += 128)
+            decay[h] = expf(-expf(p.a_log[h]) * softplus_f(p.proj[(size_t)t * p.p_stride + p.head_col + h] + p.dt_bias[h]));
+    for (int i0 = (blockIdx.y * 4 + warp) * 4; i0 < 2 * p.Hk; i0 += gridDim.y * 16) {
+        float4 x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + j;
+            float* at = row + (i < p.Hk ? p.c_q + i * p.dk : p.c_k + (i - p.Hk) * p.dk) + d;
+            x[j] = i < 2 * p.Hk && d < p.dk ? *reinterpret_cast<const float4*>(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + j;
+            const float ss = warp_sum(fmaf(x[j].w, x[j].w, fmaf(x[j].z, x[j].z, fmaf(x[j].y, x[j].y, x[j].x * x[j].x))));
+            const float inv = (i < p.Hk ? q_scale : 1.f) / sqrtf(ss + 1e-6f);
+            float* at = row + (i < p.Hk ? p.c_q + i * p.dk : p.c_k + (i - p.Hk) * p.dk) + d;
+            if (i < 2 * p.Hk && d < p.dk) *reinterpret_cast<float4*>(at) = make_float4(x[j].x * inv, x[j].y * inv, x[j].z * inv, x[j].w * inv);
+        }
+    }
+    __syncthreads();
+    float* arow = p.a + (size_t)t * p.a_stride + p.a_col;
+    const int quads = p.dk / 4;
+    for (int i = blockIdx.y * 128 + threadIdx.x; i < p.H * quads; i += gridDim.y * 128) {
+        const int h = i / quads;
+        float4* at = reinterpret_cast<float4*>(arow) + i;
+        if (p.head_col >= 0) { const float g = decay[h]; *at = make_float4(g, g, g, g); continue; }
+        const float rate = expf(p.a_log[h]);
+        const float4 z = *at, b = *reinterpret_cast<const float4*>(p.dt_bias + 4 * i);
+        *at = make_float4(expf(-rate * softplus_f(z.x + b.x)), expf(-rate * softplus_f(z.y + b.y)),
+                          expf(-rate * softplus_f(z.z + b.z)), expf(-rate * softplus_f(z.w + b.w)));
+    }
+    for (int h = blockIdx.y * 128 + threadIdx.x; h < p.H; h += gridDim.y * 128)
+        p.beta[(size_t)t * p.H + h] = 1.0f / (1.0f + expf(-p.proj[(size_t)t * p.p_stride + p.b_col + h]));
+}
+
 extern "C" int idm_delta_prep(float* c, int c_stride, int c_q, int c_k, float* a, int a_stride, int a_col,
                               const float* proj, int p_stride, int b_col, int head_col, const float* dt_bias, const float* a_log,
                               float* beta, int H, int Hk, int dk, int n_tokens, cudaStream_t stream) {
@@ -89,7 +135,9 @@ extern "C" int idm_delta_prep(float* c, int c_stride, int c_q, int c_k, float* a
     const int most = (H * dk + 127) / 128;
     if (split > most) split = most;
     if (split < 1) split = 1;
-    idm_launch(delta_prep_kernel, dim3(n_tokens, split), dim3(128), 0, stream, p);
+    const bool vec = dk % 4 == 0 && dk <= 128 && H <= DP_HEADS && c_stride % 4 == 0 && c_q % 4 == 0 && c_k % 4 == 0 && a_stride % 4 == 0 &&
+                     a_col % 4 == 0 && (((uintptr_t)c | (uintptr_t)a) & 15) == 0 && (head_col >= 0 || ((uintptr_t)dt_bias & 15) == 0);
+    idm_launch(vec ? delta_prep_vec_kernel : delta_prep_kernel, dim3(n_tokens, split), dim3(128), 0, stream, p);
     IDM_LAUNCH_CHECK("delta_prep");
     return 0;
 }
@@ -335,7 +383,80 @@ static int delta_scan_staged(const DeltaScanArgs& a, dim3 grid, cudaStream_t str
     return 0;
 }
 
-// ------------------------------------------------------------------ the recurrence, sixteen tokens at a time
+__device__ __forceinline__ float dot4(float s, float4 a, float4 b) {
+    s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s);
+    return fmaf(a.w, b.w, s);
+}
+
+// Few tokens per sequence (single tokens above all), keys of up to 128 in whole pieces of four: bound by the bytes of the state, so a
+// thread has eight 16-byte pieces of it on their way.  L lanes have a column (4 L channels), a warp 8 of them (times 32 / L); a column's
+// two sums go over its lanes by a butterfly.  64 single tokens, 32 heads of 128 x 64 (134 MB in and out): 
+// 22 us, 6.1 TB/s (55 us by the general walk).
+#define DT_COLS 8
+template <int L>
+__global__ void __launch_bounds__(128, 5) delta_token_kernel(DeltaScanArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int SIDE = 32 / L;                                // columns side by side
+    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), lane = threadIdx.x & 31, ln = lane % L;
+    const int j0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * DT_COLS * SIDE + lane / L, d = ln * 4;
+    const bool in = d < a.dk;
+    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
+    float* sp = a.state + (size_t)a.slots[s] * a.state_stride + (size_t)h * a.dv * a.dk + d;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 S[DT_COLS];
+#pragma unroll
+    for (int i = 0; i < DT_COLS; ++i) {
+        const int j = j0 + i * SIDE;
+        S[i] = in && j < a.dv ? *reinterpret_cast<const float4*>(sp + (size_t)j * a.dk) : zero;
+    }
+    for (int t = t0; t < t1; ++t) {
+        const float* row = a.c + (size_t)t * a.c_stride;
+        const float4 k = in ? *reinterpret_cast<const float4*>(row + a.c_k + hk * a.dk + d) : zero;
+        const float4 q = in ? *reinterpret_cast<const float4*>(row + a.c_q + hk * a.dk + d) : zero;
+        const float4 g = in ? *reinterpret_cast<const float4*>(a.g + (size_t)t * a.g_stride + a.g_col + h * a.dk + d) : zero;
+        const float beta = a.beta[(size_t)t * a.H + h];
+        float v[DT_COLS], ks[DT_COLS], qs[DT_COLS], kq = dot4(0.f, k, q);
+#pragma unroll
+        for (int i = 0; i < DT_COLS; ++i) {
+            const int j = j0 + i * SIDE;
+            v[i] = j < a.dv ? row[a.c_v + h * a.dv + j] : 0.f;
+            S[i] = make_float4(g.x * S[i].x, g.y * S[i].y, g.z * S[i].z, g.w * S[i].w);
+            ks[i] = dot4(0.f, k, S[i]);
+            qs[i] = dot4(0.f, q, S[i]);
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+            kq += __shfl_xor_sync(0xffffffffu, kq, o);
+#pragma unroll
+            for (int i = 0; i < DT_COLS; ++i) {
+                ks[i] += __shfl_xor_sync(0xffffffffu, ks[i], o);
+                qs[i] += __shfl_xor_sync(0xffffffffu, qs[i], o);
+            }
+        }
+        float mine = 0.f;                                       // lane i of a column's lanes stores column i's read-out
+#pragma unroll
+        for (int i = 0; i < DT_COLS; ++i) {
+            const float u = beta * (v[i] - ks[i]);
+            S[i] = make_float4(fmaf(k.x, u, S[i].x), fmaf(k.y, u, S[i].y), fmaf(k.z, u, S[i].z), fmaf(k.w, u, S[i].w));
+            if (ln == i) mine = fmaf(u, kq, qs[i]);
+        }
+        const int j = j0 + ln * SIDE;
+        if (ln < DT_COLS && j < a.dv) a.o[(size_t)t * a.o_stride + h * a.dv + j] = mine;
+    }
+#pragma unroll
+    for (int i = 0; i < DT_COLS; ++i) {
+        const int j = j0 + i * SIDE;
+        if (in && j < a.dv) *reinterpret_cast<float4*>(sp + (size_t)j * a.dk) = S[i];
+    }
+}
+template <int L>
+static void delta_token(const DeltaScanArgs& a, int n_seqs, cudaStream_t stream) {
+    constexpr int COLS = 4 * DT_COLS * (32 / L);
+    idm_launch(delta_token_kernel<L>, dim3((a.dv + COLS - 1) / COLS, a.H, n_seqs), dim3(128), 0, stream, a);
+}
+
+// ------------------------------------------------------------------ the recurrence, thirty-two tokens at a time
 // Over a chunk of C tokens that starts from the state S0, with G_t the product of the decays up to and including
 // token t (per key channel), the walk above unrolls to
 //
@@ -343,305 +464,329 @@ static int delta_scan_staged(const DeltaScanArgs& a, dim3 grid, cudaStream_t str
 //   o_t  = S0^T (G_t q_t) + sum_{s<=t} B_ts u_s,                    B_ts = sum_d k_s[d] q_t[d] G_t[d] / G_s[d]
 //   S_C  = G_C S0 + sum_s (k_s G_C / G_s) u_s^T
 //
-// so that the work against the state becomes three products with C independent sums each instead of a chain of
-// C dependent steps, and the chain that is left (the u_t, a triangular system of C unknowns per column) is C short
-// steps in registers.  The quotients G_t / G_s are never divided out: they are products of the decays between s
-// and t, in (0, 1], so a decay that underflows ends at 0 and nothing overflows.  A and B belong to (chunk, head)
-// and not to a column: a pass of its own makes them for all chunks side by side.  All of it is 32-bit; the numbers
-// are those of the walk up to the order of the sums.
-#define DC_C 16                                                 // tokens per chunk
-
-// ab[(t H + h) 2C ..]: for token s of a chunk, -A_ts for the chunk's tokens t > s (0 elsewhere), then B_ts for t >= s
-__global__ void __launch_bounds__(128) delta_pairs_kernel(DeltaScanArgs a, float* __restrict__ ab) {
-    __shared__ float sm[3][DC_C][128];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), tid = threadIdx.x;
-    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1], tb = t0 + blockIdx.x * DC_C;
-    if (tb >= t1) return;
-    const int n = min(DC_C, t1 - tb);
-    for (int e = tid; e < n * a.dk; e += 128) {
-        const int tt = e / a.dk, d = e % a.dk;
-        const float* row = a.c + (size_t)(tb + tt) * a.c_stride + hk * a.dk + d;
-        sm[0][tt][d] = row[a.c_k];
-        sm[1][tt][d] = row[a.c_q];
-        sm[2][tt][d] = a.g[(size_t)(tb + tt) * a.g_stride + a.g_col + h * a.dk + d];
-    }
-    for (int e = tid; e < n * 2 * DC_C; e += 128)
-        ab[((size_t)(tb + e / (2 * DC_C)) * a.H + h) * (2 * DC_C) + e % (2 * DC_C)] = 0.f;
-    __syncthreads();
-    // a warp takes four tokens s whose rows together are as long as every other warp's; its lanes split the channels
-    const int warp = tid >> 5, lane = tid & 31;
-#pragma unroll 1
-    for (int pass = 0; pass < 4; ++pass) {
-        const int ts = pass == 0 ? warp : pass == 1 ? 7 - warp : pass == 2 ? 8 + warp : 15 - warp;
-        if (ts >= n) continue;
-        float kr[4];                                            // k_s times the decays from s up to the token at hand
-#pragma unroll
-        for (int i = 0; i < 4; ++i) kr[i] = lane + 32 * i < a.dk ? sm[0][ts][lane + 32 * i] : 0.f;
-        float* out = ab + ((size_t)(tb + ts) * a.H + h) * (2 * DC_C);
-        for (int t = ts; t < n; ++t) {
-            float pa = 0.f, pb = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int d = lane + 32 * i;
-                if (d < a.dk) {
-                    if (t > ts) kr[i] *= sm[2][t][d];
-                    pa = fmaf(sm[0][t][d], kr[i], pa);
-                    pb = fmaf(sm[1][t][d], kr[i], pb);
-                }
-            }
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                pa += __shfl_xor_sync(0xffffffffu, pa, o);
-                pb += __shfl_xor_sync(0xffffffffu, pb, o);
-            }
-            if (lane == 0) {
-                if (t > ts) out[t] = -pa;
-                out[DC_C + t] = pb;
-            }
-        }
-    }
-}
-
-// The chunk kernel: a block owns (sequence, head, 16 columns of S), a warp four of the columns, lane L rows
-// [L RP, (L + 1) RP) of each.  Four columns a warp, because what a warp reads from shared memory (a token's scaled k or
-// q) then serves four sums, and four independent chains keep one warp per scheduler busy.  Per chunk: (1) the threads
-// turn the staged k, q, g in place into k G_C / G_t, q G_t, k G_t, a thread per channel and group of tokens, the
-// groups' products joined through shared memory; (2) the warp lays its columns of S0 into shared memory, and lane t
-// sums S0^T (G_t k_t) for token t's correction, lane 16 + t S0^T (G_t q_t) for its read-out; (3) the triangular system
-// runs down the lanes: u_s goes from lane s to all, lane L adds row s's entry L of [-A | B] times u_s to its sum; (4)
-// lanes 16.. store the read-outs, all lanes bring their rows of S behind the chunk.
-#define DC_NC 4                                                 // columns per warp
-template <int RP>
+// The u_t are a triangular system whose right-hand sides are v_t and, row by row of S0, G_t k_t: with X the solutions for
+// those, u = X_v - X_k S0.  So everything but S0 belongs to (chunk, head) and not to a column or to what came before:
+// delta_chunk_kernel makes it for all chunks side by side (X_k, X_v, G_t q_t, k_s G_C / G_s, B, G_C), and the chain that is
+// left (delta_walk_kernel) is products with S0 and with u.  The quotients G_t / G_s are never divided out: they are products
+// of the decays between s and t, in (0, 1] (inside half a chunk multiplied up from s, across its middle the product up to
+// the middle times the product from there), so a decay that underflows ends at 0 and nothing overflows.  All of it is
+// 32-bit; the numbers are those of the walk up to the order of the sums.
+//
+// A prompt of 2 048 tokens, 32 heads of 128 x 64: 257 us the chunks (two windows), 230 the walk;
+// the walk of chunks of 16 that did it all in one chain took 408 + 75 for its pairs.
+#define DC_C 32                                                 // tokens per chunk
+#define DC_H (DC_C / 2)
+#define DC_THREADS 256
+#define DC_ROW 36                                               // a row of C numbers in shared memory and scratch
+template <int DKP>
 struct DeltaChunk {
-    static constexpr int DKP = RP * 32, NT = DS_COLS / DC_NC * 32;
-    static constexpr int NG = NT / DKP < 1 ? 1 : NT / DKP;      // groups of tokens in step (1)
-    static constexpr int V_AT = 3 * DKP, BETA_AT = V_AT + DS_COLS, AB_AT = BETA_AT + 4;
-    static constexpr int ROW = AB_AT + 2 * DC_C;                // k, q, g, v of the block's columns, beta, -A and B
-    static constexpr int GC_AT = 2 * DC_C * ROW;                // the chunk's whole decay, behind the two stages
-    static constexpr int GP_AT = GC_AT + DKP;                   // the token groups' decays
-    static constexpr int SW_AT = GP_AT + NG * DKP;              // the block's columns of S
-    static constexpr int FLOATS = SW_AT + DS_COLS * DKP;
-    static_assert(DKP <= NT && DC_C % NG == 0, "a thread per channel, whole groups of tokens");
+    static constexpr int LD = DKP + 4;                          // a row of channels: eight rows' 16-byte reads in different places
+    // a chunk's numbers in scratch, in floats: X_k, G q, k G_C / G (each [C][LD]), B [C][DC_ROW], G_C, then X_v by groups of 16 columns
+    static constexpr int TILE = DC_C * LD;
+    static constexpr int B_AT = 3 * TILE, GC_AT = B_AT + DC_C * DC_ROW, XV_AT = GC_AT + DKP;
+    static constexpr int XV = DC_C * DS_COLS;
+    static constexpr int BUF = XV_AT + XV;                      // a stage of the walk: one group of columns
+    static constexpr int CHUNK_SMEM = (3 * TILE + 2 * DC_C * DC_ROW + 2 * DKP + DC_C) * 4;
+    static constexpr int WALK_SMEM = (2 * BUF + DS_COLS * LD + DC_C * (DS_COLS + 4)) * 4;
 };
-
-template <int RP>
-__device__ __forceinline__ void load_rows(const float* p, float (&x)[RP]) {
-    if constexpr (RP == 4) { const float4 v = *reinterpret_cast<const float4*>(p); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
-    else if constexpr (RP == 2) { const float2 v = *reinterpret_cast<const float2*>(p); x[0] = v.x; x[1] = v.y; }
-    else x[0] = *p;
+__host__ __device__ __forceinline__ int delta_chunk_floats(int dkp, int dv) {
+    return 3 * DC_C * (dkp + 4) + DC_C * DC_ROW + dkp + (dv + DS_COLS - 1) / DS_COLS * DC_C * DS_COLS;
 }
 
-template <int RP, bool VEC>
-__global__ void __launch_bounds__(DeltaChunk<RP>::NT) delta_scan_chunked_kernel(DeltaScanArgs a, const float* __restrict__ ab) {
-    using L = DeltaChunk<RP>;
-    constexpr int C = DC_C, NT = L::NT, NC = DC_NC, NW = NT / 32;
+// Chunks first, first + 1, ... (gridDim.x of them) of every sequence and head; chunk c of sequence s goes to scratch + (s * gridDim.x + c -
+// first) * H + h.
+template <int DKP>
+__global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArgs a, float* __restrict__ scratch, int first) {
+    using L = DeltaChunk<DKP>;
+    constexpr int C = DC_C, LD = L::LD;
     extern __shared__ __align__(16) float ds_smem[];
     pdl_launch_dependents();
-    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j0 = blockIdx.x * DS_COLS, jw = warp * NC;
-    const int row0 = lane * RP;
-    for (int e = tid; e < 2 * C * L::DKP; e += NT) {            // channels past dk: k = q = 0, g = 1, never copied
-        const int row = e / L::DKP, p = e % L::DKP;
-        if (p >= a.dk) {
-            float* base = ds_smem + row * L::ROW;
-            base[p] = 0.f; base[L::DKP + p] = 0.f; base[2 * L::DKP + p] = 1.f;
+    pdl_wait();
+    float* sk = ds_smem;                                        // k; then k times the decays behind it in its half
+    float* sq = sk + L::TILE;                                   // q; then q times the decays up to it in its half
+    float* sg = sq + L::TILE;                                   // the decays; then k times the decays up to it in its half
+    float* sA = sg + L::TILE;                                   // [t][s]
+    float* sB = sA + C * DC_ROW;
+    float* sG = sB + C * DC_ROW;                                // the halves' whole decays [2][DKP]
+    float* sbeta = sG + 2 * DKP;
+    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int t1 = a.cu_q[s + 1], tb = a.cu_q[s] + (first + (int)blockIdx.x) * C;
+    if (tb >= t1) return;
+    const int n = min(C, t1 - tb);
+    float* out = scratch + (((size_t)s * gridDim.x + blockIdx.x) * a.H + h) * delta_chunk_floats(DKP, a.dv);
+
+    // missing tokens and channels write nothing (k = q = 0, beta = 0) and decay nothing (g = 1)
+#pragma unroll 4
+    for (int e = tid; e < C * DKP; e += DC_THREADS) {
+        const int t = e / DKP, d = e % DKP;
+        const bool in = t < n && d < a.dk;
+        const float* row = a.c + (size_t)(tb + t) * a.c_stride + hk * a.dk + d;
+        sk[t * LD + d] = in ? row[a.c_k] : 0.f;
+        sq[t * LD + d] = in ? row[a.c_q] : 0.f;
+        sg[t * LD + d] = in ? a.g[(size_t)(tb + t) * a.g_stride + a.g_col + h * a.dk + d] : 1.f;
+    }
+    if (tid < C) sbeta[tid] = tid < n ? a.beta[(size_t)(tb + tid) * a.H + h] : 0.f;
+    for (int e = tid; e < 2 * C * DC_ROW; e += DC_THREADS) sA[e] = 0.f;                // (and B behind it)
+    __syncthreads();
+
+    // pairs inside a half: a warp has tokens s = w and 15 - w of both halves, its lanes the channels; k_s times the decays from s on
+    // meets k_t and q_t
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const int base = (i & 1) * DC_H, ts = base + (i < 2 ? warp : DC_H - 1 - warp);
+        constexpr int PER = DKP / 32;
+        float kr[PER];
+#pragma unroll
+        for (int m = 0; m < PER; ++m) kr[m] = sk[ts * LD + lane + 32 * m];
+        for (int t = ts; t < base + DC_H; ++t) {
+            float pa = 0.f, pb = 0.f;
+#pragma unroll
+            for (int m = 0; m < PER; ++m) {
+                const int d = lane + 32 * m;
+                if (t > ts) kr[m] *= sg[t * LD + d];
+                pa = fmaf(kr[m], sk[t * LD + d], pa);
+                pb = fmaf(kr[m], sq[t * LD + d], pb);
+            }
+            pa = warp_sum(pa); pb = warp_sum(pb);
+            if (lane == 0) {
+                if (t > ts) sA[t * DC_ROW + ts] = pa;
+                sB[t * DC_ROW + ts] = pb;
+            }
         }
     }
-    pdl_wait();
-    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
-    float* sp = a.state + (size_t)a.slots[s] * a.state_stride + ((size_t)h * a.dv + j0 + jw) * a.dk + row0;
-    float S[NC][RP];
+    __syncthreads();
+    // in place, a thread per channel and half: k behind, q and k up to a token
+    for (int e = tid; e < 2 * DKP; e += DC_THREADS) {
+        const int p = e % DKP, t0 = e / DKP * DC_H;
+        float g[DC_H], k[DC_H], G = 1.f, suf = 1.f;
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int i = 0; i < RP; ++i) S[c][i] = (j0 + jw + c < a.dv && row0 + i < a.dk) ? sp[(size_t)c * a.dk + i] : 0.f;
-
-    const int cols = min(DS_COLS, a.dv - j0);
-    auto issue = [&](int tb, int stage) {
-        const int n = min(C, t1 - tb);
-        for (int tt = warp; tt < n; tt += NW) {
-            const int t = tb + tt;
-            float* row = ds_smem + (stage * C + tt) * L::ROW;
-            const float* kp = a.c + (size_t)t * a.c_stride + hk * a.dk;
-            const float* gp = a.g + (size_t)t * a.g_stride + a.g_col + h * a.dk;
-            if (VEC) {
-                for (int d = lane * 4; d < a.dk; d += 128) {
-                    cp_async_16(row + d, kp + a.c_k + d);
-                    cp_async_16(row + L::DKP + d, kp + a.c_q + d);
-                    cp_async_16(row + 2 * L::DKP + d, gp + d);
-                }
-            } else {
-                for (int d = lane; d < a.dk; d += 32) {
-                    cp_async_4(row + d, kp + a.c_k + d);
-                    cp_async_4(row + L::DKP + d, kp + a.c_q + d);
-                    cp_async_4(row + 2 * L::DKP + d, gp + d);
-                }
-            }
-            if (lane < cols) cp_async_4(row + L::V_AT + lane, a.c + (size_t)t * a.c_stride + a.c_v + h * a.dv + j0 + lane);
-            else if (lane == 16) cp_async_4(row + L::BETA_AT, a.beta + (size_t)t * a.H + h);
-            else if (lane >= 24) cp_async_16(row + L::AB_AT + (lane - 24) * 4, ab + ((size_t)t * a.H + h) * (2 * C) + (lane - 24) * 4);
+        for (int i = 0; i < DC_H; ++i) {
+            g[i] = sg[(t0 + i) * LD + p]; k[i] = sk[(t0 + i) * LD + p];
+            G *= g[i];
+            sg[(t0 + i) * LD + p] = k[i] * G;
+            sq[(t0 + i) * LD + p] *= G;
         }
-        cp_async_commit();
-    };
-
-    const int n_chunks = (t1 - t0 + C - 1) / C;
-    if (n_chunks > 0) issue(t0, 0);
-    for (int ch = 0; ch < n_chunks; ++ch) {
-        const int tb = t0 + ch * C;
-        if (ch + 1 < n_chunks) { issue(tb + C, (ch + 1) & 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        float* st = ds_smem + (ch & 1) * C * L::ROW;
-        const int n = min(C, t1 - tb);
-        // a last chunk of fewer tokens: the missing ones write nothing (k = 0, beta = 0) and decay nothing (g = 1)
-        for (int e = tid; e < (C - n) * L::ROW; e += NT) {
-            const int c = e % L::ROW;
-            st[(n + e / L::ROW) * L::ROW + c] = (c >= 2 * L::DKP && c < 3 * L::DKP) ? 1.f : 0.f;
-        }
-        __syncthreads();
-        // (1) in place, per channel: k -> k G_C / G_t, q -> q G_t, g -> k G_t; and G_C.  Thread (channel, group of tokens).
-        {
-            constexpr int TPG = C / L::NG;
-            const int p = tid % L::DKP, grp = tid / L::DKP;
-            float gg[TPG], kk[TPG], qq[TPG];
-            if (grp < L::NG) {
-                float prod = 1.f;
+        sG[e] = G;
 #pragma unroll
-                for (int i = 0; i < TPG; ++i) {
-                    const float* row = st + (TPG * grp + i) * L::ROW;
-                    gg[i] = row[2 * L::DKP + p]; kk[i] = row[p]; qq[i] = row[L::DKP + p];
-                    prod *= gg[i];
-                }
-                if (L::NG > 1) ds_smem[L::GP_AT + grp * L::DKP + p] = prod;
-            }
-            if (L::NG > 1) __syncthreads();
-            if (grp < L::NG) {
-                float G = 1.f, suf = 1.f;
-                if (L::NG > 1) {
+        for (int i = DC_H - 1; i >= 0; --i) { sk[(t0 + i) * LD + p] = k[i] * suf; suf *= g[i]; }
+    }
+    __syncthreads();
+    // pairs across the middle: 64 tiles of 2 x 2, four threads a tile with a quarter of the channels' pieces each
+    {
+        const int tile = tid >> 2, kg = tid & 3, tr = DC_H + (tile >> 3) * 2, sr = (tile & 7) * 2;
+        float pa[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, pb[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+        for (int d = kg * 4; d < DKP; d += 16) {
+            float4 k4[2];
 #pragma unroll
-                    for (int o = 0; o < L::NG; ++o) {
-                        const float x = ds_smem[L::GP_AT + o * L::DKP + p];
-                        if (o < grp) G *= x;
-                        if (o > grp) suf *= x;
-                    }
-                }
+            for (int j = 0; j < 2; ++j) k4[j] = *reinterpret_cast<const float4*>(sk + (sr + j) * LD + d);
 #pragma unroll
-                for (int i = 0; i < TPG; ++i) {
-                    float* row = st + (TPG * grp + i) * L::ROW;
-                    G *= gg[i];
-                    row[2 * L::DKP + p] = kk[i] * G;
-                    row[L::DKP + p] = qq[i] * G;
-                }
-                if (grp == L::NG - 1) ds_smem[L::GC_AT + p] = G;
+            for (int i = 0; i < 2; ++i) {
+                const float4 kt = *reinterpret_cast<const float4*>(sg + (tr + i) * LD + d);
+                const float4 qt = *reinterpret_cast<const float4*>(sq + (tr + i) * LD + d);
 #pragma unroll
-                for (int i = TPG - 1; i >= 0; --i) {
-                    st[(TPG * grp + i) * L::ROW + p] = kk[i] * suf;
-                    suf *= gg[i];
-                }
+                for (int j = 0; j < 2; ++j) { pa[i][j] = dot4(pa[i][j], kt, k4[j]); pb[i][j] = dot4(pb[i][j], qt, k4[j]); }
             }
         }
-        __syncthreads();
-        // (2) what the state before the chunk gives token t's correction (lane t) and read-out (lane 16 + t): the columns
-        // go through shared memory, and a lane walks all of them against its token's G_t k_t or G_t q_t
-        float x[NC];
-        {
-            float* sw = ds_smem + L::SW_AT + jw * L::DKP;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                if constexpr (RP == 4) *reinterpret_cast<float4*>(sw + c * L::DKP + row0) = make_float4(S[c][0], S[c][1], S[c][2], S[c][3]);
-                else if constexpr (RP == 2) *reinterpret_cast<float2*>(sw + c * L::DKP + row0) = make_float2(S[c][0], S[c][1]);
-                else sw[c * L::DKP + row0] = S[c][0];
-            }
-            __syncwarp();
-            const float* xr = st + (lane & 15) * L::ROW + (lane < 16 ? 2 * L::DKP : L::DKP);
-            float acc[NC][4];
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
-#pragma unroll 8
-            for (int m = 0; m < L::DKP / 4; ++m) {
-                const float4 xv = *reinterpret_cast<const float4*>(xr + 4 * m);
+            for (int j = 0; j < 2; ++j) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const float4 sv = *reinterpret_cast<const float4*>(sw + c * L::DKP + 4 * m);
-                    acc[c][0] = fmaf(xv.x, sv.x, acc[c][0]); acc[c][1] = fmaf(xv.y, sv.y, acc[c][1]);
-                    acc[c][2] = fmaf(xv.z, sv.z, acc[c][2]); acc[c][3] = fmaf(xv.w, sv.w, acc[c][3]);
+                for (int m = 1; m < 4; m <<= 1) {
+                    pa[i][j] += __shfl_xor_sync(0xffffffffu, pa[i][j], m);
+                    pb[i][j] += __shfl_xor_sync(0xffffffffu, pb[i][j], m);
                 }
+                if (kg == 0) { sA[(tr + i) * DC_ROW + sr + j] = pa[i][j]; sB[(tr + i) * DC_ROW + sr + j] = pb[i][j]; }
             }
-#pragma unroll
-            for (int c = 0; c < NC; ++c) x[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
-        }
-        // (3) lane t < 16: v_t minus the sum, times beta_t when its turn comes; lane 16 + t: the read-out so far
-        float u[NC][C];
-        const float* mine = st + (lane & 15) * L::ROW;
-        const float beta = lane < 16 ? mine[L::BETA_AT] : 0.f;
-        if (lane < 16) {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) x[c] = (j0 + jw + c < a.dv ? mine[L::V_AT + jw + c] : 0.f) - x[c];
-        }
-#pragma unroll
-        for (int q = 0; q < C; ++q) {
-            const float coef = st[q * L::ROW + L::AB_AT + lane];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                u[c][q] = __shfl_sync(0xffffffffu, beta * x[c], q);
-                x[c] = fmaf(coef, u[c][q], x[c]);
-            }
-        }
-        if (lane >= 16 && lane - 16 < n) {
-            float* dst = a.o + (size_t)(tb + lane - 16) * a.o_stride + h * a.dv + j0 + jw;
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (j0 + jw + c < a.dv) dst[c] = x[c];
-        }
-        // (4) the state behind the chunk
-        {
-            float gc[RP];
-            load_rows<RP>(ds_smem + L::GC_AT + row0, gc);
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-#pragma unroll
-                for (int i = 0; i < RP; ++i) S[c][i] *= gc[i];
-        }
+    }
+    __syncthreads();
+    // what needs no solving goes out: G q, k G_C / G, B, G_C
+    for (int e = tid; e < C * DKP; e += DC_THREADS) {
+        const int t = e / DKP, d = e % DKP;
+        out[L::TILE + t * LD + d] = sq[t * LD + d] * (t < DC_H ? 1.f : sG[d]);
+        out[2 * L::TILE + t * LD + d] = sk[t * LD + d] * (t < DC_H ? sG[DKP + d] : 1.f);
+    }
+    for (int e = tid; e < C * DC_ROW; e += DC_THREADS) out[L::B_AT + e] = sB[e];
+    for (int e = tid; e < DKP; e += DC_THREADS) out[L::GC_AT + e] = sG[e] * sG[DKP + e];
+    // the triangular system, a thread per right-hand side: channels of G k, then columns of v
+    const int vcols = (a.dv + DS_COLS - 1) / DS_COLS * DS_COLS;
+    for (int col = tid; col < DKP + vcols; col += DC_THREADS) {
+        const int j = col - DKP;
+        float x[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) {
-            float kt[RP];
-            load_rows<RP>(st + t * L::ROW + row0, kt);
+            float r;
+            if (col < DKP) r = sg[t * LD + col] * (t < DC_H ? 1.f : sG[col]);
+            else r = t < n && j < a.dv ? a.c[(size_t)(tb + t) * a.c_stride + a.c_v + h * a.dv + j] : 0.f;
+            float sum[2] = {0.f, 0.f};
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-#pragma unroll
-                for (int i = 0; i < RP; ++i) S[c][i] = fmaf(kt[i], u[c][t], S[c][i]);
+            for (int i = 0; i < t; i += 4) {                    // (entries from t on are 0, their x are not made yet)
+                const float4 c4 = *reinterpret_cast<const float4*>(sA + t * DC_ROW + i);
+                sum[0] = fmaf(c4.x, x[i], sum[0]);
+                if (i + 1 < t) sum[1] = fmaf(c4.y, x[i + 1], sum[1]);
+                if (i + 2 < t) sum[0] = fmaf(c4.z, x[i + 2], sum[0]);
+                if (i + 3 < t) sum[1] = fmaf(c4.w, x[i + 3], sum[1]);
+            }
+            x[t] = sbeta[t] * (r - (sum[0] + sum[1]));
         }
-        __syncthreads();
+        float* dst = col < DKP ? out + col : out + L::XV_AT + j / DS_COLS * L::XV + j % DS_COLS;
+        const int step = col < DKP ? LD : DS_COLS;
+#pragma unroll
+        for (int t = 0; t < C; ++t) dst[t * step] = x[t];
     }
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int i = 0; i < RP; ++i)
-            if (j0 + jw + c < a.dv && row0 + i < a.dk) sp[(size_t)c * a.dk + i] = S[c][i];
 }
 
-template <int RP>
-static int delta_scan_chunked(const DeltaScanArgs& a, float* ab, dim3 grid, int max_tokens, cudaStream_t stream) {
-    const size_t smem = (size_t)DeltaChunk<RP>::FLOATS * sizeof(float);
-    const bool vec = a.dk % 4 == 0 && a.c_stride % 4 == 0 && a.c_q % 4 == 0 && a.c_k % 4 == 0 && a.g_stride % 4 == 0 &&
-                     a.g_col % 4 == 0 && ((uintptr_t)a.c & 15) == 0 && ((uintptr_t)a.g & 15) == 0;
-    static bool set[2] = {false, false};
-    if (!set[vec]) {
-        cudaError_t e = vec ? cudaFuncSetAttribute(delta_scan_chunked_kernel<RP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                            : cudaFuncSetAttribute(delta_scan_chunked_kernel<RP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        IDM_REQUIRE(e == cudaSuccess, "delta_scan: %zu bytes of shared memory were refused (%s)", smem, cudaGetErrorString(e));
-        set[vec] = true;
+// The chain: a block owns (sequence, head, 16 columns of S) and walks the chunks of one launch from and to the state.  S lies
+// transposed in shared memory, a chunk's numbers come by asynchronous copies one chunk ahead.  Per chunk: (1) X_k S0 and (G q) S0, 64 x
+// 16 sums in tiles of 4 x 4, four threads a tile with every fourth piece of four channels; u = X_v - X_k S0 to shared memory; (2) half of
+// the block brings S behind the chunk, the other half adds B u to its read-outs and stores them.
+template <int DKP>
+__global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a, const float* __restrict__ scratch, int first, int count) {
+    using L = DeltaChunk<DKP>;
+    constexpr int C = DC_C, LD = L::LD, LU = DS_COLS + 4;
+    extern __shared__ __align__(16) float ds_smem[];
+    pdl_launch_dependents();
+    float* sS = ds_smem + 2 * L::BUF;                           // [16 columns][LD]
+    float* sU = sS + DS_COLS * LD;                              // [C][LU]
+    const int s = blockIdx.z, h = blockIdx.y, grp = blockIdx.x, j0 = grp * DS_COLS, tid = threadIdx.x;
+    pdl_wait();
+    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
+    const int chunks = min(count, (t1 - t0 + C - 1) / C - first);
+    if (chunks <= 0) return;
+    const size_t per = delta_chunk_floats(DKP, a.dv);
+    const float* src = scratch + ((size_t)s * count * a.H + h) * per;
+    auto issue = [&](int ch) {
+        const float* from = src + (size_t)ch * a.H * per;
+        float* to = ds_smem + (ch & 1) * L::BUF;
+        for (int e = tid * 4; e < L::BUF; e += DC_THREADS * 4)  // (the columns' part of X_v lies further on)
+            cp_async_16(to + e, e < L::XV_AT ? from + e : from + e + (size_t)grp * L::XV);
+        cp_async_commit();
+    };
+    issue(0);
+    float* sp = a.state + (size_t)a.slots[s] * a.state_stride + ((size_t)h * a.dv + j0) * a.dk;
+    const int cols = min(DS_COLS, a.dv - j0);
+    for (int e = tid; e < DS_COLS * DKP; e += DC_THREADS) {
+        const int j = e / DKP, d = e % DKP;
+        sS[j * LD + d] = j < cols && d < a.dk ? sp[(size_t)j * a.dk + d] : 0.f;
     }
-    idm_launch(delta_pairs_kernel, dim3((max_tokens + DC_C - 1) / DC_C, grid.y, grid.z), dim3(128), 0, stream, a, ab);
-    if (vec) idm_launch(delta_scan_chunked_kernel<RP, true>, grid, dim3(DeltaChunk<RP>::NT), smem, stream, a, (const float*)ab);
-    else idm_launch(delta_scan_chunked_kernel<RP, false>, grid, dim3(DeltaChunk<RP>::NT), smem, stream, a, (const float*)ab);
+    const int tile = tid >> 2, kg = tid & 3, row = (tile >> 2) * 4, col = (tile & 3) * 4;     // rows 0..31 of X_k, 32..63 of G q
+    for (int ch = 0; ch < chunks; ++ch) {
+        if (ch + 1 < chunks) { issue(ch + 1); cp_async_wait<1>(); }
+        else cp_async_wait<0>();
+        __syncthreads();                                        // the chunk's numbers and S are there
+        const float* st = ds_smem + (ch & 1) * L::BUF;
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+        for (int d = kg * 4; d < DKP; d += 16) {
+            float4 x4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x4[i] = *reinterpret_cast<const float4*>(st + (row + i) * LD + d);   // (G q lies right behind X_k)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 s4 = *reinterpret_cast<const float4*>(sS + (col + j) * LD + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i][j] = dot4(acc[i][j], x4[i], s4);
+            }
+        }
+#pragma unroll
+        for (int m = 1; m < 4; m <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], m);
+        float mine[4];                                          // row kg of the tile
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mine[j] = kg == 0 ? acc[0][j] : kg == 1 ? acc[1][j] : kg == 2 ? acc[2][j] : acc[3][j];
+        const int t = (row + kg) % C;
+        if (row < C) {
+            const float4 v = *reinterpret_cast<const float4*>(st + L::XV_AT + t * DS_COLS + col);
+            *reinterpret_cast<float4*>(sU + t * LU + col) = make_float4(v.x - mine[0], v.y - mine[1], v.z - mine[2], v.w - mine[3]);
+        }
+        __syncthreads();                                        // u is there, everyone has read S
+        if (row < C) {
+            // S <- G_C S + (k G_C / G)^T u: four channels and DKP / 32 columns a thread
+            constexpr int NC = DKP / 32;
+            const int d = tid % (DKP / 4) * 4, c0 = tid / (DKP / 4) * NC;
+            float4 n4[NC];
+            const float4 gc = *reinterpret_cast<const float4*>(st + L::GC_AT + d);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float4 o = *reinterpret_cast<const float4*>(sS + (c0 + c) * LD + d);
+                n4[c] = make_float4(o.x * gc.x, o.y * gc.y, o.z * gc.z, o.w * gc.w);
+            }
+#pragma unroll 8
+            for (int i = 0; i < C; ++i) {
+                const float4 k4 = *reinterpret_cast<const float4*>(st + 2 * L::TILE + i * LD + d);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float u = sU[i * LU + c0 + c];
+                    n4[c].x = fmaf(k4.x, u, n4[c].x); n4[c].y = fmaf(k4.y, u, n4[c].y);
+                    n4[c].z = fmaf(k4.z, u, n4[c].z); n4[c].w = fmaf(k4.w, u, n4[c].w);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) *reinterpret_cast<float4*>(sS + (c0 + c) * LD + d) = n4[c];
+        } else {
+            const float* br = st + L::B_AT + t * DC_ROW;
+            for (int i = 0; i <= t; i += 4) {                   // (entries behind t are 0, their u are numbers of later tokens: left out)
+                const float4 b4 = *reinterpret_cast<const float4*>(br + i);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (i + e > t) break;
+                    const float b = e == 0 ? b4.x : e == 1 ? b4.y : e == 2 ? b4.z : b4.w;
+                    const float4 u = *reinterpret_cast<const float4*>(sU + (i + e) * LU + col);
+                    mine[0] = fmaf(b, u.x, mine[0]); mine[1] = fmaf(b, u.y, mine[1]);
+                    mine[2] = fmaf(b, u.z, mine[2]); mine[3] = fmaf(b, u.w, mine[3]);
+                }
+            }
+            const int tt = t0 + (first + ch) * C + t;
+            if (tt < t1) {
+                float* dst = a.o + (size_t)tt * a.o_stride + h * a.dv + j0 + col;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (col + j < cols) dst[j] = mine[j];
+            }
+        }
+        __syncthreads();                                        // S is behind the chunk; its numbers' place is free
+    }
+    for (int e = tid; e < DS_COLS * DKP; e += DC_THREADS) {
+        const int j = e / DKP, d = e % DKP;
+        if (j < cols && d < a.dk) sp[(size_t)j * a.dk + d] = sS[j * LD + d];
+    }
+}
+
+// Chunks of a launch: as many of every sequence as fit 18 M floats of scratch (a chunk of one head of 128 x 64 is 64 KB, so that a long
+// prompt's numbers are read again while they are in the L2), at least one.  The state carries over from launch to launch.
+#define DC_SCRATCH (18ll << 20)
+static int delta_window(int n_seqs, int H, int dkp, int dv, int max_tokens) {
+    const long long fit = DC_SCRATCH / ((long long)n_seqs * H * delta_chunk_floats(dkp, dv)), all = (max_tokens + DC_C - 1) / DC_C;
+    return (int)(fit < 1 ? 1 : fit < all ? fit : all);
+}
+static int delta_dkp(int dk) { return dk <= 32 ? 32 : dk <= 64 ? 64 : 128; }
+
+template <int DKP>
+static int delta_scan_chunked(const DeltaScanArgs& a, float* scratch, int n_seqs, int max_tokens, cudaStream_t stream) {
+    using L = DeltaChunk<DKP>;
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::CHUNK_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::WALK_SMEM);
+    IDM_REQUIRE(e == cudaSuccess, "delta_scan: %d bytes of shared memory were refused (%s)", L::WALK_SMEM, cudaGetErrorString(e));
+    const int window = delta_window(n_seqs, a.H, DKP, a.dv, max_tokens), groups = (a.dv + DS_COLS - 1) / DS_COLS;
+    for (int first = 0; first * DC_C < max_tokens; first += window) {
+        idm_launch(delta_chunk_kernel<DKP>, dim3(window, a.H, n_seqs), dim3(DC_THREADS), L::CHUNK_SMEM, stream, a, scratch, first);
+        idm_launch(delta_walk_kernel<DKP>, dim3(groups, a.H, n_seqs), dim3(DC_THREADS), L::WALK_SMEM, stream, a, (const float*)scratch, first, window);
+    }
     return 0;
 }
 
-// Floats of scratch that a step of `n_tokens` tokens, at most `max_tokens` of one sequence, wants (0: none).
-extern "C" long long idm_delta_scan_scratch_floats(int n_tokens, int H, int dk, int max_tokens) {
-    return (max_tokens > 4 && dk <= 128) ? (long long)n_tokens * H * 2 * DC_C : 0;
+// Floats of scratch that a step of `n_seqs` sequences, at most `max_tokens` of one of them, wants (0: none).
+extern "C" long long idm_delta_scan_scratch_floats(int n_seqs, int H, int dk, int dv, int max_tokens) {
+    if (max_tokens <= 4 || dk <= 0 || dk > 128 || dv <= 0 || n_seqs <= 0 || H <= 0) return 0;
+    return (long long)n_seqs * H * delta_window(n_seqs, H, delta_dkp(dk), dv, max_tokens) * delta_chunk_floats(delta_dkp(dk), dv);
 }
 
 // `max_tokens`: the most tokens any sequence brings to this step; steps of a few tokens walk them straight from
@@ -661,11 +806,10 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
                     H, Hk, dk, dv};
     const dim3 grid((dv + DS_COLS - 1) / DS_COLS, H, n_seqs), block(DS_COLS * 8);
     if (max_tokens > 4 && dk <= 128 && scratch != nullptr) {
-        IDM_REQUIRE(((uintptr_t)scratch & 15) == 0 && (max_tokens + DC_C - 1) / DC_C <= 0x7fffffff, "delta_scan: scratch at %p", (void*)scratch);
-        int rc;
-        if (dk <= 32) rc = delta_scan_chunked<1>(a, scratch, grid, max_tokens, stream);
-        else if (dk <= 64) rc = delta_scan_chunked<2>(a, scratch, grid, max_tokens, stream);
-        else rc = delta_scan_chunked<4>(a, scratch, grid, max_tokens, stream);
+        IDM_REQUIRE(((uintptr_t)scratch & 15) == 0, "delta_scan: scratch at %p", (void*)scratch);
+        const int rc = dk <= 32 ? delta_scan_chunked<32>(a, scratch, n_seqs, max_tokens, stream)
+                     : dk <= 64 ? delta_scan_chunked<64>(a, scratch, n_seqs, max_tokens, stream)
+                                : delta_scan_chunked<128>(a, scratch, n_seqs, max_tokens, stream);
         if (rc) return rc;
     } else if (max_tokens > 4) {
         int rc;
@@ -674,6 +818,11 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
         else if (dk <= 128) rc = delta_scan_staged<16>(a, grid, stream);
         else rc = delta_scan_staged<32>(a, grid, stream);
         if (rc) return rc;
+    } else if (dk <= 128 && dk % 4 == 0 && c_stride % 4 == 0 && c_q % 4 == 0 && c_k % 4 == 0 && g_stride % 4 == 0 && g_col % 4 == 0 &&
+               state_stride % 4 == 0 && (((uintptr_t)c | (uintptr_t)g | (uintptr_t)state) & 15) == 0) {
+        if (dk <= 32) delta_token<8>(a, n_seqs, stream);
+        else if (dk <= 64) delta_token<16>(a, n_seqs, stream);
+        else delta_token<32>(a, n_seqs, stream);
     } else if (dk <= 32) idm_launch(delta_scan_kernel<4>, grid, block, 0, stream, a);
     else if (dk <= 64) idm_launch(delta_scan_kernel<8>, grid, block, 0, stream, a);
     else if (dk <= 128) idm_launch(delta_scan_kernel<16>, grid, block, 0, stream, a);
@@ -708,6 +857,47 @@ __global__ void __launch_bounds__(128) delta_out_kernel(const float* __restrict_
     }
 }
 
+// The same with four elements a lane and load: LANES lanes have a head of up to 4 LANES NV elements, everything a head needs is on its
+// way before its sum is made.  Bound by the bytes of o and the gate.
+template <int LANES, int NV>
+__global__ void __launch_bounds__(128) delta_out_vec_kernel(const float* __restrict__ o, int o_stride, const float* __restrict__ w,
+                                                            float eps, const float* __restrict__ gate, int gate_stride,
+                                                            int gate_col, int gate_act, float scale, T* __restrict__ out,
+                                                            int out_stride, int out_col, int n_tokens, int H, int dv) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = (int)blockIdx.x * (128 / LANES) + threadIdx.x / LANES, lane = threadIdx.x % LANES;
+    const bool live = i < n_tokens * H;                          // (no lane leaves: the sums are over whole warps)
+    const int t = live ? i / H : 0, h = live ? i % H : 0;
+    const float* x = o + (size_t)t * o_stride + (size_t)h * dv;
+    const float* gr = gate + (size_t)t * gate_stride + gate_col + (size_t)h * dv;
+    float4 v[NV], z[NV];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int d = (k * LANES + lane) * 4;
+        v[k] = z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live && d < dv) { v[k] = *reinterpret_cast<const float4*>(x + d); z[k] = *reinterpret_cast<const float4*>(gr + d); }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) { ss = fmaf(v[k].x, v[k].x, ss); ss = fmaf(v[k].y, v[k].y, ss); ss = fmaf(v[k].z, v[k].z, ss); ss = fmaf(v[k].w, v[k].w, ss); }
+#pragma unroll
+    for (int m = LANES / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+    T* dst = out + (size_t)t * out_stride + out_col + (size_t)h * dv;
+    auto one = [&](float xv, float zv, float wv) {
+        const float y = w ? xv * inv * wv : xv * inv, den = 1.0f + expf(-zv);
+        return gate_act == 1 ? y * (zv * (1.0f / den)) * scale : y / den * scale;
+    };
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int d = (k * LANES + lane) * 4;
+        if (!live || d >= dv) continue;
+        const float4 wv = w ? *reinterpret_cast<const float4*>(w + d) : make_float4(1.f, 1.f, 1.f, 1.f);
+        store4(dst + d, one(v[k].x, z[k].x, wv.x), one(v[k].y, z[k].y, wv.y), one(v[k].z, z[k].z, wv.z), one(v[k].w, z[k].w, wv.w));
+    }
+}
+
 extern "C" int idm_delta_out(const float* o, int o_stride, const float* w, float eps, const float* gate, int gate_stride,
                              int gate_col, int gate_act, float scale, void* out, int out_stride, int out_col, int n_tokens, int H,
                              int dv, cudaStream_t stream) {
@@ -715,6 +905,22 @@ extern "C" int idm_delta_out(const float* o, int o_stride, const float* w, float
     IDM_REQUIRE(H > 0 && dv > 0 && out_col >= 0 && out_col + H * dv <= out_stride, "delta_out: columns %d..%d of rows of %d",
                 out_col, out_col + H * dv, out_stride);
     const long long warps = (long long)n_tokens * H;
+    // heads whose rows are whole pieces of four elements on their borders (a prompt of 2 048 tokens, 32 heads of 64: 13 us, element by element 31): others
+    // element by element
+    const bool vec = dv % 4 == 0 && dv <= 512 && o_stride % 4 == 0 && gate_stride % 4 == 0 && gate_col % 4 == 0 && out_stride % 4 == 0 &&
+                     out_col % 4 == 0 && (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 15) == 0 && warps < (1ll << 31);
+    if (vec) {
+#define DELTA_OUT(LANES_, NV_) idm_launch(delta_out_vec_kernel<LANES_, NV_>, dim3((unsigned)((warps + 128 / LANES_ - 1) / (128 / LANES_))), dim3(128), 0, \
+                                          stream, o, o_stride, w, eps, gate, gate_stride, gate_col, gate_act, scale, (T*)out, out_stride, out_col, n_tokens, H, dv)
+        if (dv <= 32) DELTA_OUT(8, 1);
+        else if (dv <= 64) DELTA_OUT(16, 1);
+        else if (dv <= 128) DELTA_OUT(32, 1);
+        else if (dv <= 256) DELTA_OUT(32, 2);
+        else DELTA_OUT(32, 4);
+#undef DELTA_OUT
+        IDM_LAUNCH_CHECK("delta_out");
+        return 0;
+    }
     idm_launch(delta_out_kernel, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, stream, o, o_stride, w, eps, gate,
                gate_stride, gate_col, gate_act, scale, (T*)out, out_stride, out_col, n_tokens, H, dv);
     IDM_LAUNCH_CHECK("delta_out");
