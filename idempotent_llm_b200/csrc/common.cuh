@@ -98,6 +98,17 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float a, float b, float
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
+// four consecutive elements by one load (the address on an 8-byte border in bfloat16, 16-byte in 32-bit)
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
+    v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
+}
+
 // 16-byte vector of T: 8 bfloat16 or 4 float
 template <typename U> struct Vec16;
 template <> struct Vec16<float> {

@@ -315,7 +315,9 @@ extern "C" int idm_rope_table(const int* positions, const double* inv_freq, floa
 __global__ void __launch_bounds__(128) qkv_finish_kernel(QkvArgs a) {
     pdl_launch_dependents();
     pdl_wait();
-    // one block per token: the token's place in the cache is looked up once, the warps share the heads
+    // a block per token: the token's place in the cache is looked up once, the warps share the heads (steps of few tokens spread a
+    // token's heads over several blocks: a warp's heads are one chain of loads and stores after another; 8 tokens of 32 heads 3.0 us, in one block
+    // a token 9.3)
     __shared__ int place[2];
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads = a.n_q + 2 * a.n_kv;
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(128) qkv_finish_kernel(QkvArgs a) {
     if (a.tiles4) {
         // whole heads inside tiles of 128 features, four features per lane (qkv_finish_tile4)
         const int width = heads * a.hd;
-        for (int f0 = warp * 128; f0 < width; f0 += 4 * 128) {
+        for (int f0 = (blockIdx.y * 4 + warp) * 128; f0 < width; f0 += gridDim.y * 4 * 128) {
             const int f = f0 + lane * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (f < width) {
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(128) qkv_finish_kernel(QkvArgs a) {
         }
         return;
     }
-    for (int head = warp; head < heads; head += 4) {
+    for (int head = blockIdx.y * 4 + warp; head < heads; head += gridDim.y * 4) {
         const size_t row = (size_t)t * heads * a.hd + (size_t)head * a.hd;
         qkv_finish_row(a, t, head, lane,
                        [&](int j) { return add_partials(0.f, a.qkv, a.n_partials, a.partial_stride, row + j); },
@@ -371,7 +373,8 @@ extern "C" int idm_qkv_finish(const float* qkv, int n_partials, long long partia
     a.write_cache = k_pool != nullptr;
     a.token_seq = token_seq; a.positions = positions; a.slots = slots;
     a.tiles4 = (128 % hd == 0 && hd >= 8 && (partial_stride % 4) == 0) ? 1 : 0;
-    idm_launch(qkv_finish_kernel, dim3(n_tokens), dim3(128), 0, stream, a);
+    const int quarters = ((n_q + 2 * n_kv) * (a.tiles4 ? hd : 128) + 511) / 512, split = (1184 + n_tokens - 1) / n_tokens;
+    idm_launch(qkv_finish_kernel, dim3(n_tokens, split < quarters ? split : quarters), dim3(128), 0, stream, a);
     IDM_LAUNCH_CHECK("qkv_finish");
     return 0;
 }
@@ -684,7 +687,7 @@ extern "C" int idm_token_gate(const float* s, const int* tokens, const void* tab
 // elements in o of which the first `out_head` count (padded heads): out and gate hold those alone.
 __global__ void __launch_bounds__(256) gate_scale_kernel(const T* __restrict__ o, const float* __restrict__ gate,
                                                          int gate_stride, int gate_group, float scale, T* __restrict__ out,
-                                                         int out_stride, int out_col, int width, int in_head, int out_head) {
+                                                         int out_stride, int out_col, int width, int in_head, int out_head, int vec) {
     pdl_launch_dependents();
     pdl_wait();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
@@ -692,6 +695,18 @@ __global__ void __launch_bounds__(256) gate_scale_kernel(const T* __restrict__ o
     const size_t t = blockIdx.x;
     const T* src = o + t * (size_t)(width / out_head * in_head);
     T* dst = out + t * out_stride + out_col + c;
+    if (vec) {                                                   // four columns of one head on their borders, a gate each or none
+        float v[4], z[4] = {0.f, 0.f, 0.f, 0.f};
+        load4(src + (in_head == out_head ? c : c / out_head * in_head + c % out_head), v);
+        if (gate) *reinterpret_cast<float4*>(z) = *reinterpret_cast<const float4*>(gate + t * gate_stride + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (gate) v[i] = v[i] / (1.0f + expf(-z[i]));
+            v[i] *= scale;
+        }
+        store4(dst, v[0], v[1], v[2], v[3]);
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (c + i >= width) break;
@@ -710,8 +725,11 @@ extern "C" int idm_gate_scale(const void* o, const float* gate, int gate_stride,
     IDM_REQUIRE(gate_group >= 1, "gate_scale: a gate serves %d columns", gate_group);
     IDM_REQUIRE(out_head >= 1 && in_head >= out_head && width % out_head == 0, "gate_scale: %d of %d elements of a head, %d columns",
                 out_head, in_head, width);
+    const int vec = width % 4 == 0 && out_head % 4 == 0 && in_head % 4 == 0 && out_stride % 4 == 0 && out_col % 4 == 0 &&
+                    (((uintptr_t)o | (uintptr_t)out) & 15) == 0 &&
+                    (gate == nullptr || (gate_group == 1 && gate_stride % 4 == 0 && ((uintptr_t)gate & 15) == 0));
     idm_launch(gate_scale_kernel, dim3(n_tokens, (width + 1023) / 1024), dim3(256), 0, stream, (const T*)o, gate, gate_stride,
-               gate_group, scale, (T*)out, out_stride, out_col, width, in_head, out_head);
+               gate_group, scale, (T*)out, out_stride, out_col, width, in_head, out_head, vec);
     IDM_LAUNCH_CHECK("gate_scale");
     return 0;
 }
