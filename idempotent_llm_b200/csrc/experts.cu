@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) experts_combine_kernel(CombineArgs a) {
     float same = 0.f;                                                        // the identity experts' weight
     if (a.x)
         for (int k = 0; k < top; ++k)
-            if (a.table[(size_t)a.tokens[t] * top + k] >= a.n_real) same += a.pair_w[t * top + k];
+            if (a.table[(a.tokens ? (size_t)a.tokens[t] : t) * top + k] >= a.n_real) same += a.pair_w[t * top + k];
     for (int d = threadIdx.x * V; d < a.width; d += blockDim.x * V) {
         float s[V];
 #pragma unroll
@@ -425,7 +425,9 @@ struct GroupArgs {
     int* place; int* offsets; float* row_w; T* xg;
 };
 __device__ __forceinline__ int pair_expert(const GroupArgs& a, int p) {      // of pair p = token * top + choice, or -1
-    const int t = p / a.top, e = a.table[(size_t)a.tokens[t] * a.top + (p - t * a.top)];
+    int e;
+    if (a.tokens) { const int t = p / a.top; e = a.table[(size_t)a.tokens[t] * a.top + (p - t * a.top)]; }
+    else e = a.table[p];                                                     // (the table's rows are the step's)
     return e >= 0 && e < a.n_experts ? e : -1;
 }
 __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) {
@@ -438,6 +440,13 @@ __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * a.block_tokens, t1 = min(t0 + a.block_tokens, a.n_tokens);
     const int pairs = a.n_tokens * a.top, p0 = t0 * a.top, p1 = t1 * a.top;
+    // this block's rows in 16-byte pieces (whole pieces, width % 8 == 0), the first four of a thread on their way while it counts
+    const int pieces = a.width / Vec16<T>::N, all = (t1 - t0) * pieces;
+    const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)t0 * a.width);
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if ((int)threadIdx.x + j * EG_THREADS < all) v[j] = src[threadIdx.x + j * EG_THREADS];
     for (int e = threadIdx.x; e < a.n_experts; e += EG_THREADS) { total[e] = 0; before[e] = 0; }
     __syncthreads();
     for (int c0 = warp * 32; c0 < pairs; c0 += 8 * EG_THREADS) {             // eight looks at the table on their way at a time
@@ -449,11 +458,11 @@ __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) 
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int e = named[j];
-            const unsigned same = __match_any_sync(0xffffffffu, e), early = __ballot_sync(0xffffffffu, c0 + j * EG_THREADS + lane < p0);
-            if (e >= 0 && lane == __ffs(same) - 1) {
-                atomicAdd(&total[e], __popc(same));
-                if (same & early) atomicAdd(&before[e], __popc(same & early));
+            const int p = c0 + j * EG_THREADS + lane;
+            if (p >= p0 && p < p1) at[p - p0] = named[j];
+            if (named[j] >= 0) {
+                atomicAdd(&total[named[j]], 1);
+                if (p < p0) atomicAdd(&before[named[j]], 1);
             }
         }
     }
@@ -474,7 +483,7 @@ __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) 
         if (blockIdx.x == 0 && lane == 0) a.offsets[a.n_experts] = rows;
         __syncwarp();
         for (int c = p0; c < p1; c += 32) {
-            const int p = c + lane, e = p < p1 ? pair_expert(a, p) : -1;
+            const int p = c + lane, e = p < p1 ? at[p - p0] : -1;
             const unsigned same = __match_any_sync(0xffffffffu, e);
             const int row = e >= 0 ? total[e] + before[e] + __popc(same & ((1u << lane) - 1u)) : -1;
             __syncwarp();
@@ -488,15 +497,8 @@ __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) 
         }
     }
     __syncthreads();
-    // 16-byte pieces of this block's rows (whole pieces, width % 8 == 0), one after another over all threads, four on their way
-    const int pieces = a.width / Vec16<T>::N, all = (t1 - t0) * pieces;
-    const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)t0 * a.width);
     uint4* dst = reinterpret_cast<uint4*>(a.xg);
     for (int i0 = threadIdx.x; i0 < all; i0 += 4 * EG_THREADS) {
-        uint4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (i0 + j * EG_THREADS < all) v[j] = src[i0 + j * EG_THREADS];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int i = i0 + j * EG_THREADS, t = i / pieces, piece = i - t * pieces;
@@ -506,6 +508,9 @@ __global__ void __launch_bounds__(EG_THREADS) experts_group_kernel(GroupArgs a) 
                 if (row >= 0) dst[(size_t)row * pieces + piece] = v[j];
             }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i0 + (4 + j) * EG_THREADS < all) v[j] = src[i0 + (4 + j) * EG_THREADS];
     }
 }
 
@@ -513,7 +518,7 @@ int gemm_experts_store(const void* x, const void* w, float* out, const int* offs
 int gemm_experts_gated(const void* x, const void* w_tiled, void* y, const int* offsets, int n_experts, int n_rows, int inter, int K, int act,
                        const float* row_w, cudaStream_t stream);
 
-// h[t] += weight * sum_k ff_e(x_t), e = table[tokens[t], k], with the pairs grouped by expert: one launch groups them, one makes every
+// h[t] += weight * sum_k ff_e(x_t), e = table[tokens[t], k] (tokens null: table[t, k]), with the pairs grouped by expert: one launch groups them, one makes every
 // expert's gated product (gate_up [E, tiles * 128, width], gate and up rows alternating), one every expert's down product (down
 // [E, width, ff]), one adds the outputs up in the order of a token's choices.  Nothing depends on the host: steps can be captured.
 // pair_w [N, top] (or null: 1) weighs the outputs, or (weight_in) the inputs; `identity`: pairs that name expert E or more add

@@ -1209,19 +1209,22 @@ class Kernels:
 
     def experts_by_expert(self, x, tokens, table, gate_up, down, h, act: int, weight: float, pair_w=None, weight_in: bool = False,
                           identity: bool = False) -> None:
-        """``h[t] += weight * sum_k ff_e(x_t)``, ``e = table[tokens[t], k]``, with the (token, choice) pairs grouped by expert on the
-        device: an expert's matrices (``gate_up`` in the layout of ``tile_gate_up``) are read once a step, by one product over
+        """``h[t] += weight * sum_k ff_e(x_t)``, ``e = table[tokens[t], k]`` (``tokens`` None: ``table[t, k]``), with the (token,
+        choice) pairs grouped by expert on the device: an expert's matrices (``gate_up`` in the layout of ``tile_gate_up``) are read once a step, by one product over
         all experts each way (bfloat16; steps of many pairs, captured ones too).  ``pair_w [N, top]`` weighs the pairs' outputs, or
         with ``weight_in`` their inputs; ``identity``: a pair that names expert ``E`` or more adds its weight times ``x_t`` itself."""
         self._need(x, self.dtype, "experts input")
         self._need(h, torch.float32, "residual stream")
         self._need(gate_up, self.dtype, "experts' gate and up rows")
         self._need(down, self.dtype, "experts' down matrices")
-        self._need(tokens, torch.int32, "tokens")
+        if tokens is not None:
+            self._need(tokens, torch.int32, "tokens")
         self._need(table, torch.int32, "expert table")
         n, width = x.shape
         E, _, ff = down.shape
         top = table.shape[1]
+        if tokens is None and table.shape[0] != n:
+            raise KernelError(f"experts: choices of {table.shape[0]} rows for {n} rows")
         if tuple(gate_up.shape) != (E, -(-ff // 64) * 128, width) or down.shape[1] != width or tuple(h.shape) != (n, width):
             raise KernelError(f"experts: gate/up {tuple(gate_up.shape)}, down {tuple(down.shape)}, stream {tuple(h.shape)} for rows of {width}")
         xg = torch.empty((n * top, width), dtype=self.dtype, device=self.device)

@@ -235,15 +235,15 @@ class RoutedExperts(FeedForward):
         elif residual is None:
             h = torch.zeros((n, s.hidden), dtype=torch.float32, device=x.device)
         if s.n_experts:
-            rows = self._row_numbers(n, x.device)
             grouped = n * s.top >= GROUP_FROM and getattr(ctx, "host_tokens", None) is not None
             if self.fused and (grouped or n * s.top >= self.dense_from):
-                K.experts_by_expert(x, rows, chosen, self.gate_up, self.down, h, self.act, 1.0, pair_w=weight, weight_in=self.weight_in,
+                K.experts_by_expert(x, None, chosen, self.gate_up, self.down, h, self.act, 1.0, pair_w=weight, weight_in=self.weight_in,
                                     identity=s.n_identity > 0)
                 return None if residual is not None else h.unsqueeze(0)
             if grouped and not self.fused and self.can_group:
                 self._grouped(x, chosen, weight, h)
             else:
+                rows = self._row_numbers(n, x.device)
                 K.experts_few(x, rows, chosen, self.gate_up, self.row_stride, self.up_off, self.down, h, self.act, 1.0,
                               pair_w=weight, weight_in=self.weight_in)
         if s.n_identity:
