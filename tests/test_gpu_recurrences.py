@@ -1,0 +1,252 @@
+"""The recurrent mixers' kernels alone at the sizes where their cuts can go wrong: chunks and tiles with one token or one column
+left over, sequences that end inside a block of tokens, launches that carry a state on, rows on and off 16-byte borders (GPU)."""
+
+import pytest
+import torch
+
+import helpers
+from idempotent_llm_b200.cache import CacheNeed, SequenceCache
+from idempotent_llm_b200.engine.batch import context_from_packed, pack_step_host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from idempotent_llm_b200.kernels import Kernels
+    return Kernels(torch.float32, torch.device("cuda:0"))
+
+
+def _randn(*shape, seed):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).cuda()
+
+
+def _ctx(starts, lens):
+    slots = list(range(len(lens)))
+    packed, n, q_lens = pack_step_host(slots, starts, [[0] * L for L in lens])
+    return context_from_packed(packed.cuda(), n, slots, q_lens, starts)
+
+
+def _pieces(lens, cut):
+    """Steps that bring each sequence at most ``cut`` tokens: (starts, counts) until all are through."""
+    at = [0] * len(lens)
+    while any(a < n for a, n in zip(at, lens)):
+        counts = [min(cut, n - a) for a, n in zip(at, lens)]
+        yield list(at), counts
+        at = [a + c for a, c in zip(at, counts)]
+
+
+def _step_rows(lens, starts, counts):
+    """Rows of the step's tokens among all sequences' rows, one after another; sequences without a token left out."""
+    first = [sum(lens[:i]) for i in range(len(lens))]
+    keep = [i for i, c in enumerate(counts) if c]
+    return keep, [first[i] + starts[i] + j for i in keep for j in range(counts[i])]
+
+
+# ------------------------------------------------------------------------------------------------ short filters
+@pytest.mark.parametrize("taps", [2, 4])
+@pytest.mark.parametrize("lens,channels", [([1601], 1500), ([3, 1, 700, 9, 801, 2], 1700), ([8, 8, 1589], 1536)])
+def test_short_conv_of_eight_tokens_a_thread(K, taps, lens, channels):
+    """A prompt long enough for eight tokens a thread gives a token the bits that single tokens get."""
+    n = sum(lens)
+    proj = _randn(n, channels + 12, seed=1)
+    w, b = _randn(channels, taps, seed=2), _randn(channels, seed=3)
+    start = _randn(len(lens), (taps - 1) * channels, seed=4)
+    starts = [5 * (i % 3) for i in range(len(lens))]               # (some sequences go on from a state, with fewer tokens than taps too)
+    out = K.short_conv(proj, 7, channels, w, b, 1, start.clone(), _ctx(starts, lens))
+    want, state = torch.empty_like(out), start.clone()
+    for at, counts in _pieces([min(L, 12) for L in lens], 1):
+        keep, rows = _step_rows(lens, at, counts)
+        slots = keep
+        packed, _, q_lens = pack_step_host(slots, [starts[i] + at[i] for i in keep], [[0]] * len(keep))
+        ctx = context_from_packed(packed.cuda(), len(keep), slots, q_lens, [starts[i] + at[i] for i in keep])
+        want[rows] = K.short_conv(proj[rows].contiguous(), 7, channels, w, b, 1, state, ctx)
+    first = [sum(lens[:i]) for i in range(len(lens))]
+    rows = [first[i] + j for i, L in enumerate(lens) for j in range(min(L, 12))]
+    # (a single token moves its state on; one-token sequences of the long step did so as well)
+    assert torch.equal(out[rows], want[rows])
+    u = torch.zeros(n, channels, dtype=torch.float64, device="cuda")
+    for j in range(taps):
+        u[taps - 1:] += w[:, j].double() * proj[j:n - taps + 1 + j, 7:7 + channels].double()
+    deep = [first[i] + j for i, L in enumerate(lens) for j in range(taps, L)]
+    z = u[deep] + b.double()
+    assert helpers.rel_err(out[deep], z * torch.sigmoid(z)) < 1e-5
+
+
+@pytest.mark.parametrize("maps,dk,half", [(1, 128, 32), (2, 128, 16), (1, 24, 0), (1, 40, 20)])
+def test_conv_qkv_of_eight_tokens_a_thread(K, maps, dk, half):
+    lens, n_q, n_kv, dv, taps = [900, 3, 701], 6, 2, 72, 3
+    n_q, n_kv = (n_q, n_kv) if dk == 128 else (20, 10)
+    n, channels = sum(lens), (n_q + n_kv) * dk + n_kv * dv
+    proj, w = _randn(n, channels + 4, seed=5), _randn(channels, taps, seed=6)
+    cs = _randn(n, half, 2, seed=7) if half else None
+    start = _randn(len(lens), (taps - 1) * channels, seed=8)
+
+    def fresh():
+        cache = SequenceCache({0: CacheNeed("full", n_kv, dk, k_row=(n_kv, dk), v_row=(n_kv, dv))}, 64 * 40, torch.float32, "cuda:0",
+                              max_seqs=3, max_seq_len=1024)
+        cache.reserve([(cache.alloc_slot(), L) for L in lens]); cache.flush()
+        return cache.view(0)
+    kv = fresh()
+    q = K.conv_qkv_cache(proj, 4, w, start.clone(), n_q, n_kv, dk, dv, cs, kv, _ctx([0] * 3, lens), maps=maps)
+    other, state, one = fresh(), start.clone(), torch.empty_like(q)
+    for at, counts in _pieces([min(L, 20) for L in lens], 1):
+        keep, rows = _step_rows(lens, at, counts)
+        packed, _, q_lens = pack_step_host(keep, [at[i] for i in keep], [[0]] * len(keep))
+        ctx = context_from_packed(packed.cuda(), len(keep), keep, q_lens, [at[i] for i in keep])
+        one[rows] = K.conv_qkv_cache(proj[rows].contiguous(), 4, w, state, n_q, n_kv, dk, dv, None if cs is None else cs[rows].contiguous(),
+                                     other, ctx, maps=maps)
+    first = [0, lens[0], lens[0] + lens[1]]
+    for i, L in enumerate(lens):
+        m = min(L, 20)
+        assert torch.equal(q[first[i]:first[i] + m], one[first[i]:first[i] + m])
+        page, page2 = int(kv.table[i, 0]), int(other.table[i, 0])
+        assert torch.equal(kv.k[page][:, :m], other.k[page2][:, :m]) and torch.equal(kv.v[page][:, :m], other.v[page2][:, :m])
+
+
+# ------------------------------------------------------------------------------------------------ delta rule
+def _delta_inputs(n, H, Hk, dk, dv, seed, pad=0):
+    k = torch.nn.functional.normalize(_randn(n, Hk, dk, seed=seed), dim=-1)
+    q = torch.nn.functional.normalize(_randn(n, Hk, dk, seed=seed + 1), dim=-1) * dk ** -0.5
+    v = _randn(n, H * dv, seed=seed + 2)
+    gap = torch.zeros(n, pad, device="cuda")
+    c = torch.cat([gap, q.reshape(n, -1), k.reshape(n, -1), v], dim=1).contiguous()
+    g = torch.exp(-3.0 * _randn(n, H * dk, seed=seed + 3).abs() ** 3)     # (some decays underflow within a chunk)
+    g[_randn(n, H * dk, seed=seed + 4) > 1.5] = 1.0
+    beta = torch.sigmoid(_randn(n, H, seed=seed + 5))
+    return c, g.contiguous(), beta, (pad, pad + Hk * dk, pad + 2 * Hk * dk)
+
+
+def _delta_64(c, cols, g, beta, S, H, Hk, dk, dv):
+    """One sequence in 64 bits from S [H, dv, dk]; returns the read-outs and moves S on."""
+    out = []
+    for t in range(c.shape[0]):
+        q, k = (c[t, a:a + Hk * dk].double().view(Hk, dk).repeat_interleave(H // Hk, dim=0) for a in cols[:2])
+        v = c[t, cols[2]:].double().view(H, dv)
+        S *= g[t].double().view(H, 1, dk)
+        u = beta[t].double()[:, None] * (v - (S @ k[:, :, None])[:, :, 0])
+        S += u[:, :, None] * k[:, None, :]
+        out.append((S @ q[:, :, None])[:, :, 0].reshape(-1))
+    return torch.stack(out)
+
+
+# chunks of 32 with one token left over or missing, a half chunk and one more, keys below and at the kernels' sizes, columns that are no
+# whole group of 16; enough sequences that a launch takes one chunk of each and the state carries over
+@pytest.mark.parametrize("lens,H,Hk,dk,dv,pad", [
+    ([5, 31, 32, 33], 4, 2, 128, 64, 0), ([16, 17, 65, 200], 2, 2, 64, 40, 4), ([100, 7], 3, 1, 20, 24, 0), ([97], 6, 3, 128, 16, 3),
+    ([40, 33], 2, 1, 100, 72, 1), ([70] * 24, 64, 16, 128, 64, 0)])
+def test_delta_chunks_against_64_bits(K, lens, H, Hk, dk, dv, pad):
+    n = sum(lens)
+    c, g, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 20, pad)
+    state = _randn(len(lens), H * dv * dk, seed=30)
+    start = state.clone()
+    o = K.delta_scan(c, *cols, g, 0, beta, state, _ctx([0] * len(lens), lens), H, Hk, dk, dv)
+    at = 0
+    for i, L in enumerate(lens[:4]):
+        S = start[i].double().view(H, dv, dk).clone()
+        want = _delta_64(c[at:at + L], cols, g[at:at + L], beta[at:at + L], S, H, Hk, dk, dv)
+        # 32-bit sums of up to 128 products over a chain of up to 200 tokens whose state does not grow
+        assert helpers.rel_err(o[at:at + L], want) < 2e-5 and helpers.rel_err(state[i].view(H, dv, dk), S) < 2e-5, f"sequence {i}"
+        at += L
+    # a later token that is not a number leaves the ones before it alone
+    bad = c.clone()
+    bad[lens[0] - 1] = float("nan")
+    o2 = K.delta_scan(bad, *cols, g, 0, beta, start.clone(), _ctx([0] * len(lens), lens), H, Hk, dk, dv)
+    assert torch.equal(o2[:lens[0] - 1], o[:lens[0] - 1])
+
+
+@pytest.mark.parametrize("dk,dv,pad", [(128, 64, 0), (64, 40, 4), (24, 9, 0), (100, 64, 0), (30, 16, 0), (128, 64, 1), (160, 16, 0)])
+def test_delta_single_tokens_against_64_bits_and_however_cut(K, dk, dv, pad):
+    H, Hk, lens = 4, 2, [8, 3, 5]
+    n = sum(lens)
+    c, g, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 40, pad)
+    start = _randn(len(lens), H * dv * dk, seed=50)
+    got = {}
+    for cut in (1, 3, 4):
+        state, o = start.clone(), torch.empty(n, H * dv, device="cuda")
+        for at, counts in _pieces(lens, cut):
+            keep, rows = _step_rows(lens, at, counts)
+            packed, _, q_lens = pack_step_host(keep, [at[i] for i in keep], [[0] * counts[i] for i in keep])
+            ctx = context_from_packed(packed.cuda(), len(rows), keep, q_lens, [at[i] for i in keep])
+            o[rows] = K.delta_scan(c[rows].contiguous(), *cols, g[rows].contiguous(), 0, beta[rows].contiguous(), state, ctx, H, Hk, dk, dv)
+        got[cut] = (o, state)
+    for cut in (3, 4):
+        assert torch.equal(got[cut][0], got[1][0]) and torch.equal(got[cut][1], got[1][1])
+    at = 0
+    for i, L in enumerate(lens):
+        S = start[i].double().view(H, dv, dk).clone()
+        want = _delta_64(c[at:at + L], cols, g[at:at + L], beta[at:at + L], S, H, Hk, dk, dv)
+        assert helpers.rel_err(got[1][0][at:at + L], want) < 5e-6 and helpers.rel_err(got[1][1][i].view(H, dv, dk), S) < 5e-6
+        at += L
+
+
+@pytest.mark.parametrize("head", [False, True])
+def test_delta_prep_and_out_on_and_off_16_byte_borders(K, head):
+    """Rows shifted by one column take the element by element kernels: the same numbers up to the order of a norm's sum."""
+    n, H, Hk, dk, dv = 37, 6, 3, 64, 40
+    qk, a, proj = _randn(n, 2 * Hk * dk, seed=60), _randn(n, H * dk, seed=61), _randn(n, 2 * H + 3, seed=62)
+    dt, rate = _randn(H if head else H * dk, seed=63), _randn(H, seed=64)
+    o, w, gate = _randn(n, H * dv, seed=65), _randn(dv, seed=66), _randn(n, H * dv, seed=67)
+    got = []
+    for shift in (0, 1):
+        c = torch.cat([torch.zeros(n, 4 * shift + shift, device="cuda"), qk], dim=1).contiguous()
+        dec = torch.cat([torch.zeros(n, shift, device="cuda"), a], dim=1).contiguous()
+        beta = K.delta_prep(c, 5 * shift, 5 * shift + Hk * dk, dec, shift, proj, 0, dt, rate, H, Hk, dk, head_col=H if head else -1)
+        gates = torch.cat([torch.zeros(n, shift, device="cuda"), gate], dim=1).contiguous()
+        out = torch.zeros(n, H * dv + 4, device="cuda")
+        K.delta_out(o, w, 1e-6, gates, shift, 0.7, out, 4 - shift, H, dv, gate_act=1)
+        got.append((c[:, 5 * shift:], dec[:, shift:], beta, out[:, 4 - shift:4 - shift + H * dv]))
+    for x, y in zip(*got):
+        assert helpers.rel_err(x, y.double()) < 1e-6
+
+
+# ------------------------------------------------------------------------------------------------ products over chunks
+# chunks of 64 with one token left over, columns and dims that are no whole tiles, heads that share keys, blocks with several panels
+@pytest.mark.parametrize("lens,heads,groups,P,N,shift", [
+    ([129, 200, 3], 4, 2, 64, 128, 0), ([257], 6, 3, 40, 36, 0), ([130, 191], 3, 1, 72, 100, 0), ([193, 64], 2, 2, 20, 7, 1), ([150], 8, 1, 64, 200, 0)])
+def test_state_space_chunks_against_the_walk(K, lens, heads, groups, P, N, shift):
+    n, inner, gn = sum(lens), heads * P, groups * N
+    xbc = torch.cat([torch.zeros(n, shift, device="cuda"), _randn(n, inner + 2 * gn, seed=70)], dim=1).contiguous()
+    cols = (shift, shift + inner, shift + inner + gn)
+    proj = _randn(n, inner + heads, seed=71)
+    dt_bias, a_log, skip = _randn(heads, seed=72) - 2.0, _randn(heads, seed=73), _randn(heads, seed=74)
+    start = _randn(len(lens), heads * N * P, seed=75)
+    out = []
+    for walk in (128, 1 << 30):
+        K.SSD_WALK = walk
+        state = start.clone()
+        out.append((K.ssd_scan(xbc, cols, proj, 0, inner, dt_bias, a_log, skip, state, _ctx([0] * len(lens), lens), heads, groups, P, N), state))
+    K.SSD_WALK = type(K).SSD_WALK
+    # the same sums of up to N + 64 products per token in another order
+    assert helpers.rel_err(out[0][0], out[1][0].double()) < 1e-5 and helpers.rel_err(out[0][1], out[1][1].double()) < 1e-5
+    bad = xbc.clone()
+    bad[lens[0] - 1] = float("nan")
+    y = K.ssd_scan(bad, cols, proj, 0, inner, dt_bias, a_log, skip, start.clone(), _ctx([0] * len(lens), lens), heads, groups, P, N)
+    assert torch.equal(y[:lens[0] - 1], out[0][0][:lens[0] - 1])       # (a later token leaves the ones before it alone)
+
+
+@pytest.mark.parametrize("lens,H,dk,dv,shift", [([65, 128, 9], 2, 128, 256, 0), ([127], 3, 64, 72, 0), ([64, 1, 193], 2, 20, 36, 0), ([130], 1, 200, 40, 1)])
+def test_retention_chunks_against_the_walk(K, lens, H, dk, dv, shift):
+    n = sum(lens)
+    proj = torch.cat([torch.zeros(n, shift, device="cuda"), _randn(n, 2 * H * dk + H * dv, seed=80)], dim=1).contiguous()
+    cols = (shift, shift + H * dk, shift + 2 * H * dk)
+    decay = torch.tensor([0.96875, 0.5, 0.9995][:H], device="cuda")
+    start = _randn(len(lens), H * dk * dv, seed=81)
+    out = []
+    for walk in (8, 1 << 30):
+        K.RETENTION_WALK = walk
+        state = start.clone()
+        out.append((K.retention(proj.clone(), cols, None, dk ** -0.5, decay, state, _ctx([0] * len(lens), lens), H, dk, dv), state))
+    K.RETENTION_WALK = type(K).RETENTION_WALK
+    assert helpers.rel_err(out[0][0], out[1][0].double()) < 1e-5 and helpers.rel_err(out[0][1], out[1][1].double()) < 1e-5
+
+
+def test_group_norm_and_gate_scale_on_and_off_16_byte_borders(K):
+    n, parts, length = 21, 5, 132
+    y, w = _randn(n, parts * length, seed=90), _randn(parts * length, seed=91)
+    got = []
+    for shift in (0, 1):
+        out = torch.zeros(n, parts * length + 4, device="cuda")
+        K.ssd_group_norm(y, parts, w, 1e-6, 0.5, out, shift)
+        got.append(out[:, shift:shift + parts * length])
+    assert helpers.rel_err(got[0], got[1].double()) < 1e-6
