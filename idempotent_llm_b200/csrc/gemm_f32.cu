@@ -1,323 +1,372 @@
-// out[M, N] = x[M, K] . w[N, K]^T in true 32-bit: plain FMA on CUDA cores, no tensor cores, no reduced-precision mode.
+// out[M, N] = x[M, K] . w[N, K]^T of 32-bit numbers to 32-bit precision, on the tensor cores.
 // (The reference's exact path is the CPU integer matmul of src/detllm/backends.py:95-96; this is its float counterpart.)
 //
-// One order of summation.  The inner axis is cut into segments of 128, dealt to eight classes in turn (class c: segments c,
-// c + 8, ...).  A class is one chain of FMAs in ascending k; an output is ((c0 + c1) + c2) + c3 plus ((c4 + c5) + c6) + c7.
-// Both kernels below do exactly that for every output, so its value does not depend on M, on the tile it falls in, on the
-// kernel, or on what else is in the batch.  Classes are what lets a step of few tokens spread the inner axis over the
-// warps of a block and a tile of outputs be worked by two halves of a block, without a second order of summation; chains
-// of an eighth of the length also round less (1.5e-7 against 4e-7 relative at 1 024 .. 3 072 k).
+// A 32-bit number is three bfloat16 parts, v = v1 + v2 + v3, to its last bit: v1 is v rounded to eight bits, v2 what that left out,
+// v3 what both left out.  x . w is then the sum of nine products of parts; the three smallest (x2 w3, x3 w2, x3 w3) are below 2^-24
+// of the largest and left out.  Products of bfloat16 numbers are exact in 32-bit, so what rounds is the adding, and that is kept
+// short: a segment of 64 k is summed by the MMAs (x1 w1 in one accumulator, x2 w1 + x1 w2 in a second, x3 w1 + x2 w2 + x1 w3 in a
+// third), and the segments are added up one after another by ordinary 32-bit adds.  Error against 64 bits, root mean square
+// relative to the two rows' norms, at 64 / 128 / 1 024 / 3 072 / 8 192 k (one chain of 32-bit FMAs over k in brackets): normal
+// numbers 0.9e-8 / 0.7e-8 / 0.3e-8 / 0.3e-8 / 0.2e-8 (1.8e-8 at all); all positive 0.6e-7 / 0.6e-7 / 0.6e-7 / 0.8e-7 / 1.2e-7
+// (0.8e-7 / 1.1e-7 / 3.2e-7 / 4.7e-7 / 8.9e-7); magnitudes spread over e^(3 z) 1.5e-8 / 1.1e-8 / 0.4e-8 / 0.3e-8 / 0.2e-8
+// (1.6e-8 / 1.5e-8 / 1.1e-8 / 0.9e-8 / 0.7e-8).  An output that is not finite is made again of plain FMAs (plain_sum): infinities
+// and numbers at the very end of the range have no parts.
 //
-// The kernels.
-//   gemm_f32_few_kernel    few tokens: bound by the weight's bytes.  A block owns 8 or 16 output features and up to 32
-//                          tokens; each of its eight warps runs one class through a cp.async ring of its own.
-//                          A head of 151936 x 1024: 131 us with 1 token (4.7 TB/s), 184 us with 8; 1024 x 3072 with 8:
-//                          14 us (some 7 of which are the measurement's).  A tile kernel of 64 x 64 with scalar loads and one
-//                          chain over k, which it replaces, took 300 us for these products whatever the tokens.
-//   gemm_f32_tile_kernel   many tokens: bound by the FMA rate (58 TFLOP/s is what FMAs from registers alone reach here).  Tiles
-//                          of 64 x 64 outputs, 64 per thread.  2 048 tokens: 4096 x 1024 432 us (39.8 TFLOP/s), 1024 x 3072
-//                          388 us (33.2).  Packed FMAs (fma.rn.f32x2) over even and odd k gave the same rate: twice the
-//                          accumulators leave 32 outputs a thread and more shared-memory reads per FMA.
+// One order of summation: an output's bits do not depend on M, on the tile it falls in, on how its segments were dealt out, or on
+// what else is in the batch.
+//
+// A block has 128 features (the MMA's lanes) and 16, 32 or 64 tokens (its columns).  Sixteen warps read both operands from memory,
+// a row's 256 bytes side by side, two segments ahead in registers, and lay the parts down in the swizzled rows that the MMA reads;
+// the token parts lie one after another, so that w1 meets x1, x2 and x3 in one MMA, w2 meets x1 and x2 in one (shared memory is
+// read twelve times a segment instead of 24).  One thread issues the MMAs; eight warps add the segments up from tensor memory, two
+// of them in turn.  Where tiles are few, the blocks of a cluster deal a tile's segments out among them and send the sums to the
+// block that adds up the feature's segments in order.  What bounds it is splitting and fetching, not the MMAs: 1.15 us a segment
+// with 64 tokens, 0.95 with 16 or 32 (more than two stages leave the L1 too little room for the loads in flight: three take 1.3).
+//   700 tokens: 4096 x 1024 64 us (92 TFLOP/s), 1024 x 3072 61 us (72); plain FMAs in tiles of 64 x 64 took 164 and 182.
+//   8 tokens: 1024 x 3072 18 us, some 7 of which are the measurement's; a head of 151936 x 1024 145 us (4.3 TB/s).
+// (A number that is split keeps its bits unless its third part leaves the exponent's range, below 2^-109 or so.)
 #include "common.cuh"
+#include "tcgen05.cuh"
 
-#define GF_SEG 128         // k per segment
-#define GF_CLASSES 8
+#define GX_FEATURES 128                // features of a tile (the MMA's M axis)
+#define GX_SEG 64                      // k per segment and stage: 64 bfloat16 = one swizzled row of 128 bytes
+#define GX_ADD 256                     // threads that add segments up (a warp: a quarter of the features, half of the tokens),
+#define GX_CONV 512                    // that split operands,
+#define GX_THREADS (GX_ADD + GX_CONV + 32)   // and the warp that issues MMAs
+#define GX_WARP_MMA ((GX_ADD + GX_CONV) / 32)
+#define GX_SMEM (226 * 1024)           // dynamic shared memory that a block may ask for (a few bytes of its own beside it)
 
-// 16 bytes of a row from element k on into shared memory, zeros behind the row's end (`rows_ok`: the row exists).  VEC: rows
-// start on 16-byte borders; else element by element.
-template <bool VEC>
-__device__ __forceinline__ void copy_piece(float* dst, const float* row, int k, int K, bool row_ok) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if (VEC) {
-        const bool in = row_ok && k < K;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(in ? row + k : row), "r"(in ? 16 : 0));
-    } else {
+__device__ int g_gemm_f32_error = 0;
+
+__device__ __forceinline__ void tc_ld8_issue(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+
+template <int TN> struct SplitTile {                                           // 128 features, TN tokens
+    static constexpr int A = GX_FEATURES * 128, B = TN * 128;                  // bytes of one part of a stage
+    static constexpr int STAGE = 3 * (A + B);
+    static constexpr int ROUNDS = 4 + (TN + 31) / 32;                   // rows of a thread that splits: features, then tokens
+    static constexpr int COLS = TN == 64 ? 512 : 8 * TN;                       // tensor memory: three sums a segment, two segments in turn
+};
+
+// two numbers side by side: v - u
+__device__ __forceinline__ float2 minus2(float2 v, float ux, float uy) {
+    unsigned long long a, b, d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(ux), "f"(uy));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(v.x), "f"(v.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(0xbf800000bf800000ull), "l"(b));       // u * -1 + v
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(d));
+    return v;
+}
+// four numbers in three bfloat16 parts each, v = p1 + p2 + p3 (to the last bit unless p3 leaves the exponent's range)
+__device__ __forceinline__ void split_four(float4 f, uint2 (&part)[3]) {
+    float2 lo = make_float2(f.x, f.y), hi = make_float2(f.z, f.w);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const bool in = row_ok && k + e < K;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * e), "l"(in ? row + k + e : row), "r"(in ? 4 : 0));
+    for (int p = 0; p < 3; ++p) {
+        const __nv_bfloat162 l = __floats2bfloat162_rn(lo.x, lo.y), h = __floats2bfloat162_rn(hi.x, hi.y);
+        const uint32_t a = *reinterpret_cast<const uint32_t*>(&l), b = *reinterpret_cast<const uint32_t*>(&h);
+        part[p] = make_uint2(a, b);
+        if (p < 2) {
+            lo = minus2(lo, __uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u));
+            hi = minus2(hi, __uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
         }
     }
 }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;"); }
-template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
-// ------------------------------------------------------------------------------------------------------ few tokens
-#define GF_WARPS GF_CLASSES
-#define GF_CHUNK 32                    // k per stage of a warp's ring
-#define GF_ROW (GF_CHUNK + 4)          // a row of a stage in floats: eight rows' 16-byte reads meet in eight different places
-template <int NG, int MT, int STAGES>
-struct FewSmem {
-    static constexpr int STAGE = (NG + MT) * GF_ROW;                          // floats of a warp's stage
-    static constexpr int TABLE = GF_WARPS * MT * NG;                          // a feature group's class sums
-    static constexpr int BYTES = (GF_WARPS * STAGES * STAGE + 2 * TABLE) * 4;
-};
+// An output that is not finite: infinities and numbers at the very end of the range have no parts (inf - inf), so its sum is made
+// of plain FMAs, which stay not finite where the product is.
+__device__ __noinline__ float plain_sum(const float* __restrict__ x, const float* __restrict__ w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K && !isnan(s); ++k) s = fmaf(x[k], w[k], s);
+    return s;
+}
 
-// Warp c runs class c of the block's features; behind a barrier, the thread that owns an output adds the eight chains (two
-// tables in turn, so one barrier per feature group).  A warp's ring runs on across feature groups.
-template <int NG, int MT, int STAGES, bool VEC>
-__global__ void __launch_bounds__(GF_WARPS * 32) gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                     float* __restrict__ out, int M, int N, int K, int n_groups) {
-    using S = FewSmem<NG, MT, STAGES>;
-    constexpr int NI = NG / 8, MI = MT / 4;
-    extern __shared__ __align__(16) float smem[];
-    pdl_launch_dependents();
+template <int TN, int ROWS>
+__global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                                       float* __restrict__ out, int M, int N, int K, int token_tiles, int tiles) {
+    using S = SplitTile<TN>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) unsigned long long bars_mem[8];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_mem;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem_u32(bars_mem);
+    uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+    float* recv = reinterpret_cast<float*>(gen + 2 * S::STAGE);             // [segment][this block's features][TN]
+    auto full = [&](int b) { return bars + 8u * b; };
+    auto empty = [&](int b) { return bars + 8u * (2 + b); };
+    auto acc_full = [&](int b) { return bars + 8u * (4 + b); };
+    auto acc_empty = [&](int b) { return bars + 8u * (6 + b); };
+    volatile int* abort_flag = &abort_mem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ln = lane & 7, lm = lane >> 3;                                  // features ln + 8 i, tokens lm + 4 j
-    float* ring = smem + warp * STAGES * S::STAGE;
-    float* tables = smem + GF_WARPS * STAGES * S::STAGE;
-    const int m0 = blockIdx.y * MT, k_first = warp * GF_SEG;
-    const int segs = (K + GF_SEG - 1) / GF_SEG, my_segs = warp < segs ? (segs - 1 - warp) / GF_CLASSES + 1 : 0;
-    const int per_group = my_segs * (GF_SEG / GF_CHUNK);                      // chunks of this warp in a feature group
-    const int total = per_group * ((n_groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1);
-    int ask_group = blockIdx.x, ask_k = k_first, ask_c = 0;                   // the chunk that is asked for next
-    auto step_ask = [&]() {
-        ask_k += GF_CHUNK;
-        if (ask_k % GF_SEG == 0) ask_k += (GF_CLASSES - 1) * GF_SEG;
-        if (++ask_c == per_group) { ask_c = 0; ask_k = k_first; ask_group += gridDim.x; }
-    };
-    auto copy_w = [&](int slot) {
-        float* dst = ring + slot * S::STAGE;
-#pragma unroll
-        for (int i = 0; i < NG / 4; ++i) {
-            const int r = i * 4 + (lane >> 3), n = ask_group * NG + r, k = ask_k + (lane & 7) * 4;
-            copy_piece<VEC>(dst + r * GF_ROW + (lane & 7) * 4, w + (size_t)min(n, N - 1) * K, k, K, n < N);
+    const int split = gridDim.z, rank = blockIdx.z;                            // blocks of a cluster deal a tile's segments out in turn
+    const int segs = (K + GX_SEG - 1) / GX_SEG;
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(full(b), GX_CONV / 32); mbar_init(empty(b), 1);
+            mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), GX_ADD / 32);
         }
-    };
-    auto copy_x = [&](int slot) {
-        float* dst = ring + slot * S::STAGE + NG * GF_ROW;
-#pragma unroll
-        for (int i = 0; i < MT / 4; ++i) {
-            const int r = i * 4 + (lane >> 3), m = m0 + r, k = ask_k + (lane & 7) * 4;
-            copy_piece<VEC>(dst + r * GF_ROW + (lane & 7) * 4, x + (size_t)min(m, M - 1) * K, k, K, m < M);
-        }
-    };
-    // the weight's first chunks are asked for before the kernel before has ended (no kernel writes a weight)
-    for (int q = 0; q < STAGES - 1 && q < total; ++q) { copy_w(q); step_ask(); }
-    pdl_wait();
-    ask_group = blockIdx.x; ask_k = k_first; ask_c = 0;
-    for (int q = 0; q < STAGES - 1; ++q) {
-        if (q < total) { copy_x(q); step_ask(); }
-        copies_commit();
+        abort_mem = 0;
+        mbar_init_fence();
     }
-    int q = 0, slot = 0, turn = 0;
-    for (int g = blockIdx.x; g < n_groups; g += gridDim.x, turn ^= 1) {
-        float acc[NI][MI];
+    if (warp == GX_WARP_MMA) tmem_alloc(smem_u32(&tmem_slot), S::COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();               // (behind the allocation: a block of the next kernel cannot hold what this one waits for)
+    if (split > 1) cluster_sync_all();     // every block of the cluster is there before one writes to another
+
+    if (warp >= GX_ADD / 32 && warp < GX_WARP_MMA) {
+        // ------------------------------------------------------------ operands: 32-bit from memory, three parts into the stage
+        // a thread has four k of rows row, row + 32, ...: sixteen threads read a row's 256 bytes side by side
+        const int ct = threadIdx.x - GX_ADD, row = ct >> 4, piece = ct & 15;
+        float4 raw[2][S::ROUNDS];
+        // rows behind the end are the last one again: their outputs are dropped
+        struct Where { int tile, seg; const float *w, *x; int dw[3], dx; };
+        auto place = [&](Where& p, int tile) {
+            p.tile = tile; p.seg = rank;
+            const int f = tile / token_tiles * GX_FEATURES + row, m = tile % token_tiles * TN + row, k = rank * GX_SEG + piece * 4;
+            p.w = w + (size_t)min(f, N - 1) * K + k;
+            p.x = x + (size_t)min(m, M - 1) * K + k;
 #pragma unroll
-        for (int i = 0; i < NI; ++i)
-#pragma unroll
-            for (int j = 0; j < MI; ++j) acc[i][j] = 0.f;
-        for (int c = 0; c < per_group; ++c, ++q) {
-            copies_wait<STAGES - 2>();
-            __syncwarp();
-            if (q + STAGES - 1 < total) {
-                const int to = slot == 0 ? STAGES - 1 : slot - 1;            // the stage that was read last
-                copy_w(to); copy_x(to); step_ask();
+            for (int i = 0; i < 3; ++i) p.dw[i] = (min(f + 32 * (i + 1), N - 1) - min(f, N - 1)) * K;
+            p.dx = (min(m + 32, M - 1) - min(m, M - 1)) * K;
+        };
+        auto step = [&](Where& p) {                                            // false behind the block's last segment
+            p.seg += split;
+            if (p.seg < segs) { p.w += split * GX_SEG; p.x += split * GX_SEG; return true; }
+            if (p.tile + (int)gridDim.x >= tiles) return false;
+            place(p, p.tile + gridDim.x);
+            return true;
+        };
+        auto load4k = [&](const float* p, int seg) {
+            const int left = K - seg * GX_SEG - piece * 4;                     // elements of the row from here on
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ROWS == 2) return __ldcg(reinterpret_cast<const float4*>(p));  // (K in whole segments)
+            if (ROWS == 1) {
+                if (left > 0) v = __ldcg(reinterpret_cast<const float4*>(p));
+            } else {
+                if (left > 0) v.x = p[0];
+                if (left > 1) v.y = p[1];
+                if (left > 2) v.z = p[2];
+                if (left > 3) v.w = p[3];
             }
-            copies_commit();
-            const float* ws = ring + slot * S::STAGE + ln * GF_ROW;
-            const float* xs = ring + slot * S::STAGE + (NG + lm) * GF_ROW;
-            slot = slot == STAGES - 1 ? 0 : slot + 1;
+            return v;
+        };
+        auto load_w = [&](float4 (&v)[S::ROUNDS], const Where& p) {
+            v[0] = load4k(p.w, p.seg);
 #pragma unroll
-            for (int k = 0; k < GF_CHUNK; k += 4) {
-                float4 a[NI];
+            for (int i = 0; i < 3; ++i) v[i + 1] = load4k(p.w + p.dw[i], p.seg);
+        };
+        auto load_x = [&](float4 (&v)[S::ROUNDS], const Where& p) {
+            if (TN >= 32 || row < TN) v[4] = load4k(p.x, p.seg);
+            if (TN > 32) v[S::ROUNDS - 1] = load4k(p.x + p.dx, p.seg);
+        };
+        if (blockIdx.x < tiles && rank < segs) {
+            Where at;
+            // the weight's first pieces are asked for before the kernel before has ended (no kernel writes a weight)
+            place(at, blockIdx.x);
+            load_w(raw[0], at);
+            if (step(at)) load_w(raw[1], at);
+            pdl_wait();
+            place(at, blockIdx.x);
+            int have = 1;                                                      // segments asked for
+            load_x(raw[0], at);
+            bool more = step(at);
+            if (more) { load_x(raw[1], at); more = step(at); have = 2; }
+            const uint32_t off = (uint32_t)(row * 128 + (((piece >> 1) ^ (row & 7)) << 4) + (piece & 1) * 8);   // (row + 32 i: the same place in its swizzle atom)
+            for (int turn = 0; have > 0; turn ^= 1) {
 #pragma unroll
-                for (int i = 0; i < NI; ++i) a[i] = *reinterpret_cast<const float4*>(ws + i * 8 * GF_ROW + k);
+                for (int b = 0; b < 2; ++b) {
+                    if (have == 0) break;
+                    if (!mbar_wait(empty(b), turn ^ 1, abort_flag, &g_gemm_f32_error)) { have = 0; break; }
+                    uint8_t* stage = gen + b * S::STAGE + off;
 #pragma unroll
-                for (int j = 0; j < MI; ++j) {
-                    const float4 b = *reinterpret_cast<const float4*>(xs + j * 4 * GF_ROW + k);
+                    for (int i = 0; i < S::ROUNDS; ++i) {
+                        if (i >= 4 && TN < 32 && row >= TN) break;
+                        uint2 part[3];
+                        split_four(raw[b][i], part);
 #pragma unroll
-                    for (int i = 0; i < NI; ++i) {
-                        acc[i][j] = fmaf(b.x, a[i].x, acc[i][j]);
-                        acc[i][j] = fmaf(b.y, a[i].y, acc[i][j]);
-                        acc[i][j] = fmaf(b.z, a[i].z, acc[i][j]);
-                        acc[i][j] = fmaf(b.w, a[i].w, acc[i][j]);
+                        for (int p = 0; p < 3; ++p)
+                            *reinterpret_cast<uint2*>(stage + (i < 4 ? p * S::A + i * 4096 : 3 * S::A + p * S::B + (i - 4) * 4096)) = part[p];
                     }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full(b));                       // (one arrival a warp: they queue up at the barrier)
+                    if (more) {
+                        load_w(raw[b], at); load_x(raw[b], at);
+                        more = step(at);
+                    } else --have;
                 }
             }
         }
-        float* table = tables + turn * S::TABLE;
-#pragma unroll
-        for (int i = 0; i < NI; ++i)
-#pragma unroll
-            for (int j = 0; j < MI; ++j) table[(warp * MT + lm + 4 * j) * NG + ln + 8 * i] = acc[i][j];
-        __syncthreads();
-        for (int at = threadIdx.x; at < MT * NG; at += GF_WARPS * 32) {
-            const int m = m0 + at / NG, n = g * NG + at % NG;
-            const float* c = table + at;
-            constexpr int D = MT * NG;
-            const float low = ((c[0] + c[D]) + c[2 * D]) + c[3 * D], high = ((c[4 * D] + c[5 * D]) + c[6 * D]) + c[7 * D];
-            if (m < M && n < N) out[(size_t)m * N + n] = low + high;
+    } else if (warp == GX_WARP_MMA) {
+        // ------------------------------------------------------------ MMAs: products of parts, by size into three sums
+        if (lane == 0) {
+            const uint32_t three = umma_idesc(GX_FEATURES, 3 * TN), two = umma_idesc(GX_FEATURES, 2 * TN), one = umma_idesc(GX_FEATURES, TN);
+            int it = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+                for (int seg = rank; ok && seg < segs; seg += split, ++it) {
+                    const int b = it & 1, turn = (it >> 1) & 1;
+                    const uint32_t d = tmem + b * 3 * TN;
+                    ok = mbar_wait(acc_empty(b), turn ^ 1, abort_flag, &g_gemm_f32_error) &&
+                         mbar_wait(full(b), turn, abort_flag, &g_gemm_f32_error);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a = base + b * S::STAGE;
+                    const uint64_t a1 = umma_desc_kmajor(a), a2 = umma_desc_kmajor(a + S::A), a3 = umma_desc_kmajor(a + 2 * S::A);
+                    const uint64_t t = umma_desc_kmajor(a + 3 * S::A);         // the token parts' rows one after another
+                    tc_mma_bf16_kblock(d, a1, t, three, 0);                    // w1 x1 | w1 x2 | w1 x3
+                    tc_mma_bf16_kblock(d + TN, a2, t, two, 1);                 //       + w2 x1 | w2 x2
+                    tc_mma_bf16_kblock(d + 2 * TN, a3, t, one, 1);             //               + w3 x1
+                    tc_commit(empty(b));
+                    tc_commit(acc_full(b));
+                }
         }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------------ many tokens
-#define GF_TILE 64
-#define GF_BK 16
-#define GF_BROW (GF_BK + 4)            // a row of a stage in floats (eight rows' 16-byte reads in eight different places)
-#define GF_TSTAGES 2
-#define GF_HALF 64                     // threads of a half of the block
-#define GF_STAGE (2 * GF_TILE * GF_BROW)
-#define GF_TILE_SMEM (2 * (GF_TSTAGES * GF_STAGE + 64 * GF_HALF) * 4)
-
-// A block is two halves of two warps, a thread 8 x 8 outputs of the tile; half h runs classes 4 h .. 4 h + 3 through a ring of its
-// own and adds them up in shared memory (64 more registers a thread would leave room for two blocks on an SM instead of
-// three); the lower half's threads add the two halves' sums at the end.
-template <bool VEC>
-__global__ void __launch_bounds__(2 * GF_HALF, 3) gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                       float* __restrict__ out, int M, int N, int K) {
-    extern __shared__ __align__(16) float smem[];
-    pdl_launch_dependents();
-    pdl_wait();
-    // a warp is 4 x 8 threads: four rows of x and eight of w per 16-byte read
-    const int half = threadIdx.x / GF_HALF, ht = threadIdx.x % GF_HALF;
-    const int tx = ht & 7, ty = ht >> 3;                                     // features tx + 8 j, tokens ty + 8 i
-    const int m0 = blockIdx.y * GF_TILE, n0 = blockIdx.x * GF_TILE;
-    float* ring = smem + half * GF_TSTAGES * GF_STAGE;
-    float* sums = smem + 2 * GF_TSTAGES * GF_STAGE + half * 64 * GF_HALF + ht;   // [8 * 8][threads of a half]
-    // a walk over this half's k: a class's segments, then the next class's
-    struct Walk { int cls, k; };
-    auto done = [&](const Walk& p) { return p.k >= K; };
-    auto step = [&](Walk& p) {                                               // true behind a class's last piece
-        p.k += GF_BK;
-        if (p.k % GF_SEG == 0) p.k += (GF_CLASSES - 1) * GF_SEG;
-        if (p.k < K) return false;
-        ++p.cls;
-        p.k = p.cls < 4 * half + 4 ? p.cls * GF_SEG : K;                     // (a class that starts behind K is empty, and so are those after it)
-        return true;
-    };
-    // this thread's pieces of a stage: 16 bytes at column lk of rows lr, lr + 16, ... of the tile's x and w
-    const int lr = ht >> 2, lk = (ht & 3) * 4;
-    const float* px = x + (size_t)(m0 + lr) * K + lk;                        // (rows behind the end are not read: zeros go there)
-    const float* pw = w + (size_t)(n0 + lr) * K + lk;
-    const size_t step16 = (size_t)16 * K;
-    auto copy_stage = [&](int slot, int k0) {
-        float* dst = ring + slot * GF_STAGE + lr * GF_BROW + lk;
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------ segments, one after another
+        constexpr int COLS = TN / 2;
+        float tot[COLS];
+        int it = 0;
+        bool ok = true;
+        const int per = (GX_FEATURES + split - 1) / split, mine = (warp & 3) * 32 + lane, owner = mine / per, spot = mine % per, c0 = (warp >> 2) * COLS;
+        pdl_wait();                        // (the kernel before may still read what is written here)
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            copy_piece<VEC>(dst + i * 16 * GF_BROW, px + i * step16, k0, K - lk, m0 + lr + i * 16 < M);
-            copy_piece<VEC>(dst + (GF_TILE + i * 16) * GF_BROW, pw + i * step16, k0, K - lk, n0 + lr + i * 16 < N);
-        }
-    };
-    float acc[8][8];
+            for (int j = 0; j < COLS; ++j) tot[j] = 0.f;
+            for (int seg = rank; seg < segs; seg += split, ++it) {
+                ok = mbar_wait(acc_full(it & 1), (it >> 1) & 1, abort_flag, &g_gemm_f32_error);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t big = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (it & 1) * 3 * TN + c0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+                for (int c = 0; c < COLS; c += 8) {
+                    uint32_t u[8], v[8], z[8];
+                    tc_ld8_issue(big + c, u); tc_ld8_issue(big + TN + c, v); tc_ld8_issue(big + 2 * TN + c, z);
+                    tc_ld_wait();
+                    float sum[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { acc[i][j] = 0.f; sums[(i * 8 + j) * GF_HALF] = 0.f; }
-    Walk ask{4 * half, 4 * half * GF_SEG}, at = ask;
-    for (int s = 0; s < GF_TSTAGES - 1; ++s) {
-        if (!done(ask)) { copy_stage(s, ask.k); step(ask); }
-        copies_commit();
-    }
-    int slot = 0;
-    while (!done(at)) {
-        copies_wait<GF_TSTAGES - 2>();
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(GF_HALF) : "memory");
-        if (!done(ask)) { copy_stage(slot == 0 ? GF_TSTAGES - 1 : slot - 1, ask.k); step(ask); }
-        copies_commit();
-        const float* xs = ring + slot * GF_STAGE + ty * GF_BROW;
-        const float* ws = ring + slot * GF_STAGE + (GF_TILE + tx) * GF_BROW;
-        slot = slot == GF_TSTAGES - 1 ? 0 : slot + 1;
+                    for (int j = 0; j < 8; ++j) sum[j] = __uint_as_float(u[j]) + (__uint_as_float(v[j]) + __uint_as_float(z[j]));
+                    if (split == 1) {
 #pragma unroll
-        for (int k = 0; k < GF_BK; k += 4) {
-            float4 a[8];
+                        for (int j = 0; j < 8; ++j) tot[c + j] += sum[j];
+                    } else {
+                        const uint32_t to = mapa_u32(smem_u32(recv + ((size_t)seg * per + spot) * TN + c0 + c), owner);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * 8 * GF_BROW + k);
+                        for (int j = 0; j < 8; j += 4)
+                            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 4 * j), "f"(sum[j]), "f"(sum[j + 1]), "f"(sum[j + 2]), "f"(sum[j + 3]) : "memory");
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(it & 1));
+            }
+            if (split == 1 && ok) {
+                const int f = tile / token_tiles * GX_FEATURES + mine, m0 = tile % token_tiles * TN + c0;
+                if (f < N)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 b = *reinterpret_cast<const float4*>(ws + j * 8 * GF_BROW + k);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+                    for (int j = 0; j < COLS; ++j)
+                        if (m0 + j < M) {
+                            float s = tot[j];
+                            if (!isfinite(s)) s = plain_sum(x + (size_t)(m0 + j) * K, w + (size_t)f * K, K);
+                            out[(size_t)(m0 + j) * N + f] = s;
+                        }
             }
         }
-        if (step(at)) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) { sums[(i * 8 + j) * GF_HALF] += acc[i][j]; acc[i][j] = 0.f; }
-        }
     }
+    __syncwarp();
+    if (split > 1) {
+        pdl_wait();
+        cluster_sync_all();                // all segments' sums are here
+        const int per = (GX_FEATURES + split - 1) / split, tile = blockIdx.x;
+        const int f0 = tile / token_tiles * GX_FEATURES + rank * per, m0 = tile % token_tiles * TN, have = min(per, GX_FEATURES - rank * per);
+        if (abort_mem == 0)
+            for (int at = threadIdx.x; at < have * TN; at += GX_THREADS) {
+                const int spot = at % have, f = f0 + spot, m = m0 + at / have;
+                if (f >= N || m >= M) continue;
+                float s = 0.f;
+#pragma unroll 8
+                for (int seg = 0; seg < segs; ++seg) s += recv[((size_t)seg * per + spot) * TN + at / have];
+                if (!isfinite(s)) s = plain_sum(x + (size_t)m * K, w + (size_t)f * K, K);
+                out[(size_t)m * N + f] = s;
+            }
+    }
+    tc_fence_before();
     __syncthreads();
-    if (half == 1) return;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty + i * 8;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int n = n0 + tx + j * 8;
-            if (n < N) out[(size_t)m * N + n] = sums[(i * 8 + j) * GF_HALF] + sums[(64 + i * 8 + j) * GF_HALF];
-        }
-    }
+    tc_fence_after();
+    if (warp == GX_WARP_MMA) tmem_dealloc(tmem, S::COLS);
 }
 
 // ------------------------------------------------------------------------------------------------------ launches
-// opt in to more than 48 KB of shared memory, once per kernel and device
-template <typename F>
-static int allow_smem(F kernel, int bytes, const char* what) {
+template <int TN> static long long split_smem(int K, int split) {
+    const long long segs = (K + GX_SEG - 1) / GX_SEG, per = (GX_FEATURES + split - 1) / split;
+    return 1024 + 2 * SplitTile<TN>::STAGE + (split > 1 ? segs * per * TN * 4 : 0);
+}
+
+template <int TN>
+static int split_launch(const float* x, const float* w, float* out, int M, int N, int K, int rows, int split, int sms, cudaStream_t stream) {
+    const int bytes = (int)split_smem<TN>(K, split);
+    auto kernel = rows == 0 ? gemm_f32_split_kernel<TN, 0> : rows == 1 ? gemm_f32_split_kernel<TN, 1> : gemm_f32_split_kernel<TN, 2>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory: %s", what, bytes, cudaGetErrorString(e));
+    IDM_REQUIRE(e == cudaSuccess, "gemm_f32: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+    const int token_tiles = (M + TN - 1) / TN;
+    const long long tiles = (long long)token_tiles * ((N + GX_FEATURES - 1) / GX_FEATURES);
+    IDM_REQUIRE(tiles < (1ll << 30), "gemm_f32: M=%d N=%d are too large for one launch", M, N);
+    if (split > 1)
+        idm_launch_cluster(kernel, dim3((unsigned)tiles, 1, split), dim3(GX_THREADS), bytes, stream, split, x, w, out, M, N, K, token_tiles, (int)tiles);
+    else
+        idm_launch(kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(GX_THREADS), bytes, stream, x, w, out, M, N, K, token_tiles, (int)tiles);
     return 0;
 }
 
-template <int NG, int MT, int STAGES>
-static int few_launch(const float* x, const float* w, float* out, int M, int N, int K, bool vec, int sms, cudaStream_t stream) {
-    constexpr int BYTES = FewSmem<NG, MT, STAGES>::BYTES;
-    auto kernel = vec ? gemm_f32_few_kernel<NG, MT, STAGES, true> : gemm_f32_few_kernel<NG, MT, STAGES, false>;
-    if (int rc = allow_smem(kernel, BYTES, "gemm_f32")) return rc;
-    const int n_groups = (N + NG - 1) / NG, per_sm = 227 * 1024 / (BYTES + 1024);
-    idm_launch(kernel, dim3(min(n_groups, sms * per_sm), (M + MT - 1) / MT), dim3(GF_WARPS * 32), BYTES, stream, x, w, out, M, N,
-               K, n_groups);
-    return 0;
+// Tokens per tile and blocks per tile: the same bits whichever, so only time decides.  A block's time is its segments, one after
+// another: 0.95 us with 16 or 32 tokens, 1.15 with 64, and about 3 us more where a tile is split (the cluster's barriers, and the sums
+// sent).  Measured (us, inputs out of the L2): 1024 x 3072 with 8 tokens split 1 / 4 / 8: 49 / 29 / 18; 4096 x 1024 split
+// 1 / 2 / 4: 25 / 20 / 16; with 700 tokens, tiles of 32 / 64 tokens: 4096 x 1024 78 / 64, 1024 x 3072 90 / 61; with 64 tokens
+// 6144 x 1024 25 / 37.  A split needs room for all segments' sums of the features that a block adds up.
+template <int TN> static void split_cost(int M, int N, int K, int sms, float per_segment, int& best_tn, int& best_split, float& best) {
+    const long long tiles = (long long)((M + TN - 1) / TN) * ((N + GX_FEATURES - 1) / GX_FEATURES), segs = (K + GX_SEG - 1) / GX_SEG;
+    for (const int split : {1, 2, 3, 4, 6, 8}) {                                 // (sizes of which the SMs of a cluster's reach hold whole numbers)
+        if (split > segs || (split > 1 && tiles * split > sms)) break;
+        if (split_smem<TN>(K, split) > GX_SMEM) continue;
+        const float t = (split == 1 ? (float)((tiles + sms - 1) / sms * segs) : (float)((segs + split - 1) / split)) * per_segment + (split > 1 ? 3.f : 0.f);
+        if (t < best) { best = t; best_tn = TN; best_split = split; }
+    }
 }
-
-static int tile_launch(const float* x, const float* w, float* out, int M, int N, int K, bool vec, cudaStream_t stream) {
-    auto kernel = vec ? gemm_f32_tile_kernel<true> : gemm_f32_tile_kernel<false>;
-    if (int rc = allow_smem(kernel, GF_TILE_SMEM, "gemm_f32")) return rc;
-    const dim3 grid((N + GF_TILE - 1) / GF_TILE, (M + GF_TILE - 1) / GF_TILE);
-    IDM_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large for one launch", M);
-    idm_launch(kernel, grid, dim3(2 * GF_HALF), GF_TILE_SMEM, stream, x, w, out, M, N, K);
-    return 0;
-}
-
-// Which kernel: the same bits either way, so only time decides.  Measured (us, inputs out of the L2, few / tile), N x K: 1024 x 2048 with
-// 613 tokens (160 tiles of 64 x 64) 114 / 140, with 1 024 (256 tiles) 185 / 143; 4096 x 1024 with 128 (128) 51 / 52, with
-// 256 (256) 96 / 78; 6144 x 1024 with 128 (192) 75 / 80, with 256 (384) 138 / 101; a head of 151936 x 1024 with 32 tokens
-// 412 / 506, with 64 807 / 521: from 200 tiles on the tiles fill the SMs, unless the step has so few tokens that half of
-// every tile is padding.
-#define GF_TILES_FROM 200
-#define GF_FEW_UP_TO 32
 
 extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
     IDM_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
-    const bool vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-    int rc, dev = 0, sms = 0;
+    IDM_REQUIRE(K < (1 << 24), "gemm_f32: rows of %d elements", K);               // (a tile's rows are reached by 32-bit offsets)
+    const int rows = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 148;
-    const long long tiles = (long long)((M + GF_TILE - 1) / GF_TILE) * ((N + GF_TILE - 1) / GF_TILE);
-    if (M > GF_FEW_UP_TO && tiles >= GF_TILES_FROM) {
-        rc = tile_launch(x, w, out, M, N, K, vec, stream);
-    } else if (N >= 16 * sms || M > 16) {
-        // 16 features a block where that still gives every SM one (or a tile of 32 tokens has work enough for a block)
-        rc = M <= 4 ? few_launch<16, 4, 4>(x, w, out, M, N, K, vec, sms, stream)
-           : M <= 8 ? few_launch<16, 8, 3>(x, w, out, M, N, K, vec, sms, stream)
-           : M <= 16 ? few_launch<16, 16, 3>(x, w, out, M, N, K, vec, sms, stream)
-                     : few_launch<16, 32, 3>(x, w, out, M, N, K, vec, sms, stream);
-    } else {
-        rc = M <= 4 ? few_launch<8, 4, 6>(x, w, out, M, N, K, vec, sms, stream)
-           : M <= 8 ? few_launch<8, 8, 6>(x, w, out, M, N, K, vec, sms, stream)
-                    : few_launch<8, 16, 4>(x, w, out, M, N, K, vec, sms, stream);
+    int tn = 64, split = 1;
+    float best = 1e30f;
+    if (M <= 16) split_cost<16>(M, N, K, sms, 0.95f, tn, split, best);
+    else {
+        split_cost<32>(M, N, K, sms, 0.95f, tn, split, best);
+        split_cost<64>(M, N, K, sms, 1.15f, tn, split, best);
     }
+    const int rc = tn == 16 ? split_launch<16>(x, w, out, M, N, K, rows, split, sms, stream)
+                 : tn == 32 ? split_launch<32>(x, w, out, M, N, K, rows, split, sms, stream)
+                            : split_launch<64>(x, w, out, M, N, K, rows, split, sms, stream);
     if (rc) return rc;
     IDM_LAUNCH_CHECK("gemm_f32");
     return 0;
 }
+
+#if defined(IDM_F32)
+// 0, or 1 if any block's bounded wait ran out since the last call (reads the flag: synchronises)
+extern "C" int idm_gemm_status() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_gemm_f32_error, sizeof(int)) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_gemm_f32_error, &zero, sizeof(int));
+    return v;
+}
+#endif

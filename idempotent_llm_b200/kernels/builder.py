@@ -31,8 +31,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]   # never --use_fast_math
 
-# sources per dtype: the 32-bit library carries the plain FMA matrix product,
-# the bfloat16 library the tensor-core kernels
+# sources per dtype: the 32-bit library carries the matrix product of operands split in three,
+# the bfloat16 library the kernels of operands that are bfloat16 themselves
 SOURCES: Dict[str, List[str]] = {
     "float32": ["runtime.cu", "elementwise.cu", "sampler.cu", "attention_generic.cu",
                 "attention_decode.cu", "short_conv.cu", "ssd_scan.cu", "head_finish.cu", "delta_rule.cu", "retention.cu", "differential.cu", "latent.cu", "experts.cu", "layer_norm.cu", "sum_norm.cu", "router.cu", "gemm_f32.cu"],

@@ -6,12 +6,12 @@ checks what the kernel cannot check itself and raises ``KernelError`` with the
 library's message when a launch is refused.  There is no CPU path: constructing
 ``Kernels`` without a CUDA device raises.
 
-Matrix products: the 32-bit library has its own FMA kernel (no tensor cores, no
+Matrix products: the 32-bit library splits its operands into three bfloat16 parts
+each and adds their products up to 32-bit precision (``csrc/gemm_f32.cu``; no
 reduced-precision mode).  In bfloat16 they run on the hand-written tcgen05
 kernels of ``csrc/gemm_tcgen05.cu`` (the reference sends every matrix product to
 a library, ``torch._int_mm``, src/detllm/backends.py:88-135).  No product is sent
-to a library here, and none is split over its inner axis: an element is one chain
-of additions whatever the step's size.
+to a library here, and an element is one sum in one order whatever the step's size.
 
 Environment switches (all default to the fast path): ``IDM_FUSED=0`` (epilogues as kernels of their
 own), ``IDM_ATTENTION=generic`` (the general attention kernel for every step), ``IDM_PDL=0`` (no
@@ -1015,8 +1015,8 @@ class Kernels:
         return bool(ran_out), int(cycles), bool(other)
 
     def gemm_status(self) -> int:
-        """0, or 1 if a bounded wait inside the tensor-core GEMM ran out since the last call (synchronises)."""
-        return 0 if self.dtype == torch.float32 else self.lib.idm_gemm_status()
+        """0, or 1 if a bounded wait inside a GEMM ran out since the last call (synchronises)."""
+        return self.lib.idm_gemm_status()
 
     # ---- a norm without statistics, one-argument activations, streams side by side, capped logits ----
     def _delta_args(self, delta, n, hidden):

@@ -521,10 +521,11 @@ def test_gemm_32_bit_is_true_32_bit_and_row_independent(kernels, M, N, K_):
     assert torch.equal(one[0, 0], out[0, M // 2]), "a row's result must not depend on the other rows"
 
 
-# few tokens on 8 and on 16 features a block; either side of the border to tiles (32 tokens; 200 tiles of 64 x 64); rows that do
-# not start on 16-byte borders; inner sizes behind one segment of 128, behind the eight classes, and that fill none
+# tiles of 16, 32 and 64 tokens, whole and not; a tile's segments of 64 k on one block and dealt out to two, three, four, six and eight; more
+# tiles than SMs; rows that do not start on 16-byte borders, that do but end inside a segment, that fill none
 @pytest.mark.parametrize("M,N,K_", [(4, 2367, 128), (9, 2400, 1153), (16, 100, 4100), (17, 33, 1025), (32, 12801, 132), (33, 12737, 260),
-                                    (65, 6401, 1029), (613, 1100, 2052), (200, 1100, 96)])
+                                    (65, 6401, 1029), (613, 1100, 2052), (200, 1100, 96), (1, 384, 3072), (8, 6144, 1024), (40, 640, 640),
+                                    (12, 3000, 384), (700, 1024, 192), (257, 9000, 68)])
 def test_gemm_32_bit_is_one_sum_in_every_kernel(kernels, M, N, K_):
     K = kernels("float32")
     x, w = _randn(M, K_, seed=74).float().cuda(), _randn(N, K_, seed=75).float().cuda()
@@ -534,6 +535,26 @@ def test_gemm_32_bit_is_one_sum_in_every_kernel(kernels, M, N, K_):
         assert torch.equal(K.gemm_store(x[m:m + 1].contiguous(), w)[0], out[m]), "a row's result must not depend on the other rows"
     half = K.gemm_store(x, w[:N // 2].contiguous())       # (fewer features: another kernel or tile for many of the sizes)
     assert torch.equal(half, out[:, :N // 2])
+
+
+@pytest.mark.parametrize("M,K_", [(5, 512), (40, 130), (700, 64)])
+def test_gemm_32_bit_with_numbers_that_have_no_parts(kernels, M, K_):
+    """Infinities, not-a-numbers and the ends of the range: what plain 32-bit sums give, and the neighbours' bits as without them."""
+    K = kernels("float32")
+    x, w = _randn(M, K_, seed=76).float().cuda(), _randn(200, K_, seed=77).float().cuda()
+    plain = K.gemm_store(x, w)
+    x2, w2 = x.clone(), w.clone()
+    x2[0, 3] = float("inf"); x2[1, 5] = float("nan"); x2[2] = 0.0; x2[2, 7] = 3.4e38; w2[9, 11] = -float("inf"); w2[:, 7] *= 0.01; w2[10] = 0.0
+    x2[3] = x2[3] * 1e-35
+    out, want = K.gemm_store(x2, w2), (x2.double() @ w2.double().T)
+    odd = ~torch.isfinite(want)
+    assert torch.equal(out[odd].isnan(), want[odd].isnan()) and torch.equal(out[odd].nan_to_num(0.0, 1.0, -1.0), want[odd].float().nan_to_num(0.0, 1.0, -1.0))
+    for row in (2, 3):                                     # (one product of 3.4e38 a sum; numbers of 1e-35, whose third parts still have an exponent)
+        keep = ~odd[row]
+        assert helpers.rel_err(out[row][keep], want[row][keep]) < 2e-6
+    w3 = w.clone(); w3[:, 7] *= 0.01                       # the same weight without the special numbers
+    assert torch.equal(out[4:, 11:], K.gemm_store(x, w3)[4:, 11:]) and torch.isfinite(plain).all()
+    assert K.gemm_status() == 0
 
 
 # Token counts on both sides of every border between kernels and tile shapes (16, 32, 64, 128 tokens on
