@@ -389,24 +389,27 @@ __device__ __forceinline__ float dot4(float s, float4 a, float4 b) {
 }
 
 // Few tokens per sequence (single tokens above all), keys of up to 128 in whole pieces of four: bound by the bytes of the state, so a
-// thread has eight 16-byte pieces of it on their way.  L lanes have a column (4 L channels), a warp 8 of them (times 32 / L); a column's
-// two sums go over its lanes by a butterfly.  64 single tokens, 32 heads of 128 x 64 (134 MB in and out): 
-// 22 us, 6.1 TB/s (55 us by the general walk).
+// thread has eight 16-byte pieces of it on their way.  L lanes have a column (4 L channels) and add its two sums up by a butterfly.
+// 64 single tokens, 32 heads of 128 x 64 (134 MB in and out): 22 us, 6.1 TB/s (55 us by the general walk).
+// A warp has COLS columns (times 32 / L): eight keep enough bytes on their way where the blocks fill the SMs, two where sequences
+// are few and it is the chain of loads, sums and stores that counts; a column's sums are the same either way.  A layer's step with
+// 1 / 4 / 16 single tokens takes 23.3 / 24.5 / 32.8 us (by the general walk 23.9 / 28.0 / 40.8).
 #define DT_COLS 8
-template <int L>
+#define DT_FILL 296                    // blocks of eight columns a warp: two an SM
+template <int L, int COLS>
 __global__ void __launch_bounds__(128, 5) delta_token_kernel(DeltaScanArgs a) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int SIDE = 32 / L;                                // columns side by side
     const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), lane = threadIdx.x & 31, ln = lane % L;
-    const int j0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * DT_COLS * SIDE + lane / L, d = ln * 4;
+    const int j0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * COLS * SIDE + lane / L, d = ln * 4;
     const bool in = d < a.dk;
     const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
     float* sp = a.state + (size_t)a.slots[s] * a.state_stride + (size_t)h * a.dv * a.dk + d;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 S[DT_COLS];
+    float4 S[COLS];
 #pragma unroll
-    for (int i = 0; i < DT_COLS; ++i) {
+    for (int i = 0; i < COLS; ++i) {
         const int j = j0 + i * SIDE;
         S[i] = in && j < a.dv ? *reinterpret_cast<const float4*>(sp + (size_t)j * a.dk) : zero;
     }
@@ -416,9 +419,9 @@ __global__ void __launch_bounds__(128, 5) delta_token_kernel(DeltaScanArgs a) {
         const float4 q = in ? *reinterpret_cast<const float4*>(row + a.c_q + hk * a.dk + d) : zero;
         const float4 g = in ? *reinterpret_cast<const float4*>(a.g + (size_t)t * a.g_stride + a.g_col + h * a.dk + d) : zero;
         const float beta = a.beta[(size_t)t * a.H + h];
-        float v[DT_COLS], ks[DT_COLS], qs[DT_COLS], kq = dot4(0.f, k, q);
+        float v[COLS], ks[COLS], qs[COLS], kq = dot4(0.f, k, q);
 #pragma unroll
-        for (int i = 0; i < DT_COLS; ++i) {
+        for (int i = 0; i < COLS; ++i) {
             const int j = j0 + i * SIDE;
             v[i] = j < a.dv ? row[a.c_v + h * a.dv + j] : 0.f;
             S[i] = make_float4(g.x * S[i].x, g.y * S[i].y, g.z * S[i].z, g.w * S[i].w);
@@ -429,31 +432,37 @@ __global__ void __launch_bounds__(128, 5) delta_token_kernel(DeltaScanArgs a) {
         for (int o = L / 2; o > 0; o >>= 1) {
             kq += __shfl_xor_sync(0xffffffffu, kq, o);
 #pragma unroll
-            for (int i = 0; i < DT_COLS; ++i) {
+            for (int i = 0; i < COLS; ++i) {
                 ks[i] += __shfl_xor_sync(0xffffffffu, ks[i], o);
                 qs[i] += __shfl_xor_sync(0xffffffffu, qs[i], o);
             }
         }
         float mine = 0.f;                                       // lane i of a column's lanes stores column i's read-out
 #pragma unroll
-        for (int i = 0; i < DT_COLS; ++i) {
+        for (int i = 0; i < COLS; ++i) {
             const float u = beta * (v[i] - ks[i]);
             S[i] = make_float4(fmaf(k.x, u, S[i].x), fmaf(k.y, u, S[i].y), fmaf(k.z, u, S[i].z), fmaf(k.w, u, S[i].w));
             if (ln == i) mine = fmaf(u, kq, qs[i]);
         }
         const int j = j0 + ln * SIDE;
-        if (ln < DT_COLS && j < a.dv) a.o[(size_t)t * a.o_stride + h * a.dv + j] = mine;
+        if (ln < COLS && j < a.dv) a.o[(size_t)t * a.o_stride + h * a.dv + j] = mine;
     }
 #pragma unroll
-    for (int i = 0; i < DT_COLS; ++i) {
+    for (int i = 0; i < COLS; ++i) {
         const int j = j0 + i * SIDE;
         if (in && j < a.dv) *reinterpret_cast<float4*>(sp + (size_t)j * a.dk) = S[i];
     }
 }
+template <int L, int COLS>
+static void delta_token_launch(const DeltaScanArgs& a, int n_seqs, cudaStream_t stream) {
+    constexpr int BLOCK = 4 * COLS * (32 / L);
+    idm_launch(delta_token_kernel<L, COLS>, dim3((a.dv + BLOCK - 1) / BLOCK, a.H, n_seqs), dim3(128), 0, stream, a);
+}
 template <int L>
 static void delta_token(const DeltaScanArgs& a, int n_seqs, cudaStream_t stream) {
-    constexpr int COLS = 4 * DT_COLS * (32 / L);
-    idm_launch(delta_token_kernel<L>, dim3((a.dv + COLS - 1) / COLS, a.H, n_seqs), dim3(128), 0, stream, a);
+    constexpr int BLOCK = 4 * DT_COLS * (32 / L);
+    if ((long long)((a.dv + BLOCK - 1) / BLOCK) * a.H * n_seqs >= DT_FILL) delta_token_launch<L, DT_COLS>(a, n_seqs, stream);
+    else delta_token_launch<L, 2>(a, n_seqs, stream);
 }
 
 // ------------------------------------------------------------------ the recurrence, thirty-two tokens at a time

@@ -123,15 +123,15 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
         const int ct = threadIdx.x - GX_ADD, row = ct >> 4, piece = ct & 15;
         float4 raw[2][S::ROUNDS];
         // rows behind the end are the last one again: their outputs are dropped
-        struct Where { int tile, seg; const float *w, *x; int dw[3], dx; };
+        struct Where { int tile, seg; const float *w, *x; int dw[3], dx; };     // (dw, dx: rows from there to this thread's others)
         auto place = [&](Where& p, int tile) {
             p.tile = tile; p.seg = rank;
             const int f = tile / token_tiles * GX_FEATURES + row, m = tile % token_tiles * TN + row, k = rank * GX_SEG + piece * 4;
             p.w = w + (size_t)min(f, N - 1) * K + k;
             p.x = x + (size_t)min(m, M - 1) * K + k;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) p.dw[i] = (min(f + 32 * (i + 1), N - 1) - min(f, N - 1)) * K;
-            p.dx = (min(m + 32, M - 1) - min(m, M - 1)) * K;
+            for (int i = 0; i < 3; ++i) p.dw[i] = min(f + 32 * (i + 1), N - 1) - min(f, N - 1);
+            p.dx = min(m + 32, M - 1) - min(m, M - 1);
         };
         auto step = [&](Where& p) {                                            // false behind the block's last segment
             p.seg += split;
@@ -157,11 +157,11 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
         auto load_w = [&](float4 (&v)[S::ROUNDS], const Where& p) {
             v[0] = load4k(p.w, p.seg);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) v[i + 1] = load4k(p.w + p.dw[i], p.seg);
+            for (int i = 0; i < 3; ++i) v[i + 1] = load4k(p.w + (long long)p.dw[i] * K, p.seg);
         };
         auto load_x = [&](float4 (&v)[S::ROUNDS], const Where& p) {
             if (TN >= 32 || row < TN) v[4] = load4k(p.x, p.seg);
-            if (TN > 32) v[S::ROUNDS - 1] = load4k(p.x + p.dx, p.seg);
+            if (TN > 32) v[S::ROUNDS - 1] = load4k(p.x + (long long)p.dx * K, p.seg);
         };
         if (blockIdx.x < tiles && rank < segs) {
             Where at;
@@ -340,7 +340,6 @@ template <int TN> static void split_cost(int M, int N, int K, int sms, float per
 extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
     IDM_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
-    IDM_REQUIRE(K < (1 << 24), "gemm_f32: rows of %d elements", K);               // (a tile's rows are reached by 32-bit offsets)
     const int rows = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

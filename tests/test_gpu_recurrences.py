@@ -180,6 +180,19 @@ def test_delta_single_tokens_against_64_bits_and_however_cut(K, dk, dv, pad):
         at += L
 
 
+def test_delta_single_tokens_are_the_same_bits_in_any_batch(K):
+    """Enough sequences for eight columns a warp, and one alone (two columns)."""
+    H, Hk, dk, dv, n = 16, 4, 128, 64, 20
+    c, g, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 55)
+    start = _randn(n, H * dv * dk, seed=56)
+    together = start.clone()
+    o = K.delta_scan(c, *cols, g, 0, beta, together, _ctx([3] * n, [1] * n), H, Hk, dk, dv)
+    for i in (0, 7, n - 1):
+        state = start[i:i + 1].clone()
+        one = K.delta_scan(c[i:i + 1].contiguous(), *cols, g[i:i + 1].contiguous(), 0, beta[i:i + 1].contiguous(), state, _ctx([3], [1]), H, Hk, dk, dv)
+        assert torch.equal(one[0], o[i]) and torch.equal(state[0], together[i])
+
+
 @pytest.mark.parametrize("head", [False, True])
 def test_delta_prep_and_out_on_and_off_16_byte_borders(K, head):
     """Rows shifted by one column take the element by element kernels: the same numbers up to the order of a norm's sum."""
