@@ -465,7 +465,7 @@ static void delta_token(const DeltaScanArgs& a, int n_seqs, cudaStream_t stream)
     else delta_token_launch<L, 2>(a, n_seqs, stream);
 }
 
-// ------------------------------------------------------------------ the recurrence, thirty-two tokens at a time
+// ------------------------------------------------------------------ the recurrence in chunks
 // Over a chunk of C tokens that starts from the state S0, with G_t the product of the decays up to and including
 // token t (per key channel), the walk above unrolls to
 //
@@ -473,40 +473,332 @@ static void delta_token(const DeltaScanArgs& a, int n_seqs, cudaStream_t stream)
 //   o_t  = S0^T (G_t q_t) + sum_{s<=t} B_ts u_s,                    B_ts = sum_d k_s[d] q_t[d] G_t[d] / G_s[d]
 //   S_C  = G_C S0 + sum_s (k_s G_C / G_s) u_s^T
 //
-// The u_t are a triangular system whose right-hand sides are v_t and, row by row of S0, G_t k_t: with X the solutions for
-// those, u = X_v - X_k S0.  So everything but S0 belongs to (chunk, head) and not to a column or to what came before:
-// delta_chunk_kernel makes it for all chunks side by side (X_k, X_v, G_t q_t, k_s G_C / G_s, B, G_C), and the chain that is
-// left (delta_walk_kernel) is products with S0 and with u.  The quotients G_t / G_s are never divided out: they are products
-// of the decays between s and t, in (0, 1] (inside half a chunk multiplied up from s, across its middle the product up to
-// the middle times the product from there), so a decay that underflows ends at 0 and nothing overflows.  All of it is
-// 32-bit; the numbers are those of the walk up to the order of the sums.
+// so that the work against the state becomes three products with C independent sums each instead of a chain of C dependent
+// steps.  The quotients G_t / G_s are never divided out: they are products of the decays between s and t, in (0, 1], so a
+// decay that underflows ends at 0 and nothing overflows.  All of it is 32-bit; the numbers are those of the walk up to the
+// order of the sums.  There are two forms (delta_split says which a step takes).
+
+// ---- chunks of 16, one chain: A and B belong to (chunk, head) and not to a column, so a pass of its own makes them for all
+// chunks side by side; the triangular system (the u_t, 16 unknowns per column) is solved on the chain's way, in registers.
+// It works on the tokens that are there, and its blocks of 65 KB share an SM: the form for steps that fill the SMs.
+#define CH_C 16                                                 // tokens per chunk
+
+// ab[(t H + h) 2C ..]: for token s of a chunk, -A_ts for the chunk's tokens t > s (0 elsewhere), then B_ts for t >= s
+__global__ void __launch_bounds__(128) delta_pairs_kernel(DeltaScanArgs a, float* __restrict__ ab) {
+    __shared__ float sm[3][CH_C][128];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), tid = threadIdx.x;
+    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1], tb = t0 + blockIdx.x * CH_C;
+    if (tb >= t1) return;
+    const int n = min(CH_C, t1 - tb);
+    for (int e = tid; e < n * a.dk; e += 128) {
+        const int tt = e / a.dk, d = e % a.dk;
+        const float* row = a.c + (size_t)(tb + tt) * a.c_stride + hk * a.dk + d;
+        sm[0][tt][d] = row[a.c_k];
+        sm[1][tt][d] = row[a.c_q];
+        sm[2][tt][d] = a.g[(size_t)(tb + tt) * a.g_stride + a.g_col + h * a.dk + d];
+    }
+    for (int e = tid; e < n * 2 * CH_C; e += 128)
+        ab[((size_t)(tb + e / (2 * CH_C)) * a.H + h) * (2 * CH_C) + e % (2 * CH_C)] = 0.f;
+    __syncthreads();
+    // a warp takes four tokens s whose rows together are as long as every other warp's; its lanes split the channels
+    const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll 1
+    for (int pass = 0; pass < 4; ++pass) {
+        const int ts = pass == 0 ? warp : pass == 1 ? 7 - warp : pass == 2 ? 8 + warp : 15 - warp;
+        if (ts >= n) continue;
+        float kr[4];                                            // k_s times the decays from s up to the token at hand
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kr[i] = lane + 32 * i < a.dk ? sm[0][ts][lane + 32 * i] : 0.f;
+        float* out = ab + ((size_t)(tb + ts) * a.H + h) * (2 * CH_C);
+        for (int t = ts; t < n; ++t) {
+            float pa = 0.f, pb = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int d = lane + 32 * i;
+                if (d < a.dk) {
+                    if (t > ts) kr[i] *= sm[2][t][d];
+                    pa = fmaf(sm[0][t][d], kr[i], pa);
+                    pb = fmaf(sm[1][t][d], kr[i], pb);
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                pa += __shfl_xor_sync(0xffffffffu, pa, o);
+                pb += __shfl_xor_sync(0xffffffffu, pb, o);
+            }
+            if (lane == 0) {
+                if (t > ts) out[t] = -pa;
+                out[CH_C + t] = pb;
+            }
+        }
+    }
+}
+
+// The chain: a block owns (sequence, head, 16 columns of S), a warp four of the columns, lane L rows
+// [L RP, (L + 1) RP) of each.  Four columns a warp, because what a warp reads from shared memory (a token's scaled k or
+// q) then serves four sums, and four independent chains keep one warp per scheduler busy.  Per chunk: (1) the threads
+// turn the staged k, q, g in place into k G_C / G_t, q G_t, k G_t, a thread per channel and group of tokens, the
+// groups' products joined through shared memory; (2) the warp lays its columns of S0 into shared memory, and lane t
+// sums S0^T (G_t k_t) for token t's correction, lane 16 + t S0^T (G_t q_t) for its read-out; (3) the triangular system
+// runs down the lanes: u_s goes from lane s to all, lane L adds row s's entry L of [-A | B] times u_s to its sum; (4)
+// lanes 16.. store the read-outs, all lanes bring their rows of S behind the chunk.
+#define CH_NC 4                                                 // columns per warp
+template <int RP>
+struct DeltaChain {
+    static constexpr int DKP = RP * 32, NT = DS_COLS / CH_NC * 32;
+    static constexpr int NG = NT / DKP < 1 ? 1 : NT / DKP;      // groups of tokens in step (1)
+    static constexpr int V_AT = 3 * DKP, BETA_AT = V_AT + DS_COLS, AB_AT = BETA_AT + 4;
+    static constexpr int ROW = AB_AT + 2 * CH_C;                // k, q, g, v of the block's columns, beta, -A and B
+    static constexpr int GC_AT = 2 * CH_C * ROW;                // the chunk's whole decay, behind the two stages
+    static constexpr int GP_AT = GC_AT + DKP;                   // the token groups' decays
+    static constexpr int SW_AT = GP_AT + NG * DKP;              // the block's columns of S
+    static constexpr int FLOATS = SW_AT + DS_COLS * DKP;
+    static_assert(DKP <= NT && CH_C % NG == 0, "a thread per channel, whole groups of tokens");
+};
+
+template <int RP>
+__device__ __forceinline__ void load_rows(const float* p, float (&x)[RP]) {
+    if constexpr (RP == 4) { const float4 v = *reinterpret_cast<const float4*>(p); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+    else if constexpr (RP == 2) { const float2 v = *reinterpret_cast<const float2*>(p); x[0] = v.x; x[1] = v.y; }
+    else x[0] = *p;
+}
+
+template <int RP, bool VEC>
+__global__ void __launch_bounds__(DeltaChain<RP>::NT) delta_chain_kernel(DeltaScanArgs a, const float* __restrict__ ab) {
+    using L = DeltaChain<RP>;
+    constexpr int C = CH_C, NT = L::NT, NC = CH_NC, NW = NT / 32;
+    extern __shared__ __align__(16) float ds_smem[];
+    pdl_launch_dependents();
+    const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j0 = blockIdx.x * DS_COLS, jw = warp * NC;
+    const int row0 = lane * RP;
+    for (int e = tid; e < 2 * C * L::DKP; e += NT) {            // channels past dk: k = q = 0, g = 1, never copied
+        const int row = e / L::DKP, p = e % L::DKP;
+        if (p >= a.dk) {
+            float* base = ds_smem + row * L::ROW;
+            base[p] = 0.f; base[L::DKP + p] = 0.f; base[2 * L::DKP + p] = 1.f;
+        }
+    }
+    pdl_wait();
+    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
+    float* sp = a.state + (size_t)a.slots[s] * a.state_stride + ((size_t)h * a.dv + j0 + jw) * a.dk + row0;
+    float S[NC][RP];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int i = 0; i < RP; ++i) S[c][i] = (j0 + jw + c < a.dv && row0 + i < a.dk) ? sp[(size_t)c * a.dk + i] : 0.f;
+
+    const int cols = min(DS_COLS, a.dv - j0);
+    auto issue = [&](int tb, int stage) {
+        const int n = min(C, t1 - tb);
+        for (int tt = warp; tt < n; tt += NW) {
+            const int t = tb + tt;
+            float* row = ds_smem + (stage * C + tt) * L::ROW;
+            const float* kp = a.c + (size_t)t * a.c_stride + hk * a.dk;
+            const float* gp = a.g + (size_t)t * a.g_stride + a.g_col + h * a.dk;
+            if (VEC) {
+                for (int d = lane * 4; d < a.dk; d += 128) {
+                    cp_async_16(row + d, kp + a.c_k + d);
+                    cp_async_16(row + L::DKP + d, kp + a.c_q + d);
+                    cp_async_16(row + 2 * L::DKP + d, gp + d);
+                }
+            } else {
+                for (int d = lane; d < a.dk; d += 32) {
+                    cp_async_4(row + d, kp + a.c_k + d);
+                    cp_async_4(row + L::DKP + d, kp + a.c_q + d);
+                    cp_async_4(row + 2 * L::DKP + d, gp + d);
+                }
+            }
+            if (lane < cols) cp_async_4(row + L::V_AT + lane, a.c + (size_t)t * a.c_stride + a.c_v + h * a.dv + j0 + lane);
+            else if (lane == 16) cp_async_4(row + L::BETA_AT, a.beta + (size_t)t * a.H + h);
+            else if (lane >= 24) cp_async_16(row + L::AB_AT + (lane - 24) * 4, ab + ((size_t)t * a.H + h) * (2 * C) + (lane - 24) * 4);
+        }
+        cp_async_commit();
+    };
+
+    const int n_chunks = (t1 - t0 + C - 1) / C;
+    if (n_chunks > 0) issue(t0, 0);
+    for (int ch = 0; ch < n_chunks; ++ch) {
+        const int tb = t0 + ch * C;
+        if (ch + 1 < n_chunks) { issue(tb + C, (ch + 1) & 1); cp_async_wait<1>(); }
+        else cp_async_wait<0>();
+        float* st = ds_smem + (ch & 1) * C * L::ROW;
+        const int n = min(C, t1 - tb);
+        // a last chunk of fewer tokens: the missing ones write nothing (k = 0, beta = 0) and decay nothing (g = 1)
+        for (int e = tid; e < (C - n) * L::ROW; e += NT) {
+            const int c = e % L::ROW;
+            st[(n + e / L::ROW) * L::ROW + c] = (c >= 2 * L::DKP && c < 3 * L::DKP) ? 1.f : 0.f;
+        }
+        __syncthreads();
+        // (1) in place, per channel: k -> k G_C / G_t, q -> q G_t, g -> k G_t; and G_C.  Thread (channel, group of tokens).
+        {
+            constexpr int TPG = C / L::NG;
+            const int p = tid % L::DKP, grp = tid / L::DKP;
+            float gg[TPG], kk[TPG], qq[TPG];
+            if (grp < L::NG) {
+                float prod = 1.f;
+#pragma unroll
+                for (int i = 0; i < TPG; ++i) {
+                    const float* row = st + (TPG * grp + i) * L::ROW;
+                    gg[i] = row[2 * L::DKP + p]; kk[i] = row[p]; qq[i] = row[L::DKP + p];
+                    prod *= gg[i];
+                }
+                if (L::NG > 1) ds_smem[L::GP_AT + grp * L::DKP + p] = prod;
+            }
+            if (L::NG > 1) __syncthreads();
+            if (grp < L::NG) {
+                float G = 1.f, suf = 1.f;
+                if (L::NG > 1) {
+#pragma unroll
+                    for (int o = 0; o < L::NG; ++o) {
+                        const float x = ds_smem[L::GP_AT + o * L::DKP + p];
+                        if (o < grp) G *= x;
+                        if (o > grp) suf *= x;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < TPG; ++i) {
+                    float* row = st + (TPG * grp + i) * L::ROW;
+                    G *= gg[i];
+                    row[2 * L::DKP + p] = kk[i] * G;
+                    row[L::DKP + p] = qq[i] * G;
+                }
+                if (grp == L::NG - 1) ds_smem[L::GC_AT + p] = G;
+#pragma unroll
+                for (int i = TPG - 1; i >= 0; --i) {
+                    st[(TPG * grp + i) * L::ROW + p] = kk[i] * suf;
+                    suf *= gg[i];
+                }
+            }
+        }
+        __syncthreads();
+        // (2) what the state before the chunk gives token t's correction (lane t) and read-out (lane 16 + t): the columns
+        // go through shared memory, and a lane walks all of them against its token's G_t k_t or G_t q_t
+        float x[NC];
+        {
+            float* sw = ds_smem + L::SW_AT + jw * L::DKP;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                if constexpr (RP == 4) *reinterpret_cast<float4*>(sw + c * L::DKP + row0) = make_float4(S[c][0], S[c][1], S[c][2], S[c][3]);
+                else if constexpr (RP == 2) *reinterpret_cast<float2*>(sw + c * L::DKP + row0) = make_float2(S[c][0], S[c][1]);
+                else sw[c * L::DKP + row0] = S[c][0];
+            }
+            __syncwarp();
+            const float* xr = st + (lane & 15) * L::ROW + (lane < 16 ? 2 * L::DKP : L::DKP);
+            float acc[NC][4];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
+#pragma unroll 8
+            for (int m = 0; m < L::DKP / 4; ++m) {
+                const float4 xv = *reinterpret_cast<const float4*>(xr + 4 * m);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float4 sv = *reinterpret_cast<const float4*>(sw + c * L::DKP + 4 * m);
+                    acc[c][0] = fmaf(xv.x, sv.x, acc[c][0]); acc[c][1] = fmaf(xv.y, sv.y, acc[c][1]);
+                    acc[c][2] = fmaf(xv.z, sv.z, acc[c][2]); acc[c][3] = fmaf(xv.w, sv.w, acc[c][3]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) x[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
+        }
+        // (3) lane t < 16: v_t minus the sum, times beta_t when its turn comes; lane 16 + t: the read-out so far
+        float u[NC][C];
+        const float* mine = st + (lane & 15) * L::ROW;
+        const float beta = lane < 16 ? mine[L::BETA_AT] : 0.f;
+        if (lane < 16) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) x[c] = (j0 + jw + c < a.dv ? mine[L::V_AT + jw + c] : 0.f) - x[c];
+        }
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const float coef = st[q * L::ROW + L::AB_AT + lane];
+            const bool behind = lane < 16 ? lane > q : lane - 16 >= q;      // (the tokens before q are not touched, whatever u_q is)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                u[c][q] = __shfl_sync(0xffffffffu, beta * x[c], q);
+                if (behind) x[c] = fmaf(coef, u[c][q], x[c]);
+            }
+        }
+        if (lane >= 16 && lane - 16 < n) {
+            float* dst = a.o + (size_t)(tb + lane - 16) * a.o_stride + h * a.dv + j0 + jw;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (j0 + jw + c < a.dv) dst[c] = x[c];
+        }
+        // (4) the state behind the chunk
+        {
+            float gc[RP];
+            load_rows<RP>(ds_smem + L::GC_AT + row0, gc);
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int i = 0; i < RP; ++i) S[c][i] *= gc[i];
+        }
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+            float kt[RP];
+            load_rows<RP>(st + t * L::ROW + row0, kt);
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int i = 0; i < RP; ++i) S[c][i] = fmaf(kt[i], u[c][t], S[c][i]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int i = 0; i < RP; ++i)
+            if (j0 + jw + c < a.dv && row0 + i < a.dk) sp[(size_t)c * a.dk + i] = S[c][i];
+}
+
+template <int RP>
+static int delta_scan_chain(const DeltaScanArgs& a, float* ab, dim3 grid, int max_tokens, cudaStream_t stream) {
+    const size_t smem = (size_t)DeltaChain<RP>::FLOATS * sizeof(float);
+    const bool vec = a.dk % 4 == 0 && a.c_stride % 4 == 0 && a.c_q % 4 == 0 && a.c_k % 4 == 0 && a.g_stride % 4 == 0 &&
+                     a.g_col % 4 == 0 && ((uintptr_t)a.c & 15) == 0 && ((uintptr_t)a.g & 15) == 0;
+    const cudaError_t e = vec ? cudaFuncSetAttribute(delta_chain_kernel<RP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                              : cudaFuncSetAttribute(delta_chain_kernel<RP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    IDM_REQUIRE(e == cudaSuccess, "delta_scan: %zu bytes of shared memory were refused (%s)", smem, cudaGetErrorString(e));
+    idm_launch(delta_pairs_kernel, dim3((max_tokens + CH_C - 1) / CH_C, grid.y, grid.z), dim3(128), 0, stream, a, ab);
+    if (vec) idm_launch(delta_chain_kernel<RP, true>, grid, dim3(DeltaChain<RP>::NT), smem, stream, a, (const float*)ab);
+    else idm_launch(delta_chain_kernel<RP, false>, grid, dim3(DeltaChain<RP>::NT), smem, stream, a, (const float*)ab);
+    return 0;
+}
+
+// ---- chunks of 32, split: the u_t are a triangular system whose right-hand sides are v_t and, row by row of S0, G_t k_t: with X
+// the solutions for those, u = X_v - X_k S0.  So everything but S0 belongs to (chunk, head) and not to a column or to what came
+// before: delta_chunk_kernel makes it for all chunks side by side (X_k, X_v, G_t q_t, k_s G_C / G_s, B, G_C), and the chain that is
+// left (delta_walk_kernel) is products with S0 and with u.  (The decays between s and t: inside half a chunk multiplied up from s,
+// across its middle the product up to the middle times the product from there.)  A walk's block has an SM to itself.
 //
-// A prompt of 2 048 tokens, 32 heads of 128 x 64: 257 us the chunks (two windows), 230 the walk;
-// the walk of chunks of 16 that did it all in one chain took 408 + 75 for its pairs.
+// A prompt of 2 048 tokens, 32 heads of 128 x 64: 257 us the chunks (two windows), 230 the walk; the chain of chunks of 16 takes
+// 408 + 75 for its pairs.
 #define DC_C 32                                                 // tokens per chunk
 #define DC_H (DC_C / 2)
 #define DC_THREADS 256
+#define DC_DKP 128                                              // channels of a key's row, rounded up (keys of 65 to 128)
 #define DC_ROW 36                                               // a row of C numbers in shared memory and scratch
-template <int DKP>
 struct DeltaChunk {
-    static constexpr int LD = DKP + 4;                          // a row of channels: eight rows' 16-byte reads in different places
+    static constexpr int LD = DC_DKP + 4;                          // a row of channels: eight rows' 16-byte reads in different places
     // a chunk's numbers in scratch, in floats: X_k, G q, k G_C / G (each [C][LD]), B [C][DC_ROW], G_C, then X_v by groups of 16 columns
     static constexpr int TILE = DC_C * LD;
-    static constexpr int B_AT = 3 * TILE, GC_AT = B_AT + DC_C * DC_ROW, XV_AT = GC_AT + DKP;
+    static constexpr int B_AT = 3 * TILE, GC_AT = B_AT + DC_C * DC_ROW, XV_AT = GC_AT + DC_DKP;
     static constexpr int XV = DC_C * DS_COLS;
     static constexpr int BUF = XV_AT + XV;                      // a stage of the walk: one group of columns
-    static constexpr int CHUNK_SMEM = (3 * TILE + 2 * DC_C * DC_ROW + 2 * DKP + DC_C) * 4;
+    static constexpr int CHUNK_SMEM = (3 * TILE + 2 * DC_C * DC_ROW + 2 * DC_DKP + DC_C) * 4;
     static constexpr int WALK_SMEM = (2 * BUF + DS_COLS * LD + DC_C * (DS_COLS + 4)) * 4;
 };
-__host__ __device__ __forceinline__ int delta_chunk_floats(int dkp, int dv) {
-    return 3 * DC_C * (dkp + 4) + DC_C * DC_ROW + dkp + (dv + DS_COLS - 1) / DS_COLS * DC_C * DS_COLS;
+__host__ __device__ __forceinline__ int delta_chunk_floats(int dv) {
+    return 3 * DC_C * (DC_DKP + 4) + DC_C * DC_ROW + DC_DKP + (dv + DS_COLS - 1) / DS_COLS * DC_C * DS_COLS;
 }
 
 // Chunks first, first + 1, ... (gridDim.x of them) of every sequence and head; chunk c of sequence s goes to scratch + (s * gridDim.x + c -
 // first) * H + h.
-template <int DKP>
 __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArgs a, float* __restrict__ scratch, int first) {
-    using L = DeltaChunk<DKP>;
+    using L = DeltaChunk;
     constexpr int C = DC_C, LD = L::LD;
     extern __shared__ __align__(16) float ds_smem[];
     pdl_launch_dependents();
@@ -516,18 +808,18 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
     float* sg = sq + L::TILE;                                   // the decays; then k times the decays up to it in its half
     float* sA = sg + L::TILE;                                   // [t][s]
     float* sB = sA + C * DC_ROW;
-    float* sG = sB + C * DC_ROW;                                // the halves' whole decays [2][DKP]
-    float* sbeta = sG + 2 * DKP;
+    float* sG = sB + C * DC_ROW;                                // the halves' whole decays [2][DC_DKP]
+    float* sbeta = sG + 2 * DC_DKP;
     const int s = blockIdx.z, h = blockIdx.y, hk = h / (a.H / a.Hk), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t1 = a.cu_q[s + 1], tb = a.cu_q[s] + (first + (int)blockIdx.x) * C;
     if (tb >= t1) return;
     const int n = min(C, t1 - tb);
-    float* out = scratch + (((size_t)s * gridDim.x + blockIdx.x) * a.H + h) * delta_chunk_floats(DKP, a.dv);
+    float* out = scratch + (((size_t)s * gridDim.x + blockIdx.x) * a.H + h) * delta_chunk_floats(a.dv);
 
     // missing tokens and channels write nothing (k = q = 0, beta = 0) and decay nothing (g = 1)
 #pragma unroll 4
-    for (int e = tid; e < C * DKP; e += DC_THREADS) {
-        const int t = e / DKP, d = e % DKP;
+    for (int e = tid; e < C * DC_DKP; e += DC_THREADS) {
+        const int t = e / DC_DKP, d = e % DC_DKP;
         const bool in = t < n && d < a.dk;
         const float* row = a.c + (size_t)(tb + t) * a.c_stride + hk * a.dk + d;
         sk[t * LD + d] = in ? row[a.c_k] : 0.f;
@@ -543,7 +835,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
         const int base = (i & 1) * DC_H, ts = base + (i < 2 ? warp : DC_H - 1 - warp);
-        constexpr int PER = DKP / 32;
+        constexpr int PER = DC_DKP / 32;
         float kr[PER];
 #pragma unroll
         for (int m = 0; m < PER; ++m) kr[m] = sk[ts * LD + lane + 32 * m];
@@ -565,8 +857,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
     }
     __syncthreads();
     // in place, a thread per channel and half: k behind, q and k up to a token
-    for (int e = tid; e < 2 * DKP; e += DC_THREADS) {
-        const int p = e % DKP, t0 = e / DKP * DC_H;
+    for (int e = tid; e < 2 * DC_DKP; e += DC_THREADS) {
+        const int p = e % DC_DKP, t0 = e / DC_DKP * DC_H;
         float g[DC_H], k[DC_H], G = 1.f, suf = 1.f;
 #pragma unroll
         for (int i = 0; i < DC_H; ++i) {
@@ -585,7 +877,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
         const int tile = tid >> 2, kg = tid & 3, tr = DC_H + (tile >> 3) * 2, sr = (tile & 7) * 2;
         float pa[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, pb[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 4
-        for (int d = kg * 4; d < DKP; d += 16) {
+        for (int d = kg * 4; d < DC_DKP; d += 16) {
             float4 k4[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) k4[j] = *reinterpret_cast<const float4*>(sk + (sr + j) * LD + d);
@@ -611,22 +903,22 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
     }
     __syncthreads();
     // what needs no solving goes out: G q, k G_C / G, B, G_C
-    for (int e = tid; e < C * DKP; e += DC_THREADS) {
-        const int t = e / DKP, d = e % DKP;
+    for (int e = tid; e < C * DC_DKP; e += DC_THREADS) {
+        const int t = e / DC_DKP, d = e % DC_DKP;
         out[L::TILE + t * LD + d] = sq[t * LD + d] * (t < DC_H ? 1.f : sG[d]);
-        out[2 * L::TILE + t * LD + d] = sk[t * LD + d] * (t < DC_H ? sG[DKP + d] : 1.f);
+        out[2 * L::TILE + t * LD + d] = sk[t * LD + d] * (t < DC_H ? sG[DC_DKP + d] : 1.f);
     }
     for (int e = tid; e < C * DC_ROW; e += DC_THREADS) out[L::B_AT + e] = sB[e];
-    for (int e = tid; e < DKP; e += DC_THREADS) out[L::GC_AT + e] = sG[e] * sG[DKP + e];
+    for (int e = tid; e < DC_DKP; e += DC_THREADS) out[L::GC_AT + e] = sG[e] * sG[DC_DKP + e];
     // the triangular system, a thread per right-hand side: channels of G k, then columns of v
     const int vcols = (a.dv + DS_COLS - 1) / DS_COLS * DS_COLS;
-    for (int col = tid; col < DKP + vcols; col += DC_THREADS) {
-        const int j = col - DKP;
+    for (int col = tid; col < DC_DKP + vcols; col += DC_THREADS) {
+        const int j = col - DC_DKP;
         float x[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) {
             float r;
-            if (col < DKP) r = sg[t * LD + col] * (t < DC_H ? 1.f : sG[col]);
+            if (col < DC_DKP) r = sg[t * LD + col] * (t < DC_H ? 1.f : sG[col]);
             else r = t < n && j < a.dv ? a.c[(size_t)(tb + t) * a.c_stride + a.c_v + h * a.dv + j] : 0.f;
             float sum[2] = {0.f, 0.f};
 #pragma unroll
@@ -639,8 +931,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
             }
             x[t] = sbeta[t] * (r - (sum[0] + sum[1]));
         }
-        float* dst = col < DKP ? out + col : out + L::XV_AT + j / DS_COLS * L::XV + j % DS_COLS;
-        const int step = col < DKP ? LD : DS_COLS;
+        float* dst = col < DC_DKP ? out + col : out + L::XV_AT + j / DS_COLS * L::XV + j % DS_COLS;
+        const int step = col < DC_DKP ? LD : DS_COLS;
 #pragma unroll
         for (int t = 0; t < C; ++t) dst[t * step] = x[t];
     }
@@ -650,9 +942,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_kernel(DeltaScanArg
 // transposed in shared memory, a chunk's numbers come by asynchronous copies one chunk ahead.  Per chunk: (1) X_k S0 and (G q) S0, 64 x
 // 16 sums in tiles of 4 x 4, four threads a tile with every fourth piece of four channels; u = X_v - X_k S0 to shared memory; (2) half of
 // the block brings S behind the chunk, the other half adds B u to its read-outs and stores them.
-template <int DKP>
 __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a, const float* __restrict__ scratch, int first, int count) {
-    using L = DeltaChunk<DKP>;
+    using L = DeltaChunk;
     constexpr int C = DC_C, LD = L::LD, LU = DS_COLS + 4;
     extern __shared__ __align__(16) float ds_smem[];
     pdl_launch_dependents();
@@ -663,7 +954,7 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
     const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1];
     const int chunks = min(count, (t1 - t0 + C - 1) / C - first);
     if (chunks <= 0) return;
-    const size_t per = delta_chunk_floats(DKP, a.dv);
+    const size_t per = delta_chunk_floats(a.dv);
     const float* src = scratch + ((size_t)s * count * a.H + h) * per;
     auto issue = [&](int ch) {
         const float* from = src + (size_t)ch * a.H * per;
@@ -675,8 +966,8 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
     issue(0);
     float* sp = a.state + (size_t)a.slots[s] * a.state_stride + ((size_t)h * a.dv + j0) * a.dk;
     const int cols = min(DS_COLS, a.dv - j0);
-    for (int e = tid; e < DS_COLS * DKP; e += DC_THREADS) {
-        const int j = e / DKP, d = e % DKP;
+    for (int e = tid; e < DS_COLS * DC_DKP; e += DC_THREADS) {
+        const int j = e / DC_DKP, d = e % DC_DKP;
         sS[j * LD + d] = j < cols && d < a.dk ? sp[(size_t)j * a.dk + d] : 0.f;
     }
     const int tile = tid >> 2, kg = tid & 3, row = (tile >> 2) * 4, col = (tile & 3) * 4;     // rows 0..31 of X_k, 32..63 of G q
@@ -691,7 +982,7 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll 4
-        for (int d = kg * 4; d < DKP; d += 16) {
+        for (int d = kg * 4; d < DC_DKP; d += 16) {
             float4 x4[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) x4[i] = *reinterpret_cast<const float4*>(st + (row + i) * LD + d);   // (G q lies right behind X_k)
@@ -718,9 +1009,9 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
         }
         __syncthreads();                                        // u is there, everyone has read S
         if (row < C) {
-            // S <- G_C S + (k G_C / G)^T u: four channels and DKP / 32 columns a thread
-            constexpr int NC = DKP / 32;
-            const int d = tid % (DKP / 4) * 4, c0 = tid / (DKP / 4) * NC;
+            // S <- G_C S + (k G_C / G)^T u: four channels and DC_DKP / 32 columns a thread
+            constexpr int NC = DC_DKP / 32;
+            const int d = tid % (DC_DKP / 4) * 4, c0 = tid / (DC_DKP / 4) * NC;
             float4 n4[NC];
             const float4 gc = *reinterpret_cast<const float4*>(st + L::GC_AT + d);
 #pragma unroll
@@ -763,39 +1054,53 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
         }
         __syncthreads();                                        // S is behind the chunk; its numbers' place is free
     }
-    for (int e = tid; e < DS_COLS * DKP; e += DC_THREADS) {
-        const int j = e / DKP, d = e % DKP;
+    for (int e = tid; e < DS_COLS * DC_DKP; e += DC_THREADS) {
+        const int j = e / DC_DKP, d = e % DC_DKP;
         if (j < cols && d < a.dk) sp[(size_t)j * a.dk + d] = sS[j * LD + d];
     }
 }
 
+// Which form a step of more than 4 tokens takes: split where the walk's blocks (an SM each) all run at once, the longest portion has more
+// than four chunks of 32, and the keys are wider than 64; else the chain.  Measured, us of the chain / split, keys of 128, values of 64:
+//   one sequence, 32 heads (128 blocks): 32 tokens 24 / 31, 64 30 / 34, 128 47 / 42, 256 92 / 57, 1 024 245 / 246, 2 048 538 / 487, 8 192
+//   1 914 / 1 889; 4 heads: 64 28 / 31, 128 41 / 38, 256 66 / 51, 2 048 425 / 245, 8 192 1 670 / 1 002;
+//   more blocks than SMs: 48 heads (192 blocks) 512 tokens 181 / 215, 64 heads 215 / 250, 2 048 769 / 974; 3 x 1 500 tokens of 64 heads
+//   1 394 / 2 263; 8 x 40 120 / 276; 2 048 tokens of 32 heads among 60 single tokens 921 / 3 756;
+//   keys of 64, 32 heads: 512 tokens 171 / 117, 1 024 198 / 241, 4 096 772 / 1 032.
+static bool delta_split(int n_seqs, int H, int dk, int dv, int max_tokens) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return dk > 64 && max_tokens > 4 * DC_C && (long long)n_seqs * H * ((dv + DS_COLS - 1) / DS_COLS) <= sms;
+}
+
 // Chunks of a launch: as many of every sequence as fit 18 M floats of scratch (a chunk of one head of 128 x 64 is 64 KB, so that a long
-// prompt's numbers are read again while they are in the L2), at least one.  The state carries over from launch to launch.
+// prompt's numbers are read again while they are in the L2), at least one (delta_split: sequences times heads are no more than the SMs).
+// The state carries over from launch to launch.
 #define DC_SCRATCH (18ll << 20)
-static int delta_window(int n_seqs, int H, int dkp, int dv, int max_tokens) {
-    const long long fit = DC_SCRATCH / ((long long)n_seqs * H * delta_chunk_floats(dkp, dv)), all = (max_tokens + DC_C - 1) / DC_C;
+static int delta_window(int n_seqs, int H, int dv, int max_tokens) {
+    const long long fit = DC_SCRATCH / ((long long)n_seqs * H * delta_chunk_floats(dv)), all = (max_tokens + DC_C - 1) / DC_C;
     return (int)(fit < 1 ? 1 : fit < all ? fit : all);
 }
-static int delta_dkp(int dk) { return dk <= 32 ? 32 : dk <= 64 ? 64 : 128; }
 
-template <int DKP>
-static int delta_scan_chunked(const DeltaScanArgs& a, float* scratch, int n_seqs, int max_tokens, cudaStream_t stream) {
-    using L = DeltaChunk<DKP>;
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::CHUNK_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::WALK_SMEM);
+static int delta_scan_split(const DeltaScanArgs& a, float* scratch, int n_seqs, int max_tokens, cudaStream_t stream) {
+    using L = DeltaChunk;
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::CHUNK_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::WALK_SMEM);
     IDM_REQUIRE(e == cudaSuccess, "delta_scan: %d bytes of shared memory were refused (%s)", L::WALK_SMEM, cudaGetErrorString(e));
-    const int window = delta_window(n_seqs, a.H, DKP, a.dv, max_tokens), groups = (a.dv + DS_COLS - 1) / DS_COLS;
+    const int window = delta_window(n_seqs, a.H, a.dv, max_tokens), groups = (a.dv + DS_COLS - 1) / DS_COLS;
     for (int first = 0; first * DC_C < max_tokens; first += window) {
-        idm_launch(delta_chunk_kernel<DKP>, dim3(window, a.H, n_seqs), dim3(DC_THREADS), L::CHUNK_SMEM, stream, a, scratch, first);
-        idm_launch(delta_walk_kernel<DKP>, dim3(groups, a.H, n_seqs), dim3(DC_THREADS), L::WALK_SMEM, stream, a, (const float*)scratch, first, window);
+        idm_launch(delta_chunk_kernel, dim3(window, a.H, n_seqs), dim3(DC_THREADS), L::CHUNK_SMEM, stream, a, scratch, first);
+        idm_launch(delta_walk_kernel, dim3(groups, a.H, n_seqs), dim3(DC_THREADS), L::WALK_SMEM, stream, a, (const float*)scratch, first, window);
     }
     return 0;
 }
 
-// Floats of scratch that a step of `n_seqs` sequences, at most `max_tokens` of one of them, wants (0: none).
-extern "C" long long idm_delta_scan_scratch_floats(int n_seqs, int H, int dk, int dv, int max_tokens) {
+// Floats of scratch that a step of `n_seqs` sequences and `n_tokens` tokens, at most `max_tokens` of one sequence, wants (0: none).
+extern "C" long long idm_delta_scan_scratch_floats(int n_seqs, int n_tokens, int H, int dk, int dv, int max_tokens) {
     if (max_tokens <= 4 || dk <= 0 || dk > 128 || dv <= 0 || n_seqs <= 0 || H <= 0) return 0;
-    return (long long)n_seqs * H * delta_window(n_seqs, H, delta_dkp(dk), dv, max_tokens) * delta_chunk_floats(delta_dkp(dk), dv);
+    if (!delta_split(n_seqs, H, dk, dv, max_tokens)) return (long long)n_tokens * H * 2 * CH_C;
+    return (long long)n_seqs * H * delta_window(n_seqs, H, dv, max_tokens) * delta_chunk_floats(dv);
 }
 
 // `max_tokens`: the most tokens any sequence brings to this step; steps of a few tokens walk them straight from
@@ -816,9 +1121,9 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
     const dim3 grid((dv + DS_COLS - 1) / DS_COLS, H, n_seqs), block(DS_COLS * 8);
     if (max_tokens > 4 && dk <= 128 && scratch != nullptr) {
         IDM_REQUIRE(((uintptr_t)scratch & 15) == 0, "delta_scan: scratch at %p", (void*)scratch);
-        const int rc = dk <= 32 ? delta_scan_chunked<32>(a, scratch, n_seqs, max_tokens, stream)
-                     : dk <= 64 ? delta_scan_chunked<64>(a, scratch, n_seqs, max_tokens, stream)
-                                : delta_scan_chunked<128>(a, scratch, n_seqs, max_tokens, stream);
+        const int rc = delta_split(n_seqs, H, dk, dv, max_tokens) ? delta_scan_split(a, scratch, n_seqs, max_tokens, stream)
+                     : dk <= 32 ? delta_scan_chain<1>(a, scratch, grid, max_tokens, stream)
+                     : dk <= 64 ? delta_scan_chain<2>(a, scratch, grid, max_tokens, stream) : delta_scan_chain<4>(a, scratch, grid, max_tokens, stream);
         if (rc) return rc;
     } else if (max_tokens > 4) {
         int rc;

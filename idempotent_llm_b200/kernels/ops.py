@@ -74,7 +74,7 @@ SIGNATURES = {
     "idm_cols_cast": (c_int, "piiipiip"),
     "idm_delta_prep": (c_int, "piiipiipiiipppiiiip"),
     "idm_delta_scan": (c_int, "piiiipiippqpippiiiiiipp"),
-    "idm_delta_scan_scratch_floats": (c_longlong, "iiiii"),
+    "idm_delta_scan_scratch_floats": (c_longlong, "iiiiii"),
     "idm_delta_out": (c_int, "pipfpiiifpiiiiip"),
     "idm_add_rmsnorm2": (c_int, "ppiqppfpppiip"),
     "idm_gemm_bf16_gated": (c_int, "pppiiiip"),
@@ -542,7 +542,7 @@ class Kernels:
         returns the read-outs ``[N, H * dv]`` in 32-bit."""
         n = c.shape[0]
         o = torch.empty((n, H * dv), dtype=torch.float32, device=self.device)
-        want = int(self.lib.idm_delta_scan_scratch_floats(ctx.n_seqs, H, dk, dv, int(ctx.max_q_len)))
+        want = int(self.lib.idm_delta_scan_scratch_floats(ctx.n_seqs, n, H, dk, dv, int(ctx.max_q_len)))
         scratch = torch.empty((want,), dtype=torch.float32, device=self.device) if want else None
         self._check(self.lib.idm_delta_scan(_p(c), c.shape[1], c_q, c_k, c_v, _p(g), g.shape[1], g_col, _p(beta), _p(state),
                                             self._state_stride(state), _p(o), H * dv, _p(ctx.cu_q), _p(ctx.slots),

@@ -155,6 +155,44 @@ def test_delta_chunks_against_64_bits(K, lens, H, Hk, dk, dv, pad):
     assert torch.equal(o2[:lens[0] - 1], o[:lens[0] - 1])
 
 
+# chunks of 32 split from the state (one sequence: 32 blocks) and the chain of chunks of 16 (six of them, 192 blocks): portions of one
+# token more than the border between them, with and without a chunk's rest, keys at and below 128, keys that lie close together
+@pytest.mark.parametrize("L,dk,dv,pad,close", [(129, 128, 64, 0, 0.0), (160, 100, 64, 1, 0.0), (201, 128, 64, 0, 0.1), (257, 72, 56, 4, 0.3)])
+def test_delta_forms_in_64_bits_and_beside_one_another(K, L, dk, dv, pad, close):
+    H, Hk, seqs = 8, 4, 6
+    c, g, beta, cols = _delta_inputs(L, H, Hk, dk, dv, 60, pad)
+    if close:
+        k = torch.nn.functional.normalize(_randn(1, Hk, dk, seed=66) + close * _randn(L, Hk, dk, seed=67), dim=-1)
+        c[:, cols[1]:cols[2]] = k.reshape(L, -1)
+        g.fill_(0.9999); beta.fill_(0.98)
+    start = _randn(1, H * dv * dk, seed=68)
+    S = start[0].double().view(H, dv, dk).clone()
+    want = _delta_64(c, cols, g, beta, S, H, Hk, dk, dv)
+    one = start.clone()
+    o = K.delta_scan(c, *cols, g, 0, beta, one, _ctx([0], [L]), H, Hk, dk, dv)
+    many = start.repeat(seqs, 1)
+    o6 = K.delta_scan(c.repeat(seqs, 1), *cols, g.repeat(seqs, 1), 0, beta.repeat(seqs, 1), many, _ctx([0] * seqs, [L] * seqs), H, Hk, dk, dv)
+    assert all(torch.equal(o6[i * L:(i + 1) * L], o6[:L]) and torch.equal(many[i], many[0]) for i in range(seqs))
+    assert not torch.equal(o, o6[:L])                              # (two orders of the same sums)
+    for mine, other, ref in ((o, o6[:L], want), (one[0].view(H, dv, dk), many[0].view(H, dv, dk), S)):
+        a, b = helpers.rel_err(mine, ref), helpers.rel_err(other, ref)
+        assert a < 2e-5 and b < 2e-5 and a < 1.5 * b + 1e-7, (a, b)    # (simulated in 32 bits: 1.0 to 1.1 times, close keys among them)
+
+
+def test_delta_scratch_is_for_the_tokens_that_are_there(K):
+    """One portion among many single tokens, and many sequences of many heads: nothing is sized by the longest portion times all."""
+    for lens, H in (([300] + [1] * 63, 32), ([40] * 64, 64)):
+        n, Hk, dk, dv = sum(lens), 8, 128, 64
+        c, g, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 80)
+        state, ctx = torch.zeros(len(lens), H * dv * dk, device="cuda"), _ctx([0] * len(lens), lens)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        o = K.delta_scan(c, *cols, g, 0, beta, state, ctx, H, Hk, dk, dv)
+        # the read-outs, and the chain's numbers: 32 floats a token and head
+        assert torch.cuda.max_memory_allocated() - before < 4 * (o.numel() + 32 * n * H) + (2 << 20)
+
+
 @pytest.mark.parametrize("dk,dv,pad", [(128, 64, 0), (64, 40, 4), (24, 9, 0), (100, 64, 0), (30, 16, 0), (128, 64, 1), (160, 16, 0)])
 def test_delta_single_tokens_against_64_bits_and_however_cut(K, dk, dv, pad):
     H, Hk, lens = 4, 2, [8, 3, 5]
