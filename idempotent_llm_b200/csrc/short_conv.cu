@@ -45,22 +45,55 @@ __device__ __forceinline__ ConvToken conv_token(const ConvStep& st, int t) {
     return m;
 }
 
-// Channel c of tokens t0 .. t0 + n - 1 (n <= TB; the number of taps is known at compile time, so that the loops unroll to
+// Tokens per thread: 8 where that still leaves blocks enough for the SMs (a thread's weights and state then serve eight outputs;
+// ConvChannel), else one, so that a few single tokens spread over as many threads as they have channels (conv_at).  Measured, short_conv of 4 096
+// channels x 4 taps: 2 048 tokens 18.6 us (one token a thread: 47), 6 000 tokens 45 us (113); conv_qkv_cache of 6 000 tokens x 6 144
+// channels 112 us (127).  With few tokens the looking up of a token's place, then loads, is the shortest chain: asked for in
+// ConvChannel's order, 1 / 8 / 64 single tokens take 2.85 / 3.18 / 6.86 us in conv_qkv_cache (20 heads of 64) against 2.40 / 2.77 / 6.36.
+#define CONV_TOKENS 8
+#define CONV_BLOCKS 1184               // eight blocks of 256 threads an SM
+
+// the convolution of token t, channel c (the number of taps known at compile time: the loops unroll to straight
+// code); moves the state on if t is its sequence's only token
+template <int TAPS>
+__device__ __forceinline__ float conv_at(const ConvSeg& g, const ConvToken& m, int t, int c) {
+    constexpr int H = TAPS - 1;
+    const float* base = g.in + (size_t)t * g.in_stride + g.col0 + c;
+    float* srow = g.state + (size_t)m.slot * g.state_stride + c;
+    float u[TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {
+        const int back = H - j;                                    // the input `back` positions before the token
+        float v = 0.f;
+        if (back <= m.avail) v = base[-(ptrdiff_t)back * g.in_stride];
+        else if (back <= m.pos) v = srow[(size_t)(H - (back - m.avail)) * g.channels];
+        u[j] = v;
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) acc = fmaf(g.w[(size_t)c * TAPS + j], u[j], acc);
+    if (g.bias) acc += g.bias[c];
+    if (m.single) {
+#pragma unroll
+        for (int j = 1; j < TAPS; ++j) srow[(size_t)(j - 1) * g.channels] = u[j];
+    }
+    return acc;
+}
+
+// Channel c of tokens t0 .. t0 + n - 1 (n <= CONV_TOKENS; the number of taps is known at compile time, so that the loops unroll to
 // straight code).  A thread keeps the channel's last inputs and its taps in registers: every input is read once for all the
 // outputs it takes part in.  load() asks for everything that does not depend on the tokens' places, the rows in front of t0 among it
 // (they count only if they are the same sequence's), so that one wait covers these loads and the looking up of the places.
-template <int TAPS, int TB>
+template <int TAPS>
 struct ConvChannel {
-    static constexpr int H = TAPS - 1;
+    static constexpr int H = TAPS - 1, TB = CONV_TOKENS;
     float front[TAPS], v[TB], w[TAPS], bias;
     __device__ __forceinline__ void load(const ConvSeg& g, int t0, int n, int c) {
         const float* base = g.in + (size_t)t0 * g.in_stride + g.col0 + c;
 #pragma unroll
         for (int i = 0; i < TB; ++i) v[i] = i < n ? base[(size_t)i * g.in_stride] : 0.f;
-        if (TB > 1) {
 #pragma unroll
-            for (int j = 0; j < H; ++j) front[j] = t0 >= H - j ? base[-(ptrdiff_t)(H - j) * g.in_stride] : 0.f;
-        }
+        for (int j = 0; j < H; ++j) front[j] = t0 >= H - j ? base[-(ptrdiff_t)(H - j) * g.in_stride] : 0.f;
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) w[j] = g.w[(size_t)c * TAPS + j];
         bias = g.bias ? g.bias[c] : 0.f;
@@ -72,12 +105,11 @@ struct ConvChannel {
         for (int i = 0; i < TB; ++i) {
             if (i >= n) break;
             if (i == 0 || m[i].avail == 0) {                           // the inputs before a first token: from the step, or from the state
-                const float* base = g.in + (size_t)t0 * g.in_stride + g.col0 + c;
                 const float* srow = g.state + (size_t)m[i].slot * g.state_stride + c;
 #pragma unroll
                 for (int j = 0; j < H; ++j) {
                     const int back = H - j;                            // the input `back` positions before the token
-                    u[j] = back <= m[i].avail ? (TB > 1 ? front[j] : base[-(ptrdiff_t)back * g.in_stride])
+                    u[j] = back <= m[i].avail ? front[j]
                          : back <= m[i].pos ? srow[(size_t)(H - (back - m[i].avail)) * g.channels] : 0.f;
                 }
             } else {
@@ -98,12 +130,6 @@ struct ConvChannel {
     }
 };
 
-// Tokens per thread: 8 where that still leaves blocks enough for the SMs (a thread's weights and state then serve eight outputs), else
-// one, so that a few single tokens spread over as many threads as they have channels.  Measured, short_conv of 4 096 channels x 4 taps:
-// 2 048 tokens 18.6 us (one token a thread: 47), 6 000 tokens 45 us (113); conv_qkv_cache of 6 000 tokens x 6 144 channels 112 us (127).
-#define CONV_TOKENS 8
-#define CONV_BLOCKS 1184               // eight blocks of 256 threads an SM
-
 // silu of a filter's output: exact in the 32-bit library; with the hardware exponential and division where the
 // result is rounded to bfloat16 operands anyway (relative error ~1e-6)
 __device__ __forceinline__ float silu_exact(float v) {
@@ -115,13 +141,28 @@ __device__ __forceinline__ float silu_exact(float v) {
 }
 
 // out [N, channels] 32-bit; act: 0 none, 1 silu
-template <int TAPS, int TB>
-__global__ void __launch_bounds__(256) short_conv_kernel(ConvSeg g, ConvStep st, float* __restrict__ out, int act, int n_tokens) {
+template <int TAPS>
+__global__ void __launch_bounds__(256) short_conv_kernel(ConvSeg g, ConvStep st, float* __restrict__ out, int act) {
     pdl_launch_dependents();
     pdl_wait();
+    __shared__ ConvToken token;                     // (one token per block: looked up by one thread)
+    const int c = blockIdx.y * blockDim.x + threadIdx.x, t = blockIdx.x;
+    if (threadIdx.x == 0) token = conv_token(st, t);
+    __syncthreads();
+    if (c >= g.channels) return;
+    const float v = conv_at<TAPS>(g, token, t, c);
+    out[(size_t)t * g.channels + c] = act == 1 ? silu_exact(v) : v;
+}
+
+// the same, eight tokens a thread
+template <int TAPS>
+__global__ void __launch_bounds__(256) short_conv_tokens_kernel(ConvSeg g, ConvStep st, float* __restrict__ out, int act, int n_tokens) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int TB = CONV_TOKENS;
     __shared__ ConvToken token[TB];                 // looked up by one thread each
     const int c = blockIdx.y * blockDim.x + threadIdx.x, t0 = blockIdx.x * TB, n = min(TB, n_tokens - t0);
-    ConvChannel<TAPS, TB> ch;
+    ConvChannel<TAPS> ch;
     if (c < g.channels) ch.load(g, t0, n, c);
     if (threadIdx.x < n) token[threadIdx.x] = conv_token(st, t0 + threadIdx.x);
     __syncthreads();
@@ -150,10 +191,55 @@ struct ConvQkvArgs {
     int n_tokens;
 };
 
-template <int TAPS, int TB>
-__global__ void __launch_bounds__(256, 3) conv_qkv_cache_kernel(ConvQkvArgs a) {
+template <int TAPS>
+__global__ void __launch_bounds__(256) conv_qkv_cache_kernel(ConvQkvArgs a) {
     pdl_launch_dependents();
     pdl_wait();
+    const int t = blockIdx.x;
+    const ConvToken m = conv_token(a.st, t);                       // (one token per block: every thread the same)
+    const size_t page = a.table[(size_t)m.slot * a.table_stride + m.pos / IDM_PAGE], prow = m.pos % IDM_PAGE;
+    const int qk_heads = a.n_q + a.n_kv;
+    const int part = a.dk / a.maps, per = part - a.half;  // work items of a part: pairs, then single dims
+    const int rest = a.maps * per;                        // work items of a q or k head
+    const int qk_items = qk_heads * rest, v_items = a.n_kv * a.dv;
+    // (steps of few tokens spread a token's items over several blocks: gridDim.y)
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < qk_items + v_items; i += gridDim.y * blockDim.x) {
+        if (i < qk_items) {
+            const int head = i / rest, mp = i % rest / per, r = i % per, d0 = mp * part;
+            const bool is_q = head < a.n_q;
+            T* row = is_q ? a.q_out + ((size_t)t * a.n_q + head) * a.maps * a.dk
+                          : a.k_pool + ((page * a.n_kv + (head - a.n_q)) * IDM_PAGE + prow) * (size_t)a.dk;
+            T* dst = row + (is_q ? mp * a.dk : 0) + d0;
+            const int other = r < a.half ? r + a.half : -1, d = r < a.half ? r : r + a.half;
+            if (other >= 0) {
+                const float u = conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + d);
+                const float v = conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + other);
+                const float2 cs = a.cs[(size_t)t * a.half + r];
+                from_f32(dst[d], u * cs.x - v * cs.y);
+                from_f32(dst[other], v * cs.x + u * cs.y);
+            } else {
+                from_f32(dst[d], conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + d));
+            }
+            if (is_q)
+                for (int z = 0; z < a.maps; ++z)
+                    if (z != mp) {
+                        from_f32(row[z * a.dk + d0 + d], 0.f);
+                        if (other >= 0) from_f32(row[z * a.dk + d0 + other], 0.f);
+                    }
+        } else {
+            const int j = i - qk_items, g = j / a.dv, d = j % a.dv;
+            T* dst = a.v_pool + ((page * a.n_kv + g) * IDM_PAGE + prow) * (size_t)a.dv;
+            from_f32(dst[d], conv_at<TAPS>(a.seg, m, t, qk_heads * a.dk + j));
+        }
+    }
+}
+
+// the same, eight tokens a thread
+template <int TAPS>
+__global__ void __launch_bounds__(256, 3) conv_qkv_cache_tokens_kernel(ConvQkvArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int TB = CONV_TOKENS;
     __shared__ ConvToken token[TB];
     __shared__ size_t place[TB];                    // a token's row among all rows of a kv-head's first page: + head * PAGE
     const int t0 = blockIdx.x * TB, n = min(TB, a.n_tokens - t0);
@@ -162,7 +248,7 @@ __global__ void __launch_bounds__(256, 3) conv_qkv_cache_kernel(ConvQkvArgs a) {
     const int rest = a.maps * per;                        // work items of a q or k head
     const int qk_items = qk_heads * rest, items = qk_items + a.n_kv * a.dv;
     bool known = false;
-    // (a block's items are spread over gridDim.y blocks where steps have few tokens; every thread comes to the barrier)
+    // (every thread comes to the barrier)
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; !known || i < items; i += gridDim.y * blockDim.x) {
         const bool value = i >= qk_items;
         const int j = value ? i - qk_items : i, head = value ? j / a.dv : j / rest;
@@ -170,7 +256,7 @@ __global__ void __launch_bounds__(256, 3) conv_qkv_cache_kernel(ConvQkvArgs a) {
         const bool is_q = !value && head < a.n_q, turned = !value && r < a.half;
         const int d = value || turned ? r : r + a.half, other = r + a.half;
         const int c = value ? qk_heads * a.dk + j : head * a.dk + d0 + d;
-        ConvChannel<TAPS, TB> one, two;
+        ConvChannel<TAPS> one, two;
         if (i < items) {
             one.load(a.seg, t0, n, c);
             if (turned) two.load(a.seg, t0, n, c + a.half);
@@ -266,10 +352,12 @@ extern "C" int idm_short_conv(const float* in, int in_stride, int col0, int chan
     const int across = (channels + 255) / 256;
     const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS;
     const dim3 grid(many ? (n_tokens + CONV_TOKENS - 1) / CONV_TOKENS : n_tokens, across);
-#define CONV_GO(TAPS_) case TAPS_: idm_launch(many ? short_conv_kernel<TAPS_, CONV_TOKENS> : short_conv_kernel<TAPS_, 1>, grid, dim3(256), 0, stream, \
-                                              g, st, out, act, n_tokens); break;
-    switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
+#define CONV_GO(TAPS_) case TAPS_: idm_launch(short_conv_kernel<TAPS_>, grid, dim3(256), 0, stream, g, st, out, act); break;
+#define CONV_MANY(TAPS_) case TAPS_: idm_launch(short_conv_tokens_kernel<TAPS_>, grid, dim3(256), 0, stream, g, st, out, act, n_tokens); break;
+    if (many) switch (taps) { CONV_MANY(1) CONV_MANY(2) CONV_MANY(3) CONV_MANY(4) CONV_MANY(5) CONV_MANY(6) CONV_MANY(7) CONV_MANY(8) }
+    else switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
 #undef CONV_GO
+#undef CONV_MANY
     IDM_LAUNCH_CHECK("short_conv");
     return 0;
 }
@@ -290,17 +378,19 @@ extern "C" int idm_conv_qkv_cache(const float* in, int in_stride, int col0, int 
     a.n_q = n_q; a.n_kv = n_kv; a.dk = dk; a.dv = dv; a.half = half; a.maps = maps; a.cs = (const float2*)cs;
     a.q_out = (T*)q_out; a.k_pool = (T*)k_pool; a.v_pool = (T*)v_pool; a.table = table; a.table_stride = table_stride;
     a.n_tokens = n_tokens;
-    // a thread per item and eight tokens; a block per token, with few tokens several, so that two blocks' worth of work per SM is about
+    // a thread per item and eight tokens; else a block per token, with few tokens several, so that two blocks' worth of work per SM is about
     const int items = (n_q + n_kv) * (dk - maps * half) + n_kv * dv, across = (items + 255) / 256;
     const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS;
     int split = many ? across : (296 + n_tokens - 1) / n_tokens;
     if (split > across) split = across;
     if (split < 1) split = 1;
     const dim3 grid(many ? (n_tokens + CONV_TOKENS - 1) / CONV_TOKENS : n_tokens, split);
-#define CONV_GO(TAPS_) case TAPS_: idm_launch(many ? conv_qkv_cache_kernel<TAPS_, CONV_TOKENS> : conv_qkv_cache_kernel<TAPS_, 1>, grid, dim3(256), 0, \
-                                              stream, a); break;
-    switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
+#define CONV_GO(TAPS_) case TAPS_: idm_launch(conv_qkv_cache_kernel<TAPS_>, grid, dim3(256), 0, stream, a); break;
+#define CONV_MANY(TAPS_) case TAPS_: idm_launch(conv_qkv_cache_tokens_kernel<TAPS_>, grid, dim3(256), 0, stream, a); break;
+    if (many) switch (taps) { CONV_MANY(1) CONV_MANY(2) CONV_MANY(3) CONV_MANY(4) CONV_MANY(5) CONV_MANY(6) CONV_MANY(7) CONV_MANY(8) }
+    else switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
 #undef CONV_GO
+#undef CONV_MANY
     IDM_LAUNCH_CHECK("conv_qkv_cache");
     return 0;
 }
