@@ -11,7 +11,7 @@
 // One order of summation.  Keys lie in blocks of 64 and runs of two blocks, both at absolute positions.  A score is one chain of
 // FMAs over the head's dims.  Inside a run (max, sum, context) start from nothing and are rescaled block by block; a block's
 // weights are added 16 apart and then by a butterfly, its values by one chain over its keys; the runs are folded in ascending
-// order.  A key that a row does not see takes no part in anything (the float analogue of the reference's integer sentinel,
+// order (a run whose scores all lie below a 32-bit number's range adds nothing).  A key that a row does not see takes no part in anything (the float analogue of the reference's integer sentinel,
 // src/detllm/ops/di_softmax.py:45-58): it is left out of the maximum and its value is not touched, whatever it holds.  So a
 // row's bits depend on its position and its visible keys alone, not on the step's batch, on the tile it falls in, on how
 // the sequence was cut into steps, or on whether one thread block walks its runs or several do.
@@ -102,12 +102,15 @@ __device__ __forceinline__ float max16(float v) {
     return v;
 }
 
+// exp(a - b) for a <= b, 1 where they are the same (also where both are minus infinity: scores below a 32-bit number's range)
+__device__ __forceinline__ float exp_below(float a, float b) { return a == b ? 1.f : expf(a - b); }
+
 // what a row has summed up so far, and a run's result onto it; the context's factors for both
 struct RowSum { float m, l; };
 __device__ __forceinline__ void fold_run(RowSum& t, float m, float l, float& keep, float& add) {
     const float mn = fmaxf(t.m, m);
-    keep = expf(t.m - mn);
-    add = expf(m - mn);
+    keep = exp_below(t.m, mn);
+    add = exp_below(m, mn);
     t.l = fmaf(l, add, t.l * keep);
     t.m = mn;
 }
@@ -299,12 +302,11 @@ __device__ __forceinline__ float block_weights(const AttnArgs& a, const Row& row
         for (int j = 0; j < 4; ++j) sc[j] = seen[j] ? 1.0f / (1.0f + expf(-(sc[j] + row.bias))) : -1.f;
         return 1.f;
     }
-    // (a row that sees nothing of the block stays as it is)
-    const float alpha = sees_any(row.pos, row.lo, row.keep, j0, j0 + AG_KEYS) ? expf(m_run - top) : 1.f;
+    const float alpha = exp_below(m_run, top);                  // (1 for a row that sees nothing of the block)
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        sc[j] = seen[j] ? expf(sc[j] - top) : -1.f;
+        sc[j] = !seen[j] ? -1.f : sc[j] == -INFINITY ? 0.f : expf(sc[j] - top);
         sum += seen[j] ? sc[j] : 0.f;
     }
     l_run = fmaf(l_run, alpha, sum16(sum));

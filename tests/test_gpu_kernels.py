@@ -496,6 +496,39 @@ def test_general_attention_is_one_sum_in_every_tile(kernels, dtype, n_q, n_kv, h
         assert torch.equal(run(rows, [n - few for n in lens], [few] * 3), whole[rows]), f"{few} tokens a sequence"
 
 
+# scores below a 32-bit number's range (minus infinity) over a whole run of 128 keys, over the first block of a run, over the sequence's
+# first keys: such keys weigh nothing and leave the others alone; prompts, and single tokens with their runs apart
+@pytest.mark.parametrize("low", [(128, 256), (128, 192), (0, 128), (250, 300)])
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_general_attention_with_scores_of_minus_infinity(kernels, dtype, low, sink):
+    K = kernels(dtype)
+    n, H, G, d = 301, 4, 2, 64
+    cache = SequenceCache({0: CacheNeed("full", G, d, k_row=(G, d), v_row=(G, d))}, 64 * 8, DT[dtype], "cuda:0", max_seqs=1)
+    slot = cache.alloc_slot()
+    cache.reserve([(slot, n)]); cache.flush()
+    kv = cache.view(0)
+    q, k, v = (_randn(n, h, d, seed=120 + i).to(DT[dtype]) for i, h in enumerate((H, G, G)))
+    q[..., 0], k[..., 0] = 1e3, 0.0
+    k[low[0]:low[1], :, 0] = -3e38
+    for j in range(n):
+        page = int(kv.table[slot, j // 64])
+        kv.k[page, :, j % 64], kv.v[page, :, j % 64] = k[j].cuda(), v[j].cuda()
+    s = _randn(H, seed=124).float() if sink else None
+
+    def run(first):
+        packed, m, q_lens = pack_step_host([slot], [first], [[0] * (n - first)])
+        out = torch.empty((m, H * d), dtype=DT[dtype], device="cuda")
+        K.attention_biased(q[first:].contiguous().cuda(), kv, context_from_packed(packed.cuda(), m, [slot], q_lens, [first]), d ** -0.5,
+                           out, 0, sink=None if s is None else s.cuda())
+        return out.view(m, H, d)
+    ref = _attention_64(q.double(), k.double(), v.double(), range(n), d ** -0.5, sink=None if s is None else s.double())
+    some = [t for t in range(n) if sink or low[0] > 0 or t >= low[1]]      # (a row that sees such keys alone has no answer without a sink)
+    whole = run(0)
+    assert helpers.rel_err(whole[some], ref[some]) < KTOL[dtype]
+    assert torch.equal(run(n - 1), whole[n - 1:]) and torch.equal(run(n - 9), whole[n - 9:])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_swiglu(kernels, dtype):
     K = kernels(dtype)
