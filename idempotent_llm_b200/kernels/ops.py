@@ -454,12 +454,12 @@ class Kernels:
         n, n_q, dk = q.shape
         dv = kv.v_head_dim
         self._check_kv(kv, kv.n_kv_heads, dk, dv)
+        step, runs = self._generic_step(ctx, n, n_q, kv.n_kv_heads, dv, False)
         self._check(self.lib.idm_attention_sink(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], _p(sink), (gate.data_ptr() if gate is not None else None), gate_stride,
             _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
-            *self._generic_step(ctx, n, n_q, kv.n_kv_heads, dv, False), n_q, kv.n_kv_heads, dk, dv, scale, 0, self._stream()),
-            self._generic_launches)
+            *step, _p(runs), n_q, kv.n_kv_heads, dk, dv, scale, 0, self._stream()), 1 if runs is None else 2)
 
     def attention_biased(self, q, kv, ctx, scale: float, out, out_col: int, out_scale: float = 1.0, sink=None,
                          slopes=None, gate=None, gate_stride: int = 0, gate_per_head: bool = False, window=None,
@@ -475,21 +475,22 @@ class Kernels:
         for name, t in (("sink", sink), ("slopes", slopes), ("score_bias", score_bias)):
             if t is not None and (t.dtype != torch.float32 or t.numel() != n_q):
                 raise KernelError(f"attention: {name} must hold one 32-bit number per head")
+        step, runs = self._generic_step(ctx, n, n_q, kv.n_kv_heads, kv.v_head_dim, bool(window or chunk))
         self._check(self.lib.idm_attention_biased(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table), kv.table.shape[1],
             kv.ring, _p(sink), _p(slopes), _p(gate), gate_stride, 1 if gate_per_head else 0, _p(ctx.token_seq),
             _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
-            *self._generic_step(ctx, n, n_q, kv.n_kv_heads, kv.v_head_dim, bool(window or chunk)), n_q, kv.n_kv_heads, dk,
-            kv.v_head_dim, float(scale), int(window) if window else 0, float(softcap or 0.0), int(keep_first or 0),
-            int(chunk or 0), _p(score_bias), self._stream()), self._generic_launches)
+            *step, _p(runs), n_q, kv.n_kv_heads, dk, kv.v_head_dim, float(scale), int(window) if window else 0,
+            float(softcap or 0.0), int(keep_first or 0), int(chunk or 0), _p(score_bias), self._stream()), 1 if runs is None else 2)
 
     def _generic_step(self, ctx, n: int, n_q: int, n_kv: int, dv: int, bounded: bool):
-        """What the general attention kernel is told of a step: tokens, sequences, bounds on a sequence's new tokens and
-        keys, and scratch for the runs of steps with few tiles (``bounded``: a window or chunks, whose walk is short)."""
+        """What the general attention kernel is told of a step: (tokens, sequences, bounds on a sequence's new tokens and
+        keys), and scratch for the runs of steps with few tiles, or None (``bounded``: a window or chunks, whose walk is
+        short).  The scratch is the call's own, so that calls of several streams or threads keep theirs apart."""
         need = self.lib.idm_attention_generic_scratch_floats(n, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, n_q, n_kv, dv,
                                                              1 if bounded else 0)
-        self._generic_launches = 2 if need else 1
-        return n, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, _p(self.scratch("attention_generic", need) if need else None)
+        runs = torch.empty((need,), dtype=torch.float32, device=self.device) if need else None
+        return (n, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len), runs
 
     def head_finish(self, proj, col_q: int, col_k: int, col_v, n_q: int, n_kv: int, dk: int, dv: int, biases, gammas,
                     eps: float, cs, mag: float, kv, ctx, norm_all: bool = False, v_norm: bool = False,
@@ -837,12 +838,13 @@ class Kernels:
         """The general kernel, whatever the step's shape (tests compare the special kernels with it)."""
         n, n_q, hd = q.shape
         out = torch.empty((n, n_q * hd), dtype=self.dtype, device=self.device)
+        step, runs = self._generic_step(ctx, n, n_q, kv.n_kv_heads, hd, bool(window))
         self._check(self.lib.idm_attention_generic(
             _p(q), _p(out), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], kv.ring, _p(k_new), _p(v_new),
             _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots),
-            _p(ctx.q_start), _p(ctx.cu_q), *self._generic_step(ctx, n, n_q, kv.n_kv_heads, hd, bool(window)),
-            n_q, kv.n_kv_heads, hd, scale, (int(window) if window else 0), self._stream()), self._generic_launches)
+            _p(ctx.q_start), _p(ctx.cu_q), *step, _p(runs),
+            n_q, kv.n_kv_heads, hd, scale, (int(window) if window else 0), self._stream()), 1 if runs is None else 2)
         return out
 
     def attention_decode(self, q, kv, slots, kv_len, max_kv_len: int, scale: float, window: int,

@@ -529,6 +529,37 @@ def test_general_attention_with_scores_of_minus_infinity(kernels, dtype, low, si
     assert torch.equal(run(n - 1), whole[n - 1:]) and torch.equal(run(n - 9), whole[n - 9:])
 
 
+def test_general_attention_of_two_streams_at_once(kernels):
+    """Single tokens whose runs of keys are walked apart, on two streams of one ``Kernels``: each has its own results."""
+    K = kernels("float32")
+    H, G, d, n = 16, 8, 128, 2000
+    cache = SequenceCache({0: CacheNeed("full", G, d, k_row=(G, d), v_row=(G, d))}, 64 * 70, torch.float32, "cuda:0", max_seqs=2)
+    slots = [cache.alloc_slot() for _ in range(2)]
+    cache.reserve([(s, n + 1) for s in slots]); cache.flush()
+    kv = cache.view(0)
+    kv.k.normal_(); kv.v.normal_()
+    steps = []
+    for i, s in enumerate(slots):
+        packed, m, q_lens = pack_step_host([s], [n], [[0]])
+        steps.append((_randn(1, H, d, seed=130 + i).float().cuda(), context_from_packed(packed.cuda(), m, [s], q_lens, [n])))
+
+    def run(i, out):
+        K.attention_biased(steps[i][0], kv, steps[i][1], d ** -0.5, out, 0)
+    want = [torch.empty((1, H * d), device="cuda") for _ in steps]
+    for i in range(2):
+        run(i, want[i])
+    got = [[torch.empty((1, H * d), device="cuda") for _ in range(50)] for _ in steps]
+    streams = [torch.cuda.Stream() for _ in steps]
+    torch.cuda.synchronize()
+    for k in range(50):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                run(i, got[i][k])
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(o, want[i]) for o in got[i])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_swiglu(kernels, dtype):
     K = kernels(dtype)
