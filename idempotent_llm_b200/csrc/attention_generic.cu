@@ -608,19 +608,21 @@ extern "C" long long idm_attention_generic_scratch_floats(int n_tokens, int n_se
     return attention_cut(n_tokens, n_seqs, max_q_len, max_kv_len, n_q, n_kv, dv, bounded != 0).scratch;
 }
 
+// (`most`: what the kernel's widest heads take.  The same limit from every call: a smaller one from another thread would have this
+// launch refused.)
 template <typename Kernel>
-static int attention_launch(Kernel kernel, const AttnArgs& a, dim3 grid, int bytes, cudaStream_t stream) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    IDM_REQUIRE(e == cudaSuccess, "attention: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+static int attention_launch(Kernel kernel, const AttnArgs& a, dim3 grid, int bytes, int most, cudaStream_t stream) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    IDM_REQUIRE(e == cudaSuccess, "attention: %d bytes of shared memory: %s", most, cudaGetErrorString(e));
     idm_launch(kernel, grid, dim3(AG_THREADS), bytes, stream, a);
     return 0;
 }
 template <int DC>
 static int attention_launch_rows(int rows, const AttnArgs& a, dim3 grid, cudaStream_t stream) {
-    const int bytes = attention_smem_bytes(rows, DC, a.hd);
-    return rows == 4 ? attention_launch(attention_rows_kernel<4, DC>, a, grid, bytes, stream)
-         : rows == 16 ? attention_launch(attention_rows_kernel<16, DC>, a, grid, bytes, stream)
-                      : attention_launch(attention_tile_kernel<2, DC>, a, grid, bytes, stream);
+    const int bytes = attention_smem_bytes(rows, DC, a.hd), most = attention_smem_bytes(rows, DC, IDM_MAX_HEAD_DIM);
+    return rows == 4 ? attention_launch(attention_rows_kernel<4, DC>, a, grid, bytes, most, stream)
+         : rows == 16 ? attention_launch(attention_rows_kernel<16, DC>, a, grid, bytes, most, stream)
+                      : attention_launch(attention_tile_kernel<2, DC>, a, grid, bytes, most, stream);
 }
 
 static int attention_generic_launch(AttnArgs& a, int n_seqs, int max_q_len, int max_kv_len, float* scratch, cudaStream_t stream) {

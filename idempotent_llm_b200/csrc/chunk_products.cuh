@@ -29,6 +29,7 @@
 #define CP_C 64                 // tokens of a chunk
 #define CP_LD 68                // row stride of a tile of 64 columns in shared memory (16-byte rows, banks spread)
 #define CP_TILE (64 * CP_LD)
+#define CP_MAX_DK 256
 #define CP_THREADS 256          // of the state's kernel
 #define CP_OUT_THREADS 128      // of the read-outs': 8 tokens x 4 columns a thread (4 x 4 read shared memory nearly as long as they multiply)
 
@@ -380,12 +381,13 @@ static int chunk_panels(int n_chunks, int groups, int panels) {
 
 template <typename W>
 static int chunk_products(ChunkArgs a, const W& w, int n_chunks, int n_seqs, const char* what, cudaStream_t stream) {
-    const int panels = a.heads / a.groups * ((a.dv + 63) / 64), out_smem = chunk_out_smem(a.dk);
-    IDM_REQUIRE(n_chunks > 0 && a.heads % a.groups == 0 && a.dk <= 256 && a.groups <= 65535 && n_seqs <= 65535, "%s: %d chunks, %d heads in %d groups, keys of %d",
+    const int panels = a.heads / a.groups * ((a.dv + 63) / 64), out_smem = chunk_out_smem(a.dk), out_most = chunk_out_smem(CP_MAX_DK);
+    IDM_REQUIRE(n_chunks > 0 && a.heads % a.groups == 0 && a.dk <= CP_MAX_DK && a.groups <= 65535 && n_seqs <= 65535, "%s: %d chunks, %d heads in %d groups, keys of %d",
                 what, n_chunks, a.heads, a.groups, a.dk);
     cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_state_smem());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem);
-    IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused (%s)", what, out_smem, cudaGetErrorString(e));
+    // (the same limit from every call: a smaller one from another thread would have this launch refused)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_most);
+    IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused (%s)", what, out_most, cudaGetErrorString(e));
     a.panels = chunk_panels(n_chunks, a.groups, panels);
     const dim3 grid(n_chunks, a.groups, (panels + a.panels - 1) / a.panels);
     idm_launch(chunk_state_kernel<W>, grid, dim3(CP_THREADS), chunk_state_smem(), stream, a, w);

@@ -419,6 +419,7 @@ extern "C" int idm_experts_major(const void* x, const int* tokens, const int* ta
 // are a few hundred KB at most, in the L2), so one launch does it all, without a count from the host; then it copies
 // its tokens' rows, each read once.  Bound by the bytes of xg.
 #define EG_THREADS 512
+#define EG_SMEM (200 * 1024)
 struct GroupArgs {
     const T* x; const int* tokens; const int* table; const float* pair_w;
     int n_tokens, top, n_experts, width, block_tokens;
@@ -542,8 +543,8 @@ extern "C" int idm_experts_by_expert(const void* x, const int* tokens, const int
     g.block_tokens = even < most ? even : most;
     g.offsets = ints; g.place = ints + n_experts + 1; g.row_w = weight_in ? row_w : nullptr; g.xg = (T*)xg;
     const size_t smem = (size_t)(2 * n_experts + g.block_tokens * top) * sizeof(int);
-    IDM_REQUIRE(smem <= 200 * 1024, "experts_by_expert: %d experts do not fit shared memory", n_experts);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(experts_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    IDM_REQUIRE(smem <= EG_SMEM, "experts_by_expert: %d experts do not fit shared memory", n_experts);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(experts_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EG_SMEM);   // (every call the same limit)
     idm_launch(experts_group_kernel, dim3((n_tokens + g.block_tokens - 1) / g.block_tokens), dim3(EG_THREADS), smem, stream, g);
     IDM_LAUNCH_CHECK("experts_group");
     const int rows = n_tokens * top;

@@ -310,8 +310,9 @@ template <int TN>
 static int split_launch(const float* x, const float* w, float* out, int M, int N, int K, int rows, int split, int sms, cudaStream_t stream) {
     const int bytes = (int)split_smem<TN>(K, split);
     auto kernel = rows == 0 ? gemm_f32_split_kernel<TN, 0> : rows == 1 ? gemm_f32_split_kernel<TN, 1> : gemm_f32_split_kernel<TN, 2>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    IDM_REQUIRE(e == cudaSuccess, "gemm_f32: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+    // (the same limit from every call: a smaller one from another thread would have this launch refused)
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GX_SMEM);
+    IDM_REQUIRE(e == cudaSuccess, "gemm_f32: %d bytes of shared memory: %s", GX_SMEM, cudaGetErrorString(e));
     const int token_tiles = (M + TN - 1) / TN;
     const long long tiles = (long long)token_tiles * ((N + GX_FEATURES - 1) / GX_FEATURES);
     IDM_REQUIRE(tiles < (1ll << 30), "gemm_f32: M=%d N=%d are too large for one launch", M, N);

@@ -621,6 +621,46 @@ def test_gemm_32_bit_with_numbers_that_have_no_parts(kernels, M, K_):
     assert K.gemm_status() == 0
 
 
+def test_calls_of_two_threads_at_once(kernels):
+    """Products and attention whose launches of one kernel take different amounts of shared memory, from two threads on streams of
+    their own: none is refused, and each gives what it gives alone."""
+    import threading
+    K = kernels("float32")
+    jobs, errors = [], []
+    for i, (N, K_, hd) in enumerate(((1024, 3072, 64), (6144, 256, 32))):
+        x, w = _randn(8, K_, seed=140 + i).float().cuda(), _randn(N, K_, seed=142 + i).float().cuda()
+        cache = SequenceCache({0: CacheNeed("full", 2, hd, k_row=(2, hd), v_row=(2, hd))}, 64 * 4, torch.float32, "cuda:0", max_seqs=1)
+        cache.reserve([(cache.alloc_slot(), 101)]); cache.flush()
+        kv = cache.view(0)
+        kv.k.normal_(); kv.v.normal_()
+        packed, m, q_lens = pack_step_host([0], [100], [[0]])
+        ctx = context_from_packed(packed.cuda(), m, [0], q_lens, [100])
+        q = _randn(1, 4, hd, seed=144 + i).float().cuda()
+
+        def run(x=x, w=w, q=q, kv=kv, ctx=ctx, hd=hd):
+            out = torch.empty((1, 4 * hd), device="cuda")
+            K.attention_biased(q, kv, ctx, hd ** -0.5, out, 0)
+            return K.gemm_store(x, w), out
+        jobs.append((run, run()))
+    torch.cuda.synchronize()
+
+    def work(run, want):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                got = [run() for _ in range(1500)][-1]
+                torch.cuda.current_stream().synchronize()
+            if not all(torch.equal(a, b) for a, b in zip(got, want)):
+                errors.append("another result")
+        except Exception as e:
+            errors.append(str(e))
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+
+
 # Token counts on both sides of every border between kernels and tile shapes (16, 32, 64, 128 tokens on
 # the lanes of one kernel; 128- and 256-token tiles of another above that).
 CUTS = (1, 2, 16, 17, 32, 33, 64, 65, 128, 129, 200, 256, 257, 300)
