@@ -82,6 +82,13 @@ __device__ __noinline__ float plain_sum(const float* __restrict__ x, const float
     return s;
 }
 
+// A block of a cluster whose wait has run out tells the others before they meet: none of them may add up sums that were not sent.
+// (The thread whose wait it was sees its own flag.)
+__device__ __forceinline__ void tell_cluster(int* abort_mem, int blocks) {
+    if (*(volatile int*)abort_mem == 0) return;
+    for (int r = 0; r < blocks; ++r) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(smem_u32(abort_mem), r)), "r"(1) : "memory");
+}
+
 template <int TN, int ROWS>
 __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ out, int M, int N, int K, int token_tiles, int tiles) {
@@ -280,6 +287,7 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
     __syncwarp();
     if (split > 1) {
         pdl_wait();
+        tell_cluster(&abort_mem, split);
         cluster_sync_all();                // all segments' sums are here
         const int per = (GX_FEATURES + split - 1) / split, tile = blockIdx.x;
         const int f0 = tile / token_tiles * GX_FEATURES + rank * per, m0 = tile % token_tiles * TN, have = min(per, GX_FEATURES - rank * per);
@@ -298,6 +306,14 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
     __syncthreads();
     tc_fence_after();
     if (warp == GX_WARP_MMA) tmem_dealloc(tmem, S::COLS);
+    if (abort_mem != 0) {                  // a wait ran out: none of the block's outputs passes for a number
+        const int per = (GX_FEATURES + split - 1) / split, have = min(per, GX_FEATURES - rank * per);
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+            for (int at = threadIdx.x; at < have * TN; at += GX_THREADS) {
+                const int f = tile / token_tiles * GX_FEATURES + rank * per + at % have, m = tile % token_tiles * TN + at / have;
+                if (f < N && m < M) out[(size_t)m * N + f] = __int_as_float(0x7fffffff);
+            }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------ launches
@@ -362,6 +378,30 @@ extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, i
 }
 
 #if defined(IDM_F32)
+// The bounded wait in a cluster, by itself: block `late` waits on a barrier that nothing arrives at, for `limit_cycles` (late < 0: no block
+// does); out[r]: whether block r knows when they have met.  The kernel ends normally either way.
+#define GX_PROBE_BLOCKS 4
+__global__ void __launch_bounds__(64) gemm_f32_wait_probe_kernel(long long limit_cycles, int late, int* out) {
+    __shared__ __align__(8) unsigned long long bar_mem;
+    __shared__ int abort_mem;
+    const uint32_t bar = smem_u32(&bar_mem);
+    if (threadIdx.x == 0) { mbar_init(bar, 1); abort_mem = 0; mbar_init_fence(); }
+    __syncthreads();
+    cluster_sync_all();
+    if ((int)blockIdx.z == late && threadIdx.x == 32) mbar_wait_limit(bar, 0, (volatile int*)&abort_mem, &g_gemm_f32_error, limit_cycles);
+    __syncwarp();
+    tell_cluster(&abort_mem, GX_PROBE_BLOCKS);
+    cluster_sync_all();
+    if (threadIdx.x == 0) out[blockIdx.z] = abort_mem;
+}
+extern "C" int idm_gemm_f32_wait_probe(long long limit_cycles, int late, int* out, cudaStream_t stream) {
+    IDM_REQUIRE(limit_cycles > 0 && limit_cycles <= 2000000000ll, "wait_probe: limit of %lld cycles (1 .. 2e9)", limit_cycles);
+    IDM_REQUIRE(out != nullptr && late < GX_PROBE_BLOCKS, "wait_probe: block %d of %d", late, GX_PROBE_BLOCKS);
+    idm_launch_cluster(gemm_f32_wait_probe_kernel, dim3(1, 1, GX_PROBE_BLOCKS), dim3(64), 0, stream, GX_PROBE_BLOCKS, limit_cycles, late, out);
+    IDM_LAUNCH_CHECK("wait_probe");
+    return 0;
+}
+
 // 0, or 1 if any block's bounded wait ran out since the last call (reads the flag: synchronises)
 extern "C" int idm_gemm_status() {
     int v = 0, zero = 0;

@@ -145,6 +145,7 @@ SIGNATURES = {
     "idm_gemm_bf16_qkv": (c_int, "ppiiiiippfppppppppiipppp"),
     "idm_gemm_status": (c_int, ""),
     "idm_wait_probe": (c_int, "qipp"),
+    "idm_gemm_f32_wait_probe": (c_int, "qipp"),
     "idm_program_layout": (c_int, "p"),
     "idm_run_program": (c_int, "pipp"),
     # only in a library compiled with -DIDM_TRACE (time stamps from inside two kernels: a measuring aid)
@@ -1016,8 +1017,18 @@ class Kernels:
         ran_out, cycles, other = out.tolist()
         return bool(ran_out), int(cycles), bool(other)
 
+    def cluster_wait_probe(self, limit_cycles: int, late: int):
+        """The 32-bit product's bounded wait in a cluster of four blocks: block ``late`` waits for what never comes (-1: none
+        does); returns which blocks know of it when they have met."""
+        if self.dtype != torch.float32:
+            raise KernelError("the cluster's wait probe lives in the 32-bit library")
+        out = torch.full((4,), -1, dtype=torch.int32, device=self.device)
+        self._check(self.lib.idm_gemm_f32_wait_probe(int(limit_cycles), int(late), _p(out), self._stream()), 1)
+        return out.tolist()
+
     def gemm_status(self) -> int:
-        """0, or 1 if a bounded wait inside a GEMM ran out since the last call (synchronises)."""
+        """0, or 1 if a bounded wait inside a GEMM ran out since the last call (synchronises).  In 32-bit the outputs of a tile
+        whose wait ran out are not numbers, so that no step's results pass for sums that were not made."""
         return self.lib.idm_gemm_status()
 
     # ---- a norm without statistics, one-argument activations, streams side by side, capped logits ----

@@ -920,6 +920,17 @@ def test_a_bounded_wait_that_runs_out_reports_and_the_kernel_ends_normally(kerne
         K.wait_probe(0)
 
 
+def test_a_wait_that_runs_out_is_known_to_the_whole_cluster(kernels):
+    """The 32-bit product deals a tile's segments out to the blocks of a cluster: when one of them gives up, none adds the tile up."""
+    K = kernels("float32")
+    assert K.cluster_wait_probe(5000, -1) == [0, 0, 0, 0] and K.gemm_status() == 0
+    for late in (0, 2, 3):
+        assert K.cluster_wait_probe(5000, late) == [1, 1, 1, 1]
+        assert K.gemm_status() == 1 and K.gemm_status() == 0
+    x, w = _randn(8, 3072, seed=1).float().cuda(), _randn(1024, 3072, seed=2).float().cuda()
+    assert helpers.rel_err(K.gemm_store(x, w), x.double().cpu() @ w.double().cpu().T) < 2e-6 and K.gemm_status() == 0
+
+
 # Mean rows per expert on either side of the tiles' sizes (32, 64, 256 rows), tiles with one row, experts without rows, one that has
 # all, pairs that name no expert, inner sizes that are no whole k-blocks, feature counts that are no whole tiles, more experts than
 # a block keeps the offsets of
