@@ -6,8 +6,9 @@
 // q, k [Hk, dk] are unit vectors per head (q also times dk^-1/2), v [H, dv], beta [H] in (0, 1), g [H, dk] in (0, 1];
 // head h reads q/k head h / (H / Hk).  Everything here is 32-bit: the state, the decays and their logarithms, the
 // unit norms, the gates.  S lives per sequence as [H][dv][dk] (a column's dk numbers side by side) and is carried
-// from step to step; tokens are walked one by one from and to it, so a token's result does not depend on how its
-// sequence was cut into steps.
+// from step to step.  Steps of up to 4 tokens a sequence walk them one by one, and a token's bits do not depend on how its
+// sequence was cut into such steps; when any sequence of a step brings more, all of the step's run in chunks, and a token's
+// result is the same sums in another order.
 //
 // The read-out is computed from the decayed state before the write: o = (g S)^T q + u (k . q), the same number
 // as S_new^T q, so that one round of shuffles per token serves both sums.

@@ -353,7 +353,8 @@ class Kernels:
                                                    self._state_stride(state), _p(ctx.slots), _p(ctx.q_start),
                                                    _p(ctx.cu_q), _p(ctx.kv_len), ctx.n_seqs, self._stream()))
 
-    # portions of up to so many tokens are walked token by token (the same bits however they are cut), longer ones run in chunks
+    # steps whose longest portion has up to so many tokens are walked token by token (the same bits however they are cut); in
+    # others every sequence runs in chunks
     SSD_WALK = 128
 
     def ssd_chunks(self, ctx):

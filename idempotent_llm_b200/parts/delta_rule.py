@@ -37,6 +37,8 @@ def _default_rank(s) -> int:
 
 @MIXERS.register("gated_delta")
 class GatedDeltaRule(Mixer):
+    same_bits_across_steps = False      # a step's longest portion decides whether it runs token by token or in chunks
+
     @staticmethod
     def _sizes(s):
         qk, v = s.kv_heads * s.key_dim, s.heads * s.value_dim

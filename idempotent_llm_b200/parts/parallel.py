@@ -82,6 +82,7 @@ class ParallelMixer(Mixer):
         for p in self.branches:                     # the joint matrices are the ones that are read
             p.in_weight = p.out_weight = None
         self.graph_safe = all(getattr(p, "graph_safe", True) for p in self.branches)
+        self.same_bits_across_steps = all(getattr(p, "same_bits_across_steps", True) for p in self.branches)
         self.stream_bias = None
         for p, scale in zip(self.branches, self.scales):
             b = getattr(p, "out_bias", None)

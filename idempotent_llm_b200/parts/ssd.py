@@ -27,6 +27,8 @@ from .base import MIXERS, Mixer
 
 @MIXERS.register("ssd")
 class SSDMixer(Mixer):
+    same_bits_across_steps = False      # a step's longest portion decides whether it runs token by token or in chunks
+
     @staticmethod
     def _sizes(s):
         inner, gn = s.heads * s.head_dim, s.groups * s.state

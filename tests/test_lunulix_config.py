@@ -156,3 +156,18 @@ def test_plain_rotation_turns_pairs_half_apart_and_leaves_the_rest():
     y = plain.rotate(x, torch.tensor([3]), f)[0, 0]
     assert torch.allclose(y[4:], x[0, 0, 4:])
     assert abs(y[0] - (1.0 * math.cos(3.0) - 3.0 * math.sin(3.0))) < 1e-12 and abs(y[3] - (4.0 * math.cos(0.3) + 2.0 * math.sin(0.3))) < 1e-12
+
+
+def test_mixers_that_run_in_chunks_say_that_their_bits_depend_on_the_step():
+    """A longer portion anywhere in a step moves all of its sequences to chunks: the same sums in another order.  A parallel mixer
+    says what its branches say."""
+    from idempotent_llm_b200.parts import MIXERS, Runtime
+    for kind in ("ssd", "gated_delta", "retention"):
+        assert MIXERS.get(kind).same_bits_across_steps is False
+    layer = LunulixConfig.from_dict(helpers.LUNULIX["P"]()).to_model_spec().layers[0]
+    cls = MIXERS.get("parallel")
+    weights = {d.name: torch.zeros([8 if n == -1 else n for n in d.shape]) for d in cls.declare(layer.mixer, layer.prefix)}
+    part = cls(layer.mixer, weights, layer.prefix, Runtime(device=torch.device("cpu"), dtype=torch.float32, kernels=None))
+    assert part.same_bits_across_steps is False
+    part.branches[1].same_bits_across_steps = True
+    assert part.branches[0].same_bits_across_steps is True
