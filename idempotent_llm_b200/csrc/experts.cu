@@ -531,6 +531,8 @@ extern "C" int idm_experts_by_expert(const void* x, const int* tokens, const int
     IDM_REQUIRE(width > 0 && ff > 0 && width % 8 == 0 && ff % 8 == 0, "experts_by_expert: width=%d ff=%d (multiples of 8)", width, ff);
     IDM_REQUIRE(n_experts > 0 && top > 0 && (long long)n_tokens * top < (1ll << 31), "experts_by_expert: %d experts, %d x %d pairs", n_experts, n_tokens, top);
     IDM_REQUIRE(!(weight_in || identity) || pair_w, "experts_by_expert: weights on the inputs, or identity experts, need the pairs' weights");
+    IDM_REQUIRE(!(weight_in && identity), "experts_by_expert: weights on the inputs and identity experts do not come together");
+    IDM_REQUIRE(!weight_in || row_w, "experts_by_expert: weights on the inputs need their scratch");
     IDM_REQUIRE(((uintptr_t)x & 15) == 0, "experts_by_expert: rows must start on 16-byte borders");
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

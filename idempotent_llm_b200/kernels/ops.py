@@ -1239,6 +1239,12 @@ class Kernels:
         top = table.shape[1]
         if tokens is None and table.shape[0] != n:
             raise KernelError(f"experts: choices of {table.shape[0]} rows for {n} rows")
+        if tokens is not None and tokens.numel() < n:
+            raise KernelError(f"experts: {tokens.numel()} tokens for {n} rows")
+        if pair_w is not None:
+            self._need(pair_w, torch.float32, "pairs' weights")
+            if pair_w.numel() != n * top:
+                raise KernelError(f"experts: {pair_w.numel()} weights for {n} x {top} pairs")
         if tuple(gate_up.shape) != (E, -(-ff // 64) * 128, width) or down.shape[1] != width or tuple(h.shape) != (n, width):
             raise KernelError(f"experts: gate/up {tuple(gate_up.shape)}, down {tuple(down.shape)}, stream {tuple(h.shape)} for rows of {width}")
         xg = torch.empty((n * top, width), dtype=self.dtype, device=self.device)

@@ -983,6 +983,28 @@ def test_experts_grouped_on_the_device(kernels, n, E, top, width, ff, spread, we
         assert torch.equal(h, out[0][7:27])
 
 
+def test_experts_grouped_on_the_device_refuse_what_they_would_read_out_of_range(kernels):
+    from idempotent_llm_b200.kernels import KernelError
+    K = kernels("bfloat16")
+    n, E, top, width, ff = 20, 3, 2, 64, 64
+    x, h = torch.zeros(n, width, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, width, device="cuda")
+    gate_up, down = (torch.zeros(E, *s, dtype=torch.bfloat16, device="cuda") for s in ((128, width), (width, ff)))
+    table, pw = torch.zeros(n, top, dtype=torch.int32, device="cuda"), torch.ones(n, top, device="cuda")
+    rows = torch.arange(n, dtype=torch.int32, device="cuda")
+    run = lambda tokens, **kw: K.experts_by_expert(x, tokens, table, gate_up, down, h, 0, 1.0, **kw)      # noqa: E731
+    with pytest.raises(KernelError, match="come together"):
+        run(rows, pair_w=pw, weight_in=True, identity=True)
+    with pytest.raises(KernelError, match="weights for"):
+        run(rows, pair_w=pw[:7].contiguous())
+    with pytest.raises(KernelError, match="weights"):
+        run(rows, pair_w=pw.double())
+    with pytest.raises(KernelError, match="tokens for"):
+        run(rows[:9].contiguous())
+    run(rows, pair_w=pw)
+    run(None, pair_w=pw, weight_in=True)
+    assert K.gemm_status() == 0 and not h.any()
+
+
 # both kernels of the router: up to 32 experts a lane each, more in shared memory; the second's choices by padding the first's logits
 @pytest.mark.parametrize("E,groups,keep,top,group_top", [(1, 1, 1, 1, 1), (16, 4, 2, 4, 2), (32, 1, 1, 8, 1), (30, 5, 3, 6, 3), (12, 12, 7, 7, 1)])
 @pytest.mark.parametrize("sigmoid", [False, True])
