@@ -75,16 +75,20 @@ def test_short_conv_of_eight_tokens_a_thread(K, taps, lens, channels):
 
 @pytest.mark.parametrize("maps,dk,half", [(1, 128, 32), (2, 128, 16), (1, 24, 0), (1, 40, 20)])
 def test_conv_qkv_of_eight_tokens_a_thread(K, maps, dk, half):
-    lens, n_q, n_kv, dv, taps = [900, 3, 701], 6, 2, 72, 3
+    """Enough tokens for eight a thread (a block of 256 threads for eight tokens and 256 items, 1 184 blocks at least): the bits
+    that single tokens get, and the same sums in 64 bits."""
+    lens, n_q, n_kv, dv, taps = [1300, 3, 1090], 6, 2, 72, 3
     n_q, n_kv = (n_q, n_kv) if dk == 128 else (20, 10)
     n, channels = sum(lens), (n_q + n_kv) * dk + n_kv * dv
+    items = (n_q + n_kv) * (dk - maps * half) + n_kv * dv
+    assert n // 8 * -(-items // 256) >= 1184
     proj, w = _randn(n, channels + 4, seed=5), _randn(channels, taps, seed=6)
     cs = _randn(n, half, 2, seed=7) if half else None
     start = _randn(len(lens), (taps - 1) * channels, seed=8)
 
     def fresh():
-        cache = SequenceCache({0: CacheNeed("full", n_kv, dk, k_row=(n_kv, dk), v_row=(n_kv, dv))}, 64 * 40, torch.float32, "cuda:0",
-                              max_seqs=3, max_seq_len=1024)
+        cache = SequenceCache({0: CacheNeed("full", n_kv, dk, k_row=(n_kv, dk), v_row=(n_kv, dv))}, 64 * 48, torch.float32, "cuda:0",
+                              max_seqs=3, max_seq_len=2048)
         cache.reserve([(cache.alloc_slot(), L) for L in lens]); cache.flush()
         return cache.view(0)
     kv = fresh()
@@ -102,6 +106,26 @@ def test_conv_qkv_of_eight_tokens_a_thread(K, maps, dk, half):
         assert torch.equal(q[first[i]:first[i] + m], one[first[i]:first[i] + m])
         page, page2 = int(kv.table[i, 0]), int(other.table[i, 0])
         assert torch.equal(kv.k[page][:, :m], other.k[page2][:, :m]) and torch.equal(kv.v[page][:, :m], other.v[page2][:, :m])
+        # all tokens of the sequence: filtered, q and k turned in every part, a q row per part with zeros outside it
+        x = proj[first[i]:first[i] + L, 4:].double()
+        u = torch.zeros_like(x)
+        for j in range(taps):
+            back = taps - 1 - j
+            u[back:] += w[:, j].double() * x[:max(L - back, 0)]
+        turned = u[:, :(n_q + n_kv) * dk].reshape(L, n_q + n_kv, maps, dk // maps).clone()
+        if half:
+            c, sn = cs[first[i]:first[i] + L].double().permute(2, 0, 1)[:, :, None, None, :]
+            a, b = turned[..., :half].clone(), turned[..., half:2 * half].clone()
+            turned[..., :half], turned[..., half:2 * half] = a * c - b * sn, b * c + a * sn
+        rows = torch.zeros(L, n_q, maps, maps, dk // maps, dtype=torch.float64, device="cuda")
+        for z in range(maps):
+            rows[:, :, z, z] = turned[:, :n_q, z]
+        pages = kv.table[i, :-(-L // 64)].long()
+        keys = kv.k[pages].transpose(1, 2).reshape(-1, n_kv, dk)[:L]
+        values = kv.v[pages].transpose(1, 2).reshape(-1, n_kv, dv)[:L]
+        assert helpers.rel_err(q[first[i]:first[i] + L].reshape(L, -1), rows.reshape(L, -1)) < 1e-6
+        assert helpers.rel_err(keys.reshape(L, -1), turned[:, n_q:].reshape(L, -1)) < 1e-6
+        assert helpers.rel_err(values.reshape(L, -1), u[:, (n_q + n_kv) * dk:]) < 1e-6
 
 
 # ------------------------------------------------------------------------------------------------ delta rule
