@@ -34,7 +34,7 @@ struct AttnArgs {
     const T* q; T* out;
     KVAddr cache;
     const T* k_new; const T* v_new;
-    const int* token_seq; const int* positions; const int* slots; const int* q_start; const int* cu_q;
+    const int* positions; const int* slots; const int* q_start; const int* cu_q;
     int n_tokens, n_q, n_kv, hd;
     float scale; int window;
     // beyond plain attention (all off in idm_attention_generic):
@@ -645,8 +645,7 @@ static int attention_generic_launch(AttnArgs& a, int n_seqs, int max_q_len, int 
 
 extern "C" int idm_attention_generic(const void* q, void* out, void* k_pool, void* v_pool, const int* table,
                                      int table_stride, int ring, const void* k_new, const void* v_new,
-                                     const int* token_seq, const int* positions, const int* slots,
-                                     const int* q_start, const int* cu_q, int n_tokens, int n_seqs, int max_q_len,
+                                     const int* positions, const int* slots, const int* q_start, const int* cu_q, int n_tokens, int n_seqs, int max_q_len,
                                      int max_kv_len, float* scratch, int n_q, int n_kv,
                                      int hd, float scale, int window, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
@@ -659,7 +658,7 @@ extern "C" int idm_attention_generic(const void* q, void* out, void* k_pool, voi
     a.q = (const T*)q; a.out = (T*)out;
     a.cache = KVAddr{(T*)k_pool, (T*)v_pool, table, table_stride, ring, n_kv, hd};
     a.k_new = (const T*)k_new; a.v_new = (const T*)v_new;
-    a.token_seq = token_seq; a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
+    a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
     a.n_tokens = n_tokens; a.n_q = n_q; a.n_kv = n_kv; a.hd = hd; a.scale = scale; a.window = window;
     a.dv = hd; a.sink = nullptr; a.gate = nullptr; a.gate_stride = 0; a.out_stride = n_q * hd; a.out_col = 0; a.out_scale = 1.f;
     a.slopes = nullptr; a.gate_per_head = 0; a.softcap = 0.f; a.keep_first = 0; a.chunk = 0; a.score_bias = nullptr;
@@ -673,8 +672,7 @@ extern "C" int idm_attention_generic(const void* q, void* out, void* k_pool, voi
 extern "C" int idm_attention_sink(const void* q, void* out, int out_stride, int out_col, float out_scale,
                                   void* k_pool, void* v_pool, const int* table, int table_stride,
                                   const float* sink, const float* gate, int gate_stride,
-                                  const int* token_seq, const int* positions, const int* slots,
-                                  const int* q_start, const int* cu_q, int n_tokens, int n_seqs, int max_q_len,
+                                  const int* positions, const int* slots, const int* q_start, const int* cu_q, int n_tokens, int n_seqs, int max_q_len,
                                      int max_kv_len, float* scratch, int n_q, int n_kv,
                                   int hd, int dv, float scale, int window, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
@@ -687,7 +685,7 @@ extern "C" int idm_attention_sink(const void* q, void* out, int out_stride, int 
     a.q = (const T*)q; a.out = (T*)out;
     a.cache = KVAddr{(T*)k_pool, (T*)v_pool, table, table_stride, 0, n_kv, hd};
     a.k_new = nullptr; a.v_new = nullptr;
-    a.token_seq = token_seq; a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
+    a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
     a.n_tokens = n_tokens; a.n_q = n_q; a.n_kv = n_kv; a.hd = hd; a.scale = scale; a.window = window;
     a.dv = dv; a.sink = sink; a.gate = gate; a.gate_stride = gate_stride; a.out_stride = out_stride; a.out_col = out_col;
     a.out_scale = out_scale;
@@ -703,7 +701,7 @@ extern "C" int idm_attention_sink(const void* q, void* out, int out_stride, int 
 extern "C" int idm_attention_biased(const void* q, void* out, int out_stride, int out_col, float out_scale,
                                     void* k_pool, void* v_pool, const int* table, int table_stride, int ring,
                                     const float* sink, const float* slopes, const float* gate, int gate_stride,
-                                    int gate_per_head, const int* token_seq, const int* positions, const int* slots,
+                                    int gate_per_head, const int* positions, const int* slots,
                                     const int* q_start, const int* cu_q, int n_tokens, int n_seqs, int max_q_len,
                                      int max_kv_len, float* scratch, int n_q, int n_kv,
                                     int hd, int dv, float scale, int window, float softcap, int keep_first, int chunk,
@@ -722,7 +720,7 @@ extern "C" int idm_attention_biased(const void* q, void* out, int out_stride, in
     a.q = (const T*)q; a.out = (T*)out;
     a.cache = KVAddr{(T*)k_pool, (T*)v_pool, table, table_stride, ring, n_kv, hd};
     a.k_new = nullptr; a.v_new = nullptr;
-    a.token_seq = token_seq; a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
+    a.positions = positions; a.slots = slots; a.q_start = q_start; a.cu_q = cu_q;
     a.n_tokens = n_tokens; a.n_q = n_q; a.n_kv = n_kv; a.hd = hd; a.scale = scale; a.window = window;
     a.dv = dv; a.sink = sink; a.gate = gate; a.gate_stride = gate_stride; a.out_stride = out_stride; a.out_col = out_col;
     a.out_scale = out_scale; a.slopes = slopes; a.gate_per_head = gate_per_head;

@@ -250,8 +250,7 @@ extern "C" int idm_ssd_scan(const float* xbc, int xbc_stride, int x_col, int b_c
                             int proj_stride, int z_col, int dt_col, const float* dt_bias, const float* a_log,
                             const float* d_skip, float* state, long long state_stride, float* y, int y_stride,
                             const int* cu_q, const int* slots, int n_seqs, int heads, int groups, int P, int N,
-                            const int* chunk_t0, const int* seq_chunk0, int n_chunks, float* scratch, int n_tokens,
-                            cudaStream_t stream) {
+                            const int* chunk_t0, const int* seq_chunk0, int n_chunks, float* scratch, cudaStream_t stream) {
     if (n_seqs == 0) return 0;
     IDM_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0 && P > 0 && N > 0 && N <= 256,
                 "ssd_scan: %d heads in %d groups, columns %d, state %d (at most 256)", heads, groups, P, N);

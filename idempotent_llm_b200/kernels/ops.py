@@ -66,10 +66,10 @@ SIGNATURES = {
     "idm_conv_qkv_cache": (c_int, "piiippqiiiiiipppppipppppip"),
     "idm_conv_state_update": (c_int, "piiiipqppppip"),
     "idm_ssd_chunk_tokens": (c_int, ""),
-    "idm_ssd_scan": (c_int, "piiiipiiippppqpippiiiiippipip"),
+    "idm_ssd_scan": (c_int, "piiiipiiippppqpippiiiiippipp"),
     "idm_ssd_group_norm": (c_int, "piipffpiiip"),
-    "idm_attention_sink": (c_int, "ppiifpppippipppppiiiipiiiifip"),
-    "idm_attention_biased": (c_int, "ppiifpppiipppiipppppiiiipiiiififiipp"),
+    "idm_attention_sink": (c_int, "ppiifpppippippppiiiipiiiifip"),
+    "idm_attention_biased": (c_int, "ppiifpppiipppiippppiiiipiiiififiipp"),
     "idm_head_finish": (c_int, "piiiipppppiiifipfiiiippppiipppip"),
     "idm_cols_cast": (c_int, "piiipiip"),
     "idm_delta_prep": (c_int, "piiipiipiiipppiiiip"),
@@ -88,7 +88,7 @@ SIGNATURES = {
     "idm_sample_scratch_floats": (c_longlong, "ii"),
     "idm_sample": (c_int, "piifpppp"),
     "idm_decode_advance": (c_int, "pppppppiip"),
-    "idm_attention_generic": (c_int, "pppppiipppppppiiiipiiifip"),
+    "idm_attention_generic": (c_int, "pppppiippppppiiiipiiifip"),
     "idm_attention_generic_scratch_floats": (c_longlong, "iiiiiiii"),
     "idm_attention_decode_supports": (c_int, "i"),
     "idm_attention_decode_chunk": (c_int, ""),
@@ -397,7 +397,7 @@ class Kernels:
                                           z_col, dt_col, _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
                                           self._state_stride(state), _p(y), heads * P, _p(ctx.cu_q), _p(ctx.slots),
                                           ctx.n_seqs, heads, groups, P, N, _p(chunk_t0), _p(seq_chunk0), n_chunks,
-                                          _p(scratch), n, self._stream()), 3 if n_chunks else 1)
+                                          _p(scratch), self._stream()), 3 if n_chunks else 1)
         return y
 
     # portions of up to so many tokens are walked token by token, longer ones run in chunks side by side
@@ -460,7 +460,7 @@ class Kernels:
         self._check(self.lib.idm_attention_sink(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], _p(sink), (gate.data_ptr() if gate is not None else None), gate_stride,
-            _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
+            _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
             *step, _p(runs), n_q, kv.n_kv_heads, dk, dv, scale, 0, self._stream()), 1 if runs is None else 2)
 
     def attention_biased(self, q, kv, ctx, scale: float, out, out_col: int, out_scale: float = 1.0, sink=None,
@@ -480,7 +480,7 @@ class Kernels:
         step, runs = self._generic_step(ctx, n, n_q, kv.n_kv_heads, kv.v_head_dim, bool(window or chunk))
         self._check(self.lib.idm_attention_biased(
             _p(q), _p(out), out.shape[1], out_col, float(out_scale), _p(kv.k), _p(kv.v), _p(kv.table), kv.table.shape[1],
-            kv.ring, _p(sink), _p(slopes), _p(gate), gate_stride, 1 if gate_per_head else 0, _p(ctx.token_seq),
+            kv.ring, _p(sink), _p(slopes), _p(gate), gate_stride, 1 if gate_per_head else 0,
             _p(ctx.positions), _p(ctx.slots), _p(ctx.q_start), _p(ctx.cu_q),
             *step, _p(runs), n_q, kv.n_kv_heads, dk, kv.v_head_dim, float(scale), int(window) if window else 0,
             float(softcap or 0.0), int(keep_first or 0), int(chunk or 0), _p(score_bias), self._stream()), 1 if runs is None else 2)
@@ -844,7 +844,7 @@ class Kernels:
         self._check(self.lib.idm_attention_generic(
             _p(q), _p(out), _p(kv.k), _p(kv.v), _p(kv.table),
             kv.table.shape[1], kv.ring, _p(k_new), _p(v_new),
-            _p(ctx.token_seq), _p(ctx.positions), _p(ctx.slots),
+            _p(ctx.positions), _p(ctx.slots),
             _p(ctx.q_start), _p(ctx.cu_q), *step, _p(runs),
             n_q, kv.n_kv_heads, hd, scale, (int(window) if window else 0), self._stream()), 1 if runs is None else 2)
         return out
