@@ -12,7 +12,7 @@
 // (chunk_carry_kernel: S_in of every chunk, from and to the sequence's state), and the read-outs (chunk_out_kernel).  The
 // sums are those of the token by token walk in another order; everything is 32-bit multiply-adds, which is what bounds it.
 //
-// A thread block has (chunk, group) and some of the group's panels: a panel is 64 columns of one head's values.  What a
+// A thread block has (chunk, group) and some of the group's panels (chunk_cut): a panel is 64 columns of one head's values.  What a
 // panel does not depend on is done once for all of them: the keys' tile, the queries' tile and the pair scores k_s . q_t
 // (a thread keeps its 4 x 4 of them in registers, and lays them down weighed for each head).  A panel's slices of the
 // state and its values come by asynchronous copies, one slice ahead.
@@ -30,8 +30,7 @@
 #define CP_LD 68                // row stride of a tile of 64 columns in shared memory (16-byte rows, banks spread)
 #define CP_TILE (64 * CP_LD)
 #define CP_MAX_DK 256
-#define CP_THREADS 256          // of the state's kernel
-#define CP_OUT_THREADS 128      // of the read-outs': 8 tokens x 4 columns a thread (4 x 4 read shared memory nearly as long as they multiply)
+#define CP_THREADS 256
 
 struct ChunkArgs {
     const float* q; const float* k; const float* v;          // rows of packed tokens: q + t * q_stride + group * dk, v + t * v_stride + head * dv
@@ -202,18 +201,18 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs a, W w) {
     for (int i = 0; i < V; ++i) st[i] = S[i];
 }
 
-// four tokens' weighed scores times their values for eight rows; FROM: of the four, row i sees those at or below i - FROM (8: all)
-template <int FROM>
-__device__ __forceinline__ void add_values(float (&out)[8][4], const float* pr, const float* vc) {
-    float4 p4[8];
+// four tokens' weighed scores times their values for four rows; OWN: the rows' own tokens, of which row i sees the first i + 1
+template <bool OWN>
+__device__ __forceinline__ void add_values(float (&out)[4][4], const float* pr, const float* vc) {
+    float4 p4[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * CP_LD);
+    for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * CP_LD);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float4 v4 = *reinterpret_cast<const float4*>(vc + e * CP_LD);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (FROM < 8 && i < e + FROM) continue;
+        for (int i = 0; i < 4; ++i) {
+            if (OWN && i < e) continue;
             const float x = e == 0 ? p4[i].x : e == 1 ? p4[i].y : e == 2 ? p4[i].z : p4[i].w;
             out[i][0] = fmaf(x, v4.x, out[i][0]); out[i][1] = fmaf(x, v4.y, out[i][1]);
             out[i][2] = fmaf(x, v4.z, out[i][2]); out[i][3] = fmaf(x, v4.w, out[i][3]);
@@ -222,11 +221,11 @@ __device__ __forceinline__ void add_values(float (&out)[8][4], const float* pr, 
 }
 
 // read-outs: pair scores once, then panel after panel: q S_in over the dims (slices of 64), times state(t), plus the masked
-// and weighed scores times v.  A thread has 8 tokens x 4 columns.
+// and weighed scores times v.  A thread has 4 tokens x 4 columns.
 __host__ __device__ __forceinline__ int cp_q_ld(int dk) { return (dk + 63) / 64 * 64 + 4; }
 static int chunk_out_smem(int dk) { return (64 * cp_q_ld(dk) + 4 * CP_TILE) * (int)sizeof(float); }
 template <typename W>
-__global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, W w) {
+__global__ void __launch_bounds__(CP_THREADS) chunk_out_kernel(ChunkArgs a, W w) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -237,38 +236,38 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
     float* sv = ss + 2 * CP_TILE;                            // [tokens][columns]
     float* sp = sv + CP_TILE;                                // [t][s]: the head's weighed scores
     const int c = blockIdx.x, g = blockIdx.y, t0 = a.chunk_t0[c], n = a.chunk_t0[c + 1] - t0;
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;  // tokens 8 ty .., columns 4 tx ..
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;  // tokens 4 ty .., columns 4 tx ..
     const int p0 = blockIdx.z * a.panels, p1 = min(p0 + a.panels, panel_count(a));
-    const int nk = (8 * (ty | 1) + 7) / 16 + 1;              // groups of 16 tokens that a warp's rows (two ty) may see
+    const int nk = (4 * (ty | 1) + 3) / 16 + 1;              // groups of 16 tokens that a warp's rows (two ty) may see
     const float* kbase = a.k + (size_t)t0 * a.k_stride + g * a.dk;
 
-    // pair[i][k]: tokens t = 8 ty + i, s = tx + 16 k
-    float pair[8][4];
+    // pair[i][k]: tokens t = 4 ty + i, s = tx + 16 k
+    float pair[4][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int k = 0; k < 4; ++k) pair[i][k] = 0.f;
-    cp_tile<CP_OUT_THREADS>(sq, ldq, ldq - 4, a.q + (size_t)t0 * a.q_stride + g * a.dk, a.q_stride, n, a.dk, a.vec);
-    cp_tile<CP_OUT_THREADS>(ss, CP_LD, 64, kbase, a.k_stride, n, a.dk, a.vec);
+    cp_tile<CP_THREADS>(sq, ldq, ldq - 4, a.q + (size_t)t0 * a.q_stride + g * a.dk, a.q_stride, n, a.dk, a.vec);
+    cp_tile<CP_THREADS>(ss, CP_LD, 64, kbase, a.k_stride, n, a.dk, a.vec);
     cp_commit();
     for (int i = 0; i < slices; ++i) {
         if (i + 1 < slices)
-            cp_tile<CP_OUT_THREADS>(ss + ((i + 1) & 1) * CP_TILE, CP_LD, 64, kbase + (i + 1) * 64, a.k_stride, n, a.dk - (i + 1) * 64, a.vec);
+            cp_tile<CP_THREADS>(ss + ((i + 1) & 1) * CP_TILE, CP_LD, 64, kbase + (i + 1) * 64, a.k_stride, n, a.dk - (i + 1) * 64, a.vec);
         cp_commit();
         cp_wait<1>();
         __syncthreads();
         const float* sk = ss + (i & 1) * CP_TILE;
 #pragma unroll 2
         for (int d = 0; d < 64; d += 4) {
-            float4 q4[8];
+            float4 q4[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) q4[u] = *reinterpret_cast<const float4*>(sq + (8 * ty + u) * ldq + i * 64 + d);
+            for (int u = 0; u < 4; ++u) q4[u] = *reinterpret_cast<const float4*>(sq + (4 * ty + u) * ldq + i * 64 + d);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (k >= nk) break;                          // (a warp's rows all lie before these tokens)
                 const float4 k4 = *reinterpret_cast<const float4*>(sk + (tx + 16 * k) * CP_LD + d);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
+                for (int u = 0; u < 4; ++u) {
                     pair[u][k] = fmaf(q4[u].x, k4.x, pair[u][k]); pair[u][k] = fmaf(q4[u].y, k4.y, pair[u][k]);
                     pair[u][k] = fmaf(q4[u].z, k4.z, pair[u][k]); pair[u][k] = fmaf(q4[u].w, k4.w, pair[u][k]);
                 }
@@ -282,13 +281,13 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
         int head, j0;
         const int p = p0 + step / slices, i = step % slices;
         panel_place(a, g, p, head, j0);
-        cp_tile<CP_OUT_THREADS>(ss + (step & 1) * CP_TILE, CP_LD, 64, a.chunk_state + (((size_t)c * a.heads + head) * a.dk + i * 64) * a.dv + j0, a.dv,
+        cp_tile<CP_THREADS>(ss + (step & 1) * CP_TILE, CP_LD, 64, a.chunk_state + (((size_t)c * a.heads + head) * a.dk + i * 64) * a.dv + j0, a.dv,
                                 a.dk - i * 64, a.dv - j0, a.vec);
     };
     auto copy_values = [&](int p) {
         int head, j0;
         panel_place(a, g, p, head, j0);
-        cp_tile<CP_OUT_THREADS>(sv, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
+        cp_tile<CP_THREADS>(sv, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
     };
     const int steps = (p1 - p0) * slices;
     copy_slice(0);
@@ -302,17 +301,17 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
             w.prepare(hd, head, t0, n);
             __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const int t = 8 * ty + i, s = tx + 16 * k;
+                    const int t = 4 * ty + i, s = tx + 16 * k;
                     sp[t * CP_LD + s] = s <= t && t < n ? pair[i][k] * w.pair(hd, t, s) : 0.f;
                 }
             last = head;
         }
-        float out[8][4];
+        float out[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int k = 0; k < 4; ++k) out[i][k] = 0.f;
         for (int i = 0; i < slices; ++i, ++step) {
@@ -321,17 +320,17 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
             cp_wait<1>();
             __syncthreads();
             const float* st = ss + (step & 1) * CP_TILE + 4 * tx;
-            const float* qr = sq + 8 * ty * ldq + i * 64;
+            const float* qr = sq + 4 * ty * ldq + i * 64;
 #pragma unroll 2
             for (int d = 0; d < 64; d += 4) {
-                float4 q4[8];
+                float4 q4[4];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) q4[u] = *reinterpret_cast<const float4*>(qr + u * ldq + d);
+                for (int u = 0; u < 4; ++u) q4[u] = *reinterpret_cast<const float4*>(qr + u * ldq + d);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float4 s4 = *reinterpret_cast<const float4*>(st + (d + e) * CP_LD);
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
+                    for (int u = 0; u < 4; ++u) {
                         const float q = e == 0 ? q4[u].x : e == 1 ? q4[u].y : e == 2 ? q4[u].z : q4[u].w;
                         out[u][0] = fmaf(q, s4.x, out[u][0]); out[u][1] = fmaf(q, s4.y, out[u][1]);
                         out[u][2] = fmaf(q, s4.z, out[u][2]); out[u][3] = fmaf(q, s4.w, out[u][3]);
@@ -341,20 +340,19 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
             __syncthreads();                                 // the slice's place is free
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float f = 8 * ty + i < n ? w.state(hd, 8 * ty + i) : 0.f;
+        for (int i = 0; i < 4; ++i) {
+            const float f = 4 * ty + i < n ? w.state(hd, 4 * ty + i) : 0.f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) out[i][k] *= f;
         }
-        const float* pr = sp + 8 * ty * CP_LD;
+        const float* pr = sp + 4 * ty * CP_LD;
         const float* vc = sv + 4 * tx;
 #pragma unroll 2
-        for (int s = 0; s < 8 * ty; s += 4) add_values<8>(out, pr + s, vc + s * CP_LD);
-        add_values<0>(out, pr + 8 * ty, vc + 8 * ty * CP_LD);      // (the tokens behind a row's own are not touched, whatever they hold)
-        add_values<4>(out, pr + 8 * ty + 4, vc + (8 * ty + 4) * CP_LD);
+        for (int s = 0; s < 4 * ty; s += 4) add_values<false>(out, pr + s, vc + s * CP_LD);
+        add_values<true>(out, pr + 4 * ty, vc + 4 * ty * CP_LD);   // (the tokens behind a row's own are not touched, whatever they hold)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = 8 * ty + i, left = a.dv - j0 - 4 * tx;
+        for (int i = 0; i < 4; ++i) {
+            const int t = 4 * ty + i, left = a.dv - j0 - 4 * tx;
             if (t >= n || left <= 0) continue;
             const float4 v4 = *reinterpret_cast<const float4*>(sv + t * CP_LD + 4 * tx);
             const float vx[4] = {v4.x, v4.y, v4.z, v4.w};
@@ -367,16 +365,114 @@ __global__ void __launch_bounds__(CP_OUT_THREADS) chunk_out_kernel(ChunkArgs a, 
     }
 }
 
-// How many of a group's panels a block takes: all that still leaves two blocks an SM (the pair scores and the keys are then read once for
-// them), at least one
-static int chunk_panels(int n_chunks, int groups, int panels) {
+// The same for one panel a block: a slice of q meets the keys' slice and the state's at once, so that only slices are in shared memory and
+// three blocks share an SM.  The same sums in the same order.
+static int chunk_out_one_smem() { return 4 * CP_TILE * (int)sizeof(float); }
+template <typename W>
+__global__ void __launch_bounds__(CP_THREADS, 3) chunk_out_one_kernel(ChunkArgs a, W w) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    __shared__ typename W::Head hd;
+    float* sq = sm;                                          // [tokens][dims of the slice]; the weighed scores [t][s] behind the last
+    float* sk = sq + CP_TILE;                                // [tokens][dims of the slice]
+    float* ss = sk + CP_TILE;                                // [dims of the slice][columns]
+    float* sv = ss + CP_TILE;                                // [tokens][columns]
+    const int c = blockIdx.x, g = blockIdx.y, t0 = a.chunk_t0[c], n = a.chunk_t0[c + 1] - t0, slices = (a.dk + 63) / 64;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int nk = (4 * (ty | 1) + 3) / 16 + 1;
+    int head, j0;
+    panel_place(a, g, blockIdx.z, head, j0);
+    w.prepare(hd, head, t0, n);
+    cp_tile<CP_THREADS>(sv, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
+    float pair[4][4], out[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) pair[i][k] = out[i][k] = 0.f;
+    for (int i = 0; i < slices; ++i) {
+        const int d0 = i * 64, nd = a.dk - d0;
+        if (i) __syncthreads();                              // everyone is through with the slice before
+        cp_tile<CP_THREADS>(sq, CP_LD, 64, a.q + (size_t)t0 * a.q_stride + g * a.dk + d0, a.q_stride, n, nd, a.vec);
+        cp_tile<CP_THREADS>(sk, CP_LD, 64, a.k + (size_t)t0 * a.k_stride + g * a.dk + d0, a.k_stride, n, nd, a.vec);
+        cp_tile<CP_THREADS>(ss, CP_LD, 64, a.chunk_state + (((size_t)c * a.heads + head) * a.dk + d0) * a.dv + j0, a.dv, nd, a.dv - j0, a.vec);
+        cp_commit();
+        cp_wait<0>();
+        __syncthreads();
+#pragma unroll 2
+        for (int d = 0; d < 64; d += 4) {
+            float4 q4[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) q4[u] = *reinterpret_cast<const float4*>(sq + (4 * ty + u) * CP_LD + d);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k >= nk) break;                          // (a warp's rows all lie before these tokens)
+                const float4 k4 = *reinterpret_cast<const float4*>(sk + (tx + 16 * k) * CP_LD + d);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    pair[u][k] = fmaf(q4[u].x, k4.x, pair[u][k]); pair[u][k] = fmaf(q4[u].y, k4.y, pair[u][k]);
+                    pair[u][k] = fmaf(q4[u].z, k4.z, pair[u][k]); pair[u][k] = fmaf(q4[u].w, k4.w, pair[u][k]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 s4 = *reinterpret_cast<const float4*>(ss + (d + e) * CP_LD + 4 * tx);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float q = e == 0 ? q4[u].x : e == 1 ? q4[u].y : e == 2 ? q4[u].z : q4[u].w;
+                    out[u][0] = fmaf(q, s4.x, out[u][0]); out[u][1] = fmaf(q, s4.y, out[u][1]);
+                    out[u][2] = fmaf(q, s4.z, out[u][2]); out[u][3] = fmaf(q, s4.w, out[u][3]);
+                }
+            }
+        }
+    }
+    __syncthreads();                                         // everyone is through with q: the scores take its place
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i;
+        const float f = t < n ? w.state(hd, t) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int s = tx + 16 * k;
+            sq[t * CP_LD + s] = s <= t && t < n ? pair[i][k] * w.pair(hd, t, s) : 0.f;
+            out[i][k] *= f;
+        }
+    }
+    __syncthreads();
+    const float* pr = sq + 4 * ty * CP_LD;
+    const float* vc = sv + 4 * tx;
+#pragma unroll 2
+    for (int s = 0; s < 4 * ty; s += 4) add_values<false>(out, pr + s, vc + s * CP_LD);
+    add_values<true>(out, pr + 4 * ty, vc + 4 * ty * CP_LD);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i, left = a.dv - j0 - 4 * tx;
+        if (t >= n || left <= 0) continue;
+        const float4 v4 = *reinterpret_cast<const float4*>(sv + t * CP_LD + 4 * tx);
+        const float vx[4] = {v4.x, v4.y, v4.z, v4.w};
+        w.finish(t0 + t, head, j0 + 4 * tx, out[i], vx, min(left, 4), a.vec);
+        store_row4(a.o + (size_t)(t0 + t) * a.o_stride + head * a.dv + j0 + 4 * tx, out[i], left, a.vec);
+    }
+}
+
+// How many of a group's panels a block takes (the pair scores and the keys are then read once for them): as few as leave at most 2.4 blocks
+// an SM, which has room for two.  Where that is more than two, the last 60 or so would run alone: then a block takes one panel, and the
+// read-outs are chunk_out_one_kernel's, three blocks an SM.  Measured, us of a retention of 8 heads of 128 x 256 (32 of 128 x 128):
+//   tokens                                    300    500    700   1 000   1 400   1 777   8 x 700
+//   this rule                             45 (58)  47 (79)  59 (101)  75 (153)  99 (189)  129 (250)  329 (702)
+//   always one panel, three an SM         51 (58)  52 (86)  59 (101)  84 (144)  99 (194)  129 (246)  350 (709)
+//   one panel, two an SM                  44 (67)  47 (89)  67 (111)  88 (162) 109 (209)  141 (270)  386 (789)
+// (The panels' blocks with 8 x 4 outputs a thread in four warps instead of 4 x 4 in eight took 71 (115) at 700 tokens and 348 (718) at 8 x 700.)
+struct ChunkCut { int panels; bool one; };
+static ChunkCut chunk_cut(int n_chunks, int groups, int panels) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int z = (int)((2ll * sms + (long long)n_chunks * groups - 1) / ((long long)n_chunks * groups));
-    if (z > panels) z = panels;
-    if (z < 1) z = 1;
-    return (panels + z - 1) / z;
+    auto blocks = [&](int p) { return (long long)n_chunks * groups * ((panels + p - 1) / p); };
+    int p = 1;
+    while (p < panels && 5 * blocks(p) > 12ll * sms) ++p;
+    const bool one = blocks(p) > 2ll * sms && 5 * blocks(p) <= 12ll * sms;
+    return ChunkCut{one ? 1 : p, one};
 }
 
 template <typename W>
@@ -386,15 +482,18 @@ static int chunk_products(ChunkArgs a, const W& w, int n_chunks, int n_seqs, con
                 what, n_chunks, a.heads, a.groups, a.dk);
     cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_state_smem());
     // (the same limit from every call: a smaller one from another thread would have this launch refused)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_one_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_out_one_smem());
     if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_most);
     IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused (%s)", what, out_most, cudaGetErrorString(e));
-    a.panels = chunk_panels(n_chunks, a.groups, panels);
+    const ChunkCut cut = chunk_cut(n_chunks, a.groups, panels);
+    a.panels = cut.panels;
     const dim3 grid(n_chunks, a.groups, (panels + a.panels - 1) / a.panels);
     idm_launch(chunk_state_kernel<W>, grid, dim3(CP_THREADS), chunk_state_smem(), stream, a, w);
     const size_t per = (size_t)a.dk * a.dv;
     if (a.vec) idm_launch(chunk_carry_kernel<4, W>, dim3((unsigned)((per / 4 + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);
     else idm_launch(chunk_carry_kernel<1, W>, dim3((unsigned)((per + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);
-    idm_launch(chunk_out_kernel<W>, grid, dim3(CP_OUT_THREADS), out_smem, stream, a, w);
+    if (cut.one) idm_launch(chunk_out_one_kernel<W>, grid, dim3(CP_THREADS), chunk_out_one_smem(), stream, a, w);
+    else idm_launch(chunk_out_kernel<W>, grid, dim3(CP_THREADS), out_smem, stream, a, w);
     IDM_LAUNCH_CHECK(what);
     return 0;
 }

@@ -316,6 +316,32 @@ def test_retention_chunks_against_the_walk(K, lens, H, dk, dv, shift):
     assert helpers.rel_err(out[0][0], out[1][0].double()) < 1e-5 and helpers.rel_err(out[0][1], out[1][1].double()) < 1e-5
 
 
+# a block of the read-outs takes one panel of 64 columns (in either kernel), two or all four of a group's, by how many chunks and heads a
+# step has: a sequence's bits are the same beside any others (148 SMs: at most 296 blocks, at most 355, more)
+@pytest.mark.parametrize("kind", ["retention", "state space"])
+def test_chunks_give_the_same_bits_however_panels_are_dealt_out(K, kind):
+    H, dk, dv, L = 8, 100, 256, 691                                # 11 chunks of 8 heads (groups): 88 x 4 panels
+    first = None
+    for others in ([], [64], [L], [L] * 2, [L] * 7, [200] * 3):
+        lens = [L] + others
+        n, ctx = sum(lens), _ctx([0] * len(lens), lens)
+        state = torch.cat([_randn(1, H * dk * dv, seed=100), _randn(len(lens), H * dk * dv, seed=101)[1:]]).contiguous()
+        if kind == "retention":
+            proj = torch.cat([_randn(L, 2 * H * dk + H * dv, seed=102), _randn(n, 2 * H * dk + H * dv, seed=103)[L:]]).contiguous()
+            decay = torch.tensor([0.96875, 0.5, 0.9995, 0.9, 0.99, 0.8, 0.999, 0.7], device="cuda")
+            o = K.retention(proj, (0, H * dk, 2 * H * dk), None, dk ** -0.5, decay, state, ctx, H, dk, dv)
+        else:
+            heads, P = 4 * H, 64                                   # four heads a group
+            width = heads * P + 2 * H * dk
+            xbc = torch.cat([_randn(L, width, seed=104), _randn(n, width, seed=105)[L:]]).contiguous()
+            proj = torch.cat([_randn(L, heads * P + heads, seed=106), _randn(n, heads * P + heads, seed=107)[L:]]).contiguous()
+            o = K.ssd_scan(xbc, (0, heads * P, heads * P + H * dk), proj, 0, heads * P, _randn(heads, seed=108) - 2.0, _randn(heads, seed=109),
+                           _randn(heads, seed=110), state, ctx, heads, H, P, dk)
+        if first is None:
+            first = (o[:L].clone(), state[0].clone())
+        assert torch.equal(o[:L], first[0]) and torch.equal(state[0], first[1]), f"beside {others}"
+
+
 def test_group_norm_and_gate_scale_on_and_off_16_byte_borders(K):
     n, parts, length = 21, 5, 132
     y, w = _randn(n, parts * length, seed=90), _randn(parts * length, seed=91)
