@@ -1069,10 +1069,11 @@ __global__ void __launch_bounds__(DC_THREADS) delta_walk_kernel(DeltaScanArgs a,
 //   1 394 / 2 263; 8 x 40 120 / 276; 2 048 tokens of 32 heads among 60 single tokens 921 / 3 756;
 //   keys of 64, 32 heads: 512 tokens 171 / 117, 1 024 198 / 241, 4 096 772 / 1 032.
 static bool delta_split(int n_seqs, int H, int dk, int dv, int max_tokens) {
+    if (dk <= 64 || max_tokens <= 4 * DC_C) return false;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return dk > 64 && max_tokens > 4 * DC_C && (long long)n_seqs * H * ((dv + DS_COLS - 1) / DS_COLS) <= sms;
+    return (long long)n_seqs * H * ((dv + DS_COLS - 1) / DS_COLS) <= sms;
 }
 
 // Chunks of a launch: as many of every sequence as fit 18 M floats of scratch (a chunk of one head of 128 x 64 is 64 KB, so that a long
