@@ -60,6 +60,9 @@ struct AttnArgs {
 #define AG_KEYS 64                // keys of a block: one page of the cache (a ring is whole pages)
 #define AG_RUN 128                // keys of a run
 #define AG_PROW (AG_KEYS + 4)     // a row of weights in shared memory
+// what a run's maximum starts from: the lowest finite number, so that scores of minus infinity (below a 32-bit number's range) weigh
+// exp(-inf) = 0 where a run has no others
+#define AG_LOWEST (-3.402823466e38f)
 static_assert(AG_KEYS == IDM_PAGE, "a block of keys lies in one page");
 
 __host__ __device__ __forceinline__ int pad4(int n) { return (n + 3) & ~3; }
@@ -102,15 +105,12 @@ __device__ __forceinline__ float max16(float v) {
     return v;
 }
 
-// exp(a - b) for a <= b, 1 where they are the same (also where both are minus infinity: scores below a 32-bit number's range)
-__device__ __forceinline__ float exp_below(float a, float b) { return a == b ? 1.f : expf(a - b); }
-
 // what a row has summed up so far, and a run's result onto it; the context's factors for both
 struct RowSum { float m, l; };
 __device__ __forceinline__ void fold_run(RowSum& t, float m, float l, float& keep, float& add) {
     const float mn = fmaxf(t.m, m);
-    keep = exp_below(t.m, mn);
-    add = exp_below(m, mn);
+    keep = expf(t.m - mn);
+    add = expf(m - mn);
     t.l = fmaf(l, add, t.l * keep);
     t.m = mn;
 }
@@ -285,7 +285,7 @@ __device__ __forceinline__ float* run_result(const AttnArgs& a, const Row& row, 
 // returns what the run's context is multiplied by first.  Called by the 16 threads of a row side by side.
 __device__ __forceinline__ float block_weights(const AttnArgs& a, const Row& row, int j0, int tx, float (&sc)[4], float& m_run, float& l_run) {
     bool seen[4];
-    float top = -INFINITY;
+    float top = AG_LOWEST;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int key = j0 + tx + 16 * j;
@@ -302,11 +302,12 @@ __device__ __forceinline__ float block_weights(const AttnArgs& a, const Row& row
         for (int j = 0; j < 4; ++j) sc[j] = seen[j] ? 1.0f / (1.0f + expf(-(sc[j] + row.bias))) : -1.f;
         return 1.f;
     }
-    const float alpha = exp_below(m_run, top);                  // (1 for a row that sees nothing of the block)
+    // (a row that sees nothing of the block stays as it is)
+    const float alpha = sees_any(row.pos, row.lo, row.keep, j0, j0 + AG_KEYS) ? expf(m_run - top) : 1.f;
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        sc[j] = !seen[j] ? -1.f : sc[j] == -INFINITY ? 0.f : expf(sc[j] - top);
+        sc[j] = seen[j] ? expf(sc[j] - top) : -1.f;
         sum += seen[j] ? sc[j] : 0.f;
     }
     l_run = fmaf(l_run, alpha, sum16(sum));
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(AG_THREADS) attention_tile_kernel(AttnArgs a) 
     for (int i = 0; i < RI; ++i) {
         row[i].set(a, tile, ty + 16 * i);
         total[i] = row[i].start(a);
-        m_run[i] = -INFINITY; l_run[i] = 0.f;
+        m_run[i] = AG_LOWEST; l_run[i] = 0.f;
 #pragma unroll
         for (int c = 0; c < 4 * DC; ++c) o_tot[i][c] = o_run[i][c] = 0.f;
     }
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(AG_THREADS) attention_tile_kernel(AttnArgs a) 
                         for (int c = 0; c < 4 * DC; ++c) o_tot[i][c] = fold_value(o_tot[i][c], o_run[i][c], kept, add);
                     }
                 }
-                m_run[i] = -INFINITY; l_run[i] = 0.f;
+                m_run[i] = AG_LOWEST; l_run[i] = 0.f;
 #pragma unroll
                 for (int c = 0; c < 4 * DC; ++c) o_run[i][c] = 0.f;
             }
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(AG_THREADS) attention_rows_kernel(AttnArgs a) 
     const int live = (tile.t1 - tile.t0) * a.tile_heads;        // rows (a part with fewer heads has some that see nothing)
     Row mine;                                                   // of the weights
     mine.set(a, tile, ty);
-    float m_run = -INFINITY, l_run = 0.f;
+    float m_run = AG_LOWEST, l_run = 0.f;
     const int col = threadIdx.x % VROW, row0 = threadIdx.x / VROW;
     Row item[ITEMS];
     RowSum total[ITEMS];
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(AG_THREADS) attention_rows_kernel(AttnArgs a) 
                 o_run[i] = 0.f;
             }
         }
-        if (run_ends) { m_run = -INFINITY; l_run = 0.f; }
+        if (run_ends) { m_run = AG_LOWEST; l_run = 0.f; }
         __syncthreads();                                        // everyone has read the values and the weights
         if (after <= tile.pos_last) tile.copy_keys(a, after, vs, VROW, true);
         copies_commit();
