@@ -455,22 +455,27 @@ __global__ void __launch_bounds__(CP_THREADS, 3) chunk_out_one_kernel(ChunkArgs 
     }
 }
 
-// How many of a group's panels a block takes (the pair scores and the keys are then read once for them): as few as leave at most 2.4 blocks
-// an SM, which has room for two.  Where that is more than two, the last 60 or so would run alone: then a block takes one panel, and the
-// read-outs are chunk_out_one_kernel's, three blocks an SM.  Measured, us of a retention of 8 heads of 128 x 256 (32 of 128 x 128):
-//   tokens                                    300    500    700   1 000   1 400   1 777   8 x 700
-//   this rule                             45 (58)  47 (79)  59 (101)  75 (153)  99 (189)  129 (250)  329 (702)
-//   always one panel, three an SM         51 (58)  52 (86)  59 (101)  84 (144)  99 (194)  129 (246)  350 (709)
-//   one panel, two an SM                  44 (67)  47 (89)  67 (111)  88 (162) 109 (209)  141 (270)  386 (789)
+// How many of a group's panels a block takes (the pair scores and the keys are then read once for them): all that still leave two blocks an
+// SM, which is what an SM has room for; more where that leaves a round of a few blocks behind the others and a larger number fills one round.
+// Where the blocks are a few more than a round (up to 2.4 an SM), a block takes one panel and the read-outs are chunk_out_one_kernel's,
+// three blocks an SM.  Measured, us of a retention of 8 heads of 128 x 256 (32 of 128 x 128):
+//   tokens                                    300    500    700   1 000   1 400   8 x 700
+//   this rule                             45 (58)  47 (79)  59 (101)  75 (153)  99 (189)  337 (703)
+//   always one panel, three an SM         51 (58)  52 (86)  59 (101)  84 (144)  99 (194)  350 (709)
+//   one panel, two an SM                  44 (67)  47 (89)  67 (111)  88 (162) 109 (209)  386 (789)
 // (The panels' blocks with 8 x 4 outputs a thread in four warps instead of 4 x 4 in eight took 71 (115) at 700 tokens and 348 (718) at 8 x 700.)
 struct ChunkCut { int panels; bool one; };
 static ChunkCut chunk_cut(int n_chunks, int groups, int panels) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto blocks = [&](int p) { return (long long)n_chunks * groups * ((panels + p - 1) / p); };
-    int p = 1;
-    while (p < panels && 5 * blocks(p) > 12ll * sms) ++p;
+    const long long pairs = (long long)n_chunks * groups;
+    auto blocks = [&](int p) { return pairs * ((panels + p - 1) / p); };
+    const long long z = (2ll * sms + pairs - 1) / pairs;
+    int p = z >= panels ? 1 : (int)((panels + z - 1) / z);
+    if (5 * blocks(p) > 12ll * sms)
+        for (int q = p + 1; q <= panels; ++q)
+            if (blocks(q) <= 2ll * sms && 10 * blocks(q) >= 17ll * sms) { p = q; break; }
     const bool one = blocks(p) > 2ll * sms && 5 * blocks(p) <= 12ll * sms;
     return ChunkCut{one ? 1 : p, one};
 }
