@@ -545,6 +545,120 @@ __global__ void __launch_bounds__(AG_THREADS) attention_rows_kernel(AttnArgs a) 
     }
 }
 
+// One row a warp, for single tokens whose tiles would have a row or two (attention_by_warps): a lane has two keys of a block for the
+// scores and every 32nd column for the context, keys and values come straight from memory.  The same sums in the same order: four
+// weights 16 apart lie in lanes 16 apart.  NC: columns of a lane.
+template <int NC>
+__global__ void __launch_bounds__(AG_THREADS) attention_warp_kernel(AttnArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    const int lane = threadIdx.x & 31;
+    const long long id = (long long)blockIdx.x * (AG_THREADS / 32) + (threadIdx.x >> 5);
+    if (id >= (long long)a.n_tokens * a.n_q) return;            // (warps leave whole; there is no block barrier)
+    const int t = (int)(id / a.n_q), head = (int)(id % a.n_q), g = head / (a.n_q / a.n_kv);
+    const int pos = a.positions[t], slot = a.slots[t];          // (every sequence has one token: sequence t)
+    const int first_new = a.k_new ? a.q_start[t] : 0x7fffffff;
+    const int lo = first_key(a, pos), keep = kept_keys(a, lo), main0 = lo / AG_KEYS * AG_KEYS, kept_end = min(keep, main0);
+    float* qs = smem + (threadIdx.x >> 5) * pad4(a.hd);
+    for (int d = lane; d < a.hd; d += 32) qs[d] = to_f32(a.q[((size_t)t * a.n_q + head) * a.hd + d]);
+    __syncwarp();
+    const float slope = a.slopes ? a.slopes[head] : 0.f, bias = a.score_bias ? a.score_bias[head] : 0.f;
+    RowSum total{a.sink ? a.sink[head] : -INFINITY, a.sink ? 1.f : 0.f};
+    float m_run = AG_LOWEST, l_run = 0.f, o_tot[NC], o_run[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) o_tot[i] = o_run[i] = 0.f;
+    for (int j0 = kept_end > 0 ? 0 : main0; j0 <= pos;) {
+        int after = j0 + AG_KEYS;
+        if (after < main0 && after >= kept_end) after = main0;
+        const size_t page_row = j0 < first_new ? kv_row(a.cache, slot, j0, g) : 0;
+        auto row_of = [&](const T* old, const T* fresh, int width, int key) {
+            return key >= first_new ? fresh + ((size_t)(t + key - first_new) * a.n_kv + g) * width : old + (page_row + (key - j0)) * width;
+        };
+        float w[2];
+        bool seen[2];
+        float top = AG_LOWEST;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int key = j0 + lane + 32 * u;
+            seen[u] = key <= pos && (key >= lo || key < keep);
+            w[u] = 0.f;
+            if (!seen[u]) continue;
+            const T* kr = row_of(a.cache.k, a.k_new, a.hd, key);
+            float dot = 0.f;
+            if (a.hd % Vec16<T>::N == 0) {
+                for (int d = 0; d < a.hd; d += Vec16<T>::N) {
+                    Vec16<T> kv; kv.load(kr + d);
+#pragma unroll
+                    for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[d + e], kv.get(e), dot);
+                }
+            } else {                                            // rows that do not start on 16-byte borders
+                for (int d = 0; d < a.hd; ++d) dot = fmaf(qs[d], to_f32(kr[d]), dot);
+            }
+            float x = dot * a.scale;
+            if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+            if (a.slopes) x -= slope * (float)(pos - key);
+            w[u] = x;
+            top = fmaxf(top, x);
+        }
+        float alpha = 1.f;
+        if (a.score_bias) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) w[u] = 1.0f / (1.0f + expf(-(w[u] + bias)));
+        } else {
+            top = fmaxf(m_run, warp_max(top));
+            alpha = expf(m_run - top);
+            float mine[2], other[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                w[u] = expf(w[u] - top);
+                mine[u] = seen[u] ? w[u] : 0.f;
+                other[u] = __shfl_xor_sync(0xffffffffu, mine[u], 16);
+            }
+            const bool low = lane < 16;                         // keys 0, 16, 32, 48 from the lane's sixteenth on, in this order
+            float sum = 0.f;
+            sum += low ? mine[0] : other[0]; sum += low ? other[0] : mine[0];
+            sum += low ? mine[1] : other[1]; sum += low ? other[1] : mine[1];
+            l_run = fmaf(l_run, alpha, sum16(sum));
+            m_run = top;
+        }
+#pragma unroll
+        for (int i = 0; i < NC; ++i) o_run[i] *= alpha;
+        const unsigned live[2] = {__ballot_sync(0xffffffffu, seen[0]), __ballot_sync(0xffffffffu, seen[1])};
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            for (int k0 = 0; k0 < 32 && live[u] >> k0; k0 += 8) {                // eight rows' loads at a time, up to the last one seen
+                float v[8][NC];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const bool in = (live[u] >> (k0 + k)) & 1u;
+                    const T* vr = in ? row_of(a.cache.v, a.v_new, a.dv, j0 + 32 * u + k0 + k) : nullptr;
+#pragma unroll
+                    for (int i = 0; i < NC; ++i) v[k][i] = in && lane + 32 * i < a.dv ? to_f32(vr[lane + 32 * i]) : 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float wk = __shfl_sync(0xffffffffu, w[u], k0 + k);
+                    if (!((live[u] >> (k0 + k)) & 1u)) continue;
+#pragma unroll
+                    for (int i = 0; i < NC; ++i) o_run[i] = fmaf(wk, v[k][i], o_run[i]);
+                }
+            }
+        if (after > pos || after / AG_RUN != j0 / AG_RUN) {     // the run's end
+            float kept = 1.f, add = 1.f;
+            if (!a.score_bias) fold_run(total, m_run, l_run, kept, add);
+#pragma unroll
+            for (int i = 0; i < NC; ++i) { o_tot[i] = fold_value(o_tot[i], o_run[i], kept, add); o_run[i] = 0.f; }
+            m_run = AG_LOWEST; l_run = 0.f;
+        }
+        j0 = after;
+    }
+    const float inv = a.score_bias ? 1.0f : 1.0f / total.l, hg = gate_of_head(a, t, head);
+#pragma unroll
+    for (int i = 0; i < NC; ++i)
+        if (lane + 32 * i < a.dv) finish_element(a, t, head, lane + 32 * i, o_tot[i], inv, hg);
+}
+
 // the runs' results of a row (a thread block) from scratch, in ascending order; a thread per column.  (Only layers without a window or
 // chunks come here: a row sees something of every run up to its own.)
 __global__ void __launch_bounds__(256) attention_runs_fold_kernel(AttnArgs a) {
@@ -626,6 +740,18 @@ static int attention_launch_rows(int rows, const AttnArgs& a, dim3 grid, cudaStr
                       : attention_launch(attention_tile_kernel<2, DC>, a, grid, bytes, most, stream);
 }
 
+// Single tokens a warp a row, from 512 rows on: where a tile would hold one row (as many kv-heads as q-heads) in bfloat16, whose rows a tile's
+// block cannot copy asynchronously, and where a window or chunks leave a short walk (bfloat16: up to three q-heads a kv-head).  Measured, us
+// by warps / in tiles, 32 heads of 64 (16 of 32) in bfloat16: 64 tokens behind 100 keys 46 / 101 (31 / 56), behind 700 420 / 885 (285 / 396),
+// 200 behind 300 391 / 1 235 (163 / 607), a window of 64 35 / 132 (23 / 64; in 32-bit 30 / 84, 16 / 48; 24 heads over 8 of 96 32 / 42);
+// 8 tokens behind 30 13 / 9 (256 rows).  Without a window in 32-bit, or with two q-heads a kv-head in either type, tiles are faster
+// (16 heads over 8 of 128, 64 tokens behind 700 keys: 276, a warp a row 643).
+static bool attention_by_warps(const AttnArgs& a, const AttnCut& c, int n_seqs, int max_q_len) {
+    const int group = a.n_q / a.n_kv;
+    const bool bounded = a.window > 0 || a.chunk > 0, wide = sizeof(T) == 4;
+    return c.scratch == 0 && max_q_len == 1 && a.n_tokens == n_seqs && (long long)a.n_tokens * a.n_q >= 512 && (wide ? bounded && group == 1 : group == 1 || (bounded && group <= 3));
+}
+
 static int attention_generic_launch(AttnArgs& a, int n_seqs, int max_q_len, int max_kv_len, float* scratch, cudaStream_t stream) {
     IDM_REQUIRE(n_seqs > 0 && max_q_len > 0 && max_kv_len > 0, "attention: %d sequences, at most %d tokens, %d keys", n_seqs, max_q_len, max_kv_len);
     IDM_REQUIRE(a.cache.ring % AG_KEYS == 0, "attention: a ring of %d keys is no multiple of %d", a.cache.ring, AG_KEYS);
@@ -634,6 +760,14 @@ static int attention_generic_launch(AttnArgs& a, int n_seqs, int max_q_len, int 
     IDM_REQUIRE((long long)a.n_kv * c.head_parts <= 65535, "attention: %d kv-heads", a.n_kv);
     a.n_seqs = n_seqs; a.tile_heads = c.tile_heads; a.head_parts = c.head_parts; a.tile_tokens = c.tile_tokens;
     a.scratch = c.scratch ? scratch : nullptr; a.max_runs = c.max_runs;
+    if (attention_by_warps(a, c, n_seqs, max_q_len)) {
+        const dim3 rows((unsigned)(((long long)a.n_tokens * a.n_q + AG_THREADS / 32 - 1) / (AG_THREADS / 32)));
+        const size_t bytes = sizeof(float) * (AG_THREADS / 32) * pad4(a.hd);
+        idm_launch(a.dv <= 32 ? attention_warp_kernel<1> : a.dv <= 64 ? attention_warp_kernel<2> : a.dv <= 128 ? attention_warp_kernel<4> : attention_warp_kernel<8>,
+                   rows, dim3(AG_THREADS), bytes, stream, a);
+        IDM_LAUNCH_CHECK("attention_generic");
+        return 0;
+    }
     const dim3 grid(c.tiles, a.n_kv * c.head_parts, c.runs_z);
     a.tile_per_seq = max_q_len <= c.tile_tokens;
     const int rc = a.dv <= 64 ? attention_launch_rows<1>(c.rows, a, grid, stream)

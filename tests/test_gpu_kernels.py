@@ -496,6 +496,52 @@ def test_general_attention_is_one_sum_in_every_tile(kernels, dtype, n_q, n_kv, h
         assert torch.equal(run(rows, [n - few for n in lens], [few] * 3), whole[rows]), f"{few} tokens a sequence"
 
 
+# single tokens of as many sequences as fill the SMs, one q-head a kv-head (a warp a row in bfloat16, and behind a window or in chunks in
+# both), two and three of them: the bits that a prompt's tiles give, and the same sums in 64 bits
+@pytest.mark.parametrize("n_q,n_kv,hd,dv,opts", [
+    (8, 8, 64, 64, {}), (8, 8, 40, 24, {"window": 70, "keep_first": 5}), (8, 8, 7, 9, {"chunk": 100}), (16, 8, 16, 256, {"window": 65}),
+    (24, 8, 96, 96, {"chunk": 64, "softcap": 3.0}), (8, 8, 32, 32, {"sink": True}), (8, 8, 16, 40, {"slopes": True, "window": 150}),
+    (8, 8, 128, 72, {"score_bias": True})])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_general_attention_of_many_single_tokens_is_the_same_sum(kernels, dtype, n_q, n_kv, hd, dv, opts):
+    K = kernels(dtype)
+    n_seqs = 70                                                    # (8 heads: 560 rows)
+    lens = [1 + (53 * i) % 290 for i in range(n_seqs)]
+    cache = SequenceCache({0: CacheNeed("full", n_kv, hd, k_row=(n_kv, hd), v_row=(n_kv, dv))}, 64 * 360, DT[dtype], "cuda:0", max_seqs=n_seqs)
+    slots = [cache.alloc_slot() for _ in lens]
+    cache.reserve(list(zip(slots, lens))); cache.flush()
+    kv = cache.view(0)
+    kv.k.fill_(float("nan")); kv.v.fill_(float("nan"))           # what no query sees is never touched
+    n = sum(lens)
+    q = _randn(n, n_q, hd, seed=150).to(DT[dtype])
+    k, v = _randn(n, n_kv, hd, seed=151).to(DT[dtype]), _randn(n, n_kv, dv, seed=152).to(DT[dtype])
+    at, first = 0, []
+    for s, L in zip(slots, lens):
+        for j in range(0, L, 64):
+            page, m = int(kv.table[s, j // 64]), min(64, L - j)
+            kv.k[page, :, :m], kv.v[page, :, :m] = k[at + j:at + j + m].transpose(0, 1).cuda(), v[at + j:at + j + m].transpose(0, 1).cuda()
+        first.append(at)
+        at += L
+    args = {m: (_randn(n_q, seed=153).float() if x is True else x) for m, x in opts.items()}
+    dev = {m: (x.cuda() if isinstance(x, torch.Tensor) else x) for m, x in args.items()}
+
+    def run(rows, starts, counts):
+        packed, m, q_lens = pack_step_host(slots, starts, [[0] * c for c in counts])
+        out = torch.empty((m, n_q * dv), dtype=DT[dtype], device="cuda")
+        K.attention_biased(q[rows].contiguous().cuda(), kv, context_from_packed(packed.cuda(), m, slots, q_lens, starts), hd ** -0.5, out, 0, **dev)
+        return out.view(m, n_q, dv)
+    last = [f + L - 1 for f, L in zip(first, lens)]
+    one = run(last, [L - 1 for L in lens], [1] * n_seqs)
+    assert torch.equal(one, run(list(range(n)), [0] * n_seqs, lens)[last])
+    for i in (0, 5, 11, 38):
+        a, b = first[i], last[i] + 1
+        ref = _attention_64(q[b - 1:b].double(), k[a:b].double(), v[a:b].double(), [lens[i] - 1], hd ** -0.5,
+                            **{m: (x.double() if isinstance(x, torch.Tensor) else x) for m, x in args.items()})
+        # (a slope times the distance is held to 2^-24 of itself, as a score is)
+        tol = max(KTOL[dtype], float(args["slopes"].abs().max()) * lens[i] * 2.0 ** -24 if "slopes" in args else 0.0)
+        assert helpers.rel_err(one[i:i + 1], ref) < tol, f"sequence {i}"
+
+
 # scores below a 32-bit number's range (minus infinity) over a whole run of 128 keys, over the first block of a run, over the sequence's
 # first keys: such keys weigh nothing and leave the others alone; prompts, and single tokens with their runs apart
 @pytest.mark.parametrize("low", [(128, 256), (128, 192), (0, 128), (250, 300)])
