@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_persistent_kernel(const __gri
 // from the host and can be captured; a block finds its tiles by walking the experts (each role for itself, from shared
 // memory).  An expert's tiles go feature tile after feature tile, so that neighbouring blocks read the same 128 rows of the
 // weight.  One product per expert and launch, which this replaces, leaves most SMs without a tile and pays 5
-// us or more each: 16 experts of 1024 x 768, 4 a token, 64 tokens 165 -> 28 us, 2 048 tokens some 350 -> 92 us (205 TFLOP/s, of
-// which 30 us are the grouping and the sum); 14 experts of 4096 x 3072 with 3 250 tokens 946 us (1 037 TFLOP/s).
+// us or more each: 16 experts of 1024 x 768, 4 a token, 64 tokens 165 -> 28 us, 2 048 tokens some 350 -> 80 us (484 TFLOP/s, of
+// which 17 us are the grouping and the sum); 14 experts of 4096 x 3072 with 3 250 tokens 926 us (1 060 TFLOP/s).
 #define GE_SMEM_EXPERTS 400        // offsets of up to so many experts wait in shared memory (what is left beside the rings)
 struct ExpertWalk {
     const int* offs;
