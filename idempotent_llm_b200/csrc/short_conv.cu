@@ -45,13 +45,18 @@ __device__ __forceinline__ ConvToken conv_token(const ConvStep& st, int t) {
     return m;
 }
 
-// Tokens per thread: 8 where that still leaves blocks enough for the SMs (a thread's weights and state then serve eight outputs;
-// ConvChannel), else one, so that a few single tokens spread over as many threads as they have channels (conv_at).  Measured, short_conv of 4 096
-// channels x 4 taps: 2 048 tokens 18.6 us (one token a thread: 47), 6 000 tokens 45 us (113); conv_qkv_cache of 6 000 tokens x 6 144
-// channels 112 us (127).  With few tokens the looking up of a token's place, then loads, is the shortest chain: asked for in
-// ConvChannel's order, 1 / 8 / 64 single tokens take 2.85 / 3.18 / 6.86 us in conv_qkv_cache (20 heads of 64) against 2.40 / 2.77 / 6.36.
+// Tokens per thread: 8, or up to CONV_ROUNDS times 8 one after another, where that still leaves blocks enough for the SMs (a thread's weights
+// and state then serve all its outputs, and looking up places and addresses, most of the instructions, is done once), else one, so that
+// a few single tokens spread over as many threads as they have channels (conv_at).  Channels per thread: two where pairs lie on 8-byte
+// borders.  Bound by latencies and instructions, not yet by memory (which would take 13 to 18 us of the last two).  Measured: short_conv of 4 096
+// channels x 4 taps, 2 048 tokens, 13.7 us (one channel and 8 tokens a thread 18.6, one token 47), 4 876 tokens 35 us (45); conv_qkv_cache of
+// 4 096 channels x 3 taps, 4 876 tokens, 53 us (112 us with each token's turn read from memory behind the stores of the one before,
+// 70 us in pairs without rounds); three blocks an SM instead of two spill and take 54.  With few tokens the looking up of a token's place, then
+// loads, is the shortest chain: asked for in ConvChannel's order, 1 / 8 / 64 single tokens take 2.85 / 3.18 / 6.86 us in conv_qkv_cache
+// (20 heads of 64) against 2.40 / 2.77 / 6.36.
 #define CONV_TOKENS 8
 #define CONV_BLOCKS 1184               // eight blocks of 256 threads an SM
+#define CONV_ROUNDS 4
 
 // the convolution of token t, channel c (the number of taps known at compile time: the loops unroll to straight
 // code); moves the state on if t is its sequence's only token
@@ -80,55 +85,97 @@ __device__ __forceinline__ float conv_at(const ConvSeg& g, const ConvToken& m, i
     return acc;
 }
 
-// Channel c of tokens t0 .. t0 + n - 1 (n <= CONV_TOKENS; the number of taps is known at compile time, so that the loops unroll to
-// straight code).  A thread keeps the channel's last inputs and its taps in registers: every input is read once for all the
+// Channels c .. c + V - 1 of tokens t0 .. t0 + n - 1 (n <= CONV_TOKENS; the number of taps is known at compile time, so that the loops
+// unroll to straight code).  A thread keeps its channels' inputs and taps in registers: every input is read once for all the
 // outputs it takes part in.  load() asks for everything that does not depend on the tokens' places, the rows in front of t0 among it
 // (they count only if they are the same sequence's), so that one wait covers these loads and the looking up of the places.
-template <int TAPS>
+template <int V> struct ConvLoad;
+template <> struct ConvLoad<1> { static __device__ __forceinline__ void at(const float* p, float* v) { v[0] = *p; } };
+template <> struct ConvLoad<2> {
+    static __device__ __forceinline__ void at(const float* p, float* v) { const float2 x = *reinterpret_cast<const float2*>(p); v[0] = x.x; v[1] = x.y; }
+};
+template <int TAPS, int V>
 struct ConvChannel {
     static constexpr int H = TAPS - 1, TB = CONV_TOKENS;
-    float front[TAPS], v[TB], w[TAPS], bias;
-    __device__ __forceinline__ void load(const ConvSeg& g, int t0, int n, int c) {
+    float x[H + TB][V], w[V][TAPS], bias[V];
+    __device__ __forceinline__ void rows(const ConvSeg& g, int t0, int n, int c) {
         const float* base = g.in + (size_t)t0 * g.in_stride + g.col0 + c;
 #pragma unroll
-        for (int i = 0; i < TB; ++i) v[i] = i < n ? base[(size_t)i * g.in_stride] : 0.f;
-#pragma unroll
-        for (int j = 0; j < H; ++j) front[j] = t0 >= H - j ? base[-(ptrdiff_t)(H - j) * g.in_stride] : 0.f;
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) w[j] = g.w[(size_t)c * TAPS + j];
-        bias = g.bias ? g.bias[c] : 0.f;
-    }
-    // the outputs; m: the tokens' places (in shared memory).  Moves the state on for a token that is its sequence's only one
-    __device__ __forceinline__ void run(const ConvSeg& g, const ConvToken* m, int t0, int n, int c, float (&y)[TB]) const {
-        float u[TAPS];
-#pragma unroll
         for (int i = 0; i < TB; ++i) {
-            if (i >= n) break;
-            if (i == 0 || m[i].avail == 0) {                           // the inputs before a first token: from the step, or from the state
-                const float* srow = g.state + (size_t)m[i].slot * g.state_stride + c;
+            if (i < n) ConvLoad<V>::at(base + (ptrdiff_t)i * g.in_stride, x[H + i]);
+            else
 #pragma unroll
-                for (int j = 0; j < H; ++j) {
-                    const int back = H - j;                            // the input `back` positions before the token
-                    u[j] = back <= m[i].avail ? front[j]
-                         : back <= m[i].pos ? srow[(size_t)(H - (back - m[i].avail)) * g.channels] : 0.f;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < H; ++j) u[j] = u[j + 1];
-            }
-            u[H] = v[i];
-            float acc = 0.f;
-#pragma unroll
-            for (int j = 0; j < TAPS; ++j) acc = fmaf(w[j], u[j], acc);
-            y[i] = g.bias ? acc + bias : acc;
-            if (m[i].single) {
-                float* srow = g.state + (size_t)m[i].slot * g.state_stride + c;
-#pragma unroll
-                for (int j = 1; j < TAPS; ++j) srow[(size_t)(j - 1) * g.channels] = u[j];
-            }
+                for (int e = 0; e < V; ++e) x[H + i][e] = 0.f;
         }
     }
+    // the next eight tokens: the last inputs of these are in front of them
+    __device__ __forceinline__ void next(const ConvSeg& g, int t0, int n, int c) {
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+#pragma unroll
+            for (int e = 0; e < V; ++e) x[i][e] = x[TB + i][e];
+        rows(g, t0, n, c);
+    }
+    __device__ __forceinline__ void load(const ConvSeg& g, int t0, int n, int c) {
+        rows(g, t0, n, c);
+        const float* base = g.in + (size_t)t0 * g.in_stride + g.col0 + c;
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            if (t0 >= H - i) ConvLoad<V>::at(base + (ptrdiff_t)(i - H) * g.in_stride, x[i]);
+            else
+#pragma unroll
+                for (int e = 0; e < V; ++e) x[i][e] = 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < V * TAPS; e += V) ConvLoad<V>::at(g.w + (size_t)c * TAPS + e, &w[0][0] + e);
+#pragma unroll
+        for (int e = 0; e < V; ++e) bias[e] = g.bias ? g.bias[c + e] : 0.f;
+    }
+    __device__ __forceinline__ void sums(const ConvSeg& g, const float (&u)[TAPS][V], float (&y)[V]) const {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            float acc = 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) acc = fmaf(w[e][j], u[j][e], acc);
+            y[e] = g.bias ? acc + bias[e] : acc;
+        }
+    }
+    // token i's outputs; m: the tokens' places (in shared memory).  PLAIN: it and the tokens before it whose inputs it takes are all of one
+    // sequence and in the step.  Else moves the state on for a token that is its sequence's only one
+    template <bool PLAIN>
+    __device__ __forceinline__ void at(const ConvSeg& g, const ConvToken* m, int i, int c, float (&y)[V]) const {
+        float u[TAPS][V];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+            for (int e = 0; e < V; ++e) u[j][e] = x[i + j][e];
+        if constexpr (!PLAIN) {
+            const int avail = m[i].avail, pos = m[i].pos;
+            float* srow = g.state + (size_t)m[i].slot * g.state_stride + c;
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                const int back = H - j;                                // the input `back` positions before the token
+                if (back <= avail) continue;
+#pragma unroll
+                for (int e = 0; e < V; ++e) u[j][e] = back <= pos ? srow[(size_t)(H - (back - avail)) * g.channels + e] : 0.f;
+            }
+            if (m[i].single)
+#pragma unroll
+                for (int j = 1; j < TAPS; ++j)
+#pragma unroll
+                    for (int e = 0; e < V; ++e) srow[(size_t)(j - 1) * g.channels + e] = u[j][e];
+        }
+        sums(g, u, y);
+    }
+    // whether that holds for eight tokens of a block
+    static __device__ __forceinline__ bool plain(const ConvToken* m, int n) { return n == TB && m[0].avail >= H && m[TB - 1].avail == m[0].avail + TB - 1; }
 };
+__device__ __forceinline__ void conv_store(float* p, const float (&y)[1]) { *p = y[0]; }
+__device__ __forceinline__ void conv_store(float* p, const float (&y)[2]) { *reinterpret_cast<float2*>(p) = make_float2(y[0], y[1]); }
+__device__ __forceinline__ void conv_store(__nv_bfloat16* p, const float (&y)[1]) { from_f32(*p, y[0]); }
+__device__ __forceinline__ void conv_store(__nv_bfloat16* p, const float (&y)[2]) {
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(y[0], y[1]);
+}
 
 // silu of a filter's output: exact in the 32-bit library; with the hardware exponential and division where the
 // result is rounded to bfloat16 operands anyway (relative error ~1e-6)
@@ -154,24 +201,51 @@ __global__ void __launch_bounds__(256) short_conv_kernel(ConvSeg g, ConvStep st,
     out[(size_t)t * g.channels + c] = act == 1 ? silu_exact(v) : v;
 }
 
-// the same, eight tokens a thread
-template <int TAPS>
-__global__ void __launch_bounds__(256) short_conv_tokens_kernel(ConvSeg g, ConvStep st, float* __restrict__ out, int act, int n_tokens) {
+// the same, V channels and `rounds` times eight tokens a thread
+template <int TAPS, int V>
+__global__ void __launch_bounds__(256) short_conv_tokens_kernel(ConvSeg g, ConvStep st, float* __restrict__ out, int act, int n_tokens, int rounds) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int TB = CONV_TOKENS;
-    __shared__ ConvToken token[TB];                 // looked up by one thread each
-    const int c = blockIdx.y * blockDim.x + threadIdx.x, t0 = blockIdx.x * TB, n = min(TB, n_tokens - t0);
-    ConvChannel<TAPS> ch;
-    if (c < g.channels) ch.load(g, t0, n, c);
-    if (threadIdx.x < n) token[threadIdx.x] = conv_token(st, t0 + threadIdx.x);
+    __shared__ ConvToken places[TB * CONV_ROUNDS];  // looked up by one thread each
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    int t0 = blockIdx.x * TB * rounds;
+    const int t1 = min(t0 + TB * rounds, n_tokens);
+    ConvChannel<TAPS, V> ch;
+    if (c < g.channels) ch.load(g, t0, min(TB, t1 - t0), c);
+    if (threadIdx.x < t1 - t0) places[threadIdx.x] = conv_token(st, t0 + threadIdx.x);
     __syncthreads();
     if (c >= g.channels) return;
-    float y[TB];
-    ch.run(g, token, t0, n, c, y);
+    float* dst = out + (size_t)t0 * g.channels + c;
+    auto finish = [&](float (&y)[V]) {
+        if (act == 1)
 #pragma unroll
-    for (int i = 0; i < TB; ++i)
-        if (i < n) out[(size_t)(t0 + i) * g.channels + c] = act == 1 ? silu_exact(y[i]) : y[i];
+            for (int e = 0; e < V; ++e) y[e] = silu_exact(y[e]);
+        conv_store(dst, y);
+        dst += g.channels;
+    };
+    for (const ConvToken* token = places;; token += TB) {
+        const int n = min(TB, t1 - t0);
+        if (ch.plain(token, n)) {
+#pragma unroll
+            for (int i = 0; i < TB; ++i) {
+                float y[V];
+                ch.template at<true>(g, token, i, c, y);
+                finish(y);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < TB; ++i) {
+                if (i >= n) break;
+                float y[V];
+                ch.template at<false>(g, token, i, c, y);
+                finish(y);
+            }
+        }
+        t0 += TB;
+        if (t0 >= t1) break;
+        ch.next(g, t0, min(TB, t1 - t0), c);
+    }
 }
 
 // The attention side: q, k and v channels [n_q * dk | n_kv * dk | n_kv * dv] are filtered, the first
@@ -181,6 +255,10 @@ __global__ void __launch_bounds__(256) short_conv_tokens_kernel(ConvSeg g, ConvS
 // With `maps` > 1 a q or k head is that many parts side by side, each turned like a head of dk / maps dims, and q goes out as
 // one row per part, [N, n_q * maps, dk], zero outside its part: against the same key rows each such row scores its part
 // alone.
+// (u, v) turned by (cos, sin): one order of rounding in both kernels
+__device__ __forceinline__ float2 conv_turned(float u, float v, float2 cs) {
+    return make_float2(fmaf(u, cs.x, -__fmul_rn(v, cs.y)), fmaf(v, cs.x, __fmul_rn(u, cs.y)));
+}
 struct ConvQkvArgs {
     ConvSeg seg; ConvStep st;
     int n_q, n_kv, dk, dv, half;
@@ -215,8 +293,9 @@ __global__ void __launch_bounds__(256) conv_qkv_cache_kernel(ConvQkvArgs a) {
                 const float u = conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + d);
                 const float v = conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + other);
                 const float2 cs = a.cs[(size_t)t * a.half + r];
-                from_f32(dst[d], u * cs.x - v * cs.y);
-                from_f32(dst[other], v * cs.x + u * cs.y);
+                const float2 y = conv_turned(u, v, cs);
+                from_f32(dst[d], y.x);
+                from_f32(dst[other], y.y);
             } else {
                 from_f32(dst[d], conv_at<TAPS>(a.seg, m, t, head * a.dk + d0 + d));
             }
@@ -234,70 +313,92 @@ __global__ void __launch_bounds__(256) conv_qkv_cache_kernel(ConvQkvArgs a) {
     }
 }
 
-// the same, eight tokens a thread
-template <int TAPS>
-__global__ void __launch_bounds__(256, 3) conv_qkv_cache_tokens_kernel(ConvQkvArgs a) {
+// the same, V channels (pairs of them in what is turned) and `rounds` times eight tokens a thread: first all that is turned, then what is
+// left of the q and k heads, then the values, so that a warp's threads do the same.  The tokens' (cos, sin) rows lie in shared memory: behind the
+// stores of the tokens before, a load of them would be a wait of its own for every token.
+template <int TAPS, int V>
+__global__ void __launch_bounds__(256, 2) conv_qkv_cache_tokens_kernel(ConvQkvArgs a, int rounds) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int TB = CONV_TOKENS;
-    __shared__ ConvToken token[TB];
-    __shared__ size_t place[TB];                    // a token's row among all rows of a kv-head's first page: + head * PAGE
-    const int t0 = blockIdx.x * TB, n = min(TB, a.n_tokens - t0);
-    const int qk_heads = a.n_q + a.n_kv;
-    const int part = a.dk / a.maps, per = part - a.half;  // work items of a part: pairs, then single dims
-    const int rest = a.maps * per;                        // work items of a q or k head
-    const int qk_items = qk_heads * rest, items = qk_items + a.n_kv * a.dv;
-    bool known = false;
-    // (every thread comes to the barrier)
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; !known || i < items; i += gridDim.y * blockDim.x) {
-        const bool value = i >= qk_items;
-        const int j = value ? i - qk_items : i, head = value ? j / a.dv : j / rest;
-        const int mp = value ? 0 : j % rest / per, r = value ? j % a.dv : j % per, d0 = mp * part;
-        const bool is_q = !value && head < a.n_q, turned = !value && r < a.half;
-        const int d = value || turned ? r : r + a.half, other = r + a.half;
-        const int c = value ? qk_heads * a.dk + j : head * a.dk + d0 + d;
-        ConvChannel<TAPS> one, two;
-        if (i < items) {
-            one.load(a.seg, t0, n, c);
-            if (turned) two.load(a.seg, t0, n, c + a.half);
-        }
-        if (!known) {
-            if (threadIdx.x < n) {
-                const ConvToken m = conv_token(a.st, t0 + threadIdx.x);
-                token[threadIdx.x] = m;
-                place[threadIdx.x] = (size_t)a.table[(size_t)m.slot * a.table_stride + m.pos / IDM_PAGE] * a.n_kv * IDM_PAGE + m.pos % IDM_PAGE;
-            }
-            __syncthreads();
-            known = true;
-            if (i >= items) break;
-        }
-        float u[TB], v[TB];
-        one.run(a.seg, token, t0, n, c, u);
-        if (turned) two.run(a.seg, token, t0, n, c + a.half, v);
+    extern __shared__ __align__(16) float2 conv_cs[];               // [TB rounds][half]
+    __shared__ ConvToken places[TB * CONV_ROUNDS];
+    __shared__ unsigned place[TB * CONV_ROUNDS];    // a token's row among all rows of a kv-head's first page: + head * PAGE
+    int t0 = blockIdx.x * TB * rounds;
+    const int t1 = min(t0 + TB * rounds, a.n_tokens);
+    const int parts = (a.n_q + a.n_kv) * a.maps, part = a.dk / a.maps, rest = part - 2 * a.half;
+    const int turned = parts * (a.half / V), straight = turned + parts * (rest / V), items = straight + a.n_kv * a.dv / V;
+    const int i = blockIdx.y * blockDim.x + threadIdx.x;
+    const bool turn = i < turned, value = i >= straight;
+    const int across = turn ? a.half / V : value ? a.dv / V : rest / V, j = i - (turn ? 0 : value ? straight : turned);
+    const int unit = j / across, r = (j - unit * across) * V, d = r + (turn || value ? 0 : 2 * a.half);   // (unit: part of a q or k head, or kv-head)
+    const int c = value ? parts * part + unit * a.dv + d : unit * part + d;
+    ConvChannel<TAPS, V> one, two;
+    if (i < items) {
+        one.load(a.seg, t0, min(TB, t1 - t0), c);
+        if (turn) two.load(a.seg, t0, min(TB, t1 - t0), c + a.half);
+    }
+    if (threadIdx.x < t1 - t0) {
+        const ConvToken m = conv_token(a.st, t0 + threadIdx.x);
+        places[threadIdx.x] = m;
+        place[threadIdx.x] = (unsigned)a.table[(size_t)m.slot * a.table_stride + m.pos / IDM_PAGE] * a.n_kv * IDM_PAGE + m.pos % IDM_PAGE;
+    }
+    for (int e = threadIdx.x; e < (t1 - t0) * a.half; e += blockDim.x) conv_cs[e] = a.cs[(size_t)t0 * a.half + e];
+    __syncthreads();
+    if (i >= items) return;
+    const int head = unit / a.maps, mp = unit - head * a.maps, at = value ? d : mp * part + d;
+    const bool is_q = !value && head < a.n_q;
+    // where a token goes: rows of q one after another, of a cache by the token's place
+    T* base = value ? a.v_pool + (size_t)unit * IDM_PAGE * a.dv + at
+              : is_q ? a.q_out + ((size_t)t0 * a.n_q + head) * a.maps * a.dk + mp * a.dk + at
+                     : a.k_pool + (size_t)(head - a.n_q) * IDM_PAGE * a.dk + at;
+    const unsigned row = value ? a.dv : is_q ? a.n_q * a.maps * a.dk : a.dk;
+    for (int k0 = 0;; k0 += TB) {
+        const ConvToken* token = places + k0;
+        const int n = min(TB, t1 - t0);
+        auto finish = [&](int k, float (&u)[V], float (&v)[V]) {
+            T* dst = base + (unsigned long long)row * (is_q ? k0 + k : place[k0 + k]);
+            if (turn) {
+                const float2* cs = conv_cs + (k0 + k) * a.half + r;
 #pragma unroll
-        for (int k = 0; k < TB; ++k) {
-            if (k >= n) break;
-            if (value) {
-                from_f32(a.v_pool[(place[k] + (size_t)head * IDM_PAGE) * a.dv + d], u[k]);
-                continue;
+                for (int e = 0; e < V; ++e) {
+                    const float2 y = conv_turned(u[e], v[e], cs[e]);
+                    u[e] = y.x;
+                    v[e] = y.y;
+                }
+                conv_store(dst + a.half, v);
             }
-            T* row = is_q ? a.q_out + ((size_t)(t0 + k) * a.n_q + head) * a.maps * a.dk
-                          : a.k_pool + (place[k] + (size_t)(head - a.n_q) * IDM_PAGE) * a.dk;
-            T* dst = row + (is_q ? mp * a.dk : 0) + d0;
-            if (turned) {
-                const float2 cs = a.cs[(size_t)(t0 + k) * a.half + r];
-                from_f32(dst[d], u[k] * cs.x - v[k] * cs.y);
-                from_f32(dst[other], v[k] * cs.x + u[k] * cs.y);
-            } else {
-                from_f32(dst[d], u[k]);
-            }
+            conv_store(dst, u);
             if (is_q)
                 for (int z = 0; z < a.maps; ++z)
                     if (z != mp) {
-                        from_f32(row[z * a.dk + d0 + d], 0.f);
-                        if (turned) from_f32(row[z * a.dk + d0 + other], 0.f);
+                        const float zero[V] = {};
+                        conv_store(dst + (z - mp) * a.dk, zero);
+                        if (turn) conv_store(dst + (z - mp) * a.dk + a.half, zero);
                     }
+        };
+        if (one.plain(token, n)) {
+#pragma unroll
+            for (int k = 0; k < TB; ++k) {
+                float u[V], v[V];
+                one.template at<true>(a.seg, token, k, c, u);
+                if (turn) two.template at<true>(a.seg, token, k, c + a.half, v);
+                finish(k, u, v);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < TB; ++k) {
+                if (k >= n) break;
+                float u[V], v[V];
+                one.template at<false>(a.seg, token, k, c, u);
+                if (turn) two.template at<false>(a.seg, token, k, c + a.half, v);
+                finish(k, u, v);
+            }
         }
+        t0 += TB;
+        if (t0 >= t1) break;
+        one.next(a.seg, t0, min(TB, t1 - t0), c);
+        if (turn) two.next(a.seg, t0, min(TB, t1 - t0), c + a.half);
     }
 }
 
@@ -341,6 +442,20 @@ static int conv_seg(ConvSeg& g, const char* what, const float* in, int in_stride
     return 0;
 }
 
+// whether two neighbouring channels lie on 8-byte borders in the projection's rows, in the taps and among the channels
+static bool conv_pairs(const ConvSeg& g) {
+    return g.channels % 2 == 0 && g.in_stride % 2 == 0 && g.col0 % 2 == 0 && (((uintptr_t)g.in | (uintptr_t)g.w) & 7) == 0;
+}
+
+// A block of the kernels of eight tokens a thread goes on with the next eight, up to CONV_ROUNDS times, where that leaves the SMs
+// enough blocks: looking up places and addresses is most of what a thread does for eight.
+static dim3 conv_cut(int n_tokens, int across, int& rounds) {
+    const long long blocks = (long long)((n_tokens + CONV_TOKENS - 1) / CONV_TOKENS) * across;
+    rounds = (int)(blocks / 592);
+    rounds = rounds < 1 ? 1 : rounds > CONV_ROUNDS ? CONV_ROUNDS : rounds;
+    return dim3((n_tokens + CONV_TOKENS * rounds - 1) / (CONV_TOKENS * rounds), across);
+}
+
 extern "C" int idm_short_conv(const float* in, int in_stride, int col0, int channels, int taps, const float* w,
                               const float* bias, int act, float* state, long long state_stride, float* out,
                               const int* token_seq, const int* positions, const int* slots, const int* q_start,
@@ -351,9 +466,15 @@ extern "C" int idm_short_conv(const float* in, int in_stride, int col0, int chan
     ConvStep st{token_seq, positions, slots, q_start, cu_q};
     const int across = (channels + 255) / 256;
     const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS;
-    const dim3 grid(many ? (n_tokens + CONV_TOKENS - 1) / CONV_TOKENS : n_tokens, across);
+    const dim3 grid(n_tokens, across);
+    const bool pairs = conv_pairs(g) && ((uintptr_t)out & 7) == 0;
+    int rounds;
+    const dim3 cut = conv_cut(n_tokens, pairs ? (channels + 511) / 512 : across, rounds);
 #define CONV_GO(TAPS_) case TAPS_: idm_launch(short_conv_kernel<TAPS_>, grid, dim3(256), 0, stream, g, st, out, act); break;
-#define CONV_MANY(TAPS_) case TAPS_: idm_launch(short_conv_tokens_kernel<TAPS_>, grid, dim3(256), 0, stream, g, st, out, act, n_tokens); break;
+#define CONV_MANY(TAPS_) case TAPS_: \
+        if (pairs) idm_launch(short_conv_tokens_kernel<TAPS_, 2>, cut, dim3(256), 0, stream, g, st, out, act, n_tokens, rounds); \
+        else idm_launch(short_conv_tokens_kernel<TAPS_, 1>, cut, dim3(256), 0, stream, g, st, out, act, n_tokens, rounds); \
+        break;
     if (many) switch (taps) { CONV_MANY(1) CONV_MANY(2) CONV_MANY(3) CONV_MANY(4) CONV_MANY(5) CONV_MANY(6) CONV_MANY(7) CONV_MANY(8) }
     else switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
 #undef CONV_GO
@@ -380,13 +501,21 @@ extern "C" int idm_conv_qkv_cache(const float* in, int in_stride, int col0, int 
     a.n_tokens = n_tokens;
     // a thread per item and eight tokens; else a block per token, with few tokens several, so that two blocks' worth of work per SM is about
     const int items = (n_q + n_kv) * (dk - maps * half) + n_kv * dv, across = (items + 255) / 256;
-    const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS;
-    int split = many ? across : (296 + n_tokens - 1) / n_tokens;
+    const size_t smem = (size_t)CONV_TOKENS * half * sizeof(float2);
+    const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS && smem * CONV_ROUNDS <= 40960;
+    const bool pairs = conv_pairs(a.seg) && half % 2 == 0 && (dk / maps) % 2 == 0 && dv % 2 == 0 &&
+                       (((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 7) == 0;
+    int rounds;
+    const dim3 cut = conv_cut(n_tokens, pairs ? (items + 511) / 512 : across, rounds);
+    int split = (296 + n_tokens - 1) / n_tokens;
     if (split > across) split = across;
     if (split < 1) split = 1;
-    const dim3 grid(many ? (n_tokens + CONV_TOKENS - 1) / CONV_TOKENS : n_tokens, split);
+    const dim3 grid(n_tokens, split);
 #define CONV_GO(TAPS_) case TAPS_: idm_launch(conv_qkv_cache_kernel<TAPS_>, grid, dim3(256), 0, stream, a); break;
-#define CONV_MANY(TAPS_) case TAPS_: idm_launch(conv_qkv_cache_tokens_kernel<TAPS_>, grid, dim3(256), 0, stream, a); break;
+#define CONV_MANY(TAPS_) case TAPS_: \
+        if (pairs) idm_launch(conv_qkv_cache_tokens_kernel<TAPS_, 2>, cut, dim3(256), smem * rounds, stream, a, rounds); \
+        else idm_launch(conv_qkv_cache_tokens_kernel<TAPS_, 1>, cut, dim3(256), smem * rounds, stream, a, rounds); \
+        break;
     if (many) switch (taps) { CONV_MANY(1) CONV_MANY(2) CONV_MANY(3) CONV_MANY(4) CONV_MANY(5) CONV_MANY(6) CONV_MANY(7) CONV_MANY(8) }
     else switch (taps) { CONV_GO(1) CONV_GO(2) CONV_GO(3) CONV_GO(4) CONV_GO(5) CONV_GO(6) CONV_GO(7) CONV_GO(8) }
 #undef CONV_GO

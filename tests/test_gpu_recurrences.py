@@ -275,6 +275,41 @@ def test_delta_prep_and_out_on_and_off_16_byte_borders(K, head):
         assert helpers.rel_err(x, y.double()) < 1e-6
 
 
+# pairs of channels a thread (even columns) and one to four rounds of eight tokens: the bits of the kernels of one token a thread, which steps
+# of few tokens take.  Ends of rounds and of sequences everywhere, sequences that go on from a state
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("lens,n_q,dk", [([1601, 7, 40], 20, 64), ([1300, 3, 9, 1, 1090], 12, 128), ([31, 33, 1, 2600], 20, 128)])
+def test_filters_in_pairs_and_rounds(K, lens, n_q, dk, shift):
+    n_kv, dv, half, taps = n_q // 2, 72, 16, 4
+    n, channels, starts = sum(lens), (n_q + n_kv) * dk + n_kv * dv, [6 * (i % 2) for i in range(len(lens))]
+    items = (n_q + n_kv) * (dk - half) + n_kv * dv
+    assert n // 8 * -(-items // 256) >= 1184
+    proj, w = _randn(n, channels + 2 + shift, seed=11), _randn(channels, taps, seed=12)
+    cs, start = _randn(n, half, 2, seed=13), _randn(len(lens), (taps - 1) * channels, seed=14)
+    got = []
+    for cut in (1 << 30, 64):
+        cache = SequenceCache({0: CacheNeed("full", n_kv, dk, k_row=(n_kv, dk), v_row=(n_kv, dv))}, 64 * 64, torch.float32, "cuda:0",
+                              max_seqs=8, max_seq_len=4096)
+        cache.reserve([(cache.alloc_slot(), s + L) for s, L in zip(starts, lens)]); cache.flush()
+        kv = cache.view(0)
+        kv.k.zero_(); kv.v.zero_()
+        state, state2 = start.clone(), start.clone()
+        q, y = torch.empty(n, n_q, dk, device="cuda"), torch.empty(n, channels, device="cuda")
+        for at, counts in _pieces(lens, cut):
+            keep, rows = _step_rows(lens, at, counts)
+            packed, tokens, q_lens = pack_step_host(keep, [starts[i] + at[i] for i in keep], [[0] * counts[i] for i in keep])
+            ctx = context_from_packed(packed.cuda(), tokens, keep, q_lens, [starts[i] + at[i] for i in keep])
+            piece = proj[rows].contiguous()
+            q[rows] = K.conv_qkv_cache(piece, 2 + shift, w, state, n_q, n_kv, dk, dv, cs[rows].contiguous(), kv, ctx)
+            K.conv_state_update(piece, 2 + shift, channels, taps, state, ctx)
+            y[rows] = K.short_conv(piece, 2 + shift, channels, w, None, 0, state2, ctx)
+            K.conv_state_update(piece, 2 + shift, channels, taps, state2, ctx)
+        table = [kv.table[i, :-(-(starts[i] + L) // 64)].long() for i, L in enumerate(lens)]
+        got.append([q, y, state, state2] + [pool[t] for t in table for pool in (kv.k, kv.v)])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 # ------------------------------------------------------------------------------------------------ products over chunks
 # chunks of 64 with one token left over, columns and dims that are no whole tiles, heads that share keys, blocks with several panels
 @pytest.mark.parametrize("lens,heads,groups,P,N,shift", [
