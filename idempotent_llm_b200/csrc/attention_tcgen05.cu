@@ -8,7 +8,7 @@
 //   S = Q . K^T        tcgen05.mma, both operands in shared memory, S [128 x 64] in tensor memory
 //   softmax            one thread per row reads its row of S (tcgen05.ld): scale, causal mask, running
 //                      maximum, p = 2^(s - m), running sum -- all 32-bit, no shuffles
-//   O += P . V         P written to shared memory as bfloat16 in the MMA's swizzled layout, V read in
+//   O += P . V         P written to tensor memory as bfloat16, where its S was; V read in
 //                      place ([keys, head_dim] = MN-major operand); O stays in tensor memory
 // The running maximum is only moved when the block's maximum exceeds it by more than 2^8 (then O and
 // the sum are rescaled); p and the sum always use the same reference.
@@ -32,6 +32,10 @@
 // so stale page contents cannot leak.  Rows of a tile beyond its tokens are not worked on.
 // The reference's paths are src/detllm/model.py:382-402 (prompts: query-chunked integer GEMMs) and
 // src/detllm/ops/fused_attn.py:47-115 (single tokens: one program per (batch, q-head)).
+//
+// What bounds it: the chain of a row's block (scores read 0.2 us, maximum 0.25, exponentials 0.45 to 0.65, hand-over 0.2; two blocks of
+// threads an SM), then a run's end (3 us every eighth block) and the fold.  With P in shared memory the softmax waited for the product before
+// it (0.3 us) and the hand-over took 0.35: 2 048 tokens of 16 heads of 128 over 8 52.6 us, so 42.9.
 //
 // Roles: warps 0-3 softmax + epilogue (thread = row = tensor-memory lane), warp 4 TMA, warp 5 MMA.
 // All mbarrier waits are bounded; a wait that runs out sets the error word (idm_attention_tc_status).
@@ -109,13 +113,10 @@ struct AttnTcSmem {
     static constexpr int Q_BYTES = HT * AP_BM * 128;
     static constexpr int K_BYTES = HT * AP_BN * 128;   // per stage, two stages
     static constexpr int V_BYTES = HT * AP_BN * 128;   // per stage, two stages
-    static constexpr int P_BYTES = AP_BM * 128;
-    static constexpr int Q_OFF = 0, K_OFF = Q_BYTES, V_OFF = K_OFF + 2 * K_BYTES, P_OFF = V_OFF + 2 * V_BYTES;
-    static constexpr int BAR_OFF = P_OFF + P_BYTES;
-    static constexpr int NEED = BAR_OFF + 256;         // from the first 1024-byte border on
-    // two blocks per SM: 2 x (TOTAL + 1 KB the system keeps per block) must stay within 228 KB, which
-    // leaves 512 bytes to reach the border (the array is declared with that alignment; the kernel checks)
-    static constexpr int TOTAL = NEED + (HD == 128 ? 512 : 1024);
+    static constexpr int Q_OFF = 0, K_OFF = Q_BYTES, V_OFF = K_OFF + 2 * K_BYTES;
+    static constexpr int BAR_OFF = V_OFF + 2 * V_BYTES;
+    static constexpr int NEED = BAR_OFF + 256;         // from the first 1024-byte border on (two blocks per SM fit)
+    static constexpr int TOTAL = NEED + 1024;
 };
 
 // the first key a query at position p sees, kept first keys aside
@@ -302,13 +303,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t bars = base + S::BAR_OFF;
     // barriers (8 bytes each)
-    const uint32_t q_full = bars, p_full = bars + 40, o_done = bars + 48;
+    const uint32_t q_full = bars;
+    // (two of each: a warp may be a block behind or ahead of who counts there)
+    auto o_done = [&](int b) { return bars + 40 + 8u * (b & 1); };
+    auto p_full = [&](int b) { return bars + 104 + 8u * (b & 1); };
     auto k_full = [&](int i) { return bars + 8 + 8u * i; };
     auto k_empty = [&](int i) { return bars + 24 + 8u * i; };
     auto v_full = [&](int i) { return bars + 56 + 8u * i; };
     auto v_empty = [&](int i) { return bars + 72 + 8u * i; };
     auto s_full = [&](int i) { return bars + 88 + 8u * i; };
-    auto s_empty = [&](int i) { return bars + 104 + 8u * i; };
     volatile uint32_t* tmem_slot = (volatile uint32_t*)(gbase + S::BAR_OFF + 120);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
@@ -369,10 +372,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int n_hg = a.n_q >> gs;
 
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1); mbar_init(p_full, 4); mbar_init(o_done, 1);
+        mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) {
+            mbar_init(p_full(i), 4); mbar_init(o_done(i), 1);
             mbar_init(k_full(i), 1); mbar_init(k_empty(i), 1);
-            mbar_init(v_full(i), 1); mbar_init(v_empty(i), 1); mbar_init(s_full(i), 1); mbar_init(s_empty(i), 4);
+            mbar_init(v_full(i), 1); mbar_init(v_empty(i), 1); mbar_init(s_full(i), 1);
         }
         *abort_flag = 0;
         mbar_init_fence();
@@ -382,7 +386,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_o = tmem + 128;                          // S buffers at columns 0 and 64, O from 128
+    const uint32_t tmem_o = tmem + 128;                          // S buffers at columns 0 and 64 (P takes the place of its S), O from 128
     pdl_wait();                                                  // set-up done; now the previous kernel's results
     if (threadIdx.x == 0) attn_stamp(1);                         // set-up done, the kernel before too
 
@@ -445,13 +449,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int b = 0; b < nb && ok; ++b) {
                 if (b + 1 < nb) {
                     ok = mbar_wait(k_full((b + 1) & 1), ((b + 1) >> 1) & 1, abort_flag, &g_attn_tc_error);
-                    if (ok && b + 1 >= 2)
-                        ok = mbar_wait(s_empty((b + 1) & 1), (((b + 1) >> 1) - 1) & 1, abort_flag, &g_attn_tc_error);
+                    if (ok && b >= 1)                            // P of block b - 1 lies where these scores go
+                        ok = mbar_wait(o_done(b - 1), ((b - 1) >> 1) & 1, abort_flag, &g_attn_tc_error);
                     if (!ok) break;
                     tc_fence_after();
                     mma_s(b + 1);
                 }
-                ok = mbar_wait(p_full, b & 1, abort_flag, &g_attn_tc_error) &&
+                ok = mbar_wait(p_full(b), (b >> 1) & 1, abort_flag, &g_attn_tc_error) &&
                      mbar_wait(v_full(b & 1), (b >> 1) & 1, abort_flag, &g_attn_tc_error);
                 if (!ok) break;
                 tc_fence_after();
@@ -459,11 +463,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const bool fresh = block_of(b_first + b) % R == 0;   // a run's first block starts its context from nothing
 #pragma unroll
                 for (int kk = 0; kk < AP_BN / 16; ++kk) {        // O (+)= P . V_b
-                    const uint64_t ad = umma_desc_kmajor(base + S::P_OFF) + 2 * kk;
                     const uint64_t bd = umma_desc_mnmajor(vbase + kk * 16 * 128, AP_BN * 128);
-                    tc_mma_bf16(tmem_o, ad, bd, idesc_o, (!fresh || kk > 0) ? 1u : 0u);
+                    tc_mma_bf16_ts(tmem_o, tmem + (uint32_t)((b & 1) * AP_BN + 8 * kk), bd, idesc_o, (!fresh || kk > 0) ? 1u : 0u);
                 }
-                tc_commit(o_done);
+                tc_commit(o_done(b));
                 tc_commit(v_empty(b & 1));
             }
         }
@@ -479,12 +482,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // the slope in units of the raw score (the scale is positive): raw + slope_raw * (j - p) is what is scaled
         const float slope_raw = a.slopes ? __fdiv_rn(__fmul_rn(a.slopes[head0 + (r & (gp - 1))], 1.4426950408889634f), a.scale_log2) : 0.f;
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-        uint8_t* prow = gbase + S::P_OFF + r * 128;
-        if (!row_live) {
-            // the row's P stays zero: its part of O is never read, and nothing undefined meets the MMA
-#pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(prow + (c << 4)) = make_uint4(0, 0, 0, 0);
-        }
         // one block per tile, more than one run: the row's context so far lives in scratch of this block's own
         float* tot = (!through_scratch && !shared && n_runs > 1) ? a.parts + (size_t)(tile * n_hg + hg) * (AP_BM * HD) : nullptr;
         // where the runs of this tile and head group leave their results (a block per run, or a tile shared by several blocks)
@@ -528,13 +525,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc_ld32_issue(tmem + lane_base + (uint32_t)(b & 1) * AP_BN + 32, sr + 32);
                 tc_ld_wait();
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(s_empty(b & 1));
             const int key0 = block_of(b_first + b) * AP_BN;       // position of the block's first key
             float alpha = 1.f, row_sum = 0.f;
-            uint32_t packed[AP_BN / 2];
-            if (row_live) {
+            // P goes where S was, 32 keys as soon as they are made (the scores are all in registers)
+            const uint32_t p_at = tmem + lane_base + (uint32_t)(b & 1) * AP_BN;
+            if (warp_live) {                                     // (a row beyond the tile's gets whatever its scores make: its part of O is never read)
                 if (a.cap_in > 0.f) {                             // the cap, before any key is masked (tanh of -inf is -1)
 #pragma unroll
                     for (int j = 0; j < AP_BN; ++j) {
@@ -562,10 +557,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
                 if constexpr (SIG) {
 #pragma unroll
-                    for (int j = 0; j < AP_BN; j += 2) {
-                        const __nv_bfloat162 pk = __floats2bfloat162_rn(sigmoid_weight(__uint_as_float(sr[j]), neg_scale, neg_bias),
-                                                                        sigmoid_weight(__uint_as_float(sr[j + 1]), neg_scale, neg_bias));
-                        packed[j / 2] = *reinterpret_cast<const uint32_t*>(&pk);
+                    for (int h = 0; h < AP_BN; h += 32) {
+                        uint32_t packed[16];
+#pragma unroll
+                        for (int j = h; j < h + 32; j += 2) {
+                            const __nv_bfloat162 pk = __floats2bfloat162_rn(sigmoid_weight(__uint_as_float(sr[j]), neg_scale, neg_bias),
+                                                                            sigmoid_weight(__uint_as_float(sr[j + 1]), neg_scale, neg_bias));
+                            packed[(j - h) / 2] = *reinterpret_cast<const uint32_t*>(&pk);
+                        }
+                        tc_st16(p_at + h / 2, packed);
                     }
                 } else {
                     // the maximum of the raw scores (the scale is positive), four chains side by side
@@ -587,22 +587,31 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
                     float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int j = 0; j < AP_BN; j += 4) {
-                        const float p0 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j]), a.scale_log2, neg_m));
-                        const float p1 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 1]), a.scale_log2, neg_m));
-                        const float p2 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 2]), a.scale_log2, neg_m));
-                        const float p3 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 3]), a.scale_log2, neg_m));
-                        sum4[0] = __fadd_rn(sum4[0], p0); sum4[1] = __fadd_rn(sum4[1], p1);
-                        sum4[2] = __fadd_rn(sum4[2], p2); sum4[3] = __fadd_rn(sum4[3], p3);
-                        const __nv_bfloat162 pa = __floats2bfloat162_rn(p0, p1), pb = __floats2bfloat162_rn(p2, p3);
-                        packed[j / 2] = *reinterpret_cast<const uint32_t*>(&pa);
-                        packed[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&pb);
+                    for (int h = 0; h < AP_BN; h += 32) {
+                        uint32_t packed[16];
+#pragma unroll
+                        for (int j = h; j < h + 32; j += 4) {
+                            const float p0 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j]), a.scale_log2, neg_m));
+                            const float p1 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 1]), a.scale_log2, neg_m));
+                            const float p2 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 2]), a.scale_log2, neg_m));
+                            const float p3 = ex2_hw(__fmaf_rn(__uint_as_float(sr[j + 3]), a.scale_log2, neg_m));
+                            sum4[0] = __fadd_rn(sum4[0], p0); sum4[1] = __fadd_rn(sum4[1], p1);
+                            sum4[2] = __fadd_rn(sum4[2], p2); sum4[3] = __fadd_rn(sum4[3], p3);
+                            const __nv_bfloat162 pa = __floats2bfloat162_rn(p0, p1), pb = __floats2bfloat162_rn(p2, p3);
+                            packed[(j - h) / 2] = *reinterpret_cast<const uint32_t*>(&pa);
+                            packed[(j - h) / 2 + 1] = *reinterpret_cast<const uint32_t*>(&pb);
+                        }
+                        tc_st16(p_at + h / 2, packed);
                     }
                     row_sum = __fadd_rn(__fadd_rn(sum4[0], sum4[1]), __fadd_rn(sum4[2], sum4[3]));
                 }
             }
-            if (b >= 1) {
-                ok = mbar_wait(o_done, (b - 1) & 1, abort_flag, &g_attn_tc_error);   // P is free, O is settled
+            // the O of block b - 1 is waited for where it is read or rescaled, that of block b - 2 always (a barrier's phases are not skipped)
+            const bool rescale = !run_start && __any_sync(0xffffffffu, row_live && alpha != 1.f);
+            if (b >= 2) ok = mbar_wait(o_done(b), ((b >> 1) - 1) & 1, abort_flag, &g_attn_tc_error);
+            if (!ok) break;
+            if (b >= 1 && (run_start || rescale)) {
+                ok = mbar_wait(o_done(b - 1), ((b - 1) >> 1) & 1, abort_flag, &g_attn_tc_error);
                 if (!ok) break;
                 tc_fence_after();
                 if (run_start && shared) {
@@ -639,7 +648,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                             }
                         }
                     }
-                } else if (__any_sync(0xffffffffu, alpha != 1.f)) {
+                } else if (rescale) {
 #pragma unroll 1
                     for (int c = 0; c < HD; c += 16) {
                         uint32_t o[16];
@@ -653,14 +662,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
             }
             l = __fmaf_rn(l, alpha, row_sum);
-            if (row_live) {
-                // P row: 8 chunks of 16 bytes, chunk c stored at (c ^ (row & 7)) -- the 128-byte swizzle
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) =
-                        make_uint4(packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
-                }
-            }
             // rows of V past the sequence's end hold whatever the page held before: zero them
             if (key0 + AP_BN > kv_len) {
                 ok = mbar_wait(v_full(b & 1), (b >> 1) & 1, abort_flag, &g_attn_tc_error);
@@ -672,14 +673,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const int row = first_bad + rest % (AP_BN - first_bad), h = rest / (AP_BN - first_bad);
                     *reinterpret_cast<uint4*>(vb + h * AP_BN * 128 + row * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
                 }
+                fence_proxy_async();
             }
-            fence_proxy_async();
+            tc_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full);
+            if (lane == 0) mbar_arrive(p_full(b));
             if (threadIdx.x == 0) attn_stamp(3 + 2 * b);         // p of block b handed over
         }
-        if (ok) ok = mbar_wait(o_done, (nb - 1) & 1, abort_flag, &g_attn_tc_error);
+        if (ok && nb >= 2) ok = mbar_wait(o_done(nb), ((nb >> 1) - 1) & 1, abort_flag, &g_attn_tc_error);
+        if (ok) ok = mbar_wait(o_done(nb - 1), ((nb - 1) >> 1) & 1, abort_flag, &g_attn_tc_error);
         ok = __all_sync(0xffffffffu, ok);                          // (one answer per warp for what follows)
         if (threadIdx.x == 0) attn_stamp(40);                    // the last context is complete
         T* orow = a.out + ((size_t)(tok0 + (r >> gs)) * a.n_q + head0 + (r & (gp - 1))) * HD;
