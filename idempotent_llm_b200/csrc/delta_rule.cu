@@ -13,6 +13,7 @@
 // The read-out is computed from the decayed state before the write: o = (g S)^T q + u (k . q), the same number
 // as S_new^T q, so that one round of shuffles per token serves both sums.
 #include "common.cuh"
+#include "delta_heads.cuh"
 
 // ------------------------------------------------------------------ columns of a 32-bit buffer as a matrix operand
 // out[t, c] = in[t, col0 + c] for c < width, 0 for width <= c < out_width, in the storage type
@@ -43,14 +44,15 @@ extern "C" int idm_cols_cast(const float* in, int stride, int col0, int width, v
 // x / sqrt(sum x^2 + 1e-6), q also times dk^-1/2.  a [N, a_stride]: columns [a_col, a_col + H dk) hold the decay's
 // projection and become g = exp(-exp(A_log[h]) * softplus(a + dt_bias)).  beta[t, h] = sigmoid(proj[t, b_col + h]).
 // With one decay per head (head_col >= 0) the projection is proj[t, head_col + h], dt_bias has H entries, and the
-// head's decay is written to all dk of its columns of `a`, which the recurrence reads as it reads decays per channel.
+// head's decay is written to all dk of its columns of `a`, which the recurrence reads as it reads decays per channel, or (a_dk == 1) to
+// column a_col + h alone.
 struct DeltaPrepArgs {
     float* c; int c_stride, c_q, c_k;
     float* a; int a_stride, a_col;
     const float* proj; int p_stride, b_col, head_col;
     const float* dt_bias; const float* a_log;
     float* beta;
-    int H, Hk, dk;
+    int H, Hk, dk, a_dk;                            // a_dk: columns of a head's decays
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -70,8 +72,8 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(DeltaPrepArgs p) {
         for (int d = lane; d < p.dk; d += 32) x[d] *= inv;
     }
     float* arow = p.a + (size_t)t * p.a_stride + p.a_col;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < p.H * p.dk; i += gridDim.y * blockDim.x) {
-        const int hh = i / p.dk;
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < p.H * p.a_dk; i += gridDim.y * blockDim.x) {
+        const int hh = i / p.a_dk;
         const float rate = expf(p.a_log[hh]);
         const float z = p.head_col >= 0 ? p.proj[(size_t)t * p.p_stride + p.head_col + hh] + p.dt_bias[hh] : arow[i] + p.dt_bias[i];
         arow[i] = expf(-rate * softplus_f(z));
@@ -112,7 +114,9 @@ __global__ void __launch_bounds__(128) delta_prep_vec_kernel(DeltaPrepArgs p) {
     }
     __syncthreads();
     float* arow = p.a + (size_t)t * p.a_stride + p.a_col;
-    const int quads = p.dk / 4;
+    if (p.a_dk == 1)
+        for (int h = blockIdx.y * 128 + threadIdx.x; h < p.H; h += gridDim.y * 128) arow[h] = decay[h];
+    const int quads = p.a_dk / 4;
     for (int i = blockIdx.y * 128 + threadIdx.x; i < p.H * quads; i += gridDim.y * 128) {
         const int h = i / quads;
         float4* at = reinterpret_cast<float4*>(arow) + i;
@@ -128,16 +132,17 @@ __global__ void __launch_bounds__(128) delta_prep_vec_kernel(DeltaPrepArgs p) {
 
 extern "C" int idm_delta_prep(float* c, int c_stride, int c_q, int c_k, float* a, int a_stride, int a_col,
                               const float* proj, int p_stride, int b_col, int head_col, const float* dt_bias, const float* a_log,
-                              float* beta, int H, int Hk, int dk, int n_tokens, cudaStream_t stream) {
+                              float* beta, int H, int Hk, int dk, int a_dk, int n_tokens, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
     IDM_REQUIRE(H > 0 && Hk > 0 && H % Hk == 0 && dk > 0, "delta_prep: %d heads over %d key heads of %d", H, Hk, dk);
-    DeltaPrepArgs p{c, c_stride, c_q, c_k, a, a_stride, a_col, proj, p_stride, b_col, head_col, dt_bias, a_log, beta, H, Hk, dk};
+    IDM_REQUIRE(a_dk == dk || (a_dk == 1 && head_col >= 0), "delta_prep: %d decays of a head, keys of %d", a_dk, dk);
+    DeltaPrepArgs p{c, c_stride, c_q, c_k, a, a_stride, a_col, proj, p_stride, b_col, head_col, dt_bias, a_log, beta, H, Hk, dk, a_dk};
     int split = (296 + n_tokens - 1) / n_tokens;
     const int most = (H * dk + 127) / 128;
     if (split > most) split = most;
     if (split < 1) split = 1;
-    const bool vec = dk % 4 == 0 && dk <= 128 && H <= DP_HEADS && c_stride % 4 == 0 && c_q % 4 == 0 && c_k % 4 == 0 && a_stride % 4 == 0 &&
-                     a_col % 4 == 0 && (((uintptr_t)c | (uintptr_t)a) & 15) == 0 && (head_col >= 0 || ((uintptr_t)dt_bias & 15) == 0);
+    const bool vec = dk % 4 == 0 && dk <= 128 && H <= DP_HEADS && c_stride % 4 == 0 && c_q % 4 == 0 && c_k % 4 == 0 &&
+                     (a_dk == 1 || (a_stride % 4 == 0 && a_col % 4 == 0 && ((uintptr_t)a & 15) == 0)) && ((uintptr_t)c & 15) == 0 && (head_col >= 0 || ((uintptr_t)dt_bias & 15) == 0);
     idm_launch(vec ? delta_prep_vec_kernel : delta_prep_kernel, dim3(n_tokens, split), dim3(128), 0, stream, p);
     IDM_LAUNCH_CHECK("delta_prep");
     return 0;
@@ -1144,6 +1149,39 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
     else if (dk <= 128) idm_launch(delta_scan_kernel<16>, grid, block, 0, stream, a);
     else idm_launch(delta_scan_kernel<32>, grid, block, 0, stream, a);
     IDM_LAUNCH_CHECK("delta_scan");
+    return 0;
+}
+
+// ------------------------------------------------------------------ a decay per head, chunks of 32
+// Floats of scratch that a step of `n_seqs` sequences and `n_tokens` tokens, at most `max_tokens` of one sequence, wants; 0: the step's
+// decays are wanted per channel (idm_delta_scan).  Keys of 65 to 128 channels in rows of whole 16-byte pieces, portions of more than 48 tokens.
+// Measured, us of a layer with 64 heads (32 heads), this form / the chain of chunks of 16: 8 x 12 tokens 146 / 115 (91 / 93), 8 x 40 195 / 193
+// (101 / 107), 2 x 60 114 / 120 (92 / 106), 8 x 130 337 / 402 (167 / 212), 3 x 1 000 807 / 1 094 (380 / 536).
+extern "C" long long idm_delta_heads_scratch_floats(int n_seqs, int n_tokens, int H, int Hk, int dk, int dv, int max_tokens, int c_stride, int c_q, int c_k) {
+    if (max_tokens <= 48 || n_seqs <= 0 || H <= 0 || Hk <= 0 || H % Hk || dk <= 64 || dk > DH_DK || dv <= 0) return 0;
+    if (dk % 4 || c_stride % 4 || c_q % 4 || c_k % 4 || H > 65535 || n_seqs > 65535 || Hk > 65535) return 0;
+    const long long want = ((long long)n_tokens / DH_C + n_seqs) * H * delta_heads_floats(dv);
+    return want <= DH_MOST ? want : 0;
+}
+
+// The delta rule with a decay per head, g [n_tokens, H]; scratch of idm_delta_heads_scratch_floats.
+extern "C" int idm_delta_heads(const float* c, int c_stride, int c_q, int c_k, int c_v, const float* g, const float* beta, float* state,
+                               long long state_stride, float* o, int o_stride, const int* cu_q, const int* slots, int n_seqs, int n_tokens, int H,
+                               int Hk, int dk, int dv, int max_tokens, float* scratch, cudaStream_t stream) {
+    if (n_seqs == 0 || n_tokens == 0) return 0;
+    IDM_REQUIRE(idm_delta_heads_scratch_floats(n_seqs, n_tokens, H, Hk, dk, dv, max_tokens, c_stride, c_q, c_k) > 0,
+                "delta_heads: %d heads over %d key heads, keys of %d, values of %d, %d tokens of %d sequences, columns %d and %d of rows of %d", H, Hk,
+                dk, dv, n_tokens, n_seqs, c_q, c_k, c_stride);
+    IDM_REQUIRE(state != nullptr && state_stride >= (long long)H * dk * dv, "delta_heads: a slot's state must hold %d x %d x %d floats", H, dv, dk);
+    IDM_REQUIRE(scratch != nullptr && (((uintptr_t)scratch | (uintptr_t)c) & 15) == 0, "delta_heads: scratch at %p, rows at %p", (void*)scratch, (const void*)c);
+    const DeltaHeadsScan a{c, c_stride, c_q, c_k, c_v, g, beta, state, state_stride, o, o_stride, cu_q, slots, n_seqs, H, Hk, dk, dv, scratch};
+    constexpr int chunk_smem = (int)sizeof(DeltaHeadsChunkSmem), walk_smem = (int)sizeof(DeltaHeadsWalkSmem);
+    cudaError_t e = cudaFuncSetAttribute(delta_heads_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_heads_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
+    IDM_REQUIRE(e == cudaSuccess, "delta_heads: %d bytes of shared memory were refused (%s)", walk_smem, cudaGetErrorString(e));
+    idm_launch(delta_heads_chunk_kernel, dim3(n_tokens / DH_C + n_seqs, Hk), dim3(256), chunk_smem, stream, a);
+    idm_launch(delta_heads_walk_kernel, dim3((dv + DH_COLS - 1) / DH_COLS, H, n_seqs), dim3(256), walk_smem, stream, a);
+    IDM_LAUNCH_CHECK("delta_heads");
     return 0;
 }
 

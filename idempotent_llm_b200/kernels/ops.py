@@ -72,9 +72,11 @@ SIGNATURES = {
     "idm_attention_biased": (c_int, "ppiifpppiipppiippppiiiipiiiififiipp"),
     "idm_head_finish": (c_int, "piiiipppppiiifipfiiiippppiipppip"),
     "idm_cols_cast": (c_int, "piiipiip"),
-    "idm_delta_prep": (c_int, "piiipiipiiipppiiiip"),
+    "idm_delta_prep": (c_int, "piiipiipiiipppiiiiip"),
     "idm_delta_scan": (c_int, "piiiipiippqpippiiiiiipp"),
     "idm_delta_scan_scratch_floats": (c_longlong, "iiiiii"),
+    "idm_delta_heads": (c_int, "piiiipppqpippiiiiiiipp"),
+    "idm_delta_heads_scratch_floats": (c_longlong, "iiiiiiiiii"),
     "idm_delta_out": (c_int, "pipfpiiifpiiiiip"),
     "idm_add_rmsnorm2": (c_int, "ppiqppfpppiip"),
     "idm_gemm_bf16_gated": (c_int, "pppiiiip"),
@@ -532,12 +534,28 @@ class Kernels:
                    dk: int, head_col: int = -1) -> torch.Tensor:
         """In place: q and k heads of ``c`` become unit vectors (q times ``dk ** -0.5``), columns ``a_col ..`` of ``a``
         become decays (``head_col`` >= 0: one decay per head from ``proj[:, head_col + h]``, written to all of the head's
-        columns of ``a``); returns ``beta [N, H]``."""
+        columns of ``a``, or to its one column where ``a`` holds one a head); returns ``beta [N, H]``."""
         n = c.shape[0]
+        a_dk = 1 if head_col >= 0 and a.shape[1] == H and dk > 1 else dk
         beta = torch.empty((n, H), dtype=torch.float32, device=self.device)
         self._check(self.lib.idm_delta_prep(_p(c), c.shape[1], c_q, c_k, _p(a), a.shape[1], a_col, _p(proj), proj.shape[1],
-                                            b_col, int(head_col), _p(dt_bias), _p(a_log), _p(beta), H, Hk, dk, n, self._stream()))
+                                            b_col, int(head_col), _p(dt_bias), _p(a_log), _p(beta), H, Hk, dk, a_dk, n, self._stream()))
         return beta
+
+    def delta_by_heads(self, c, c_q: int, c_k: int, ctx, H: int, Hk: int, dk: int, dv: int) -> int:
+        """Floats of scratch with which the step's delta rule runs on one decay per head (``delta_heads``); 0: it wants them per
+        channel (``delta_scan``)."""
+        return int(self.lib.idm_delta_heads_scratch_floats(ctx.n_seqs, c.shape[0], H, Hk, dk, dv, int(ctx.max_q_len), c.shape[1], c_q, c_k))
+
+    def delta_heads(self, c, c_q: int, c_k: int, c_v: int, g, beta, state, ctx, H: int, Hk: int, dk: int, dv: int, want: int) -> torch.Tensor:
+        """``delta_scan`` with one decay per head, ``g [N, H]``; ``want``: what ``delta_by_heads`` returned."""
+        n = c.shape[0]
+        o = torch.empty((n, H * dv), dtype=torch.float32, device=self.device)
+        scratch = torch.empty((want,), dtype=torch.float32, device=self.device)
+        self._check(self.lib.idm_delta_heads(_p(c), c.shape[1], c_q, c_k, c_v, _p(g), _p(beta), _p(state), self._state_stride(state), _p(o),
+                                             H * dv, _p(ctx.cu_q), _p(ctx.slots), ctx.n_seqs, n, H, Hk, dk, dv, int(ctx.max_q_len),
+                                             _p(scratch), self._stream()), 2)
+        return o
 
     def delta_scan(self, c, c_q: int, c_k: int, c_v: int, g, g_col: int, beta, state, ctx, H: int, Hk: int, dk: int,
                    dv: int) -> torch.Tensor:

@@ -138,19 +138,26 @@ class GatedDeltaRule(Mixer):
         c = K.short_conv(proj, col0, self.channels, self.w_conv, None, 1, conv_state, ctx)      # [q | k | v], silu
         if s.conv_taps > 1 and not ctx.single_token:
             K.conv_state_update(proj, col0, self.channels, s.conv_taps, conv_state, ctx)
+        # chunks of a prompt take a decay per head as it is; else it is spread over the head's channels
+        heads = K.delta_by_heads(c, 0, self.qk, ctx, s.heads, s.kv_heads, s.key_dim, s.value_dim) if self.head_decay else 0
+        decay_cols = s.heads if heads else self.decay_cols
         if self.up_weight is not None:
             low = K.cols_cast(proj, col0 + self.col_low, sum(self.ranks), self.low_width)
             ag = K.gemm_store(low, self.up_weight)                                              # [decay | gate], 32-bit
             if self.head_decay:                                                                 # (gate columns only: decays beside them)
-                g = torch.empty((proj.shape[0], self.decay_cols), dtype=torch.float32, device=proj.device)
+                g = torch.empty((proj.shape[0], decay_cols), dtype=torch.float32, device=proj.device)
             else:
                 g = ag
         else:
-            ag, g = None, torch.empty((proj.shape[0], self.decay_cols), dtype=torch.float32, device=proj.device)
+            ag, g = None, torch.empty((proj.shape[0], decay_cols), dtype=torch.float32, device=proj.device)
         beta = K.delta_prep(c, 0, self.qk, g, 0, proj, col0 + self.col_beta, self.dt_bias, self.a_log, s.heads,
                             s.kv_heads, s.key_dim, head_col=col0 + self.col_decay if self.head_decay else -1)
-        y = K.delta_scan(c, 0, self.qk, 2 * self.qk, g, 0, beta, state[:, self.conv_floats:], ctx, s.heads, s.kv_heads,
-                         s.key_dim, s.value_dim)
+        if heads:
+            y = K.delta_heads(c, 0, self.qk, 2 * self.qk, g, beta, state[:, self.conv_floats:], ctx, s.heads, s.kv_heads, s.key_dim,
+                              s.value_dim, heads)
+        else:
+            y = K.delta_scan(c, 0, self.qk, 2 * self.qk, g, 0, beta, state[:, self.conv_floats:], ctx, s.heads, s.kv_heads,
+                             s.key_dim, s.value_dim)
         if self.silu_gate:
             K.delta_out(y, self.norm, s.norm_eps, proj, col0 + self.col_gate, out_scale, out, out_col, s.heads, s.value_dim,
                         gate_act=1)

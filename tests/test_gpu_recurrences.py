@@ -203,6 +203,57 @@ def test_delta_forms_in_64_bits_and_beside_one_another(K, L, dk, dv, pad, close)
         assert a < 2e-5 and b < 2e-5 and a < 1.5 * b + 1e-7, (a, b)    # (simulated in 32 bits: 1.0 to 1.1 times, close keys among them)
 
 
+# a decay per head: chunks of 32 with one token left over or missing, keys below 128, columns that are no whole group of 16, key heads of one to
+# nine heads (a warp weighs a head: eight at a time), sequences that share places of 32 tokens, keys that lie close together
+@pytest.mark.parametrize("lens,H,Hk,dk,dv,close", [
+    ([5, 31, 32, 33, 1, 49], 4, 2, 128, 64, 0.0), ([97, 64], 6, 3, 100, 40, 0.0), ([200], 9, 1, 68, 17, 0.0), ([161, 7], 8, 2, 128, 64, 0.1),
+    ([257], 3, 3, 128, 16, 0.3)])
+def test_delta_by_heads_against_64_bits(K, lens, H, Hk, dk, dv, close):
+    n = sum(lens)
+    c, _, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 120)
+    g = torch.exp(-3.0 * _randn(n, H, seed=125).abs() ** 3)        # (some underflow within a chunk)
+    g[_randn(n, H, seed=126) > 1.5] = 1.0
+    if close:
+        c[:, cols[1]:cols[2]] = torch.nn.functional.normalize(_randn(1, Hk, dk, seed=127) + close * _randn(n, Hk, dk, seed=128), dim=-1).reshape(n, -1)
+        g.fill_(0.9999); beta.fill_(0.98)
+    c = torch.cat([c, torch.zeros(n, -c.shape[1] % 4, device="cuda")], dim=1).contiguous()    # (rows of whole pieces)
+    wide = g.repeat_interleave(dk, dim=1).contiguous()
+    start = _randn(len(lens), H * dv * dk, seed=130)
+
+    def run(c, start, lens, g=g, beta=beta):
+        ctx, state = _ctx([0] * len(lens), lens), start.clone()
+        want = K.delta_by_heads(c, *cols[:2], ctx, H, Hk, dk, dv)
+        assert want > 0
+        return K.delta_heads(c, *cols, g.contiguous(), beta.contiguous(), state, ctx, H, Hk, dk, dv, want), state
+    o, state = run(c, start, lens)
+    other = start.clone()
+    o2 = K.delta_scan(c, *cols, wide, 0, beta, other, _ctx([0] * len(lens), lens), H, Hk, dk, dv)
+    at = 0
+    for i, L in enumerate(lens):
+        S, rows = start[i].double().view(H, dv, dk).clone(), slice(at, at + L)
+        want = _delta_64(c[rows, :cols[2] + H * dv], cols, wide[rows], beta[rows], S, H, Hk, dk, dv)
+        # 32-bit sums of up to 128 products over a chain whose state does not grow; no further off than the chain of decays per channel
+        for mine, theirs, ref in ((o[rows], o2[rows], want), (state[i].view(H, dv, dk), other[i].view(H, dv, dk), S)):
+            a, b = helpers.rel_err(mine, ref), helpers.rel_err(theirs, ref)
+            assert a < 2e-5 and a < 1.5 * b + 1e-7, (i, a, b)
+        alone = run(c[rows].contiguous(), start[i:i + 1], [L], g[rows], beta[rows]) if L > 48 else None
+        assert alone is None or (torch.equal(alone[0], o[rows]) and torch.equal(alone[1][0], state[i]))
+        at += L
+    # a later token that is not a number leaves the ones before it alone, in the sequence before it in the step too; a value that is
+    # infinite reaches its own column and goes on as a number, as sums of products make it
+    bad, last = c.clone(), lens[0] - 1
+    bad[last] = float("nan")
+    o3, state3 = run(bad, start, lens)
+    assert torch.equal(o3[:last], o[:last]) and torch.isnan(o3[last]).all() and torch.isnan(state3[0]).all()
+    assert torch.equal(o3[lens[0]:], o[lens[0]:]) and torch.equal(state3[1:], state[1:])
+    bad = c.clone()
+    bad[last, cols[2]] = float("inf")                               # head 0, column 0 of its last token
+    o4, state4 = run(bad, start, lens)
+    keep = torch.ones(H * dv, dtype=torch.bool, device="cuda"); keep[0] = False
+    assert torch.equal(o4[:last], o[:last]) and helpers.rel_err(o4[:, keep], o[:, keep].double()) < 1e-5
+    assert torch.isinf(o4[last, 0]) and torch.isinf(state4[0].view(H, dv, dk)[0, 0]).all()
+
+
 def test_delta_scratch_is_for_the_tokens_that_are_there(K):
     """One portion among many single tokens, and many sequences of many heads: nothing is sized by the longest portion times all."""
     for lens, H in (([300] + [1] * 63, 32), ([40] * 64, 64)):
