@@ -1156,11 +1156,11 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
 // Floats of scratch that a step of `n_seqs` sequences and `n_tokens` tokens, at most `max_tokens` of one sequence, wants; 0: the step's
 // decays are wanted per channel (idm_delta_scan).  Keys of 65 to 128 channels in rows of whole 16-byte pieces, portions of more than 48 tokens.
 // Measured, us of a layer with 64 heads (32 heads), this form / the chain of chunks of 16: 8 x 12 tokens 146 / 115 (91 / 93), 8 x 40 195 / 193
-// (101 / 107), 2 x 60 114 / 120 (92 / 106), 8 x 130 337 / 402 (167 / 212), 3 x 1 000 807 / 1 094 (380 / 536).
+// (101 / 107), 2 x 60 117 / 121 (92 / 103), 8 x 130 308 / 403 (152 / 212), 3 x 1 000 717 / 1 097 (335 / 538).
 extern "C" long long idm_delta_heads_scratch_floats(int n_seqs, int n_tokens, int H, int Hk, int dk, int dv, int max_tokens, int c_stride, int c_q, int c_k) {
     if (max_tokens <= 48 || n_seqs <= 0 || H <= 0 || Hk <= 0 || H % Hk || dk <= 64 || dk > DH_DK || dv <= 0) return 0;
     if (dk % 4 || c_stride % 4 || c_q % 4 || c_k % 4 || H > 65535 || n_seqs > 65535 || Hk > 65535) return 0;
-    const long long want = ((long long)n_tokens / DH_C + n_seqs) * H * delta_heads_floats(dv);
+    const long long want = ((long long)n_tokens / DH_C + n_seqs) * (delta_heads_chunk_bytes(H, Hk, dv) / 4);
     return want <= DH_MOST ? want : 0;
 }
 
@@ -1174,12 +1174,12 @@ extern "C" int idm_delta_heads(const float* c, int c_stride, int c_q, int c_k, i
                 dk, dv, n_tokens, n_seqs, c_q, c_k, c_stride);
     IDM_REQUIRE(state != nullptr && state_stride >= (long long)H * dk * dv, "delta_heads: a slot's state must hold %d x %d x %d floats", H, dv, dk);
     IDM_REQUIRE(scratch != nullptr && (((uintptr_t)scratch | (uintptr_t)c) & 15) == 0, "delta_heads: scratch at %p, rows at %p", (void*)scratch, (const void*)c);
-    const DeltaHeadsScan a{c, c_stride, c_q, c_k, c_v, g, beta, state, state_stride, o, o_stride, cu_q, slots, n_seqs, H, Hk, dk, dv, scratch};
+    const DeltaHeadsScan a{c, c_stride, c_q, c_k, c_v, g, beta, state, state_stride, o, o_stride, cu_q, slots, n_seqs, H, Hk, dk, dv, (char*)scratch};
     constexpr int chunk_smem = (int)sizeof(DeltaHeadsChunkSmem), walk_smem = (int)sizeof(DeltaHeadsWalkSmem);
     cudaError_t e = cudaFuncSetAttribute(delta_heads_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_heads_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
     IDM_REQUIRE(e == cudaSuccess, "delta_heads: %d bytes of shared memory were refused (%s)", walk_smem, cudaGetErrorString(e));
-    idm_launch(delta_heads_chunk_kernel, dim3(n_tokens / DH_C + n_seqs, Hk), dim3(256), chunk_smem, stream, a);
+    idm_launch(delta_heads_chunk_kernel, dim3(n_tokens / DH_C + n_seqs, Hk), dim3(DH_THREADS), chunk_smem, stream, a);
     idm_launch(delta_heads_walk_kernel, dim3((dv + DH_COLS - 1) / DH_COLS, H, n_seqs), dim3(256), walk_smem, stream, a);
     IDM_LAUNCH_CHECK("delta_heads");
     return 0;

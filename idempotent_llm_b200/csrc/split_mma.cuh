@@ -109,7 +109,34 @@ struct SplitSum {
     __device__ __forceinline__ float sum(int j, int i) const { return big[j][i] + small[j][i]; }
 };
 
-// four neighbours into the three planes, at an 8-byte border
+// the same with three sums (by the products' sizes): no instruction waits for the one before it where a warp has few tiles
+template <int N>
+struct SplitSum3 {
+    float big[N][4], mid[N][4], low[N][4];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) big[j][i] = mid[j][i] = low[j][i] = 0.f;
+    }
+    __device__ __forceinline__ void add(int j, const SplitA& a, const SplitB& b) {
+        mma_bf16(big[j], a.p[0], b.p[0][0], b.p[0][1]);
+        mma_bf16(big[j + 1], a.p[0], b.p[0][2], b.p[0][3]);
+        mma_bf16(low[j], a.p[0], b.p[2][0], b.p[2][1]);
+        mma_bf16(low[j + 1], a.p[0], b.p[2][2], b.p[2][3]);
+        mma_bf16(mid[j], a.p[0], b.p[1][0], b.p[1][1]);
+        mma_bf16(mid[j + 1], a.p[0], b.p[1][2], b.p[1][3]);
+        mma_bf16(low[j], a.p[1], b.p[1][0], b.p[1][1]);
+        mma_bf16(low[j + 1], a.p[1], b.p[1][2], b.p[1][3]);
+        mma_bf16(mid[j], a.p[1], b.p[0][0], b.p[0][1]);
+        mma_bf16(mid[j + 1], a.p[1], b.p[0][2], b.p[0][3]);
+        mma_bf16(low[j], a.p[2], b.p[0][0], b.p[0][1]);
+        mma_bf16(low[j + 1], a.p[2], b.p[0][2], b.p[0][3]);
+    }
+    __device__ __forceinline__ float sum(int j, int i) const { return big[j][i] + (mid[j][i] + low[j][i]); }
+};
+
+// four neighbours into the three planes (shared memory or scratch), at an 8-byte border
 __device__ __forceinline__ void store_split4(__nv_bfloat16* at, int plane, float4 x) {
     uint32_t a[3], b[3];
     split3(x.x, x.y, a[0], a[1], a[2]);
