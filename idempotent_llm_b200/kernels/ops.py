@@ -28,8 +28,10 @@ from __future__ import annotations
 import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from operator import itemgetter
 from typing import Optional
 
+import numpy as np
 import torch
 
 from . import builder
@@ -235,6 +237,11 @@ class Kernels:
             raise KernelError(f"{what}: expected a contiguous CUDA tensor of {dtype}, got {t.dtype} "
                               f"{'cuda' if t.is_cuda else 'cpu'} contiguous={t.is_contiguous()}")
 
+    def _uploaded(self, numbers) -> torch.Tensor:
+        """A step's list of integers on the device.  The copy is from pageable memory: the call returns when the numbers are staged, and
+        the host does not wait for the GPU (waiting, a step of a few long kernels cost the gap until its next launch)."""
+        return torch.from_numpy(np.array(numbers, dtype=np.int32)).to(self.device, non_blocking=True)
+
     def scratch(self, key: str, n_floats: int) -> torch.Tensor:
         """A 32-bit scratch buffer that only grows (its address is stable across steps once large enough)."""
         buf = self._scratch.get(key)
@@ -376,7 +383,7 @@ class Kernels:
                 at += n
                 first.append(len(borders))
             borders.append(at)
-            dev = torch.tensor(borders + first, dtype=torch.int32).to(self.device)
+            dev = self._uploaded(borders + first)
             plan = ctx.memo[key] = (dev, dev[:len(borders)], dev[len(borders):], len(borders) - 1)
         return plan
 
@@ -791,32 +798,32 @@ class Kernels:
         if tiles is None:
             # (sequence, first token of the tile); tiles with the most keys first, so that the longest
             # blocks start first
-            items = []
-            for i, L in enumerate(ctx.host_q_lens):
-                for st in range(0, L, tok):
-                    first, last = ctx.host_starts[i] + st, ctx.host_starts[i] + min(st + tok - 1, L - 1)
-                    left_out = (first - first % chunk) // (self.page * R) * (self.page * R) if chunk else 0
-                    items.append((last - left_out, i, st))             # (the tile's last position counted from its first run)
-            items.sort(key=lambda t: -t[0])
+            items, page, run = [], self.page, self.page * R
+            for i, (L, at) in enumerate(zip(ctx.host_q_lens, ctx.host_starts)):
+                end = at + L
+                for first in range(at, end, tok):                      # (the tile's last position counted from its first run)
+                    left_out = (first - first % chunk) // run * run if chunk else 0
+                    items.append(((first + tok if first + tok < end else end) - 1 - left_out, i, first - at))
+            items.sort(key=itemgetter(0), reverse=True)                # (tiles of equal length stay in order)
             rows_cap = min(tok, max(ctx.host_q_lens)) * gp
             # Tiles with more key blocks than a fair share of the step's are shared by several blocks, each
             # walking `per` runs and leaving every run's result in a pool; the last block to arrive folds them
             # in the order of the runs (the same bits as one block walking them all: the runs are the same).
             n_hg = n_q // gp
-            blocks_of = [last // self.page + 1 for last, _, _ in items]
+            blocks_of = [last // page + 1 for last, _, _ in items]
             fair = -(-int(sum(blocks_of) * n_hg * self.attention_share_scale) // (2 * self.sm_count))
             per = max(self.attention_share_min_runs, -(-fair // R))   # runs a block walks
             pool, slots_used, max_parts = [], 0, 1
+            share_tiles, most = self.attention_share_tiles and rows_cap == 128, self.attention_pool_slots
             for nb in blocks_of:
                 runs = -(-nb // R)
-                if self.attention_share_tiles and rows_cap == 128 and runs > per and slots_used + runs * n_hg <= self.attention_pool_slots:
+                if share_tiles and runs > per and slots_used + runs * n_hg <= most:
                     pool.append(slots_used)
                     slots_used += runs * n_hg
                     max_parts = max(max_parts, -(-runs // per))
                 else:
                     pool.append(-1)
-            host = torch.tensor([[i for _, i, _ in items], [st for _, _, st in items], pool], dtype=torch.int32)
-            dev = host.to(self.device)
+            dev = self._uploaded([i for _, i, _ in items] + [st for _, _, st in items] + pool).view(3, len(items))
             plan = (dev[2].data_ptr(), max_parts, per, slots_used) if slots_used else (None, 0, 0, 0)
             tiles = ctx.memo[memo_key] = (dev, dev[0].data_ptr(), dev[1].data_ptr(), len(items), rows_cap, plan)
         _, tile_seq, tile_start, n_tiles, rows_cap = tiles[:5]
