@@ -316,6 +316,229 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
     }
 }
 
+// ------------------------------------------------------------------------------------------------------ many tokens
+// The same sums where there are tokens enough: the tokens' parts are made once, by a kernel in front, for all the feature tiles that meet them,
+// and come as tiles by TMA; a block has 128 features and SUBS times 64 tokens, so that a split weight meets all of them.  A segment's
+// 64 tokens are an accumulator's, as above: with SUBS of 2 the two take turns in tensor memory, with 1 neighbouring segments do.
+// Eight warps split the weight, eight add up 64 tokens, one thread issues the MMAs and one the copies.
+// Bound by shared memory: a segment's 128 tokens move 192 KB into the MMAs, 48 in from the weight's split and 48 from the copies, 1.2 of
+// the 1.4 us it takes (64 tokens: 0.95 us, of which some 0.7).  700 tokens: 4096 x 1024 55 us (split by every tile 62), 6144 x 1024 56 (81), 1024 x
+// 3072 54 (58); 1 400 tokens: 79 (100), 103 (157), 77 (112).
+#define GW_CONV 256
+template <int SUBS> struct WideTile {
+    static constexpr int ADD = SUBS * GX_ADD, THREADS = ADD + GW_CONV + 64, WARP_MMA = (ADD + GW_CONV) / 32;
+    static constexpr int AHEAD = SUBS == 1 ? 2 : 1;                            // segments of the weight on their way in registers
+    static constexpr int A = GX_FEATURES * 128, PART = 64 * 128, B = 3 * PART;     // bytes: one part of the weight, of 64 tokens; 64 tokens' parts
+    static constexpr int STAGE = 3 * A + SUBS * B;
+};
+
+// parts [3][M][Kp] of x [M][K], zeros from K to Kp (a multiple of 64)
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ parts, int M, int K, int Kp, int vec) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int quads = Kp / 4;
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= (long long)M * quads) return;
+    const int m = (int)(i / quads), k = (int)(i - (long long)m * quads) * 4;
+    const float* p = x + (size_t)m * K + k;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+        if (k < K) v = *reinterpret_cast<const float4*>(p);
+    } else {
+        if (k < K) v.x = p[0];
+        if (k + 1 < K) v.y = p[1];
+        if (k + 2 < K) v.z = p[2];
+        if (k + 3 < K) v.w = p[3];
+    }
+    uint2 part[3];
+    split_four(v, part);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(parts + ((size_t)j * M + m) * Kp + k) = part[j];
+}
+
+template <int SUBS, int ROWS>
+__global__ void __launch_bounds__(WideTile<SUBS>::THREADS, 1) gemm_f32_wide_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restrict__ x,
+                                                                      const float* __restrict__ w, float* __restrict__ out, int M, int N, int K,
+                                                                      int token_tiles, int tiles) {
+    using S = WideTile<SUBS>;
+    constexpr int TN = 64;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) unsigned long long bars_mem[8];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_mem;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem_u32(bars_mem);
+    uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+    auto full = [&](int b) { return bars + 8u * b; };
+    auto empty = [&](int b) { return bars + 8u * (2 + b); };
+    auto acc_full = [&](int b) { return bars + 8u * (4 + b); };
+    auto acc_empty = [&](int b) { return bars + 8u * (6 + b); };
+    volatile int* abort_flag = &abort_mem;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, segs = (K + GX_SEG - 1) / GX_SEG;
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(full(b), GW_CONV / 32 + 1); mbar_init(empty(b), 1);
+            mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), GX_ADD / 32);
+        }
+        abort_mem = 0;
+        mbar_init_fence();
+    }
+    if (warp == S::WARP_MMA) tmem_alloc(smem_u32(&tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();               // (behind the allocation: a block of the next kernel cannot hold what this one waits for)
+    // the n-th segment of a block (over all its tiles) is in stage n & 1; its tokens' sums in accumulator (SUBS == 2 ? which 64 of them : n & 1)
+    auto acc_of = [&](int n, int sub) { return SUBS == 2 ? sub : n & 1; };
+    auto acc_turn = [&](int n) { return (SUBS == 2 ? n : n >> 1) & 1; };
+
+    if (warp >= S::ADD / 32 && warp < S::WARP_MMA) {
+        // ------------------------------------------------------------ the weight: 32-bit from memory, three parts into the stage
+        // a thread has four k of rows row, row + 16, ...: sixteen threads read a row's 256 bytes side by side
+        constexpr int ROUNDS = GX_FEATURES / 16;
+        const int ct = threadIdx.x - S::ADD, row = ct >> 4, piece = ct & 15;
+        float4 raw[S::AHEAD][ROUNDS];
+        auto load = [&](float4 (&v)[ROUNDS], int tile, int seg) {              // (rows behind the end are the last one again: their outputs are dropped)
+            const int f = tile / token_tiles * GX_FEATURES + row, k = seg * GX_SEG + piece * 4, left = K - k;
+#pragma unroll
+            for (int i = 0; i < ROUNDS; ++i) {
+                const float* p = w + (size_t)min(f + 16 * i, N - 1) * K + k;
+                if (ROWS == 2) v[i] = __ldcg(reinterpret_cast<const float4*>(p));
+                else if (ROWS == 1) v[i] = left > 0 ? __ldcg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                else v[i] = make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+            }
+        };
+        int tile = blockIdx.x, seg = 0, have = 0;                              // the next segment to ask for, and how many have been
+        auto ask = [&](float4 (&v)[ROUNDS]) {
+            if (tile >= tiles) return;
+            load(v, tile, seg);
+            ++have;
+            if (++seg == segs) { seg = 0; tile += gridDim.x; }
+        };
+        ask(raw[0]);                       // (no kernel writes a weight: nothing to wait for)
+        if (S::AHEAD == 2) ask(raw[S::AHEAD - 1]);
+        const uint32_t off = (uint32_t)(row * 128 + (((piece >> 1) ^ (row & 7)) << 4) + (piece & 1) * 8);   // (row + 16 i: the same place in its swizzle atom)
+        for (int turn = 0; have > 0; turn ^= 1) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (have == 0) break;
+                if (!mbar_wait(empty(b), turn ^ 1, abort_flag, &g_gemm_f32_error)) { have = 0; break; }
+                uint8_t* stage = gen + b * S::STAGE + off;
+#pragma unroll
+                for (int i = 0; i < ROUNDS; ++i) {
+                    uint2 part[3];
+                    split_four(raw[b % S::AHEAD][i], part);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(stage + p * S::A + i * 2048) = part[p];
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full(b));
+                --have;
+                ask(raw[b % S::AHEAD]);
+            }
+        }
+    } else if (warp == S::WARP_MMA + 1) {
+        // ------------------------------------------------------------ the tokens' parts, by TMA
+        pdl_wait();
+        if (lane == 0) {
+            int n = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+                for (int seg = 0; ok && seg < segs; ++seg, ++n) {
+                    const int b = n & 1;
+                    ok = mbar_wait(empty(b), ((n >> 1) & 1) ^ 1, abort_flag, &g_gemm_f32_error);
+                    if (!ok) break;
+                    mbar_expect_tx(full(b), SUBS * S::B);
+#pragma unroll
+                    for (int i = 0; i < 3 * SUBS; ++i)
+                        tma_load_3d(base + b * S::STAGE + 3 * S::A + i * S::PART, &map_x, seg * GX_SEG,
+                                    tile % token_tiles * (TN * SUBS) + i / 3 * TN, i % 3, full(b));
+                }
+        }
+        __syncwarp();
+    } else if (warp == S::WARP_MMA) {
+        // ------------------------------------------------------------ MMAs: products of parts, by size into three sums
+        if (lane == 0) {
+            const uint32_t three = umma_idesc(GX_FEATURES, 3 * TN), two = umma_idesc(GX_FEATURES, 2 * TN), one = umma_idesc(GX_FEATURES, TN);
+            int n = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+                for (int seg = 0; ok && seg < segs; ++seg, ++n) {
+                    const int b = n & 1;
+                    ok = mbar_wait(full(b), (n >> 1) & 1, abort_flag, &g_gemm_f32_error);
+                    const uint32_t a = base + b * S::STAGE;
+                    const uint64_t a1 = umma_desc_kmajor(a), a2 = umma_desc_kmajor(a + S::A), a3 = umma_desc_kmajor(a + 2 * S::A);
+                    for (int sub = 0; ok && sub < SUBS; ++sub) {
+                        const int acc = acc_of(n, sub);
+                        ok = mbar_wait(acc_empty(acc), acc_turn(n) ^ 1, abort_flag, &g_gemm_f32_error);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t d = tmem + acc * 3 * TN;
+                        const uint64_t t = umma_desc_kmajor(a + 3 * S::A + sub * S::B);   // the token parts' rows one after another
+                        tc_mma_bf16_kblock(d, a1, t, three, 0);                // w1 x1 | w1 x2 | w1 x3
+                        tc_mma_bf16_kblock(d + TN, a2, t, two, 1);             //       + w2 x1 | w2 x2
+                        tc_mma_bf16_kblock(d + 2 * TN, a3, t, one, 1);         //               + w3 x1
+                        if (sub == SUBS - 1) tc_commit(empty(b));
+                        tc_commit(acc_full(acc));
+                    }
+                }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------ segments, one after another
+        // (with SUBS of 2 eight warps for each 64 tokens)
+        constexpr int COLS = TN / 2;
+        float tot[COLS];
+        int n = 0;
+        bool ok = true;
+        const int sub = warp >> 3, mine = (warp & 3) * 32 + lane, c0 = (warp >> 2 & 1) * COLS;
+        pdl_wait();                        // (the kernel before may still read what is written here)
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) tot[j] = 0.f;
+            for (int seg = 0; seg < segs; ++seg, ++n) {
+                const int acc = acc_of(n, sub);
+                ok = mbar_wait(acc_full(acc), acc_turn(n), abort_flag, &g_gemm_f32_error);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t big = tmem + ((uint32_t)((warp & 3) * 32) << 16) + acc * 3 * TN + c0;
+#pragma unroll
+                for (int c = 0; c < COLS; c += 8) {
+                    uint32_t u[8], v[8], z[8];
+                    tc_ld8_issue(big + c, u); tc_ld8_issue(big + TN + c, v); tc_ld8_issue(big + 2 * TN + c, z);
+                    tc_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) tot[c + j] += __uint_as_float(u[j]) + (__uint_as_float(v[j]) + __uint_as_float(z[j]));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(acc));
+            }
+            const int f = tile / token_tiles * GX_FEATURES + mine, m0 = tile % token_tiles * (TN * SUBS) + sub * TN + c0;
+            if (ok && f < N)
+#pragma unroll
+                for (int j = 0; j < COLS; ++j)
+                    if (m0 + j < M) {
+                        float s = tot[j];
+                        if (!isfinite(s)) s = plain_sum(x + (size_t)(m0 + j) * K, w + (size_t)f * K, K);
+                        out[(size_t)(m0 + j) * N + f] = s;
+                    }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == S::WARP_MMA) tmem_dealloc(tmem, 512);
+    if (abort_mem != 0)                    // a wait ran out: none of the block's outputs passes for a number
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+            for (int at = threadIdx.x; at < GX_FEATURES * TN * SUBS; at += S::THREADS) {
+                const int f = tile / token_tiles * GX_FEATURES + at % GX_FEATURES, m = tile % token_tiles * (TN * SUBS) + at / GX_FEATURES;
+                if (f < N && m < M) out[(size_t)m * N + f] = __int_as_float(0x7fffffff);
+            }
+}
+
 // ------------------------------------------------------------------------------------------------------ launches
 template <int TN> static long long split_smem(int K, int split) {
     const long long segs = (K + GX_SEG - 1) / GX_SEG, per = (GX_FEATURES + split - 1) / split;
@@ -354,24 +577,78 @@ template <int TN> static void split_cost(int M, int N, int K, int sms, float per
     }
 }
 
-extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
-    if (M == 0 || N == 0) return 0;
-    IDM_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
-    const int rows = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
+struct F32Choice { int tn, split, subs; };                    // subs > 0: gemm_f32_wide_kernel with so many times 64 tokens
+static F32Choice f32_choice(int M, int N, int K) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 148;
-    int tn = 64, split = 1;
+    F32Choice c{64, 1, 0};
     float best = 1e30f;
-    if (M <= 16) split_cost<16>(M, N, K, sms, 0.95f, tn, split, best);
-    else {
-        split_cost<32>(M, N, K, sms, 0.95f, tn, split, best);
-        split_cost<64>(M, N, K, sms, 1.15f, tn, split, best);
+    if (M <= 16) {
+        split_cost<16>(M, N, K, sms, 0.95f, c.tn, c.split, best);
+        return c;
     }
-    const int rc = tn == 16 ? split_launch<16>(x, w, out, M, N, K, rows, split, sms, stream)
-                 : tn == 32 ? split_launch<32>(x, w, out, M, N, K, rows, split, sms, stream)
-                            : split_launch<64>(x, w, out, M, N, K, rows, split, sms, stream);
+    split_cost<32>(M, N, K, sms, 0.95f, c.tn, c.split, best);
+    split_cost<64>(M, N, K, sms, 1.15f, c.tn, c.split, best);
+    // measured: 1.0 us a segment of 64 tokens and 1.4 of 128 with all SMs at it, and 5 us for the kernel in front and the start
+    const long long features = (N + GX_FEATURES - 1) / GX_FEATURES, segs = (K + GX_SEG - 1) / GX_SEG;
+    for (int subs = 1; subs <= 2; ++subs) {
+        const long long tiles = features * ((M + 64 * subs - 1) / (64 * subs));
+        const float t = (float)((tiles + sms - 1) / sms * segs) * (subs == 1 ? 1.0f : 1.5f) + 5.f;
+        if (t < best) { best = t; c.subs = subs; }
+    }
+    return c;
+}
+
+// Bytes of scratch that a product wants: the parts of x, or 0
+extern "C" long long idm_gemm_f32_scratch_bytes(int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0 || f32_choice(M, N, K).subs == 0) return 0;
+    return 3ll * M * ((K + GX_SEG - 1) / GX_SEG * GX_SEG) * 2;
+}
+
+template <int SUBS>
+static int wide_launch(const float* x, const float* w, float* out, int M, int N, int K, int rows, void* scratch, cudaStream_t stream) {
+    const int Kp = (K + GX_SEG - 1) / GX_SEG * GX_SEG, bytes = 1024 + 2 * WideTile<SUBS>::STAGE;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 148;
+    auto kernel = rows == 0 ? gemm_f32_wide_kernel<SUBS, 0> : rows == 1 ? gemm_f32_wide_kernel<SUBS, 1> : gemm_f32_wide_kernel<SUBS, 2>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    IDM_REQUIRE(e == cudaSuccess, "gemm_f32: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+    const int token_tiles = (M + 64 * SUBS - 1) / (64 * SUBS);
+    const long long tiles = (long long)token_tiles * ((N + GX_FEATURES - 1) / GX_FEATURES), pieces = (long long)M * (Kp / 4);
+    IDM_REQUIRE(tiles < (1ll << 30) && pieces < (1ll << 38), "gemm_f32: M=%d N=%d K=%d are too large for one launch", M, N, K);
+    CUtensorMap map;
+    const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)M, 3}, strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)M * Kp * 2};
+    const cuuint32_t box[3] = {GX_SEG, 64, 1};
+    const int rc = tc_make_map_bf16(&map, scratch, 3, dims, strides, box);
+    IDM_REQUIRE(rc == 0, "gemm_f32: no tensor map for %d x %d parts (%d)", M, Kp, rc);
+    idm_launch(split_rows_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, x, (__nv_bfloat16*)scratch, M, K, Kp,
+               (int)(K % 4 == 0 && ((uintptr_t)x & 15) == 0));
+    idm_launch(kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(WideTile<SUBS>::THREADS), bytes, stream, map, x, w, out, M, N, K, token_tiles, (int)tiles);
+    return 0;
+}
+
+// scratch: idm_gemm_f32_scratch_bytes, on a 16-byte border
+extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, void* scratch, cudaStream_t stream) {
+    if (M == 0 || N == 0) return 0;
+    IDM_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
+    const F32Choice c = f32_choice(M, N, K);
+    int dev = 0, sms = 0, rc;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (c.subs) {
+        IDM_REQUIRE(scratch != nullptr && ((uintptr_t)scratch & 15) == 0, "gemm_f32: scratch at %p", scratch);
+        const int rows = K % 4 == 0 && ((uintptr_t)w & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
+        rc = c.subs == 1 ? wide_launch<1>(x, w, out, M, N, K, rows, scratch, stream) : wide_launch<2>(x, w, out, M, N, K, rows, scratch, stream);
+    } else {
+        const int rows = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
+        rc = c.tn == 16 ? split_launch<16>(x, w, out, M, N, K, rows, c.split, sms, stream)
+           : c.tn == 32 ? split_launch<32>(x, w, out, M, N, K, rows, c.split, sms, stream)
+                        : split_launch<64>(x, w, out, M, N, K, rows, c.split, sms, stream);
+    }
     if (rc) return rc;
     IDM_LAUNCH_CHECK("gemm_f32");
     return 0;

@@ -135,7 +135,8 @@ SIGNATURES = {
     "idm_act_cast": (c_int, "ppqip"),
     "idm_concat_cast": (c_int, "ppiqppiip"),
     "idm_logit_cap": (c_int, "pqffp"),
-    "idm_gemm_f32": (c_int, "pppiiip"),
+    "idm_gemm_f32": (c_int, "pppiiipp"),
+    "idm_gemm_f32_scratch_bytes": (c_longlong, "iii"),
     "idm_gemm_set_small": (None, "iii"),
     "idm_gemm_set_small_max": (None, "i"),
     "idm_gemm_set_small_tiles": (None, "i"),
@@ -959,7 +960,9 @@ class Kernels:
                 raise KernelError(f"gemm: output {tuple(out.shape)} does not match the product {(M, N)}")
         if M:
             if self.dtype == torch.float32:
-                self._check(self.lib.idm_gemm_f32(_p(x), _p(w), _p(out), M, N, Kd, self._stream()))
+                want = int(self.lib.idm_gemm_f32_scratch_bytes(M, N, Kd)) if M > 16 else 0
+                scratch = torch.empty((want,), dtype=torch.uint8, device=self.device) if want else None
+                self._check(self.lib.idm_gemm_f32(_p(x), _p(w), _p(out), M, N, Kd, _p(scratch), self._stream()), 2 if want else 1)
             else:
                 self._check(self.lib.idm_gemm_bf16(_p(x), _p(w), _p(out), M, N, Kd, self._stream()))
         return out

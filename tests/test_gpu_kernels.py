@@ -647,6 +647,23 @@ def test_gemm_32_bit_is_one_sum_in_every_kernel(kernels, M, N, K_):
     assert torch.equal(half, out[:, :N // 2])
 
 
+# products of tokens enough for parts made in front: 64 and 128 tokens a block, rows and inner sizes that end inside tiles and segments, several
+# tiles a block, rows of x and of the weight on and off 16-byte borders; a row's bits are those that sixteen rows get
+@pytest.mark.parametrize("M,N,K_", [(1300, 1100, 1030), (1291, 1100, 1032), (700, 4096, 1024), (577, 4200, 1100), (4200, 260, 640), (641, 1024, 3072)])
+def test_gemm_32_bit_of_many_tokens_is_the_same_sum(kernels, M, N, K_):
+    k = kernels("float32")
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = torch.randn(M, K_, generator=g, device="cuda"), torch.randn(N, K_, generator=g, device="cuda")
+    x[M - 1, K_ - 1] = float("inf")                                    # (an output that is not finite is made again of plain FMAs)
+    assert int(k.lib.idm_gemm_f32_scratch_bytes(M, N, K_)) > 0
+    out = k.gemm_store(x, w)
+    for rows in (slice(0, 16), slice(60, 70), slice(M // 2, M // 2 + 7), slice(M - 9, M)):
+        assert torch.equal(out[rows], k.gemm_store(x[rows].contiguous(), w))
+    want = x[:M - 1].double() @ w.double().T
+    assert helpers.rel_err(out[:M - 1], want) < 1e-6                   # (0.3e-8 of the rows' norms, as the tiles that split both operands)
+    assert torch.isinf(out[M - 1]).all()
+
+
 @pytest.mark.parametrize("M,K_", [(5, 512), (40, 130), (700, 64)])
 def test_gemm_32_bit_with_numbers_that_have_no_parts(kernels, M, K_):
     """Infinities, not-a-numbers and the ends of the range: what plain 32-bit sums give, and the neighbours' bits as without them."""
