@@ -10,7 +10,7 @@
 //
 // so the work is what a chunk adds to the state (chunk_state_kernel), the chunks' states one after another
 // (chunk_carry_kernel: S_in of every chunk, from and to the sequence's state), and the read-outs (chunk_out_kernel).  The
-// sums are those of the token by token walk in another order; everything is 32-bit multiply-adds, which is what bounds it.
+// sums are those of the token by token walk in another order; everything is 32-bit, multiply-adds in the read-outs, which is what bounds them.
 //
 // A thread block has (chunk, group) and some of the group's panels (chunk_cut): a panel is 64 columns of one head's values.  What a
 // panel does not depend on is done once for all of them: the keys' tile, the queries' tile and the pair scores k_s . q_t
@@ -24,7 +24,7 @@
 //   store_end(Head&, chunk, head, n), end_factor(chunk, head, n)     F(n-1, -1), stored by chunk_state_kernel, read by the carry
 //   finish(t, head, j, o, v)                     what goes out for column j of a head's read-out o, given the token's v
 #pragma once
-#include "common.cuh"
+#include "split_mma.cuh"
 
 #define CP_C 64                 // tokens of a chunk
 #define CP_LD 68                // row stride of a tile of 64 columns in shared memory (16-byte rows, banks spread)
@@ -83,80 +83,147 @@ __device__ __forceinline__ void store_row4(float* p, const float* x, int left, i
         if (k < left) p[k] = x[k];
 }
 
-// chunk_state[c, head, d, j] = sum_s end(s) k_s[d] v_s[j]: 128 dims at a time, 8 x 4 of them a thread
-static int chunk_state_smem() { return (64 * (128 + 4) + 2 * CP_TILE) * (int)sizeof(float); }
+#define CS_LD 72                // row stride of a tile of 64 columns in three planes, bfloat16 (an odd number of 16-byte pieces)
+#define CS_LDK 136              // of a tile of 128 columns
+#define CS_PLANE (64 * CS_LD)
+#define CS_PLANE_K (64 * CS_LDK)
+// A tile of 64 x 64 numbers on its way: rows r < n_rows at src + r * ld, columns c < n_cols, zeros elsewhere.  A thread brings 16 of them as
+// they are into a place of its own by asynchronous copies (issue), and later, behind its own wait alone, lays their parts down (split).
+struct TileFrom { const float* src; size_t ld; int n_rows, n_cols; };
+__device__ __forceinline__ void cs_issue(float* raw, const TileFrom& f, int vec) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int e = threadIdx.x + u * CP_THREADS, r = e >> 4, c = (e & 15) * 4;
+        float* to = raw + e * 4;
+        const float* from = f.src + (size_t)r * f.ld + c;
+        const int left = r < f.n_rows ? f.n_cols - c : 0;
+        if (vec) {                                           // (whole pieces are there or not)
+            if (left > 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+            else *reinterpret_cast<float4*>(to) = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) to[i] = i < left ? from[i] : 0.f;
+        }
+    }
+}
+// dst: the first of three planes of 64 rows, LD apart.  SCALE: times scale[row]
+template <int LD, bool SCALE>
+__device__ __forceinline__ void cs_split(__nv_bfloat16* dst, const float* raw, const float* scale) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int e = threadIdx.x + u * CP_THREADS, r = e >> 4, c = (e & 15) * 4;
+        float4 x = *reinterpret_cast<const float4*>(raw + e * 4);
+        if (SCALE) { const float f = scale[r]; x = make_float4(x.x * f, x.y * f, x.z * f, x.w * f); }
+        store_split4(dst + r * LD + c, 64 * LD, x);
+    }
+}
+// planes of 64 x 128 and of 64 x 64 numbers, and two tiles on their way.  Two blocks an SM.
+struct ChunkStateSmem {
+    __nv_bfloat16 wide[3 * CS_PLANE_K];
+    __nv_bfloat16 tile[3 * CS_PLANE];
+    float raw[2][64 * 64];
+};
+
+// chunk_state[c, head, d, j] = sum_s end(s) k_s[d] v_s[j], 128 dims at a time, of which a warp has 32, and 32 columns: products of operands in three
+// bfloat16 parts on the tensor cores (split_mma.cuh).  76 chunks of 32 heads of 128 x 64 87 us, 28 of 8 of 128 x 256 35 (by FMAs, 8 x 4 outputs a
+// thread, 119 and 39).  Bound by a block's three barriers a panel and the splitting; two blocks an SM.
 template <typename W>
-__global__ void __launch_bounds__(CP_THREADS) chunk_state_kernel(ChunkArgs a, W w) {
+__global__ void __launch_bounds__(CP_THREADS, 2) chunk_state_kernel(ChunkArgs a, W w) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) char cp_sm[];
+    ChunkStateSmem& sm = *reinterpret_cast<ChunkStateSmem*>(cp_sm);          // wide: [tokens][128 dims]; tile: [tokens][columns], weighed
     __shared__ typename W::Head hd;
     __shared__ float weight[CP_C];
-    constexpr int LDK = 128 + 4;
-    float* sk = sm;                                          // [tokens][128 dims]
-    float* sv2 = sk + 64 * LDK;                              // [tokens][columns] of this panel and the next
     const int c = blockIdx.x, g = blockIdx.y, t0 = a.chunk_t0[c], n = a.chunk_t0[c + 1] - t0;
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int p0 = blockIdx.z * a.panels, p1 = min(p0 + a.panels, panel_count(a));
-    for (int d0 = 0; d0 < a.dk; d0 += 128) {
-        __syncthreads();
-        cp_tile<CP_THREADS>(sk, LDK, 128, a.k + (size_t)t0 * a.k_stride + g * a.dk + d0, a.k_stride, n, a.dk - d0, a.vec);
-        auto copy_values = [&](int p) {
-            int head, j0;
-            panel_place(a, g, p, head, j0);
-            cp_tile<CP_THREADS>(sv2 + (p & 1) * CP_TILE, CP_LD, 64, a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, a.v_stride, n, a.dv - j0, a.vec);
-            cp_commit();
-        };
-        copy_values(p0);
-        int last = -1;
-        for (int p = p0; p < p1; ++p) {
-            int head, j0;
-            panel_place(a, g, p, head, j0);
-            const float* sv = sv2 + (p & 1) * CP_TILE;
-            if (p + 1 < p1) copy_values(p + 1); else cp_commit();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, row = lane >> 2;
+    const int p0 = blockIdx.z * a.panels, p1 = min(p0 + a.panels, panel_count(a)), col = (warp >> 2) * 32, wide = (a.dk + 127) / 128;
+    // 128 dims' two tiles of keys, then the panels' values; and again for the other dims
+    const int per = 2 + p1 - p0, steps = wide * per;
+    auto issue = [&](int step) {
+        if (step < steps) {
+            const int d0 = step / per * 128, i = step % per;
+            TileFrom f;
+            if (i < 2) f = TileFrom{a.k + (size_t)t0 * a.k_stride + g * a.dk + d0 + i * 64, (size_t)a.k_stride, n, a.dk - d0 - i * 64};
+            else {
+                int head, j0;
+                panel_place(a, g, p0 + i - 2, head, j0);
+                f = TileFrom{a.v + (size_t)t0 * a.v_stride + head * a.dv + j0, (size_t)a.v_stride, n, a.dv - j0};
+            }
+            cs_issue(sm.raw[step & 1], f, a.vec);
+        }
+        cp_commit();
+    };
+    issue(0);
+    issue(1);
+    int last = -1;
+    for (int step = 0; step < steps; ++step) {
+        const int d0 = step / per * 128, i = step % per;
+        int head = 0, j0 = 0;
+        if (i >= 2) {
+            panel_place(a, g, p0 + i - 2, head, j0);
             if (head != last) {
+                __syncthreads();
                 w.prepare(hd, head, t0, n);
                 __syncthreads();
                 if (threadIdx.x < CP_C) weight[threadIdx.x] = threadIdx.x < n ? w.end(hd, n, threadIdx.x) : 0.f;
-                if (threadIdx.x == 0 && d0 == 0) w.store_end(hd, c, head, n);
+                if (threadIdx.x == 0) w.store_end(hd, c, head, n);
                 last = head;
             }
-            cp_wait<1>();
-            __syncthreads();
-            const bool two = a.dk - d0 > 64;                 // (a second tile of 64 dims)
-            float acc[2][4][4];
+        }
+        cp_wait<1>();
+        __syncthreads();                                     // the weights are there, everyone is through with the planes before
+        if (i < 2) cs_split<CS_LDK, false>(sm.wide + i * 64, sm.raw[step & 1], nullptr);
+        else cs_split<CS_LD, true>(sm.tile, sm.raw[step & 1], weight);
+        issue(step + 2);
+        if (i < 2) continue;
+        __syncthreads();
+        const int m0 = (warp & 3) * 32;
+        if (d0 + m0 >= a.dk) continue;
+        SplitSum<4> sum[2];
+        sum[0].clear();
+        sum[1].clear();
+#pragma unroll 1
+        for (int kk = 0; kk < n; kk += 16) {                 // 16 tokens
+            SplitA A[2];
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+            for (int m = 0; m < 2; ++m) A[m].load_t(sm.wide + kk * CS_LDK + m0 + 16 * m, CS_PLANE_K, CS_LDK, lane);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; j += 2) {
+                SplitB B;
+                B.load_t(sm.tile + kk * CS_LD + col + 8 * j, CS_PLANE, CS_LD, lane);
+                sum[0].add(j, A[0], B);
+                sum[1].add(j, A[1], B);
+            }
+        }
+        float* dst = a.chunk_state + ((size_t)c * a.heads + head) * a.dk * a.dv + j0;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) acc[m][i][k] = 0.f;
-#pragma unroll 4
-            for (int t = 0; t < n; ++t) {
-                const float4 v4 = *reinterpret_cast<const float4*>(sv + t * CP_LD + tx * 4);
-                const float f = weight[t];
-                const float vx[4] = {v4.x * f, v4.y * f, v4.z * f, v4.w * f};
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    if (m == 1 && !two) break;
-                    const float4 k4 = *reinterpret_cast<const float4*>(sk + t * LDK + m * 64 + ty * 4);
-                    const float kx[4] = {k4.x, k4.y, k4.z, k4.w};
+            for (int h = 0; h < 2; ++h) {
+                const int d = d0 + m0 + 16 * m + row + 8 * h;
+                if (d >= a.dk) continue;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) acc[m][i][k] = fmaf(kx[i], vx[k], acc[m][i][k]);
+                for (int j = 0; j < 4; ++j) {
+                    const int jj = col + 8 * j + 2 * q, left = a.dv - j0 - jj;
+                    float y[2] = {sum[m].sum(j, 2 * h), sum[m].sum(j, 2 * h + 1)};
+                    if (!isfinite(y[0] + y[1]))              // (a number that has no parts): made again of plain FMAs
+                        for (int u = 0; u < min(left, 2); ++u) {
+                            if (isfinite(y[u])) continue;
+                            const float* kd = a.k + (size_t)t0 * a.k_stride + g * a.dk + d;
+                            const float* vd = a.v + (size_t)t0 * a.v_stride + head * a.dv + j0 + jj + u;
+                            float s = 0.f;
+                            for (int t = 0; t < n; ++t) s = fmaf(kd[(size_t)t * a.k_stride], vd[(size_t)t * a.v_stride] * weight[t], s);
+                            y[u] = s;
+                        }
+                    float* to = dst + (size_t)d * a.dv + jj;
+                    if (a.vec && left >= 2) *reinterpret_cast<float2*>(to) = make_float2(y[0], y[1]);
+                    else {
+                        if (left > 0) to[0] = y[0];
+                        if (left > 1) to[1] = y[1];
+                    }
                 }
             }
-            float* dst = a.chunk_state + ((size_t)c * a.heads + head) * a.dk * a.dv + j0 + tx * 4;
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int d = d0 + 64 * m + ty * 4 + i;
-                    if (d < a.dk) store_row4(dst + (size_t)d * a.dv, acc[m][i], a.dv - j0 - tx * 4, a.vec);
-                }
-            __syncthreads();                                 // everyone is through with the values
-        }
     }
 }
 
@@ -480,20 +547,35 @@ static ChunkCut chunk_cut(int n_chunks, int groups, int panels) {
     return ChunkCut{one ? 1 : p, one};
 }
 
+// The same for what the chunks add to the state (chunk_state_kernel, two blocks an SM, in which a panel counts 5 and the keys' split 2): as few
+// rounds of blocks times a block's length as there can be.  76 chunks of 8 groups of 4 panels: four a block 97 us, two 87.
+static int chunk_state_panels(int n_chunks, int groups, int panels) {
+    int dev = 0, sms = 0, best = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    long long least = 0;
+    for (int p = 1; p <= panels; ++p) {
+        const long long blocks = (long long)n_chunks * groups * ((panels + p - 1) / p), cost = (blocks + 2 * sms - 1) / (2 * sms) * (5 * p + 2);
+        if (p == 1 || cost < least) { best = p; least = cost; }
+    }
+    return best;
+}
+
 template <typename W>
 static int chunk_products(ChunkArgs a, const W& w, int n_chunks, int n_seqs, const char* what, cudaStream_t stream) {
     const int panels = a.heads / a.groups * ((a.dv + 63) / 64), out_smem = chunk_out_smem(a.dk), out_most = chunk_out_smem(CP_MAX_DK);
     IDM_REQUIRE(n_chunks > 0 && a.heads % a.groups == 0 && a.dk <= CP_MAX_DK && a.groups <= 65535 && n_seqs <= 65535, "%s: %d chunks, %d heads in %d groups, keys of %d",
                 what, n_chunks, a.heads, a.groups, a.dk);
-    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_state_smem());
+    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkStateSmem));
     // (the same limit from every call: a smaller one from another thread would have this launch refused)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_one_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_out_one_smem());
     if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_most);
     IDM_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused (%s)", what, out_most, cudaGetErrorString(e));
+    a.panels = chunk_state_panels(n_chunks, a.groups, panels);
+    idm_launch(chunk_state_kernel<W>, dim3(n_chunks, a.groups, (panels + a.panels - 1) / a.panels), dim3(CP_THREADS), (int)sizeof(ChunkStateSmem), stream, a, w);
     const ChunkCut cut = chunk_cut(n_chunks, a.groups, panels);
     a.panels = cut.panels;
     const dim3 grid(n_chunks, a.groups, (panels + a.panels - 1) / a.panels);
-    idm_launch(chunk_state_kernel<W>, grid, dim3(CP_THREADS), chunk_state_smem(), stream, a, w);
     const size_t per = (size_t)a.dk * a.dv;
     if (a.vec) idm_launch(chunk_carry_kernel<4, W>, dim3((unsigned)((per / 4 + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);
     else idm_launch(chunk_carry_kernel<1, W>, dim3((unsigned)((per + 127) / 128), a.heads, n_seqs), dim3(128), 0, stream, a, w);

@@ -402,6 +402,33 @@ def test_retention_chunks_against_the_walk(K, lens, H, dk, dv, shift):
     assert helpers.rel_err(out[0][0], out[1][0].double()) < 1e-5 and helpers.rel_err(out[0][1], out[1][1].double()) < 1e-5
 
 
+# what a chunk adds to the state, as products of parts: a value that has none (infinite, not a number, at the end of the range) moves the state as
+# the walk of plain sums moves it, and leaves the other columns' bits alone; dims behind the first 128, columns that are no whole tile
+@pytest.mark.parametrize("dk,dv", [(128, 256), (200, 40), (36, 70)])
+def test_chunk_states_with_numbers_that_have_no_parts(K, dk, dv):
+    H, L = 2, 150
+    proj = _randn(L, 2 * H * dk + H * dv, seed=140)
+    cols, decay = (0, H * dk, 2 * H * dk), torch.tensor([0.97, 0.5], device="cuda")
+    start = _randn(1, H * dk * dv, seed=141)
+
+    def run(proj, walk):
+        K.RETENTION_WALK, state = walk, start.clone()
+        o = K.retention(proj.clone(), cols, None, dk ** -0.5, decay, state, _ctx([0], [L]), H, dk, dv)
+        K.RETENTION_WALK = type(K).RETENTION_WALK
+        return o, state.view(H, dk, dv)
+    clean = run(proj, 8)[1]
+    bad = proj.clone()
+    for t, j, x in ((5, 3, float("inf")), (70, 7, float("nan")), (149, dv + 1, -float("inf")), (148, 9, 3.4e38)):
+        bad[t, cols[2] + j] = x
+    got, want = run(bad, 8)[1], run(bad, 1 << 30)[1]
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    keep = torch.ones(H, 1, dv, dtype=torch.bool, device="cuda")
+    for j in (3, 7, 9): keep[0, 0, j] = False
+    keep[1, 0, 1] = False
+    assert torch.equal(got[keep.expand_as(got)], clean[keep.expand_as(got)])
+    assert helpers.rel_err(got[0, :, 9] / 1e38, want[0, :, 9].double() / 1e38) < 1e-5
+
+
 # a block of the read-outs takes one panel of 64 columns (in either kernel), two or all four of a group's, by how many chunks and heads a
 # step has: a sequence's bits are the same beside any others (148 SMs: at most 296 blocks, at most 355, more)
 @pytest.mark.parametrize("kind", ["retention", "state space"])
