@@ -44,14 +44,10 @@ __device__ __forceinline__ void ldmatrix4_t(uint32_t (&r)[4], const __nv_bfloat1
                  : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
 
-// 16 rows x 16 k of the left operand, as lanes hold them: x[i] are the pairs (row g, k 2q), (g + 8, 2q), (g, 2q + 8), (g + 8, 2q + 8) of
+// 16 rows x 16 k of the left operand, as lanes hold them: p[part][i] are the pairs (row g, k 2q), (g + 8, 2q), (g, 2q + 8), (g + 8, 2q + 8) of
 // lane 4 g + q
 struct SplitA {
     uint32_t p[3][4];
-    __device__ __forceinline__ void set(const float2 (&x)[4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) split3(x[i].x, x[i].y, p[0][i], p[1][i], p[2][i]);
-    }
     // planes of `plane` elements, rows `ld` apart with k side by side; at: row 0, k 0
     __device__ __forceinline__ void load(const __nv_bfloat16* at, int plane, int ld, int lane) {
         const __nv_bfloat16* mine = at + (lane & 15) * ld + (lane >> 4) * 8;
@@ -68,13 +64,7 @@ struct SplitA {
 // 16 k x 16 columns of the right operand, two tiles of 8 columns
 struct SplitB {
     uint32_t p[3][4];                                        // [part][tile 0: k 0.., k 8..; tile 1: k 0.., k 8..]
-    // planes of `plane` elements: rows are columns (n), k side by side, `ld` apart; at: row n0, k k0
-    __device__ __forceinline__ void load(const __nv_bfloat16* at, int plane, int ld, int lane) {
-        const __nv_bfloat16* mine = at + ((lane >> 4) * 8 + (lane & 7)) * ld + (lane >> 3 & 1) * 8;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) ldmatrix4(p[i], mine + i * plane);
-    }
-    // rows are k, columns (n) side by side; at: row k0, column n0
+    // planes of `plane` elements: rows are k, columns (n) side by side; at: row k0, column n0
     __device__ __forceinline__ void load_t(const __nv_bfloat16* at, int plane, int ld, int lane) {
         const __nv_bfloat16* mine = at + ((lane >> 3 & 1) * 8 + (lane & 7)) * ld + (lane >> 4) * 8;
 #pragma unroll
