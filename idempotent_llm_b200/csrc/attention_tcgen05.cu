@@ -316,7 +316,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
     if (threadIdx.x == 0) attn_stamp(0);                         // block started
 
     // blocks start in this order: all head groups (and runs) of the longest tile first.  What is read
@@ -387,6 +386,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t tmem_o = tmem + 128;                          // S buffers at columns 0 and 64 (P takes the place of its S), O from 128
+    pdl_launch_dependents();                                     // (behind the allocation)
     pdl_wait();                                                  // set-up done; now the previous kernel's results
     if (threadIdx.x == 0) attn_stamp(1);                         // set-up done, the kernel before too
 

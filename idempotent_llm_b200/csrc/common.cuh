@@ -40,6 +40,8 @@ int idm_fail(const char* fmt, ...);   // records the message, returns 1
 // Every kernel of this library starts with pdl_launch_dependents() (but the one that moves a captured
 // step's lengths and positions on, which lets nothing start before it is done) and executes pdl_wait()
 // before its first access to global memory that an earlier kernel may have written (or may still read).
+// A kernel that takes tensor memory calls it only behind the barrier that says the block has it: a block of
+// the next kernel beside it could else take columns that it waits for, and hold them until this kernel ends.
 // Launched with the programmatic-serialization attribute, the next kernel's blocks are scheduled
 // while this one still runs and do their set-up (and, in the matrix product, fetch weights, which
 // no kernel writes) before the wait returns.  Without the attribute both instructions do nothing.

@@ -259,7 +259,6 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_persistent_kernel(const __gri
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), GP_EPI_WARPS); }
@@ -271,6 +270,7 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_persistent_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
     pdl_wait();
 
     if (warp == GP_EPI_WARPS) {
@@ -398,7 +398,6 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_experts_kernel(const __grid_c
     int* held = (int*)(gen_base + S::BAR_OFF + 256);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), GP_EPI_WARPS); }
@@ -406,13 +405,15 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_experts_kernel(const __grid_c
         mbar_init_fence();
     }
     if (warp == GP_EPI_WARPS + 1) tmem_alloc(smem_u32((const void*)tmem_slot), TMEM_COLS);
-    pdl_wait();
-    if (n_experts <= GE_SMEM_EXPERTS)
-        for (int i = threadIdx.x; i <= n_experts; i += GP_THREADS) held[i] = offsets[i];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
+    pdl_wait();
+    if (n_experts <= GE_SMEM_EXPERTS)
+        for (int i = threadIdx.x; i <= n_experts; i += GP_THREADS) held[i] = offsets[i];
+    __syncthreads();
     ExpertWalk walk(n_experts <= GE_SMEM_EXPERTS ? held : offsets, n_experts, tiles_x, BN);
     int fx, t0;
 
@@ -520,7 +521,6 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_pair_kernel(const __grid_cons
     const uint32_t rank = cluster_rank();                          // 0: issues the MMAs
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 2 * GP_EPI_WARPS); }
@@ -533,6 +533,7 @@ __global__ void __launch_bounds__(GP_THREADS) gemm_pair_kernel(const __grid_cons
     cluster_sync_all();                                            // the other block's barriers exist before anything arrives there
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
     pdl_wait();
 
     if (warp == GP_EPI_WARPS) {
@@ -762,7 +763,6 @@ __global__ void __launch_bounds__(GQ_THREADS) gemm_qkv_tokens_kernel(const __gri
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), GQ_EPI_WARPS); }
@@ -774,6 +774,7 @@ __global__ void __launch_bounds__(GQ_THREADS) gemm_qkv_tokens_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
     pdl_wait();
 
     if (warp == GQ_EPI_WARPS) {
@@ -1004,7 +1005,6 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_small_kernel(const __grid_con
                                                                 const GemmEpi e, int n_tokens, int n_features,
                                                                 int kb_total, int bf, int tbox, int gk, int grouped,
                                                                 int stages, int tmem_cols) {
-    pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
@@ -1035,6 +1035,7 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_small_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
 #if defined(IDM_TRACE)
     // (stamps of the four fused products of a layer side by side: residual with a short / long inner axis, SwiGLU, q/k/v)
     if (blockIdx.x == 0 && threadIdx.x == 0) g_gemm_trace_base = EPI == EPI_RESIDUAL ? (kb_total > 32 ? 10 : 0) : EPI == EPI_SWIGLU || EPI == EPI_GATED ? 20 : EPI == EPI_QKV ? 30 : 40;
@@ -1289,7 +1290,6 @@ __global__ void __launch_bounds__(GW_THREADS) gemm_wide_kernel(const __grid_cons
                                                                float* out, int n_tokens, int n_features, int kb_total) {
     using S = WideSmem<BN, STAGES>;
     constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
-    pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
@@ -1313,6 +1313,7 @@ __global__ void __launch_bounds__(GW_THREADS) gemm_wide_kernel(const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = *tmem_slot;
+    pdl_launch_dependents();                                       // (behind the allocation)
 
     if (warp == 4) {
         if (lane == 0) {
