@@ -240,8 +240,11 @@ class Kernels:
 
     def _uploaded(self, numbers) -> torch.Tensor:
         """A step's list of integers on the device.  The copy is from pageable memory: the call returns when the numbers are staged, and
-        the host does not wait for the GPU (waiting, a step of a few long kernels cost the gap until its next launch)."""
-        return torch.from_numpy(np.array(numbers, dtype=np.int32)).to(self.device, non_blocking=True)
+        the host does not wait for the GPU (waiting, a step of a few long kernels cost the gap until its next launch).  Refused under
+        capture: a graph would read the numbers again, from host memory that is gone by then."""
+        if torch.cuda.is_current_stream_capturing():
+            raise KernelError("a step's plan cannot be made under capture: run the step once before, or capture steps of single tokens")
+        return torch.from_numpy(np.asarray(numbers, dtype=np.int32)).to(self.device, non_blocking=True)
 
     def scratch(self, key: str, n_floats: int) -> torch.Tensor:
         """A 32-bit scratch buffer that only grows (its address is stable across steps once large enough)."""

@@ -107,7 +107,7 @@ class TableExperts(FeedForward):
         counts = np.bincount(choice, minlength=s.n_experts)
         place = np.empty(n * top, dtype=np.int32)
         place[order] = np.arange(n * top, dtype=np.int32)                  # (token, k) -> grouped row
-        both = torch.from_numpy(np.concatenate([(order // top).astype(np.int32), place])).to(x.device, non_blocking=True)
+        both = K._uploaded(np.concatenate([order // top, place]))
         xg = K.rows_gather(x, both[:n * top])
         z = torch.empty((n * top, s.hidden), dtype=torch.float32, device=x.device)
         at = 0
@@ -260,7 +260,7 @@ class RoutedExperts(FeedForward):
         n_rows = int(counts.sum())
         place = np.full(n * top, -1, dtype=np.int32)
         place[order[:n_rows]] = np.arange(n_rows, dtype=np.int32)           # (token, k) -> grouped row, or -1
-        both = torch.from_numpy(np.concatenate([(order // top).astype(np.int32), place])).to(x.device, non_blocking=True)
+        both = K._uploaded(np.concatenate([order // top, place]))
         src, place_d = both[:n * top], both[n * top:].view(n, top)
         row_w = K.rows_weight(weight, place_d) if self.weight_in else None
         xg = K.rows_gather(x, src)

@@ -464,3 +464,17 @@ def test_group_norm_and_gate_scale_on_and_off_16_byte_borders(K):
         K.ssd_group_norm(y, parts, w, 1e-6, 0.5, out, shift)
         got.append(out[:, shift:shift + parts * length])
     assert helpers.rel_err(got[0], got[1].double()) < 1e-6
+
+
+def test_a_plan_is_not_made_under_capture(K):
+    """The lists of a step of long portions go up from host memory that does not outlive the call: a graph must not read them again."""
+    from idempotent_llm_b200.kernels.ops import KernelError
+    H, dk, dv, L = 2, 64, 64, 200
+    proj, state, ctx = _randn(L, H * (2 * dk + dv), seed=120), torch.zeros(1, H * dk * dv, device="cuda"), _ctx([0], [L])
+    decay = torch.tensor([0.5, 0.9], device="cuda")
+    torch.cuda.synchronize()
+    with pytest.raises(KernelError, match="capture"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            K.retention(proj, (0, H * dk, 2 * H * dk), None, dk ** -0.5, decay, state, ctx, H, dk, dv)
+    o = K.retention(proj, (0, H * dk, 2 * H * dk), None, dk ** -0.5, decay, state, ctx, H, dk, dv)      # as before, not captured
+    assert torch.isfinite(o).all()

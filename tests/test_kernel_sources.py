@@ -37,3 +37,16 @@ def test_the_next_kernel_starts_only_behind_an_allocation_of_tensor_memory():
         assert barrier > 0 and min(starts) > barrier, f"{file}: {name}"
     assert {"attention_tc_kernel", "gemm_persistent_kernel", "gemm_experts_kernel", "gemm_pair_kernel", "gemm_qkv_tokens_kernel",
             "gemm_small_kernel", "gemm_wide_kernel", "gemm_f32_split_kernel", "gemm_f32_wide_kernel"} <= set(seen), seen
+
+
+def test_uploads_are_refused_under_capture(monkeypatch):
+    """A captured copy would be made again from host memory that is gone by then (the copy does not wait, so nothing else refuses it)."""
+    import pytest
+    import torch
+    K = ops.Kernels.__new__(ops.Kernels)
+    K.device = torch.device("cpu")
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert K._uploaded([3, 1, 2]).tolist() == [3, 1, 2]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    with pytest.raises(ops.KernelError, match="capture"):
+        K._uploaded([3, 1, 2])
