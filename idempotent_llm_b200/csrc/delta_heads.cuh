@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(DH_THREADS, 2) delta_heads_chunk_kernel(DeltaH
 #pragma unroll
                     for (int m = 0; m < 3; ++m) *reinterpret_cast<uint32_t*>(to + (m * DH_C + t) * DH_LDW) = p[m];
                 }
-            } else if (j < a.dv) {
+            } else if (j < (a.dv + DH_COLS - 1) / DH_COLS * DH_COLS) {   // (the walk takes whole groups: zeros behind the last column)
                 float* to = reinterpret_cast<float*>(out + hh * bytes + DH_HEAD + j / DH_COLS * DH_XV) + j % DH_COLS;
 #pragma unroll
                 for (int t = 0; t < DH_C; ++t) *reinterpret_cast<float2*>(to + t * DH_COLS) = make_float2(x[t], y[t]);

@@ -254,6 +254,26 @@ def test_delta_by_heads_against_64_bits(K, lens, H, Hk, dk, dv, close):
     assert torch.isinf(o4[last, 0]) and torch.isinf(state4[0].view(H, dv, dk)[0, 0]).all()
 
 
+def test_delta_by_heads_lays_down_whole_groups_of_columns(K):
+    """What the walk reads is all written: as many words of the scratch are touched with 17 columns as with 32 (groups of 16), with 40 as with 48."""
+    H, Hk, dk, lens = 4, 2, 128, [65, 50]
+    left = {}
+    for dv in (17, 32, 40, 48):
+        n = sum(lens)
+        c, g, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 130)
+        g = g.view(n, H, dk)[:, :, 0].contiguous()
+        state, ctx = torch.zeros(len(lens), H * dv * dk, device="cuda"), _ctx([0] * len(lens), lens)
+        want = K.delta_by_heads(c, *cols[:2], ctx, H, Hk, dk, dv)
+        scratch = torch.full((want,), 0x7FC12345, dtype=torch.int32, device="cuda")     # (a number that is not one)
+        o = torch.empty(n, H * dv, device="cuda")
+        rc = K.lib.idm_delta_heads(c.data_ptr(), c.shape[1], *cols, g.data_ptr(), beta.data_ptr(), state.data_ptr(), state.shape[1], o.data_ptr(),
+                                   H * dv, ctx.cu_q.data_ptr(), ctx.slots.data_ptr(), ctx.n_seqs, n, H, Hk, dk, dv, max(lens), scratch.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and torch.isfinite(o).all()
+        left[dv] = int((scratch == 0x7FC12345).sum())
+    assert left[17] == left[32] and left[40] == left[48], left
+
+
 def test_delta_scratch_is_for_the_tokens_that_are_there(K):
     """One portion among many single tokens, and many sequences of many heads: nothing is sized by the longest portion times all."""
     for lens, H in (([300] + [1] * 63, 32), ([40] * 64, 64)):
