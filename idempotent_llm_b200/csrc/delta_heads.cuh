@@ -19,6 +19,11 @@
 // A prompt of 2 048 tokens, 32 heads of 128 x 64 over 8 keys: 51 us the chunks (their system's chains, two blocks of six warps an SM), 132 the walk:
 // 2.06 us a chunk, for which the tensor cores need 0.7 and the 88 KB that each of 128 blocks takes in from the L2 some 1.7.  With operands
 // split where they are used, 32-bit in scratch, the two took 39 and 186; decays per channel 258 and 230.
+//
+// A chunk of 32 heads over 8 keys leaves 1.8 MB.  So that a call's scratch does not grow with the prompt, places of chunks (a sequence's one
+// after another, sequence after sequence) go through a window: chunks, walk, the next places' chunks, their walk; the state in between is the
+// sequence's own in memory, in the 32 bits that the registers hold.  Layers of 64 heads, all places at once / windows of 32 M floats / 18 M: 2 048 tokens
+// 576 / 577 / 612 us, 4 x 1 500 and fewer 1 290 / 1 389 / 1 437; 32 heads 261 / 260 / 267 and 596 / 620 / 621.
 #pragma once
 #include "split_mma.cuh"
 
@@ -27,7 +32,7 @@
 #define DH_COLS 16                                              // columns of S of a block of the walk
 #define DH_HEADS 4                                              // heads that a block of the chunks weighs at a time, a warp each
 #define DH_THREADS 192                                          // its threads: two heads of 128 channels and 64 columns, two right-hand sides a thread
-#define DH_MOST (256ll << 20)                                   // floats of scratch
+#define DH_SCRATCH (32ll << 20)                                 // floats of scratch at most, whatever the prompt: about what the L2 holds
 struct DeltaHeadsScan {
     const float* c; int c_stride, c_q, c_k, c_v;                // rows of packed tokens: q, k [Hk, dk], v [H, dv]
     const float* g;                                             // [n, H] decays
@@ -37,6 +42,7 @@ struct DeltaHeadsScan {
     const int* cu_q; const int* slots;
     int n_seqs, H, Hk, dk, dv;
     char* scratch;
+    int first, window;                                          // of the chunks' places: those of this launch
 };
 // What the chunks leave for the walk, in bytes.  Operands as the walk's products read them: three planes of bfloat16 parts, rows as they lie in
 // its shared memory.  Of a chunk and key head: q and k [C][channels].  Of a chunk and head: X_k [C][channels], B [t][s], G and E [C] in 32-bit,
@@ -52,6 +58,15 @@ __host__ __device__ __forceinline__ long long delta_heads_chunk_bytes(int H, int
 // the place of a sequence's first chunk: chunks of sequence s are no more than the tokens' places from there to the next one's
 __host__ __device__ __forceinline__ long long delta_heads_slot(int cu_q, int s) { return (cu_q >> 5) + s; }
 static_assert(DH_C == 32, "the places count tokens by 32");
+// the last sequence whose place is at or before this one
+__device__ __forceinline__ int delta_heads_sequence(const int* cu_q, int n_seqs, int slot) {
+    int lo = 0, hi = n_seqs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (delta_heads_slot(cu_q[mid], mid) <= slot) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
 
 #define DH_LD (DH_DK + 4)
 #define DH_LDP 36
@@ -59,7 +74,7 @@ struct DeltaHeadsChunkSmem {
     float k[DH_C * DH_LD], q[DH_C * DH_LD];
     float kk[DH_C * DH_LDP], qk[DH_C * DH_LDP];
     float A[DH_HEADS][DH_C * DH_LDP];                           // [t][s], 0 from the diagonal on
-    float d[DH_HEADS][DH_C], beta[DH_HEADS][DH_C], G[DH_HEADS][DH_C];
+    float beta[DH_HEADS][DH_C], G[DH_HEADS][DH_C];
 };
 
 __global__ void __launch_bounds__(DH_THREADS, 2) delta_heads_chunk_kernel(DeltaHeadsScan a) {
@@ -67,16 +82,12 @@ __global__ void __launch_bounds__(DH_THREADS, 2) delta_heads_chunk_kernel(DeltaH
     pdl_wait();
     extern __shared__ __align__(16) char dh_sm[];
     DeltaHeadsChunkSmem& sm = *reinterpret_cast<DeltaHeadsChunkSmem*>(dh_sm);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hk = blockIdx.y, slot = blockIdx.x;
-    int lo = 0, hi = a.n_seqs - 1;                              // the last sequence whose place is at or before this one
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (delta_heads_slot(a.cu_q[mid], mid) <= slot) lo = mid; else hi = mid - 1;
-    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hk = blockIdx.y, slot = a.first + blockIdx.x;
+    const int lo = delta_heads_sequence(a.cu_q, a.n_seqs, slot);
     const int t1 = a.cu_q[lo + 1], tb = a.cu_q[lo] + (slot - (int)delta_heads_slot(a.cu_q[lo], lo)) * DH_C;
     if (tb >= t1) return;
     const int n = min(DH_C, t1 - tb), per = a.H / a.Hk;
-    char* mine = a.scratch + slot * delta_heads_chunk_bytes(a.H, a.Hk, a.dv);
+    char* mine = a.scratch + blockIdx.x * delta_heads_chunk_bytes(a.H, a.Hk, a.dv);
 
     // missing tokens and channels: k = q = 0, beta = 0, d = 1
     {
@@ -247,13 +258,17 @@ __global__ void __launch_bounds__(256, 1) delta_heads_walk_kernel(DeltaHeadsScan
     extern __shared__ __align__(16) char dh_sm[];
     DeltaHeadsWalkSmem& sm = *reinterpret_cast<DeltaHeadsWalkSmem*>(dh_sm);
     constexpr int WIDE = DH_C * DH_LDW;                         // elements of a plane
-    const int s = blockIdx.z, h = blockIdx.y, grp = blockIdx.x, hk = h / (a.H / a.Hk), j0 = grp * DH_COLS;
+    const int h = blockIdx.y, grp = blockIdx.x, hk = h / (a.H / a.Hk), j0 = grp * DH_COLS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, row = lane >> 2;
     pdl_wait();
-    const int t0 = a.cu_q[s], t1 = a.cu_q[s + 1], chunks = (t1 - t0 + DH_C - 1) / DH_C;
-    if (chunks <= 0) return;
+    // the sequences from the one that the window's first place belongs to on; of a sequence the chunks that have their places there
+    const int s = (a.first ? delta_heads_sequence(a.cu_q, a.n_seqs, a.first) : 0) + blockIdx.z;
+    if (s >= a.n_seqs) return;
+    const int t1 = a.cu_q[s + 1], slot0 = (int)delta_heads_slot(a.cu_q[s], s), c0 = max(a.first - slot0, 0), t0 = a.cu_q[s] + c0 * DH_C;
+    const int chunks = min((t1 - t0 + DH_C - 1) / DH_C, a.first + a.window - slot0 - c0);
+    if (t0 >= t1 || chunks <= 0) return;
     const long long chunk_bytes = delta_heads_chunk_bytes(a.H, a.Hk, a.dv);
-    const char* from = a.scratch + delta_heads_slot(t0, s) * chunk_bytes;
+    const char* from = a.scratch + (slot0 + c0 - a.first) * chunk_bytes;
     const char* shared = from + (long long)hk * 2 * DH_WIDE;                   // q and k
     const char* head = from + (long long)a.Hk * 2 * DH_WIDE + h * delta_heads_head_bytes(a.dv);
     // (by the upper four warps, while the others make u)

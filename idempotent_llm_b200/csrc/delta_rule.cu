@@ -1153,6 +1153,17 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
 }
 
 // ------------------------------------------------------------------ a decay per head, chunks of 32
+// Places of a launch, as in delta_window: what fits the scratch (0: not one), in whole rounds of the chunks' blocks (two an SM) where there are more
+// launches than one.  The state carries over from launch to launch.
+static long long delta_heads_window(int n_seqs, int n_tokens, int H, int Hk, int dv) {
+    const long long fit = DH_SCRATCH * 4 / delta_heads_chunk_bytes(H, Hk, dv), all = (long long)n_tokens / DH_C + n_seqs;
+    if (fit >= all) return all;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long round = 2 * sms / Hk;
+    return round > 0 && fit > round ? fit / round * round : fit;
+}
 // Floats of scratch that a step of `n_seqs` sequences and `n_tokens` tokens, at most `max_tokens` of one sequence, wants; 0: the step's
 // decays are wanted per channel (idm_delta_scan).  Keys of 65 to 128 channels in rows of whole 16-byte pieces, portions of more than 48 tokens.
 // Measured, us of a layer with 64 heads (32 heads), this form / the chain of chunks of 16: 8 x 12 tokens 146 / 115 (91 / 93), 8 x 40 195 / 193
@@ -1160,8 +1171,7 @@ extern "C" int idm_delta_scan(const float* c, int c_stride, int c_q, int c_k, in
 extern "C" long long idm_delta_heads_scratch_floats(int n_seqs, int n_tokens, int H, int Hk, int dk, int dv, int max_tokens, int c_stride, int c_q, int c_k) {
     if (max_tokens <= 48 || n_seqs <= 0 || H <= 0 || Hk <= 0 || H % Hk || dk <= 64 || dk > DH_DK || dv <= 0) return 0;
     if (dk % 4 || c_stride % 4 || c_q % 4 || c_k % 4 || H > 65535 || n_seqs > 65535 || Hk > 65535) return 0;
-    const long long want = ((long long)n_tokens / DH_C + n_seqs) * (delta_heads_chunk_bytes(H, Hk, dv) / 4);
-    return want <= DH_MOST ? want : 0;
+    return delta_heads_window(n_seqs, n_tokens, H, Hk, dv) * (delta_heads_chunk_bytes(H, Hk, dv) / 4);
 }
 
 // The delta rule with a decay per head, g [n_tokens, H]; scratch of idm_delta_heads_scratch_floats.
@@ -1174,13 +1184,16 @@ extern "C" int idm_delta_heads(const float* c, int c_stride, int c_q, int c_k, i
                 dk, dv, n_tokens, n_seqs, c_q, c_k, c_stride);
     IDM_REQUIRE(state != nullptr && state_stride >= (long long)H * dk * dv, "delta_heads: a slot's state must hold %d x %d x %d floats", H, dv, dk);
     IDM_REQUIRE(scratch != nullptr && (((uintptr_t)scratch | (uintptr_t)c) & 15) == 0, "delta_heads: scratch at %p, rows at %p", (void*)scratch, (const void*)c);
-    const DeltaHeadsScan a{c, c_stride, c_q, c_k, c_v, g, beta, state, state_stride, o, o_stride, cu_q, slots, n_seqs, H, Hk, dk, dv, (char*)scratch};
+    const int all = n_tokens / DH_C + n_seqs, window = (int)delta_heads_window(n_seqs, n_tokens, H, Hk, dv);
+    DeltaHeadsScan a{c, c_stride, c_q, c_k, c_v, g, beta, state, state_stride, o, o_stride, cu_q, slots, n_seqs, H, Hk, dk, dv, (char*)scratch, 0, window};
     constexpr int chunk_smem = (int)sizeof(DeltaHeadsChunkSmem), walk_smem = (int)sizeof(DeltaHeadsWalkSmem);
     cudaError_t e = cudaFuncSetAttribute(delta_heads_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_heads_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
     IDM_REQUIRE(e == cudaSuccess, "delta_heads: %d bytes of shared memory were refused (%s)", walk_smem, cudaGetErrorString(e));
-    idm_launch(delta_heads_chunk_kernel, dim3(n_tokens / DH_C + n_seqs, Hk), dim3(DH_THREADS), chunk_smem, stream, a);
-    idm_launch(delta_heads_walk_kernel, dim3((dv + DH_COLS - 1) / DH_COLS, H, n_seqs), dim3(256), walk_smem, stream, a);
+    for (; a.first < all; a.first += window) {                  // (a window's places are those of no more sequences)
+        idm_launch(delta_heads_chunk_kernel, dim3(window < all - a.first ? window : all - a.first, Hk), dim3(DH_THREADS), chunk_smem, stream, a);
+        idm_launch(delta_heads_walk_kernel, dim3((dv + DH_COLS - 1) / DH_COLS, H, n_seqs < window ? n_seqs : window), dim3(256), walk_smem, stream, a);
+    }
     IDM_LAUNCH_CHECK("delta_heads");
     return 0;
 }

@@ -274,6 +274,39 @@ def test_delta_by_heads_lays_down_whole_groups_of_columns(K):
     assert left[17] == left[32] and left[40] == left[48], left
 
 
+def test_delta_by_heads_through_a_window(K):
+    """More chunks than the scratch holds: the bits that each sequence gets alone, and no more memory for a longer prompt."""
+    H, Hk, dk, dv, lens = 64, 8, 128, 64, [700, 33, 900, 1, 50, 400]      # 70 places of 3.1 MB
+    n = sum(lens)
+    c, _, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 140)
+    g = torch.exp(-3.0 * _randn(n, H, seed=145).abs() ** 3)
+    start = _randn(len(lens), H * dv * dk, seed=146)
+
+    def run(rows, start, lens):
+        ctx, state = _ctx([0] * len(lens), lens), start.clone()
+        want = K.delta_by_heads(c, *cols[:2], ctx, H, Hk, dk, dv)
+        assert 0 < want <= 32 << 20
+        args = c[rows].contiguous(), g[rows].contiguous(), beta[rows].contiguous()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        o = K.delta_heads(args[0], *cols, args[1], args[2], state, ctx, H, Hk, dk, dv, want)
+        assert torch.cuda.max_memory_allocated() - before <= 4 * (o.numel() + (32 << 20)) + (2 << 20)
+        return o, state
+    o, state = run(slice(0, n), start, lens)
+    at = 0
+    for i, L in enumerate(lens):
+        rows = slice(at, at + L)
+        if L > 48:
+            alone = run(rows, start[i:i + 1], [L])
+            assert torch.equal(alone[0], o[rows]) and torch.equal(alone[1][0], state[i]), i
+        if i in (0, 3):
+            S = start[i].double().view(H, dv, dk).clone()
+            want = _delta_64(c[rows], cols, g[rows].repeat_interleave(dk, dim=1), beta[rows], S, H, Hk, dk, dv)
+            assert helpers.rel_err(o[rows], want) < 2e-5 and helpers.rel_err(state[i].view(H, dv, dk), S) < 2e-5, i
+        at += L
+
+
 def test_delta_scratch_is_for_the_tokens_that_are_there(K):
     """One portion among many single tokens, and many sequences of many heads: nothing is sized by the longest portion times all."""
     for lens, H in (([300] + [1] * 63, 32), ([40] * 64, 64)):
