@@ -553,13 +553,10 @@ class Kernels:
                                             b_col, int(head_col), _p(dt_bias), _p(a_log), _p(beta), H, Hk, dk, a_dk, n, self._stream()))
         return beta
 
-    # portions of up to so many tokens take decays per channel (idm_delta_heads_scratch_floats says the same)
-    DELTA_BY_CHANNEL = 48
-
     def delta_by_heads(self, c, c_q: int, c_k: int, ctx, H: int, Hk: int, dk: int, dv: int) -> int:
         """Floats of scratch with which the step's delta rule runs on one decay per head (``delta_heads``); 0: it wants them per
         channel (``delta_scan``)."""
-        if ctx.max_q_len <= self.DELTA_BY_CHANNEL:
+        if ctx.single_token:
             return 0
         return int(self.lib.idm_delta_heads_scratch_floats(ctx.n_seqs, c.shape[0], H, Hk, dk, dv, int(ctx.max_q_len), c.shape[1], c_q, c_k))
 

@@ -321,6 +321,18 @@ def test_delta_scratch_is_for_the_tokens_that_are_there(K):
         assert torch.cuda.max_memory_allocated() - before < 4 * (o.numel() + 32 * n * H) + (2 << 20)
 
 
+# the forms' border by the tokens of a sequence on average: 16 with 32 heads, 24 with 64
+@pytest.mark.parametrize("lens,H,by_heads", [([300] + [1] * 63, 32, False), ([300] + [1] * 63, 64, False), ([2048] + [1] * 60, 32, True), ([2048] + [1] * 60, 64, True),
+                                             ([241] + [1] * 15, 32, True), ([240] + [1] * 15, 32, False), ([369] + [1] * 15, 64, True),
+                                             ([368] + [1] * 15, 64, False), ([48] * 8, 32, False), ([49] * 8, 64, True)])
+def test_delta_form_of_a_portion_among_single_tokens(K, lens, H, by_heads):
+    """A portion among many single tokens takes no chunk for each of those, in time or in memory."""
+    Hk, dk, dv, n = 8, 128, 64, sum(lens)
+    c, _, beta, cols = _delta_inputs(n, H, Hk, dk, dv, 150)
+    ctx = _ctx([0] * len(lens), lens)
+    assert (K.delta_by_heads(c, *cols[:2], ctx, H, Hk, dk, dv) > 0) == by_heads
+
+
 @pytest.mark.parametrize("dk,dv,pad", [(128, 64, 0), (64, 40, 4), (24, 9, 0), (100, 64, 0), (30, 16, 0), (128, 64, 1), (160, 16, 0)])
 def test_delta_single_tokens_against_64_bits_and_however_cut(K, dk, dv, pad):
     H, Hk, lens = 4, 2, [8, 3, 5]
