@@ -57,6 +57,7 @@ __device__ __forceinline__ ConvToken conv_token(const ConvStep& st, int t) {
 #define CONV_TOKENS 8
 #define CONV_BLOCKS 1184               // eight blocks of 256 threads an SM
 #define CONV_ROUNDS 4
+#define CONV_TABLE 40960               // bytes of shared memory for the turns' table
 
 // the convolution of token t, channel c (the number of taps known at compile time: the loops unroll to straight
 // code); moves the state on if t is its sequence's only token
@@ -448,10 +449,11 @@ static bool conv_pairs(const ConvSeg& g) {
 }
 
 // A block of the kernels of eight tokens a thread goes on with the next eight, up to CONV_ROUNDS times, where that leaves the SMs
-// enough blocks: looking up places and addresses is most of what a thread does for eight.
-static dim3 conv_cut(int n_tokens, int across, int& rounds) {
+// enough blocks: looking up places and addresses is most of what a thread does for eight.  (`most`: as many as there is room for.)
+static dim3 conv_cut(int n_tokens, int across, int most, int& rounds) {
     const long long blocks = (long long)((n_tokens + CONV_TOKENS - 1) / CONV_TOKENS) * across;
     rounds = (int)(blocks / 592);
+    rounds = rounds > most ? most : rounds;
     rounds = rounds < 1 ? 1 : rounds > CONV_ROUNDS ? CONV_ROUNDS : rounds;
     return dim3((n_tokens + CONV_TOKENS * rounds - 1) / (CONV_TOKENS * rounds), across);
 }
@@ -469,7 +471,7 @@ extern "C" int idm_short_conv(const float* in, int in_stride, int col0, int chan
     const dim3 grid(n_tokens, across);
     const bool pairs = conv_pairs(g) && ((uintptr_t)out & 7) == 0;
     int rounds;
-    const dim3 cut = conv_cut(n_tokens, pairs ? (channels + 511) / 512 : across, rounds);
+    const dim3 cut = conv_cut(n_tokens, pairs ? (channels + 511) / 512 : across, CONV_ROUNDS, rounds);
 #define CONV_GO(TAPS_) case TAPS_: idm_launch(short_conv_kernel<TAPS_>, grid, dim3(256), 0, stream, g, st, out, act); break;
 #define CONV_MANY(TAPS_) case TAPS_: \
         if (pairs) idm_launch(short_conv_tokens_kernel<TAPS_, 2>, cut, dim3(256), 0, stream, g, st, out, act, n_tokens, rounds); \
@@ -502,11 +504,12 @@ extern "C" int idm_conv_qkv_cache(const float* in, int in_stride, int col0, int 
     // a thread per item and eight tokens; else a block per token, with few tokens several, so that two blocks' worth of work per SM is about
     const int items = (n_q + n_kv) * (dk - maps * half) + n_kv * dv, across = (items + 255) / 256;
     const size_t smem = (size_t)CONV_TOKENS * half * sizeof(float2);
-    const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS && smem * CONV_ROUNDS <= 40960;
+    // (rounds whose rows of the table have room: heads of 384, all turned, 4 000 tokens of 16 over 4: 89 us, a token a block 221, eight tokens a thread without a table 162)
+    const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS && smem <= CONV_TABLE;
     const bool pairs = conv_pairs(a.seg) && half % 2 == 0 && (dk / maps) % 2 == 0 && dv % 2 == 0 &&
                        (((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 7) == 0;
     int rounds;
-    const dim3 cut = conv_cut(n_tokens, pairs ? (items + 511) / 512 : across, rounds);
+    const dim3 cut = conv_cut(n_tokens, pairs ? (items + 511) / 512 : across, smem ? (int)(CONV_TABLE / smem) : CONV_ROUNDS, rounds);
     int split = (296 + n_tokens - 1) / n_tokens;
     if (split > across) split = across;
     if (split < 1) split = 1;

@@ -128,6 +128,12 @@ def test_conv_qkv_of_eight_tokens_a_thread(K, maps, dk, half):
         assert helpers.rel_err(values.reshape(L, -1), u[:, (n_q + n_kv) * dk:]) < 1e-6
 
 
+# rows of the turns' table that leave room for three rounds of eight tokens, for one, and for none (a token a block)
+@pytest.mark.parametrize("dk,half", [(344, 170), (800, 400), (1284, 641)])
+def test_conv_qkv_with_wide_turns(K, dk, half):
+    test_conv_qkv_of_eight_tokens_a_thread(K, 1, dk, half)
+
+
 # ------------------------------------------------------------------------------------------------ delta rule
 def _delta_inputs(n, H, Hk, dk, dv, seed, pad=0):
     k = torch.nn.functional.normalize(_randn(n, Hk, dk, seed=seed), dim=-1)
