@@ -577,13 +577,13 @@ template <int TN> static void split_cost(int M, int N, int K, int sms, float per
     }
 }
 
-struct F32Choice { int tn, split, subs; };                    // subs > 0: gemm_f32_wide_kernel with so many times 64 tokens
+struct F32Choice { int tn, split, subs, sms; };               // subs > 0: gemm_f32_wide_kernel with so many times 64 tokens
 static F32Choice f32_choice(int M, int N, int K) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 148;
-    F32Choice c{64, 1, 0};
+    F32Choice c{64, 1, 0, sms};
     float best = 1e30f;
     if (M <= 16) {
         split_cost<16>(M, N, K, sms, 0.95f, c.tn, c.split, best);
@@ -608,12 +608,8 @@ extern "C" long long idm_gemm_f32_scratch_bytes(int M, int N, int K) {
 }
 
 template <int SUBS>
-static int wide_launch(const float* x, const float* w, float* out, int M, int N, int K, int rows, void* scratch, cudaStream_t stream) {
+static int wide_launch(const float* x, const float* w, float* out, int M, int N, int K, int rows, void* scratch, int sms, cudaStream_t stream) {
     const int Kp = (K + GX_SEG - 1) / GX_SEG * GX_SEG, bytes = 1024 + 2 * WideTile<SUBS>::STAGE;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
     auto kernel = rows == 0 ? gemm_f32_wide_kernel<SUBS, 0> : rows == 1 ? gemm_f32_wide_kernel<SUBS, 1> : gemm_f32_wide_kernel<SUBS, 2>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     IDM_REQUIRE(e == cudaSuccess, "gemm_f32: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
@@ -636,18 +632,16 @@ extern "C" int idm_gemm_f32(const float* x, const float* w, float* out, int M, i
     if (M == 0 || N == 0) return 0;
     IDM_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     const F32Choice c = f32_choice(M, N, K);
-    int dev = 0, sms = 0, rc;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int rc;
     if (c.subs) {
         IDM_REQUIRE(scratch != nullptr && ((uintptr_t)scratch & 15) == 0, "gemm_f32: scratch at %p", scratch);
         const int rows = K % 4 == 0 && ((uintptr_t)w & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
-        rc = c.subs == 1 ? wide_launch<1>(x, w, out, M, N, K, rows, scratch, stream) : wide_launch<2>(x, w, out, M, N, K, rows, scratch, stream);
+        rc = c.subs == 1 ? wide_launch<1>(x, w, out, M, N, K, rows, scratch, c.sms, stream) : wide_launch<2>(x, w, out, M, N, K, rows, scratch, c.sms, stream);
     } else {
         const int rows = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 ? (K % GX_SEG == 0 ? 2 : 1) : 0;
-        rc = c.tn == 16 ? split_launch<16>(x, w, out, M, N, K, rows, c.split, sms, stream)
-           : c.tn == 32 ? split_launch<32>(x, w, out, M, N, K, rows, c.split, sms, stream)
-                        : split_launch<64>(x, w, out, M, N, K, rows, c.split, sms, stream);
+        rc = c.tn == 16 ? split_launch<16>(x, w, out, M, N, K, rows, c.split, c.sms, stream)
+           : c.tn == 32 ? split_launch<32>(x, w, out, M, N, K, rows, c.split, c.sms, stream)
+                        : split_launch<64>(x, w, out, M, N, K, rows, c.split, c.sms, stream);
     }
     if (rc) return rc;
     IDM_LAUNCH_CHECK("gemm_f32");
