@@ -322,8 +322,9 @@ __global__ void __launch_bounds__(GX_THREADS, 1) gemm_f32_split_kernel(const flo
 // 64 tokens are an accumulator's, as above: with SUBS of 2 the two take turns in tensor memory, with 1 neighbouring segments do.
 // Eight warps split the weight, eight add up 64 tokens, one thread issues the MMAs and one the copies.
 // Bound by shared memory: a segment's 128 tokens move 192 KB into the MMAs, 48 in from the weight's split and 48 from the copies, 1.2 of
-// the 1.4 us it takes (64 tokens: 0.95 us, of which some 0.7).  700 tokens: 4096 x 1024 55 us (split by every tile 62), 6144 x 1024 56 (81), 1024 x
-// 3072 54 (58); 1 400 tokens: 79 (100), 103 (157), 77 (112).
+// the 1.4 us it takes (64 tokens: 0.95 us, of which some 0.7).  700 tokens, with the kernel
+// in front and inputs out of the L2: 4096 x 1024 58 us (split by every tile 68), 6144 x 1024 60 (86), 1024 x 3072 58 (64); 1 400 tokens: 83 (107),
+// 108 (162), 85 (118).
 #define GW_CONV 256
 template <int SUBS> struct WideTile {
     static constexpr int ADD = SUBS * GX_ADD, THREADS = ADD + GW_CONV + 64, WARP_MMA = (ADD + GW_CONV) / 32;
@@ -591,11 +592,13 @@ static F32Choice f32_choice(int M, int N, int K) {
     }
     split_cost<32>(M, N, K, sms, 0.95f, c.tn, c.split, best);
     split_cost<64>(M, N, K, sms, 1.15f, c.tn, c.split, best);
-    // measured: 1.0 us a segment of 64 tokens and 1.4 of 128 with all SMs at it, and 5 us for the kernel in front and the start
+    // measured: 1.0 us a segment of 64 tokens and 1.4 of 128 with all SMs at it, and 5 us for the kernel in front and the start (us of tiles that
+    // split both operands / 64 / 128 tokens: 180 x 4096 x 1024 28.7 / 27.6 / 35.8, 350 48.1 / 44.0 / 35.8, 700 67.6 / 60.4 / 58.4; 700 x 1024 x 3072
+    // 63.5 / 58.4 / 80.9; 577 x 4200 x 1101 96.3 / 82.9 / 74.8; 1 400 x 2048 x 1024 67.6 / 60.4 / 60.4; inputs out of the L2)
     const long long features = (N + GX_FEATURES - 1) / GX_FEATURES, segs = (K + GX_SEG - 1) / GX_SEG;
     for (int subs = 1; subs <= 2; ++subs) {
         const long long tiles = features * ((M + 64 * subs - 1) / (64 * subs));
-        const float t = (float)((tiles + sms - 1) / sms * segs) * (subs == 1 ? 1.0f : 1.5f) + 5.f;
+        const float t = (float)((tiles + sms - 1) / sms * segs) * (subs == 1 ? 1.0f : 1.4f) + 5.f;
         if (t < best) { best = t; c.subs = subs; }
     }
     return c;

@@ -649,7 +649,7 @@ def test_gemm_32_bit_is_one_sum_in_every_kernel(kernels, M, N, K_):
 
 # products of tokens enough for parts made in front: 64 and 128 tokens a block, rows and inner sizes that end inside tiles and segments, several
 # tiles a block, rows of x and of the weight on and off 16-byte borders; a row's bits are those that sixteen rows get
-@pytest.mark.parametrize("M,N,K_", [(1300, 1100, 1030), (1291, 1100, 1032), (700, 4096, 1024), (577, 4200, 1100), (4200, 260, 640), (641, 1024, 3072)])
+@pytest.mark.parametrize("M,N,K_", [(1300, 1100, 1030), (1291, 1100, 1032), (700, 4096, 1024), (577, 4200, 1100), (180, 9550, 1300), (180, 9600, 1301), (4200, 260, 640), (641, 1024, 3072)])
 def test_gemm_32_bit_of_many_tokens_is_the_same_sum(kernels, M, N, K_):
     k = kernels("float32")
     g = torch.Generator(device="cuda").manual_seed(M + N)
