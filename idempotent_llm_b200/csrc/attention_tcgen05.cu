@@ -397,8 +397,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // (the whole warp walks the loop: its lanes fetch the page numbers of 32 key blocks at a time, so that
         // no request waits for a look-up of its own; lane 0 issues the requests)
         if (lane == 0) {
-            // (only the rows that some tile of the step has are fetched; the rest of the tile is whatever was there,
-            // makes rows of scores nobody reads, and gets p = 0)
+            // (only the rows that some tile of the step has are fetched; the rest of the tile is whatever was there and
+            // makes rows of scores, and of the context, that nobody reads)
             mbar_expect_tx(q_full, (uint32_t)(HT * a.rows_cap * 128));
             for (int h = 0; h < HT; ++h)
                 tma_load_3d(base + S::Q_OFF + h * AP_BM * 128, &map_q, h * 64, head0, tok0, q_full);

@@ -125,7 +125,7 @@ struct ChunkStateSmem {
 };
 
 // chunk_state[c, head, d, j] = sum_s end(s) k_s[d] v_s[j], 128 dims at a time, of which a warp has 32, and 32 columns: products of operands in three
-// bfloat16 parts on the tensor cores (split_mma.cuh).  76 chunks of 32 heads of 128 x 64 87 us, 28 of 8 of 128 x 256 35 (by FMAs, 8 x 4 outputs a
+// bfloat16 parts on the tensor cores (split_mma.cuh).  76 chunks of 32 heads of 128 x 64 87 us, 28 of 8 of 128 x 256 33 (by FMAs, 8 x 4 outputs a
 // thread, 119 and 39).  Bound by a block's three barriers a panel and the splitting; two blocks an SM.
 template <typename W>
 __global__ void __launch_bounds__(CP_THREADS, 2) chunk_state_kernel(ChunkArgs a, W w) {

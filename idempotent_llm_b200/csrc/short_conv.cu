@@ -504,7 +504,8 @@ extern "C" int idm_conv_qkv_cache(const float* in, int in_stride, int col0, int 
     // a thread per item and eight tokens; else a block per token, with few tokens several, so that two blocks' worth of work per SM is about
     const int items = (n_q + n_kv) * (dk - maps * half) + n_kv * dv, across = (items + 255) / 256;
     const size_t smem = (size_t)CONV_TOKENS * half * sizeof(float2);
-    // (rounds whose rows of the table have room: heads of 384, all turned, 4 000 tokens of 16 over 4: 89 us, a token a block 221, eight tokens a thread without a table 162)
+    // (as many rounds as the table has room for: heads of 384, all turned, 4 000 tokens of 16 over 4, 89 us; a token a block 221, eight tokens
+    // a thread without a table 162)
     const bool many = (long long)(n_tokens / CONV_TOKENS) * across >= CONV_BLOCKS && smem <= CONV_TABLE;
     const bool pairs = conv_pairs(a.seg) && half % 2 == 0 && (dk / maps) % 2 == 0 && dv % 2 == 0 &&
                        (((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 7) == 0;

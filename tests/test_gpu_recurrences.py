@@ -210,7 +210,7 @@ def test_delta_forms_in_64_bits_and_beside_one_another(K, L, dk, dv, pad, close)
 
 
 # a decay per head: chunks of 32 with one token left over or missing, keys below 128, columns that are no whole group of 16, key heads of one to
-# nine heads (a warp weighs a head: eight at a time), sequences that share places of 32 tokens, keys that lie close together
+# nine heads (a warp weighs a head: four at a time), sequences that share places of 32 tokens, keys that lie close together
 @pytest.mark.parametrize("lens,H,Hk,dk,dv,close", [
     ([5, 31, 32, 33, 1, 49], 4, 2, 128, 64, 0.0), ([97, 64], 6, 3, 100, 40, 0.0), ([200], 9, 1, 68, 17, 0.0), ([161, 7], 8, 2, 128, 64, 0.1),
     ([257], 3, 3, 128, 16, 0.3)])
