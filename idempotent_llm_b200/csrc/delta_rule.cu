@@ -1168,16 +1168,19 @@ static long long delta_heads_window(int n_seqs, int n_tokens, int H, int Hk, int
     const long long round = 2 * delta_sms() / Hk;
     return round > 0 && fit > round ? fit / round * round : fit;
 }
+
+#define DH_PORTION 48
 // Floats of scratch that a step of `n_seqs` sequences and `n_tokens` tokens, at most `max_tokens` of one sequence, wants; 0: the step's
-// decays are wanted per channel (idm_delta_scan).  Keys of 65 to 128 channels in rows of whole 16-byte pieces, portions of more than 48 tokens, and of 24
+// decays are wanted per channel (idm_delta_scan).  Keys of 65 to 128 channels in rows of whole 16-byte pieces, portions of more than DH_PORTION tokens, and of 24
 // tokens a sequence on average (16 where a sequence's blocks of the walk are no more than the SMs: 32 heads): a sequence of one token costs a block of
 // the walk, an SM each, as much as one of 32.
 // Measured, us of a layer with 64 heads (32 heads), this form / the chain of chunks of 16: 8 x 12 tokens 146 / 115 (91 / 93), 8 x 40 195 / 193
 // (101 / 107), 2 x 60 117 / 121 (92 / 103), 8 x 130 386 / 493 (195 / 254), 3 x 1 000 826 / 1 296 (391 / 598).  One portion among single tokens:
 // 2 048 among 60 1 158 / 1 645 (538 / 1 018), 1 000 among 31 609 / 729 (282 / 456), 700 among 31 526 / 535 (252 / 342), 400 among 20 331 / 325 (172 / 200), 300 among 15
 // 286 / 263 (141 / 177), 200 among 15 259 / 219 (131 / 131), 60 among 15 214 / 164 (111 / 97), 300 among 63 674 / 519 (352 / 250), 64 among 60 573 / 353 (302 / 194).
+extern "C" int idm_delta_heads_portion() { return DH_PORTION; }
 extern "C" long long idm_delta_heads_scratch_floats(int n_seqs, int n_tokens, int H, int Hk, int dk, int dv, int max_tokens, int c_stride, int c_q, int c_k) {
-    if (max_tokens <= 48 || n_seqs <= 0 || H <= 0 || Hk <= 0 || H % Hk || dk <= 64 || dk > DH_DK || dv <= 0) return 0;
+    if (max_tokens <= DH_PORTION || n_seqs <= 0 || H <= 0 || Hk <= 0 || H % Hk || dk <= 64 || dk > DH_DK || dv <= 0) return 0;
     if (dk % 4 || c_stride % 4 || c_q % 4 || c_k % 4 || H > 65535 || n_seqs > 65535 || Hk > 65535) return 0;
     const bool at_once = (long long)H * ((dv + DH_COLS - 1) / DH_COLS) <= delta_sms();
     if (n_tokens < (at_once ? 16ll : 24ll) * n_seqs) return 0;

@@ -79,6 +79,7 @@ SIGNATURES = {
     "idm_delta_scan_scratch_floats": (c_longlong, "iiiiii"),
     "idm_delta_heads": (c_int, "piiiipppqpippiiiiiiipp"),
     "idm_delta_heads_scratch_floats": (c_longlong, "iiiiiiiiii"),
+    "idm_delta_heads_portion": (c_int, ""),
     "idm_delta_out": (c_int, "pipfpiiifpiiiiip"),
     "idm_add_rmsnorm2": (c_int, "ppiqppfpppiip"),
     "idm_gemm_bf16_gated": (c_int, "pppiiiip"),
@@ -210,6 +211,7 @@ class Kernels:
         self.attention_pool_slots = 4096
         self.sm_count = torch.cuda.get_device_properties(device).multi_processor_count
         self.page = L.idm_page_tokens()
+        self._delta_portion = L.idm_delta_heads_portion()        # portions of up to so many tokens take decays per channel
         # a model whose parts can emit their calls runs a step by one call into the library (program.py);
         # switched off (IDM_PROGRAM=0, or this attribute), every kernel is called from Python: the same bits
         self.use_programs = self.fused and os.environ.get("IDM_PROGRAM", "1") != "0"
@@ -556,7 +558,7 @@ class Kernels:
     def delta_by_heads(self, c, c_q: int, c_k: int, ctx, H: int, Hk: int, dk: int, dv: int) -> int:
         """Floats of scratch with which the step's delta rule runs on one decay per head (``delta_heads``); 0: it wants them per
         channel (``delta_scan``)."""
-        if ctx.single_token:
+        if ctx.max_q_len <= self._delta_portion:             # (no call for it)
             return 0
         return int(self.lib.idm_delta_heads_scratch_floats(ctx.n_seqs, c.shape[0], H, Hk, dk, dv, int(ctx.max_q_len), c.shape[1], c_q, c_k))
 
