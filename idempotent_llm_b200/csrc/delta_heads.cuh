@@ -17,7 +17,8 @@
 // parts is 0 in the products; what meets it (a column from its token on) is made again of plain FMAs over the tokens a row may see.
 //
 // A prompt of 2 048 tokens, 32 heads of 128 x 64 over 8 keys: 51 us the chunks (their system's chains, two blocks of six warps an SM), 132 the walk:
-// 2.06 us a chunk, for which the tensor cores need 0.7 and the 88 KB that each of 128 blocks takes in from the L2 some 1.7.  With operands
+// 2.06 us a chunk, of which the tensor instructions' pipe is busy for 0.7; the block's warps wait for instructions with fixed latencies and for one
+// another (three barriers a chunk), L1 at half its rate, the 88 KB that a block takes in a chunk at 8 % of the L2's.  With operands
 // split where they are used, 32-bit in scratch, the two took 39 and 186; decays per channel 258 and 230.
 //
 // A chunk of 32 heads over 8 keys leaves 1.8 MB.  So that a call's scratch does not grow with the prompt, places of chunks (a sequence's one
