@@ -51,7 +51,9 @@ __device__ __forceinline__ ConvToken conv_token(const ConvStep& st, int t) {
 // borders.  Bound by latencies and instructions, not yet by memory (which would take 13 to 18 us of the last two).  Measured: short_conv of 4 096
 // channels x 4 taps, 2 048 tokens, 13.7 us (one channel and 8 tokens a thread 18.6, one token 47), 4 876 tokens 35 us (45); conv_qkv_cache of
 // 4 096 channels x 3 taps, 4 876 tokens, 53 us (112 us with each token's turn read from memory behind the stores of the one before,
-// 70 us in pairs without rounds); three blocks an SM instead of two spill and take 54.  With few tokens the looking up of a token's place, then
+// 70 us in pairs without rounds); three blocks an SM instead of two spill and take 54.  At
+// 6 to 8 taps pairs spill some registers and are the faster form all the same: 3 584 channels, 4 876 tokens, 4 / 6 / 7 / 8 taps into the cache
+// 42 / 46 / 49 / 55 us (one channel and 8 tokens a thread 84 / 103 / 130 / 152), short_conv 25 / 31 / 36 / 38 (36 / 37 / 41 / 48).  With few tokens the looking up of a token's place, then
 // loads, is the shortest chain: asked for in ConvChannel's order, 1 / 8 / 64 single tokens take 2.85 / 3.18 / 6.86 us in conv_qkv_cache
 // (20 heads of 64) against 2.40 / 2.77 / 6.36.
 #define CONV_TOKENS 8
